@@ -27,31 +27,15 @@ WBTE_INL Fp fp_one() { Fp r; _Pragma("unroll") for (int i = 0; i < 12; i++) r.v[
 #if defined(WBTE_FP_NOINLINE)
 // One out-of-line copy of the 12-limb product keeps every kernel's hot loop
 // inside the instruction cache.
-#if defined(WBTE_FP_ROLLED) && WBTE_FP_ROLLED == 4
-// the same product as a loop of rows, WBTE_FP_ROLLED rows per iteration:
-// less code per product for kernels bound by instruction fetch
-static __device__ __noinline__ Fp fp_mul_ool(Fp a, Fp b) { Fp r; fp_mont_mul_r4(r.v, a.v, b.v); return r; }
-#elif defined(WBTE_FP_ROLLED) && WBTE_FP_ROLLED == 6
-static __device__ __noinline__ Fp fp_mul_ool(Fp a, Fp b) { Fp r; fp_mont_mul_r6(r.v, a.v, b.v); return r; }
-#else
 static __device__ __noinline__ Fp fp_mul_ool(Fp a, Fp b) { Fp r; fp_mont_mul(r.v, a.v, b.v); return r; }
-#endif
 WBTE_INL Fp fp_mul(const Fp& a, const Fp& b) { return fp_mul_ool(a, b); }
 WBTE_INL Fp fp_sqr(const Fp& a) { return fp_mul_ool(a, a); }
 #else
 WBTE_INL Fp fp_mul(const Fp& a, const Fp& b) { Fp r; fp_mont_mul(r.v, a.v, b.v); return r; }
 WBTE_INL Fp fp_sqr(const Fp& a) { Fp r; fp_mont_mul(r.v, a.v, a.v); return r; }
 #endif
-#if defined(WBTE_FPADD_NOINLINE)
-// out-of-line sums: smaller code for kernels bound by instruction fetch
-static __device__ __noinline__ Fp fp_add_ool(Fp a, Fp b) { Fp r; fp_add_raw(r.v, a.v, b.v); return r; }
-static __device__ __noinline__ Fp fp_sub_ool(Fp a, Fp b) { Fp r; fp_sub_raw(r.v, a.v, b.v); return r; }
-WBTE_INL Fp fp_add(const Fp& a, const Fp& b) { return fp_add_ool(a, b); }
-WBTE_INL Fp fp_sub(const Fp& a, const Fp& b) { return fp_sub_ool(a, b); }
-#else
 WBTE_INL Fp fp_add(const Fp& a, const Fp& b) { Fp r; fp_add_raw(r.v, a.v, b.v); return r; }
 WBTE_INL Fp fp_sub(const Fp& a, const Fp& b) { Fp r; fp_sub_raw(r.v, a.v, b.v); return r; }
-#endif
 // a + b without reduction: only valid as a multiplication input (< 2p).
 WBTE_INL Fp fp_add_lazy(const Fp& a, const Fp& b) { Fp r; fp_add_nored(r.v, a.v, b.v); return r; }
 WBTE_INL Fp fp_dbl(const Fp& a) { return fp_add(a, a); }
