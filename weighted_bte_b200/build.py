@@ -23,7 +23,7 @@ CSRC = os.path.join(PKG, "csrc")
 INCLUDE = os.path.join(ROOT, "include")
 BUILD = os.path.join(PKG, "_build")
 LIB = os.path.join(PKG, "libwbte.so")
-SOURCES = ["k_arith.cu", "k_gt.cu", "k_hash.cu", "k_msm.cu", "k_opening.cu", "k_pairing.cu", "runtime.cu", "server.cu"]
+SOURCES = ["k_arith.cu", "k_gt.cu", "k_hash.cu", "k_msm.cu", "k_pairing.cu", "runtime.cu", "server.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", CSRC, "-I", INCLUDE]
 # Code-layout variant of the shipped library (see fields.cuh): one out-of-line
@@ -31,12 +31,13 @@ FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-I", CSRC, "-
 # B = 512): 2.5x the throughput of fully inlined arithmetic, whose hot loops
 # overflow the instruction cache (ncu: "no instruction" stalls dominate).
 DEFAULT_DEFINES: list = ["WBTE_FP_NOINLINE", "WBTE_FP2_NOINLINE"]
-# Per-file exceptions: the pairing kernels (Fp6/Fp12 towers over inlined Fp2
-# products calling the one out-of-line Fp product) measured 5-16 % faster with
-# Fp2 inlined, while the curve kernels (MSM, transforms) are faster with it
-# out of line.  Each .cu is its own translation unit with internal-linkage
-# field functions, so the layouts do not mix.
+# Per-file exceptions: the line tables and GT encodings of k_pairing.cu take
+# inlined Fp2 products over the one out-of-line Fp product (5-16 % faster),
+# while the curve kernels (MSM, transforms) are faster with it out of line.
+# Each .cu is its own translation unit with internal-linkage field functions,
+# so the layouts do not mix.
 SOURCE_UNDEFINES: dict = {"k_pairing.cu": ["WBTE_FP2_NOINLINE"]}
+
 
 def nvcc() -> str:
     path = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"

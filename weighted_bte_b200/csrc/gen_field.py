@@ -226,6 +226,108 @@ def gen_mont_mul_rolled(name, modulus, n, unroll):
     )
 
 
+def _asm_function(name, args, lines, outs, ins):
+    body = "\n".join("        \"" + l + "\\n\\t\"" for l in lines)
+    o = ", ".join('"=r"(%s[%d])' % x for x in outs)
+    i = ", ".join('"r"(%s[%d])' % x for x in ins)
+    return ("__device__ __forceinline__ void %s(%s) {\n    asm(\"{\\n\\t\"\n%s\n        \"}\"\n        : %s\n        : %s);\n}\n"
+            % (name, args, body, o, i))
+
+
+def gen_mul_wide(name, n):
+    """r (2n words) = a b, any n-word a and b."""
+    lines = []
+    w = lines.append
+    w(Window.regs(n, ""))
+    w(".reg .u32 t<%d>;" % (2 * n))
+    a = ["%%%d" % (2 * n + i) for i in range(n)]
+    b = ["%%%d" % (3 * n + i) for i in range(n)]
+    win = Window(w, n, "")
+    for i in range(n):
+        if i:
+            win.shift()
+        win.add_row(a, b[i])
+        w("mov.u32 t%d, %s;" % (i, win.E[0]))
+    win.merge(["t%d" % (n + i) for i in range(n)])
+    for i in range(2 * n):
+        w("mov.u32 %%%d, t%d;" % (i, i))
+    return _asm_function(name, "uint32_t r[%d], const uint32_t a[%d], const uint32_t b[%d]" % (2 * n, n, n), lines,
+                         [("r", i) for i in range(2 * n)], [("a", i) for i in range(n)] + [("b", i) for i in range(n)])
+
+
+def gen_redc(name, modulus, n):
+    """r (n words) = (t + k m) / 2^(32n) for the k < 2^(32n) that makes it
+    whole, t of 2n words in two's complement, modulo 2^(32n): the reduced low
+    half lies in [0, m], the high half is added as it stands."""
+    pinv = (-pow(modulus, -1, 1 << 32)) % (1 << 32)
+    mw = ["0x%08x" % x for x in limbs32(modulus, n)]
+    lines = []
+    w = lines.append
+    w(Window.regs(n, ""))
+    w(".reg .u32 u<%d>, m;" % n)
+    t = ["%%%d" % (n + i) for i in range(2 * n)]
+    win = Window(w, n, "")
+    win.Ein = t[:n]
+    w("mul.lo.u32 m, %s, 0x%08x;" % (t[0], pinv))
+    win.add_row(mw, "m")
+    for i in range(1, n):
+        win.shift()
+        w("mul.lo.u32 m, %s, 0x%08x;" % (win.E[0], pinv))
+        # the even chain of the row absorbs E as it stands, the odd chain the
+        # carry of the shift: nothing else touches the flag in between
+        win.add_row(mw, "m")
+    u = ["u%d" % i for i in range(n)]
+    win.merge(u)
+    for j in range(n):
+        op = "add.cc" if j == 0 else ("addc.cc" if j < n - 1 else "addc")
+        w("%s.u32 u%d, u%d, %s;" % (op, j, j, t[n + j]))
+    for j in range(n):
+        w("mov.u32 %%%d, u%d;" % (j, j))
+    return _asm_function(name, "uint32_t r[%d], const uint32_t t[%d]" % (n, 2 * n), lines,
+                         [("r", i) for i in range(n)], [("t", i) for i in range(2 * n)])
+
+
+def gen_cond_sub(name, c, n):
+    """r = a - c if a >= c else a."""
+    lines = []
+    w = lines.append
+    w(".reg .u32 d<%d>, bw;" % n)
+    w(".reg .pred nb;")
+    emit_cond_sub(w, ["%%%d" % i for i in range(n)], ["%%%d" % (n + i) for i in range(n)], limbs32(c, n))
+    return _asm_function(name, "uint32_t r[%d], const uint32_t a[%d]" % (n, n), lines, [("r", i) for i in range(n)],
+                         [("a", i) for i in range(n)])
+
+
+def gen_add_const(name, c, n):
+    """r = a + c modulo 2^(32n)."""
+    cl = limbs32(c, n)
+    lines = []
+    w = lines.append
+    w(".reg .u32 d<%d>;" % n)
+    for j in range(n):
+        op = "add.cc" if j == 0 else ("addc.cc" if j < n - 1 else "addc")
+        w("%s.u32 d%d, %%%d, 0x%08x;" % (op, j, n + j, cl[j]))
+    for j in range(n):
+        w("mov.u32 %%%d, d%d;" % (j, j))
+    return _asm_function(name, "uint32_t r[%d], const uint32_t a[%d]" % (n, n), lines, [("r", i) for i in range(n)],
+                         [("a", i) for i in range(n)])
+
+
+def gen_addsub_nr(name, n, sub):
+    """r = a + b or a - b modulo 2^(32n)."""
+    o = "sub" if sub else "add"
+    lines = []
+    w = lines.append
+    w(".reg .u32 d<%d>;" % n)
+    for j in range(n):
+        op = "%s.cc" % o if j == 0 else ("%sc.cc" % o if j < n - 1 else "%sc" % o)
+        w("%s.u32 d%d, %%%d, %%%d;" % (op, j, n + j, 2 * n + j))
+    for j in range(n):
+        w("mov.u32 %%%d, d%d;" % (j, j))
+    return _asm_function(name, "uint32_t r[%d], const uint32_t a[%d], const uint32_t b[%d]" % (n, n, n), lines,
+                         [("r", i) for i in range(n)], [("a", i) for i in range(n)] + [("b", i) for i in range(n)])
+
+
 def gen_add(name, modulus, n):
     """r = a + b mod m (inputs < m)."""
     ml = limbs32(modulus, n)
@@ -597,6 +699,14 @@ def main():
         gen_add("fp_add_raw", P, 12),
         gen_sub("fp_sub_raw", P, 12),
         gen_add_nr("fp_add_nored", 12),
+        gen_mul_wide("fp_mul_wide", 12),
+        gen_redc("fp_redc", P, 12),
+        gen_cond_sub("fp_csub_p", P, 12),
+        gen_cond_sub("fp_csub_2p", 2 * P, 12),
+        gen_add_const("fp_add_p", P, 12),
+        gen_add_const("fp_add_2p", 2 * P, 12),
+        gen_addsub_nr("wide_add", 24, False),
+        gen_addsub_nr("wide_sub", 24, True),
         gen_fp2_mul_lazy("fp2_mont_mul_lazy"),
         gen_mont_mul_rolled("fp_mont_mul_r4", P, 12, 4),
         gen_mont_mul_rolled("fp_mont_mul_r6", P, 12, 6),

@@ -6,27 +6,16 @@
 #include <cstdlib>
 
 #include "launch.h"
-#include "pairing.cuh"
+#include "team.cuh"
 
 namespace wbte {
 
 namespace {
-constexpr int TPB = 64;
+constexpr int TPB = 64, WARP = 32;
 inline unsigned blocks_for(int64_t n, int tpb = TPB) { return (unsigned)((n + tpb - 1) / tpb); }
 
 WBTE_INL Fp12* as_gt(uint8_t* p) { return reinterpret_cast<Fp12*>(p); }
 WBTE_INL const Fp12* as_gt(const uint8_t* p) { return reinterpret_cast<const Fp12*>(p); }
-
-// resident 64-thread blocks per SM the Miller-loop and final-exponentiation
-// kernels are compiled for (0: no bound, the compiler's 255 registers)
-#ifndef WBTE_PAIR_MINBLOCKS
-#define WBTE_PAIR_MINBLOCKS 0
-#endif
-#if WBTE_PAIR_MINBLOCKS > 0
-#define WBTE_PAIR_BOUNDS __launch_bounds__(TPB, WBTE_PAIR_MINBLOCKS)
-#else
-#define WBTE_PAIR_BOUNDS
-#endif
 
 __global__ void k_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -47,141 +36,155 @@ __global__ void k_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n) {
     }
 }
 
-// pair i uses line table i % lines_n (tables stored line-major, stride lines_n)
-__global__ void WBTE_PAIR_BOUNDS k_miller_lines(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, int64_t lines_n) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    G1A P = load_affine(reinterpret_cast<const G1A*>(p + G1_AFF * i));
-    Fp12 f;
-    miller_loop_lines(f, reinterpret_cast<const Line*>(lines) + i % lines_n, (size_t)lines_n, P);
-    store_vec(as_gt(out) + i, f);
+// this lane's team in the launch (shadow lanes belong to the warp's last one);
+// teams past the end take the last value again without storing it, which is
+// their own warp's, so that a call may work in place
+__device__ __forceinline__ int64_t team_index() {
+    const int tm = (int)(threadIdx.x & 31) / TEAM_LANES;
+    return (int64_t)blockIdx.x * TEAMS + (tm < TEAMS ? tm : TEAMS - 1);
 }
 
-__global__ void WBTE_PAIR_BOUNDS k_miller(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t n, int64_t p_mod, int64_t q_mod) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    G1A P = load_affine(reinterpret_cast<const G1A*>(p + G1_AFF * (p_mod ? i % p_mod : i)));
-    G2A Q = load_affine(reinterpret_cast<const G2A*>(q + G2_AFF * (q_mod ? i % q_mod : i)));
-    Fp12 f;
-    miller_loop(f, P, Q);
-    store_vec(as_gt(out) + i, f);
+// out[o chunks + ch] = prod over run ch (at most C of t < T) of
+// Miller(P[(o / p_per) T + t], lines of table (o % per) T + t), one team per
+// run: the opening of K batches against one committee's prepared opening keys
+// (tables line-major with stride per T), each batch with its own T shares
+// (p_per = per: weighted_btx) or each slot with its own T points (p_per = 1:
+// weighted_pfe, and single pairs with T = 1).  The pairs of a run share the 62
+// squarings.
+__global__ void __launch_bounds__(WARP) k_miller_lines_multi(uint8_t* out, const uint8_t* lines, const uint8_t* p,
+                                                             int64_t n, int64_t per, int64_t p_per, int64_t T, int64_t C,
+                                                             int64_t chunks) {
+    __shared__ uint4 sh[T6_ROWS * 32];
+    const Team t = team_init(sh);
+    int64_t g = team_index();
+    const bool active = g < n * chunks;
+    if (!active) g = n * chunks - 1;
+    const int64_t o = g / chunks, lo = (g % chunks) * C;
+    const int64_t cnt = T - lo < C ? T - lo : C;
+    const Fp* L = reinterpret_cast<const Fp*>(lines + LINE_SZ * ((o % per) * T + lo)) + t.k;
+    const int64_t stride = per * T * (int64_t)(LINE_SZ / sizeof(Fp));
+    const G1A* P = reinterpret_cast<const G1A*>(p) + (o / p_per) * T + lo;
+    Fp2 f = t6_one(t);
+    for (int i = 62; i >= 0; i--) {
+        if (i != 62) f = t6_sqr(t, f);
+        for (int step = 0; step <= (t6_bit(i) ? 1 : 0); step++) {
+            // runs of one launch differ in length only at the end of T; the
+            // shorter ones take lines of value one
+            for (int64_t r = 0; r < C; r++) {
+                const int64_t x = r < cnt ? r : 0;
+                T6Point pt = t6_point(t, load_affine(P + x));
+                pt.inf |= r >= cnt;
+                f = t6_mul_line(t, f, t6_line_value(t, load_vec(L + x * (int64_t)(LINE_SZ / sizeof(Fp))), pt));
+            }
+            L += stride;
+        }
+    }
+    f = t6_conj(t, f);
+    if (active) t6_store(t, out + GT_SZ * g, f);
 }
 
 // Segment s of `per` consecutive pairs is split into `chunks` runs of at most
-// C pairs; thread (s, ch) writes the product of its run's Miller loops, one
-// multi-Miller loop sharing the squarings.
-__global__ void WBTE_PAIR_BOUNDS k_miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t per,
-                                                 int64_t K, int C, int64_t chunks) {
-    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (g >= K * chunks) return;
+// C pairs; the team of (s, ch) writes the product of its run's Miller loops,
+// lines computed on the fly, one multi-Miller loop sharing the squarings.
+// Pair i is (P[p_mod ? i % p_mod : i], Q[q_mod ? i % q_mod : i]).
+__global__ void __launch_bounds__(WARP) k_miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t per,
+                                                        int64_t K, int C, int64_t chunks, int64_t p_mod, int64_t q_mod) {
+    __shared__ uint4 sh[T6_ROWS * 32];
+    const Team t = team_init(sh);
+    int64_t g = team_index();
+    const bool active = g < K * chunks;
+    if (!active) g = K * chunks - 1;
     const int64_t s = g / chunks, lo = (g % chunks) * C;
     const int cnt = (int)(per - lo < C ? per - lo : C);
-    G1A P[MULTI_MILLER_MAX];
-    G2A Q[MULTI_MILLER_MAX];
-    for (int t = 0; t < cnt; t++) {
-        P[t] = load_affine(reinterpret_cast<const G1A*>(p + G1_AFF * (s * per + lo + t)));
-        Q[t] = load_affine(reinterpret_cast<const G2A*>(q + G2_AFF * (s * per + lo + t)));
+    Fp2 T[MULTI_MILLER_MAX];
+    auto P_of = [&](int r) {
+        const int64_t i = s * per + lo + (r < cnt ? r : 0);
+        return load_affine(reinterpret_cast<const G1A*>(p) + (p_mod ? i % p_mod : i));
+    };
+    auto Q_of = [&](int r) {
+        const int64_t i = s * per + lo + (r < cnt ? r : 0);
+        return load_affine(reinterpret_cast<const G2A*>(q) + (q_mod ? i % q_mod : i));
+    };
+    uint32_t dead = 0;  // pairs past the run or with an identity: lines of value one
+    for (int r = 0; r < C; r++) {
+        const G2A Q = Q_of(r);
+        T[r] = t.k == 0 ? Q.x : (t.k == 1 ? Q.y : fp2_one());
+        if (r >= cnt || is_inf(Q)) dead |= 1u << r;
     }
-    Fp12 f;
-    multi_miller_loop(f, P, Q, cnt);
-    store_vec(as_gt(out) + g, f);
+    Fp2 f = t6_one(t);
+    for (int i = 62; i >= 0; i--) {
+        if (i != 62) f = t6_sqr(t, f);
+        for (int step = 0; step <= (t6_bit(i) ? 1 : 0); step++)
+            for (int r = 0; r < C; r++) {
+                const Fp c = step ? t6_line_add(t, T[r], Q_of(r)) : t6_line_double(t, T[r]);
+                T6Point pt = t6_point(t, P_of(r));
+                pt.inf |= (dead >> r) & 1;
+                f = t6_mul_line(t, f, t6_line_value(t, c, pt));
+            }
+    }
+    f = t6_conj(t, f);
+    if (active) t6_store(t, out + GT_SZ * g, f);
 }
 
-__global__ void k_fp12_segment_product(uint8_t* out, const uint8_t* in, const int64_t* offsets, int64_t k) {
-    int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= k) return;
-    Fp12 acc = fp12_one();
-    for (int64_t t = offsets[j]; t < offsets[j + 1]; t++) {
-        Fp12 x = load_vec(as_gt(in) + t);
-        fp12_mul(acc, acc, x);
+__global__ void __launch_bounds__(WARP) k_fp12_segment_product(uint8_t* out, const uint8_t* in, const int64_t* offsets,
+                                                               int64_t k) {
+    __shared__ uint4 sh[T6_ROWS * 32];
+    const Team t = team_init(sh);
+    int64_t j = team_index();
+    const bool active = j < k;
+    if (!active) j = k - 1;
+    const int64_t lo = offsets[j], len = active ? offsets[j + 1] - lo : 0;
+    const int64_t longest = __reduce_max_sync(0xffffffffu, (unsigned)len);
+    Fp2 acc = t6_one(t);
+    for (int64_t i = 0; i < longest; i++) {
+        const Fp2 x = i < len ? t6_load(t, in + GT_SZ * (lo + i)) : t6_one(t);
+        acc = i ? t6_mul(t, acc, x) : x;
     }
-    store_vec(as_gt(out) + j, acc);
+    if (active) t6_store(t, out + GT_SZ * j, acc);
 }
 
-__global__ void WBTE_PAIR_BOUNDS k_final_exp(uint8_t* out, const uint8_t* in, int64_t n, int mode) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Fp12 f = load_vec(as_gt(in) + i), r;
-    if (mode == FE_EASY) {
-        final_exp_easy(r, f);
-    } else if (mode == FE_HARD) {
-        final_exp_hard(r, f);
-    } else {
-        final_exp_easy(r, f);
-        final_exp_hard(r, r);
-    }
-    store_vec(as_gt(out) + i, r);
+__global__ void __launch_bounds__(WARP) k_final_exp(uint8_t* out, const uint8_t* in, int64_t n, int mode) {
+    __shared__ uint4 sh[T6_ROWS * 32];
+    const Team t = team_init(sh);
+    int64_t i = team_index();
+    const bool active = i < n;
+    if (!active) i = n - 1;
+    Fp2 f = t6_load(t, in + GT_SZ * i);
+    if (mode != FE_HARD) f = t6_final_exp_easy(t, f);
+    if (mode != FE_EASY) f = t6_final_exp_hard(t, f);
+    if (active) t6_store(t, out + GT_SZ * i, f);
 }
 
-WBTE_INL bool fp12_is_zero(const Fp12& a) {
-    const uint32_t* x = reinterpret_cast<const uint32_t*>(&a);
-    uint32_t d = 0;
-    for (int i = 0; i < 144; i++) d |= x[i];
-    return d == 0;
+__global__ void __launch_bounds__(WARP) k_fp12_mul(uint8_t* out, const uint8_t* a, int64_t sa, const uint8_t* b,
+                                                   int64_t sb, bool conj_b, int64_t n) {
+    __shared__ uint4 sh[T6_ROWS * 32];
+    const Team t = team_init(sh);
+    int64_t i = team_index();
+    const bool active = i < n;
+    if (!active) i = n - 1;
+    Fp2 y = t6_load(t, b + GT_SZ * sb * i);
+    if (conj_b) y = t6_conj(t, y);
+    const Fp2 r = t6_mul(t, t6_load(t, a + GT_SZ * sa * i), y);
+    if (active) t6_store(t, out + GT_SZ * i, r);
 }
 
-// The easy part f^((p^6 - 1)(p^2 + 1)) of C consecutive values per thread
-// sharing one Fp12 inversion (batch_easy_final_exponentiation,
-// btx/src/final_exponentiation.rs:228-252): the forward pass keeps the prefix
-// products in `pre`, one inversion of the chunk's product, and each value's
-// inverse falls out on the way back.  A zero value (no inverse) is left out
-// of the product and gives zero, as the per-value kernel does.  full: the
-// hard part follows.  in may equal out.
-__global__ void WBTE_PAIR_BOUNDS k_final_exp_easy_batch(uint8_t* out, const uint8_t* in, uint8_t* pre, int64_t n,
-                                                        int64_t C, int full) {
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t lo = t * C, hi = lo + C < n ? lo + C : n;
-    if (lo >= n) return;
-    Fp12 acc = fp12_one();
-    for (int64_t i = lo; i < hi; i++) {
-        const Fp12 f = load_vec(as_gt(in) + i);
-        store_vec(as_gt(pre) + i, acc);
-        if (!fp12_is_zero(f)) fp12_mul(acc, acc, f);
-    }
-    Fp12 inv;
-    fp12_inv(inv, acc);
-    for (int64_t i = hi - 1; i >= lo; i--) {
-        const Fp12 f = load_vec(as_gt(in) + i);
-        Fp12 r;
-        if (fp12_is_zero(f)) {
-            r = f;
-        } else {
-            Fp12 fi, u;
-            fp12_mul(fi, inv, load_vec(as_gt(pre) + i));  // 1 / f_i
-            fp12_mul(inv, inv, f);
-            fp12_conj(r, f);
-            fp12_mul(r, r, fi);  // f^(p^6 - 1)
-            fp12_frobenius(u, r, 2);
-            fp12_mul(r, r, u);  // ^(p^2 + 1)
-            if (full) final_exp_hard(r, r);
-        }
-        store_vec(as_gt(out) + i, r);
-    }
+__global__ void __launch_bounds__(WARP) k_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha,
+                                                 const uint8_t* beta, const uint8_t* valid, int64_t n) {
+    __shared__ uint4 sh[T6_ROWS * 32];
+    const Team t = team_init(sh);
+    int64_t i = team_index();
+    const bool active = i < n;
+    if (!active) i = n - 1;
+    Fp2 r = t6_mul(t, t6_load(t, second + GT_SZ * i), t6_conj(t, t6_load(t, alpha + GT_SZ * i)));
+    r = t6_mul(t, r, t6_load(t, beta + GT_SZ * i));
+    if (!valid[i]) r = t6_one(t);
+    if (active) t6_store(t, out + GT_SZ * i, r);
 }
 
-__global__ void k_fp12_mul(uint8_t* out, const uint8_t* a, int64_t sa, const uint8_t* b, int64_t sb, bool conj_b, int64_t n) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Fp12 x = load_vec(as_gt(a) + sa * i), y = load_vec(as_gt(b) + sb * i), r;
-    if (conj_b) fp12_conj(y, y);
-    fp12_mul(r, x, y);
-    store_vec(as_gt(out) + i, r);
-}
-
-__global__ void k_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha, const uint8_t* beta,
-                         const uint8_t* valid, int64_t n) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Fp12 r;
-    if (valid[i]) {
-        Fp12 c2 = load_vec(as_gt(second) + i), al = load_vec(as_gt(alpha) + i), be = load_vec(as_gt(beta) + i);
-        fp12_conj(al, al);
-        fp12_mul(r, c2, al);
-        fp12_mul(r, r, be);
-    } else {
-        r = fp12_one();
-    }
-    store_vec(as_gt(out) + i, r);
+// off[i] = i step
+__global__ void k_offsets(int64_t* off, int64_t n, int64_t step) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i < n) off[i] = i * step;
 }
 
 WBTE_INL void fp_store_be48(uint8_t* out, const Fp& m) {
@@ -240,39 +243,76 @@ void launch_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n, cudaStrea
     note_launch();
     k_prepare_lines<<<blocks_for(n), TPB, 0, s>>>(lines, q, n);
 }
+// Pairs per team of a launch of `outputs` products of T Miller loops each.
+// Sharing the 62 squarings saves 73 of a first pair's wide multiply-adds (in
+// thousands per lane: 62 squarings of 1,176; `line` for one pair's 68 lines),
+// but one warp keeps a scheduler's pipe only 0.6 busy, so runs are cut while
+// the launch has fewer than 1.6 warps for each scheduler.
+static int64_t miller_run(int64_t outputs, int64_t T, double line, int64_t most) {
+    static std::atomic<int> schedulers{0};
+    int sc = schedulers.load();
+    if (sc == 0) {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        sc = 4 * (sms > 0 ? sms : 148);
+        schedulers.store(sc);
+    }
+    int64_t best = 1;
+    double best_t = 0;
+    for (int64_t C = 1; C <= std::min(T, most); C++) {
+        const int64_t chunks = (T + C - 1) / C;
+        const double warps = (double)(outputs * chunks) / TEAMS / sc;
+        const double time = (73.0 + line * C) * std::max(1.6, warps);
+        if (C == 1 || time < best_t) best = C, best_t = time;
+    }
+    return best;
+}
+static constexpr double LINE_PREPARED = 130.0, LINE_COMPUTED = 245.0;
+
+static bool miller_lines(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, int64_t per, int64_t p_per,
+                         int64_t T, cudaStream_t s) {
+    const int64_t C = miller_run(n, T, LINE_PREPARED, T), chunks = (T + C - 1) / C;
+    uint8_t* runs = out;
+    int64_t* offs = nullptr;
+    if (chunks > 1 && (cudaMallocAsync(&runs, GT_SZ * (size_t)(n * chunks), s) != cudaSuccess ||
+                       cudaMallocAsync(&offs, sizeof(int64_t) * (size_t)(n + 1), s) != cudaSuccess))
+        return false;
+    note_launch();
+    k_miller_lines_multi<<<blocks_for(n * chunks, TEAMS), WARP, 0, s>>>(runs, lines, p, n, per, p_per, T, C, chunks);
+    if (chunks > 1) {
+        note_launch(2);
+        k_offsets<<<blocks_for(n + 1), TPB, 0, s>>>(offs, n + 1, chunks);
+        k_fp12_segment_product<<<blocks_for(n, TEAMS), WARP, 0, s>>>(out, runs, offs, n);
+        cudaFreeAsync(runs, s);
+        cudaFreeAsync(offs, s);
+    }
+    return true;
+}
 void launch_miller_lines(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, cudaStream_t s,
                          int64_t lines_n) {
     ProfScope prof_("miller_lines", s);
     if (n <= 0) return;
-    note_launch();
-    k_miller_lines<<<blocks_for(n), TPB, 0, s>>>(out, lines, p, n, lines_n > 0 ? lines_n : n);
+    miller_lines(out, lines, p, n, lines_n > 0 ? lines_n : n, 1, 1, s);
+}
+bool launch_miller_lines_multi(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, int64_t per, int T,
+                               cudaStream_t s, int64_t p_per) {
+    ProfScope prof_("miller_lines_multi", s);
+    if (T < 1 || per < 1) return false;
+    if (n <= 0) return true;
+    miller_lines(out, lines, p, n, per, p_per > 0 ? p_per : per, T, s);
+    return true;
 }
 void launch_miller(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t n, cudaStream_t s, int64_t p_mod,
                    int64_t q_mod) {
     ProfScope prof_("miller", s);
     if (n <= 0) return;
     note_launch();
-    k_miller<<<blocks_for(n), TPB, 0, s>>>(out, p, q, n, p_mod, q_mod);
+    k_miller_chunks<<<blocks_for(n, TEAMS), WARP, 0, s>>>(out, p, q, 1, n, 1, 1, p_mod, q_mod);
 }
-// Pairs per thread of the chunked unprepared Miller loops: sharing the 62
-// squarings over C pairs saves 2,232 Fp products per extra pair (about a
-// third of a loop), but a launch of fewer threads than the device holds
-// takes as long as the longest thread, so chunks grow only while the launch
-// still fills the resident threads.
 int miller_chunk(int64_t pairs) {
     if (g_tune.miller_chunk > 0) return g_tune.miller_chunk;
-    static std::atomic<int64_t> resident{0};
-    int64_t r = resident.load();
-    if (r == 0) {
-        int dev = 0, sms = 0, blocks = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_miller_chunks, TPB, 0);
-        r = (int64_t)(sms > 0 ? sms : 148) * (blocks > 0 ? blocks : 1) * TPB;
-        resident.store(r);
-    }
-    const int64_t C = pairs / r;
-    return (int)(C < 1 ? 1 : (C > MULTI_MILLER_MAX ? MULTI_MILLER_MAX : C));
+    return (int)miller_run(1, pairs, LINE_COMPUTED, MULTI_MILLER_MAX);
 }
 int64_t launch_miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t per, int64_t K, int C,
                              cudaStream_t s) {
@@ -285,7 +325,7 @@ int64_t launch_miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, i
     ProfScope prof_(tags[C], s);
     const int64_t chunks = (per + C - 1) / C;
     note_launch();
-    k_miller_chunks<<<blocks_for(K * chunks), TPB, 0, s>>>(out, p, q, per, K, C, chunks);
+    k_miller_chunks<<<blocks_for(K * chunks, TEAMS), WARP, 0, s>>>(out, p, q, per, K, C, chunks, 0, 0);
     return chunks;
 }
 void launch_fp12_mask(uint8_t* io, const uint8_t* valid, int64_t n, cudaStream_t s) {
@@ -297,54 +337,26 @@ void launch_fp12_segment_product(uint8_t* out, const uint8_t* in, const int64_t*
     ProfScope prof_("fp12_product", s);
     if (k <= 0) return;
     note_launch();
-    k_fp12_segment_product<<<blocks_for(k), TPB, 0, s>>>(out, in, offsets, k);
+    k_fp12_segment_product<<<blocks_for(k, TEAMS), WARP, 0, s>>>(out, in, offsets, k);
 }
-// Values per thread of the batched easy part: one Fp12 inversion (about 600
-// Fp products) per chunk against three products per value, so chunks grow
-// only while the launch still fills the resident threads.
-static int64_t easy_chunk(int64_t n) {
-    static std::atomic<int64_t> resident{0};
-    int64_t r = resident.load();
-    if (r == 0) {
-        int dev = 0, sms = 0, blocks = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_final_exp_easy_batch, TPB, 0);
-        r = (int64_t)(sms > 0 ? sms : 148) * (blocks > 0 ? blocks : 1) * TPB;
-        resident.store(r);
-    }
-    const int64_t C = n / r;
-    return C < 1 ? 1 : (C > 8 ? 8 : C);
-}
-
 void launch_final_exp(uint8_t* out, const uint8_t* in, int64_t n, FinalExpMode mode, cudaStream_t s) {
     ProfScope prof_(mode == FE_EASY ? "final_exp_easy" : (mode == FE_HARD ? "final_exp_hard" : "final_exp"), s);
     if (n <= 0) return;
-    const int64_t C = mode == FE_HARD ? 1 : easy_chunk(n);
-    uint8_t* pre = nullptr;
-    if (C > 1 && cudaMallocAsync(&pre, GT_SZ * (size_t)n, s) == cudaSuccess) {
-        const int64_t threads = (n + C - 1) / C;
-        note_launch();
-        k_final_exp_easy_batch<<<blocks_for(threads), TPB, 0, s>>>(out, in, pre, n, C, mode == FE_FULL ? 1 : 0);
-        cudaFreeAsync(pre, s);
-        return;
-    }
-    cudaGetLastError();
     note_launch();
-    k_final_exp<<<blocks_for(n), TPB, 0, s>>>(out, in, n, (int)mode);
+    k_final_exp<<<blocks_for(n, TEAMS), WARP, 0, s>>>(out, in, n, (int)mode);
 }
 
 void launch_fp12_mul(uint8_t* out, const uint8_t* a, int64_t sa, const uint8_t* b, int64_t sb, bool conj_b, int64_t n, cudaStream_t s) {
     if (n <= 0) return;
     note_launch();
-    k_fp12_mul<<<blocks_for(n), TPB, 0, s>>>(out, a, sa, b, sb, conj_b, n);
+    k_fp12_mul<<<blocks_for(n, TEAMS), WARP, 0, s>>>(out, a, sa, b, sb, conj_b, n);
 }
 void launch_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha, const uint8_t* beta, const uint8_t* valid,
                    int64_t n, cudaStream_t s) {
     ProfScope prof_("unmask", s);
     if (n <= 0) return;
     note_launch();
-    k_unmask<<<blocks_for(n), TPB, 0, s>>>(out, second, alpha, beta, valid, n);
+    k_unmask<<<blocks_for(n, TEAMS), WARP, 0, s>>>(out, second, alpha, beta, valid, n);
 }
 void launch_gt_compress(uint8_t* out, const uint8_t* in, int64_t n, cudaStream_t s) {
     ProfScope prof_("gt_compress", s);

@@ -62,165 +62,10 @@ static __device__ __noinline__ Line line_add(G2Proj& T, const G2A& Q) {
     return l;
 }
 
-WBTE_INL void mul_by_line(Fp12& f, const Line& l, const G1A& P) {
-    fp12_mul_line(f, f, l.c0, fp2_mul_fp(l.c1, P.x), fp2_mul_fp(l.c2, P.y));
-}
-
 WBTE_INL G2Proj g2proj_from_affine(const G2A& q) { return G2Proj{q.x, q.y, fp2_one()}; }
 
-// Miller loop computing lines on the fly; identities give 1.
-static __device__ __noinline__ void miller_loop(Fp12& f, const G1A& P, const G2A& Q) {
-    f = fp12_one();
-    if (is_inf(P) || is_inf(Q)) return;
-    G2Proj T = g2proj_from_affine(Q);
-    for (int i = 62; i >= 0; i--) {
-        if (i != 62) fp12_sqr(f, f);
-        Line l = line_double(T);
-        mul_by_line(f, l, P);
-        if ((X_ABS >> i) & 1) {
-            l = line_add(T, Q);
-            mul_by_line(f, l, P);
-        }
-    }
-    fp12_conj(f, f);  // the BLS12-381 parameter is negative
-}
-
-// Miller loop over precomputed lines.  `lines` points at this pair's first
-// line; consecutive lines of one pair are `stride` Line records apart.
-static __device__ __noinline__ void miller_loop_lines(Fp12& f, const Line* lines, size_t stride, const G1A& P) {
-    f = fp12_one();
-    if (is_inf(P)) return;
-    int idx = 0;
-    for (int i = 62; i >= 0; i--) {
-        if (i != 62) fp12_sqr(f, f);
-        Line l = load_vec(lines + stride * idx++);
-        mul_by_line(f, l, P);
-        if ((X_ABS >> i) & 1) {
-            l = load_vec(lines + stride * idx++);
-            mul_by_line(f, l, P);
-        }
-    }
-    fp12_conj(f, f);
-}
-
-// Product of T <= MULTI_MILLER_MAX Miller loops over precomputed lines
-// sharing one accumulator, so the 62 Fp12 squarings are paid once for all T
-// pairs.  Pair t uses the G1 point at points[t] (device memory) and the line
-// table at lines + t * pair_stride (lines of one table `stride` apart);
-// identities contribute 1.
+// pairs of one run of a Miller loop that computes its lines
 constexpr int MULTI_MILLER_MAX = 8;
-static __device__ __noinline__ void multi_miller_loop_lines(Fp12& f, const Line* lines, size_t stride,
-                                                            size_t pair_stride, const G1A* points, int T) {
-    G1A P[MULTI_MILLER_MAX];
-    for (int t = 0; t < T; t++) P[t] = load_affine(points + t);
-    f = fp12_one();
-    int idx = 0;
-    for (int i = 62; i >= 0; i--) {
-        if (i != 62) fp12_sqr(f, f);
-        for (int t = 0; t < T; t++) {
-            if (is_inf(P[t])) continue;
-            Line l = load_vec(lines + t * pair_stride + stride * idx);
-            mul_by_line(f, l, P[t]);
-        }
-        idx++;
-        if ((X_ABS >> i) & 1) {
-            for (int t = 0; t < T; t++) {
-                if (is_inf(P[t])) continue;
-                Line l = load_vec(lines + t * pair_stride + stride * idx);
-                mul_by_line(f, l, P[t]);
-            }
-            idx++;
-        }
-    }
-    fp12_conj(f, f);
-}
-
-// Product of C <= MULTI_MILLER_MAX Miller loops with lines computed on the
-// fly (unprepared_multi_miller_loop, weighted_btx/src/final_exponentiation.rs:
-// 229-274): pairs (P[t], Q[t]) share one accumulator, so the 62 Fp12
-// squarings are paid once for all C pairs; identities contribute 1.
-static __device__ __noinline__ void multi_miller_loop(Fp12& f, const G1A* P, const G2A* Q, int C) {
-    G2Proj T[MULTI_MILLER_MAX];
-    bool live[MULTI_MILLER_MAX];
-    for (int t = 0; t < C; t++) {
-        live[t] = !is_inf(P[t]) && !is_inf(Q[t]);
-        if (live[t]) T[t] = g2proj_from_affine(Q[t]);
-    }
-    f = fp12_one();
-    for (int i = 62; i >= 0; i--) {
-        if (i != 62) fp12_sqr(f, f);
-        for (int t = 0; t < C; t++) {
-            if (!live[t]) continue;
-            Line l = line_double(T[t]);
-            mul_by_line(f, l, P[t]);
-        }
-        if ((X_ABS >> i) & 1) {
-            for (int t = 0; t < C; t++) {
-                if (!live[t]) continue;
-                Line l = line_add(T[t], Q[t]);
-                mul_by_line(f, l, P[t]);
-            }
-        }
-    }
-    fp12_conj(f, f);
-}
-
-// ------------------------------------------------- final exponentiation
-// f^((p^6 - 1)(p^2 + 1))
-static __device__ __noinline__ void final_exp_easy(Fp12& r, const Fp12& f) {
-    Fp12 inv, t, u;
-    fp12_inv(inv, f);
-    fp12_conj(t, f);
-    fp12_mul(t, t, inv);
-    fp12_frobenius(u, t, 2);
-    fp12_mul(r, t, u);
-}
-
-WBTE_INL void mul_then_square(Fp12& acc, const Fp12& m, int n) {
-    fp12_mul(acc, acc, m);
-    for (int i = 0; i < n; i++) fp12_cyclotomic_sqr(acc, acc);
-}
-// x^(|z|/2) followed by conjugation, i.e. x^(z/2) for the negative parameter
-static __device__ __noinline__ void raise_to_z_div_by_2(Fp12& r, const Fp12& x) {
-    Fp12 acc;
-    fp12_cyclotomic_sqr(acc, x);
-    mul_then_square(acc, x, 2);
-    mul_then_square(acc, x, 3);
-    mul_then_square(acc, x, 9);
-    mul_then_square(acc, x, 32);
-    mul_then_square(acc, x, 15);
-    fp12_conj(r, acc);
-}
-WBTE_INL void raise_to_z(Fp12& r, const Fp12& x) {
-    Fp12 t;
-    raise_to_z_div_by_2(t, x);
-    fp12_cyclotomic_sqr(r, t);
-}
-
-static __device__ __noinline__ void final_exp_hard(Fp12& out, const Fp12& in) {
-    Fp12 result = in, y0, y1, y2, y3;
-    fp12_cyclotomic_sqr(y0, result);
-    raise_to_z(y1, y0);
-    raise_to_z_div_by_2(y2, y1);
-    fp12_conj(y3, result);
-    fp12_mul(y1, y1, y3);
-    fp12_conj(y1, y1);
-    fp12_mul(y1, y1, y2);
-    raise_to_z(y2, y1);
-    raise_to_z(y3, y2);
-    fp12_conj(y1, y1);
-    fp12_mul(y3, y3, y1);
-    fp12_conj(y1, y1);
-    fp12_frobenius(y1, y1, 3);
-    fp12_frobenius(y2, y2, 2);
-    fp12_mul(y1, y1, y2);
-    raise_to_z(y2, y3);
-    fp12_mul(y2, y2, y0);
-    fp12_mul(y2, y2, result);
-    fp12_mul(y1, y1, y2);
-    fp12_frobenius(y2, y3, 1);
-    fp12_mul(out, y1, y2);
-}
 
 // ------------------------------------------ decomposed GT exponentiation
 // A canonical scalar s < r is written s = d0 + d1|x| + d2|x|^2 + d3|x|^3
@@ -285,49 +130,6 @@ WBTE_INL void make_cyc_plan(CycPlan& pl, const uint32_t s_in[8]) {
     }
 }
 
-static __device__ __noinline__ void cyc_pow_plan(Fp12& out, const Fp12& value, const CycPlan& pl) {
-    if (pl.digits == 0) { out = fp12_one(); return; }
-    Fp12 tab[4][4], two;
-    fp12_cyclotomic_sqr(two, value);
-    tab[0][0] = value;
-    for (int i = 1; i < 4; i++) fp12_mul(tab[0][i], tab[0][i - 1], two);
-    for (int pw = 1; pw < 4; pw++)
-        for (int i = 0; i < 4; i++) {
-            fp12_frobenius(tab[pw][i], tab[0][i], pw);
-            if (pw & 1) fp12_conj(tab[pw][i], tab[pw][i]);
-        }
-    Fp12 acc = fp12_one();
-    bool started = false;
-    for (int pos = pl.digits - 1; pos >= 0; pos--) {
-        if (started) fp12_cyclotomic_sqr(acc, acc);
-        for (int c = 0; c < 4; c++) {
-            int d = pl.naf[c][pos];
-            if (!d) continue;
-            int ad = d < 0 ? -d : d;
-            if (started) {
-                if (d < 0) {
-                    Fp12 m;
-                    fp12_conj(m, tab[c][(ad - 1) >> 1]);
-                    fp12_mul(acc, acc, m);
-                } else {
-                    fp12_mul(acc, acc, tab[c][(ad - 1) >> 1]);
-                }
-            } else {
-                if (d < 0) fp12_conj(acc, tab[c][(ad - 1) >> 1]);
-                else acc = tab[c][(ad - 1) >> 1];
-                started = true;
-            }
-        }
-    }
-    out = acc;
-}
-
-WBTE_INL void gt_pow(Fp12& out, const Fp12& value, const uint32_t s[8]) {
-    CycPlan pl;
-    make_cyc_plan(pl, s);
-    cyc_pow_plan(out, value, pl);
-}
-
 // ------------------------------------------------ lane-split exponentiation
 // The transforms split one exponentiation across a few threads of a warp, one
 // base-|x| digit each, so that every thread of the warp runs the same fixed
@@ -378,75 +180,6 @@ WBTE_INL int r16_digit(uint64_t lo, uint64_t hi, int k, int top) {
     if (k < top) nib = (int)(((k < 16) ? (lo >> (4 * k)) : (hi >> (4 * (k - 16)))) & 15u);
     int cout = k < top ? r16_carry(lo, hi, k + 1) : 0;
     return nib + r16_carry(lo, hi, k) - 16 * cout;
-}
-
-// out = (+-Frobenius^c(v))^d for one base-|x| digit d (conjugated for odd
-// c), i.e. v^(d |x|^c) on GT; v must be cyclotomic.
-static __device__ __noinline__ void gt_pow_lane(Fp12& out, const Fp12& v, uint64_t d, int c) {
-    Fp12 tab[8];  // base^1 .. base^8
-    if (c == 0) {
-        tab[0] = v;
-    } else {
-        fp12_frobenius(tab[0], v, c);
-        if (c & 1) fp12_conj(tab[0], tab[0]);
-    }
-    fp12_cyclotomic_sqr(tab[1], tab[0]);
-    for (int k = 2; k < 8; k++) fp12_mul(tab[k], tab[k - 1], tab[0]);
-    Fp12 acc = fp12_one();
-    for (int k = 16; k >= 0; k--) {
-        if (k != 16) {
-            fp12_cyclotomic_sqr(acc, acc);
-            fp12_cyclotomic_sqr(acc, acc);
-            fp12_cyclotomic_sqr(acc, acc);
-            fp12_cyclotomic_sqr(acc, acc);
-        }
-        int dd = r16_digit(d, 0, k, 16);
-        int ad = dd < 0 ? -dd : dd;
-        if (ad) {
-            Fp12 m = tab[ad - 1];
-            if (dd < 0) fp12_conj(m, m);
-            fp12_mul(acc, acc, m);
-        }
-    }
-    out = acc;
-}
-
-// out = prod over the digits c = c0, c0 + step, ... < 4 of v^(d_c |x|^c):
-// one run of 64 cyclotomic squarings shared by the selected digits (Straus),
-// over one table of powers of phi^c0(v), phi = conj o Frobenius acting as
-// |x|; a later digit c applies phi^(c - c0) to the entry it multiplies in.
-// step 4 is gt_pow_lane (one digit); step 1 is the whole exponentiation.
-static __device__ __noinline__ void gt_pow_digits(Fp12& out, const Fp12& v, const uint64_t d[4], int c0, int step) {
-    Fp12 tab[8];  // phi^c0(v)^1 .. ^8
-    if (c0 == 0) {
-        tab[0] = v;
-    } else {
-        fp12_frobenius(tab[0], v, c0);
-        if (c0 & 1) fp12_conj(tab[0], tab[0]);
-    }
-    fp12_cyclotomic_sqr(tab[1], tab[0]);
-    for (int k = 2; k < 8; k++) fp12_mul(tab[k], tab[k - 1], tab[0]);
-    Fp12 acc = fp12_one();
-    for (int k = 16; k >= 0; k--) {
-        if (k != 16) {
-            fp12_cyclotomic_sqr(acc, acc);
-            fp12_cyclotomic_sqr(acc, acc);
-            fp12_cyclotomic_sqr(acc, acc);
-            fp12_cyclotomic_sqr(acc, acc);
-        }
-        for (int c = c0; c < 4; c += step) {
-            const int dd = r16_digit(d[c], 0, k, 16);
-            const int ad = dd < 0 ? -dd : dd;
-            if (!ad) continue;
-            const int rel = c - c0;
-            Fp12 m;
-            if (rel == 0) m = tab[ad - 1];
-            else fp12_frobenius(m, tab[ad - 1], rel);
-            if (((rel & 1) != 0) != (dd < 0)) fp12_conj(m, m);
-            fp12_mul(acc, acc, m);
-        }
-    }
-    out = acc;
 }
 
 // out = [w]p for w = hi 2^64 + lo < 16^top, over the signed radix-16 digits

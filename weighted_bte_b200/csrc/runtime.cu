@@ -1590,11 +1590,10 @@ static bool wpfe_open_core(Call& c, uint8_t* dm, const uint8_t* ds, uint64_t T, 
                            const uint8_t* dpc, const uint8_t* d2, const uint8_t* dap, uint64_t B, uint64_t K) {
     const uint64_t n = B * K, nt = n * T;
     const uint8_t* d2b = c.in_vec(fr_small_signed(std::vector<int64_t>(T * K, 2 * (int64_t)B)));
-    std::vector<int32_t> idx_share(nt), idx_slot(nt), idx_ap(n);
+    std::vector<int32_t> idx_share(nt), idx_slot(nt);
     // segment offsets carry k + 1 entries for k segments
     std::vector<int64_t> offs_2(nt + 1);
     for (uint64_t o = 0; o < n; o++) {
-        idx_ap[o] = (int32_t)(o % B);
         for (uint64_t k = 0; k < T; k++) {
             idx_share[o * T + k] = (int32_t)((o / B) * T + k);
             idx_slot[o * T + k] = (int32_t)o;
@@ -1603,7 +1602,6 @@ static bool wpfe_open_core(Call& c, uint8_t* dm, const uint8_t* ds, uint64_t T, 
     for (uint64_t x = 0; x <= nt; x++) offs_2[x] = (int64_t)(2 * x);
     const int32_t* dis = c.in_vec(idx_share);
     const int32_t* dil = c.in_vec(idx_slot);
-    const int32_t* dia = c.in_vec(idx_ap);
     const int64_t* do2 = c.in_vec(offs_2);
     uint8_t* scaled = c.alloc(G1_AFF * T * K);
     uint8_t* negfc = c.alloc(G1_AFF * n);
@@ -1613,7 +1611,6 @@ static bool wpfe_open_core(Call& c, uint8_t* dm, const uint8_t* ds, uint64_t T, 
     uint8_t* left = c.alloc(G1_AFF * nt);
     uint8_t* ft = c.alloc(GT_SZ * n);
     uint8_t* mp = c.alloc(GT_SZ * n);
-    uint8_t* apr = c.alloc(FR_SZ * n);
     const bool prepared = by_lines != nullptr;
     const uint8_t* dbl = prepared ? c.in(by_lines, LINE_SZ * LINES_PER_POINT * B * T) : nullptr;
     uint8_t* f = c.alloc(GT_SZ * (prepared ? n : nt));
@@ -1643,11 +1640,8 @@ static bool wpfe_open_core(Call& c, uint8_t* dm, const uint8_t* ds, uint64_t T, 
     launch_final_exp(mp, mp, (int64_t)n, FE_EASY, c.s);
     // mask = hard(mp / (ft pairing_cauchy)^(alpha (alpha + 1))); message = second / mask (:614-643)
     launch_fp12_mul(ft, ft, 1, dpc, 1, false, (int64_t)n, c.s);
-    // the slot's exponent is shared by the K batches: warp-uniform plans when K allows
-    if (!launch_gt_pow_shared(f, ft, dap, (int64_t)B, (int64_t)K, c.s)) {
-        launch_gather(apr, dap, dia, (int64_t)n, FR_SZ, c.s);
-        launch_gt_pow(f, ft, 1, apr, (int64_t)n, c.s);
-    }
+    // the slot's exponent is shared by the K batches
+    launch_gt_pow_shared(f, ft, dap, (int64_t)B, (int64_t)K, c.s);
     launch_fp12_mul(mp, mp, 1, f, 1, true, (int64_t)n, c.s);
     launch_final_exp(mp, mp, (int64_t)n, FE_HARD, c.s);
     launch_fp12_mul(dm, d2, 1, mp, 1, true, (int64_t)n, c.s);
