@@ -656,15 +656,21 @@ def gen_constants():
     w("// (p - 1) / 2, canonical, for the compressed-point sign flag")
     w("__device__ __constant__ const uint32_t C_P_HALF[12] = {%s};" % ", ".join(
         "0x%08xu" % l for l in limbs32((P - 1) // 2, 12)))
-    w("__device__ __constant__ const uint32_t C_P_MINUS_2[12] = {%s};" % ", ".join(
-        "0x%08xu" % l for l in limbs32(P - 2, 12)))
     w("// square-root exponents: (p + 1) / 4 in Fp, (p - 3) / 4 in Fp2 (p = 3 mod 4)")
     w("__device__ __constant__ const uint32_t C_P_PLUS1_DIV4[12] = {%s};" % ", ".join(
         "0x%08xu" % l for l in limbs32((P + 1) // 4, 12)))
     w("__device__ __constant__ const uint32_t C_P_MINUS3_DIV4[12] = {%s};" % ", ".join(
         "0x%08xu" % l for l in limbs32((P - 3) // 4, 12)))
-    w("__device__ __constant__ const uint32_t C_R_MINUS_2[8] = {%s};" % ", ".join(
-        "0x%08xu" % l for l in limbs32(R - 2, 8)))
+    # 30-bit limbs of k p and k r, k = 1, 2, 4, 8, 16, for the inversions
+    for name, m, n in (("P30", P, 13), ("R30", R, 9)):
+        rows = ["{" + ", ".join(str((k * m >> (30 * i)) & ((1 << 30) - 1)) for i in range(n)) + "}" for k in (1, 2, 4, 8, 16)]
+        w("// C_%s[j]: 30-bit limbs of 2^j times the modulus" % name)
+        w("__device__ __constant__ const int32_t C_%s[5][%d] = {%s};" % (name, n, ", ".join(rows)))
+        w("constexpr uint32_t %s_NEG_INV = 0x%08xu;  // -1 / modulus mod 2^30" % (name, -pow(m, -1, 1 << 30) % (1 << 30)))
+    w("__device__ __constant__ const uint32_t C_FP_R3[12] = {%s};" % ", ".join(
+        "0x%08xu" % l for l in limbs32((1 << 1152) % P, 12)))
+    w("__device__ __constant__ const uint32_t C_FR_R3[8] = {%s};" % ", ".join(
+        "0x%08xu" % l for l in limbs32((1 << 768) % R, 8)))
     # Radix-2 domain generators: the two-adic root 7^((r-1)/2^32), squared down.
     root = pow(7, (R - 1) >> 32, R)
     assert pow(root, 1 << 32, R) == 1 and pow(root, 1 << 31, R) != 1
