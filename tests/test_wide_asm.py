@@ -42,3 +42,12 @@ def test_wide_sums_wrap():
         a, b = rng.randrange(1 << 768), rng.randrange(1 << 768)
         assert value(call("wide_add", a=limbs(a, 24), b=limbs(b, 24))["r"]) == (a + b) % (1 << 768)
         assert value(call("wide_sub", a=limbs(a, 24), b=limbs(b, 24))["r"]) == (a - b) % (1 << 768)
+
+
+def test_sum_of_two_products():
+    rng = random.Random(5)
+    ri = pow(R384, -1, P)
+    for k in range(60):
+        a, b, c, d = ([0, 1, P - 1, P][rng.randrange(4)] if k < 30 else rng.randrange(P) for _ in range(4))
+        got = call("fp_mont_mul2", a=limbs(a, 12), b=limbs(b, 12), c=limbs(c, 12), d=limbs(d, 12))["r"]
+        assert value(got) == (a * b + c * d) * ri % P

@@ -234,6 +234,34 @@ def _asm_function(name, args, lines, outs, ins):
             % (name, args, body, o, i))
 
 
+def gen_mont_mul2(name, modulus, n):
+    """r = (a b + c d) / 2^(32n) mod m for factors up to m (the sum before each
+    shift stays below 5 m 2^32 < 2^(32(n+1)), the result before the last
+    subtraction below 1.3 m)."""
+    pinv = (-pow(modulus, -1, 1 << 32)) % (1 << 32)
+    ml = limbs32(modulus, n)
+    mw = ["0x%08x" % x for x in ml]
+    lines = []
+    w = lines.append
+    w(Window.regs(n, ""))
+    w(".reg .u32 t<%d>, m, bw, d<%d>;" % (n, n))
+    w(".reg .pred nb;")
+    a, b, c, d = ([("%%%d" % (k * n + i)) for i in range(n)] for k in range(1, 5))
+    win = Window(w, n, "")
+    for i in range(n):
+        if i:
+            win.shift()
+        win.add_row(a, b[i])
+        win.add_row(c, d[i])
+        w("mul.lo.u32 m, %s, 0x%08x;" % (win.E[0], pinv))
+        win.add_row(mw, "m")
+    t = ["t%d" % i for i in range(n)]
+    win.merge(t)
+    emit_cond_sub(w, ["%%%d" % i for i in range(n)], t, ml)
+    return _asm_function(name, ", ".join(["uint32_t r[%d]" % n] + ["const uint32_t %s[%d]" % (v, n) for v in "abcd"]), lines,
+                         [("r", i) for i in range(n)], [(v, i) for v in "abcd" for i in range(n)])
+
+
 def gen_mul_wide(name, n):
     """r (2n words) = a b, any n-word a and b."""
     lines = []
@@ -705,6 +733,7 @@ def main():
         gen_add("fp_add_raw", P, 12),
         gen_sub("fp_sub_raw", P, 12),
         gen_add_nr("fp_add_nored", 12),
+        gen_mont_mul2("fp_mont_mul2", P, 12),
         gen_mul_wide("fp_mul_wide", 12),
         gen_redc("fp_redc", P, 12),
         gen_cond_sub("fp_csub_p", P, 12),

@@ -227,61 +227,7 @@ __global__ void k_ntt_load(uint8_t* work, const uint8_t* in, int64_t n, int bits
     store_vec(reinterpret_cast<Xyzz<F>*>(work) + q * n + bitrev64(j, bits), p);
 }
 
-// One radix-2 butterfly per group of L lanes (blocks of one warp); twiddle
-// index j * (n / size).  The twiddle multiplication is split along the
-// base-|x| digits of the twiddle: four lanes on G2 ([d_c] (-1)^c psi^c(v)),
-// two lanes on G1 ([a]v and [b](phi(v) + v)); the parts are summed in shared
-// memory before the butterfly.
-template <class F> struct NttLanes;
-template <> struct NttLanes<Fp> { static constexpr int L = 2; };
-template <> struct NttLanes<Fp2> { static constexpr int L = 4; };
 constexpr int WARP = 32;
-
-WBTE_INL void ntt_part(G1X& out, const G1X& v, const uint64_t d[4], int c) { g1_mul_lane(out, v, d, c); }
-WBTE_INL void ntt_part(G2X& out, const G2X& v, const uint64_t d[4], int c) { g2_mul_lane(out, v, d, c); }
-
-template <class F>
-__global__ void __launch_bounds__(WARP) k_ntt_stage(uint8_t* work, const uint8_t* tw, int64_t n, int64_t half,
-                                                   int64_t count) {
-    constexpr int L = NttLanes<F>::L;
-    __shared__ Xyzz<F> sh[WARP];
-    const int lane = threadIdx.x, c = lane % L;
-    const int64_t t = ((int64_t)blockIdx.x * WARP + lane) / L;
-    const bool active = t < (n / 2) * count;
-    const int64_t q = active ? t / (n / 2) : 0, tt = active ? t % (n / 2) : 0;
-    const int64_t chunk = tt / half, j = tt % half;
-    const int64_t a = q * n + chunk * 2 * half + j, b = a + half;
-    Xyzz<F>* w = reinterpret_cast<Xyzz<F>*>(work);
-    Xyzz<F> part;
-    set_inf(part);
-    if (active) {
-        Xyzz<F> v = load_vec(w + b);
-        if (j != 0) {
-            uint32_t s[8];
-            load_scalar(s, tw + FR_SZ * (j * (n / (2 * half))));
-            uint64_t d[4];
-            decompose_base_x(d, s);
-            ntt_part(part, v, d, c);
-        } else if (c == 0) {
-            part = v;
-        }
-    }
-    store_vec(sh + lane, part);
-    __syncwarp();
-    for (int step = 1; step < L; step *= 2) {
-        if (c % (2 * step) == 0) store_vec(sh + lane, xyzz_add(load_vec(sh + lane), load_vec(sh + lane + step)));
-        __syncwarp();
-    }
-    // lanes 0 and 1 both read u before either output is written
-    Xyzz<F> u;
-    if (active && c < 2) u = load_vec(w + a);
-    __syncwarp();
-    if (active && c < 2) {
-        Xyzz<F> tv = load_vec(sh + (lane - c));
-        if (c == 1) tv = neg(tv);
-        store_vec(w + (c == 0 ? a : b), xyzz_add(u, tv));
-    }
-}
 
 // MSMs of a few terms (the share checks' per-slot aggregates): out[o] =
 // sum_t scalars[vsel[o] n + t] points[pbase[o] + idx[t]].  Every scalar is
@@ -913,6 +859,14 @@ void launch_domain_twiddles(uint8_t* tw, int64_t n, int64_t count, bool inverse,
 void launch_mul_batch(Group g, uint8_t* out, const uint8_t* pts, int64_t stride, const uint8_t* scalars, int64_t n, cudaStream_t s) {
     ProfScope prof_("mul_batch", s);
     if (n <= 0) return;
+    // 252 doublings and 76 additions by one thread or one quad (the measures
+    // of ntt_joint)
+    const bool g1 = g == GROUP_G1;
+    if (launch_time((252 * 3 + 76 * 4) * (g1 ? 360.0 : 530.0), (double)n / (g1 ? 8 : 4)) <
+        launch_time((252 * 9 + 76 * 14) * (g1 ? 300.0 : 1800.0), (double)n / 32)) {
+        launch_quad_mul_batch(g, out, pts, stride, scalars, n, s);
+        return;
+    }
     note_launch();
     if (g == GROUP_G1) k_mul_batch<Fp><<<blocks_for(n), TPB, 0, s>>>(out, pts, stride, scalars, n);
     else k_mul_batch<Fp2><<<blocks_for(n), TPB, 0, s>>>(out, pts, stride, scalars, n);
@@ -974,40 +928,21 @@ void launch_negate(Group g, uint8_t* out, const uint8_t* in, int64_t n, cudaStre
 }
 
 // Whether a transform stage of `butterflies` butterflies runs one thread per
-// butterfly (k_ntt_stage_joint) rather than the lane split: a cost model of one
-// thread's Fp products (G1: 128 doublings and 66 additions joint, against 128
-// and 33 per lane on 2 lanes; G2: 64 and 68 against 64 and 17 per lane on 4
-// lanes) times max(1, threads / resident threads).  WBTE_NTT_JOINT = 0 or 1
-// overrides the choice, and so does the calling context's tuning knob.
+// butterfly (k_ntt_stage_joint) rather than quads: a cost model of one
+// thread's products (G1: 128 doublings and 81 additions of 9 and 14 products
+// of 300 wide multiply-adds; G2: 64 and 75 of 9 and 14 Fp2 products of 900, at
+// half the pipe rate for their spills) and of a quad lane's rounds (G1: 128
+// doublings of three and 41 additions of four rounds, a fifth more for the
+// exchanges, eight lanes a butterfly; G2: 64 and 24 rounds of 444, 32 lanes).
+// WBTE_NTT_JOINT = 0 or 1 overrides the choice, and so does the calling
+// context's tuning knob.
 static bool ntt_joint(Group g, int64_t butterflies) {
     if (const char* env = getenv("WBTE_NTT_JOINT")) return atoi(env) != 0;
     if (g_tune.ntt_joint == 0 || g_tune.ntt_joint == 1) return g_tune.ntt_joint == 1;
-    static std::atomic<int64_t> cap[2][2] = {{{0}, {0}}, {{0}, {0}}};
-    const int gi = g == GROUP_G1 ? 0 : 1;
-    int64_t c[2];
-    for (int v = 0; v < 2; v++) {
-        c[v] = cap[gi][v].load();
-        if (c[v] == 0) {
-            int dev = 0, sms = 0, blocks = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            if (g == GROUP_G1)
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &blocks, v ? (const void*)k_ntt_stage_joint<Fp> : (const void*)k_ntt_stage<Fp>, WARP, 0);
-            else
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                    &blocks, v ? (const void*)k_ntt_stage_joint<Fp2> : (const void*)k_ntt_stage<Fp2>, WARP, 0);
-            c[v] = (int64_t)(blocks > 0 ? blocks : 1) * WARP * (sms > 0 ? sms : 1);
-            cap[gi][v].store(c[v]);
-        }
-    }
-    const bool g1 = g == GROUP_G1;
-    const int L = g1 ? NttLanes<Fp>::L : NttLanes<Fp2>::L;
-    const double dbl = g1 ? 9.0 : 30.0, add = g1 ? 12.0 : 42.0, dbls = g1 ? 128.0 : 64.0;
-    const double adds_joint = g1 ? 66.0 + 15.0 : 68.0 + 7.0, adds_lane = g1 ? 33.0 + 8.0 : 17.0 + 7.0;
-    const double joint = std::max(1.0, (double)butterflies / (double)c[1]) * (dbls * dbl + adds_joint * add);
-    const double lane = std::max(1.0, (double)(butterflies * L) / (double)c[0]) * (dbls * dbl + adds_lane * add);
-    return joint < lane;
+    const double n = (double)butterflies;
+    if (g == GROUP_G1)
+        return launch_time((128 * 9 + 81 * 14) * 300.0, n / 32) < launch_time((128 * 3 + 41 * 4) * 360.0, n / 4);
+    return launch_time((64 * 9 + 75 * 14) * 1800.0, n / 32) < launch_time((64 * 3 + 24 * 4) * 530.0, n);
 }
 
 // work[i] = [c_i] in[i] for small signed c_i (XYZZ out): double-and-add over
@@ -1094,11 +1029,12 @@ void launch_group_ntt(Group g, uint8_t* io, uint8_t* work, const uint8_t* tw, in
         // with at most a quarter of the lanes idle
         const int64_t pad = count >= 24 && count < WARP ? (int64_t)WARP : count;
         for (int64_t half = 1; half < n; half *= 2) {
-            note_launch();
-            if (joint)
+            if (joint) {
+                note_launch();
                 k_ntt_stage_joint<Fp><<<blocks_for((n / 2) * pad, WARP), WARP, 0, s>>>(work, tw, n, half, count, pad);
-            else
-                k_ntt_stage<Fp><<<blocks_for(NttLanes<Fp>::L * butterflies, WARP), WARP, 0, s>>>(work, tw, n, half, count);
+            } else {
+                launch_quad_ntt_stage(g, work, tw, n, half, count, s);
+            }
         }
         launch_xyzz_to_affine(GROUP_G1, io, work, total, s);
     } else {
@@ -1106,11 +1042,12 @@ void launch_group_ntt(Group g, uint8_t* io, uint8_t* work, const uint8_t* tw, in
         k_ntt_load<Fp2><<<blocks_for(total), TPB, 0, s>>>(work, io, n, bits, count);
         const bool joint = ntt_joint(g, butterflies);
         for (int64_t half = 1; half < n; half *= 2) {
-            note_launch();
-            if (joint)
+            if (joint) {
+                note_launch();
                 k_ntt_stage_joint<Fp2><<<blocks_for(butterflies, WARP), WARP, 0, s>>>(work, tw, n, half, count, count);
-            else
-                k_ntt_stage<Fp2><<<blocks_for(NttLanes<Fp2>::L * butterflies, WARP), WARP, 0, s>>>(work, tw, n, half, count);
+            } else {
+                launch_quad_ntt_stage(g, work, tw, n, half, count, s);
+            }
         }
         launch_xyzz_to_affine(GROUP_G2, io, work, total, s);
     }
@@ -1187,43 +1124,38 @@ __global__ void __launch_bounds__(WARP) k_fixed_msm_g2(uint8_t* out, const uint8
     store_affine(reinterpret_cast<G2A*>(out + G2_AFF * o), to_affine(acc));
 }
 
-// Lanes per small-MSM output, from a cost model: a lane's work is its
-// tables (7 additions per term it touches; 15 on G1, two tables), the shared
-// doublings and one addition per window and pair it holds; the launch takes
-// about max(1, k L / resident threads) times one lane's work.  The lanes run
-// from 1 up to one per (term, digit) pair, rounded up to a power of two.
-// WBTE_SMALL_MSM_LANES (a power of two up to 32) overrides the choice.
-static int small_msm_lanes(Group g, int64_t k, int64_t n) {
+// How a small MSM's outputs are spread: over L lanes of one thread per pair
+// group (quads false) or over L quads.
+struct SmallMsmSpread { bool quads; int L; };
+// From a cost model of one lane's work: its tables (7 additions per term it
+// touches; 15 on G1, two tables; on quads 7 per pair), the shared doublings and
+// one addition per window and pair it holds, in the measures of ntt_joint.
+// Lanes run from 1 up to one per (term, digit) pair, rounded up to a power of
+// two; quads up to a warp's.  WBTE_SMALL_MSM_LANES (a power of two up to 32)
+// forces lanes.
+static SmallMsmSpread small_msm_spread(Group g, int64_t k, int64_t n) {
     if (const char* env = getenv("WBTE_SMALL_MSM_LANES")) {
         const int v = atoi(env);
-        if (v >= 1 && v <= WARP && (v & (v - 1)) == 0) return v;
-    }
-    static std::atomic<int64_t> cap[2] = {{0}, {0}};
-    const int gi = g == GROUP_G1 ? 0 : 1;
-    int64_t c = cap[gi].load();
-    if (c == 0) {
-        int dev = 0, sms = 0, blocks = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (g == GROUP_G1) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_small_msm<Fp>, WARP, 0);
-        else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_small_msm<Fp2>, WARP, 0);
-        c = (int64_t)(blocks > 0 ? blocks : 1) * WARP * (sms > 0 ? sms : 1);
-        cap[gi].store(c);
+        if (v >= 1 && v <= WARP && (v & (v - 1)) == 0) return {false, v};
     }
     const bool g1 = g == GROUP_G1;
     const int D = g1 ? SmallMsmDigits<Fp>::D : SmallMsmDigits<Fp2>::D;
     const int windows = (g1 ? SmallMsmDigits<Fp>::TOP : SmallMsmDigits<Fp2>::TOP) + 1;
-    const double add = g1 ? 12.0 : 42.0, dbl = g1 ? 9.0 : 30.0, table = g1 ? 15.0 : 7.0;  // Fp products
+    const double product = g1 ? 300.0 : 1800.0, round = g1 ? 360.0 : 530.0, table = g1 ? 15.0 : 7.0;
     const int64_t pairs = n * D;
-    int best = 1;
+    SmallMsmSpread best = {false, 1};
     double best_t = 0;
     for (int L = 1; L <= WARP; L *= 2) {
         int terms = 0, prev = -1;
         for (int64_t p = 0; p < pairs; p += L)
             if (p / D != prev) prev = (int)(p / D), terms++;
-        const double lane = terms * table * add + 4.0 * (windows - 1) * dbl + (double)((pairs + L - 1) / L) * windows * add;
-        const double t = std::max(1.0, (double)(k * L) / (double)c) * lane;
-        if (L == 1 || t < best_t) best = L, best_t = t;
+        const double mine = (double)((pairs + L - 1) / L), dbls = 4.0 * (windows - 1);
+        const double t = launch_time((dbls * 9 + (terms * table + mine * windows) * 14) * product, (double)(k * L) / 32);
+        if (L == 1 || t < best_t) best = {false, L}, best_t = t;
+        if (L <= (g1 ? 8 : 4)) {
+            const double q = launch_time((dbls * 3 + mine * (windows + 7) * 4) * round, (double)(k * L) / (g1 ? 8 : 4));
+            if (q < best_t) best = {true, L}, best_t = q;
+        }
         if (L >= pairs) break;
     }
     return best;
@@ -1234,7 +1166,12 @@ void launch_small_msm(Group g, uint8_t* out, const uint8_t* points, const int64_
     ProfScope prof_(g == GROUP_G1 ? "small_msm_g1" : "small_msm_g2", s);
     if (k <= 0) return;
     if (n < 1 || n > SMALL_MSM_MAX) return;
-    const int L = small_msm_lanes(g, k, n);
+    const SmallMsmSpread spread = small_msm_spread(g, k, n);
+    const int L = spread.L;
+    if (spread.quads) {
+        launch_quad_small_msm(g, out, points, pbase, idx, scalars, vsel, k, n, L, s);
+        return;
+    }
     note_launch();
     if (g == GROUP_G1)
         k_small_msm<Fp><<<blocks_for(L * k, WARP), WARP, 0, s>>>(out, points, pbase, idx, scalars, vsel, k, n, L);
@@ -1278,9 +1215,15 @@ void launch_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t* R, c
                            int64_t n, cudaStream_t st) {
     ProfScope prof_("schnorr_verify", st);
     if (n <= 0) return;
-    note_launch();
     const uint8_t* table = generator_table(GROUP_G1, st);
     if (!table) return;
+    // 128 doublings and about 130 additions by one thread, or 128 and 60 on
+    // each of four quads
+    if (launch_time((128 * 3 + 60 * 4) * 360.0, (double)n / 2) < launch_time((128 * 9 + 130 * 13) * 300.0, (double)n / 32)) {
+        launch_quad_schnorr_verify(valid, X, R, sresp, c, n, table, st);
+        return;
+    }
+    note_launch();
     k_schnorr_verify<<<blocks_for(n), TPB, 0, st>>>(valid, X, R, sresp, c, n, table);
 }
 

@@ -265,9 +265,7 @@ __global__ void __launch_bounds__(WARP) k_gt_pow_small(uint8_t* out, const uint8
 // Teams per exponentiation for E of them, from a cost model: the wide
 // multiply-adds of one lane, in thousands (64 squarings of 888; products of
 // 1,608: 52 and three for the table with the warp-uniform NAF, 17 a digit and
-// seven for the table in radix 16; table images of 744), times the warps per
-// scheduler.  One warp alone keeps the pipe 0.6 busy, so fewer than that
-// cost nothing.  WBTE_GT_LANES = 1, 2 or 4 overrides it, and so does the
+// seven for the table in radix 16; table images of 744).  WBTE_GT_LANES = 1, 2 or 4 overrides it, and so does the
 // calling context's tuning knob.
 int gt_pow_teams(int64_t E, bool uniform) {
     if (const char* env = getenv("WBTE_GT_LANES")) {
@@ -275,22 +273,12 @@ int gt_pow_teams(int64_t E, bool uniform) {
         if (v == 1 || v == 2 || v == 4) return v;
     }
     if (g_tune.gt_lanes == 1 || g_tune.gt_lanes == 2 || g_tune.gt_lanes == 4) return g_tune.gt_lanes;
-    static std::atomic<int> schedulers{0};
-    int sc = schedulers.load();
-    if (sc == 0) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        sc = 4 * (sms > 0 ? sms : 148);
-        schedulers.store(sc);
-    }
     const double work[3] = {uniform ? 156.0 : 195.0, 130.0, 98.0};
     const int per[3] = {TEAMS, 4, 4};
     int best = 1;
     double best_t = 0;
     for (int i = 0, L = 1; L <= 4; i++, L *= 2) {
-        const double warps = (double)(E * L) / per[i] / sc;
-        const double time = work[i] * std::max(1.6, warps);
+        const double time = launch_time(work[i], (double)(E * L) / per[i]);
         if (L == 1 || time < best_t) best = L, best_t = time;
     }
     return best;

@@ -260,21 +260,6 @@ __global__ void k_reduce_warp(uint8_t* out, const uint8_t* in, int64_t rows, int
     if (lane == 0) store_vec(reinterpret_cast<Xyzz<F>*>(out) + wid, acc);
 }
 
-template <class F>
-__global__ void k_combine(uint8_t* out, const uint8_t* wins, int64_t k, int windows, int c) {
-    int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= k) return;
-    const Xyzz<F>* W = reinterpret_cast<const Xyzz<F>*>(wins) + j * windows;
-    Xyzz<F> acc;
-    set_inf(acc);
-    for (int w = windows - 1; w >= 0; w--) {
-        if (!is_inf(acc))
-            for (int i = 0; i < c; i++) acc = xyzz_dbl(acc);
-        acc = xyzz_add(acc, load_vec(W + w));
-    }
-    store_affine(reinterpret_cast<Affine<F>*>(out + Aff<F>::SZ * j), to_affine(acc));
-}
-
 struct ScratchLayout {
     size_t digits, entries, nnz, seg, red, total;
 };
@@ -348,8 +333,7 @@ void run_family(uint8_t* out, const uint8_t* points, const int64_t* pbase, const
         flip ^= 1;
         len = out_len;
     }
-    note_launch();
-    k_combine<F><<<blocks_for(k, 64), 64, 0, s>>>(out, src, k, p.windows, p.c);
+    launch_msm_combine(g1 ? GROUP_G1 : GROUP_G2, out, src, k, p.windows, p.c, s);
     prof_end(tok, s);
 }
 }  // namespace

@@ -246,24 +246,13 @@ void launch_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n, cudaStrea
 // Pairs per team of a launch of `outputs` products of T Miller loops each.
 // Sharing the 62 squarings saves 73 of a first pair's wide multiply-adds (in
 // thousands per lane: 62 squarings of 1,176; `line` for one pair's 68 lines),
-// but one warp keeps a scheduler's pipe only 0.6 busy, so runs are cut while
-// the launch has fewer than 1.6 warps for each scheduler.
+// so runs are cut only while the launch leaves schedulers idle.
 static int64_t miller_run(int64_t outputs, int64_t T, double line, int64_t most) {
-    static std::atomic<int> schedulers{0};
-    int sc = schedulers.load();
-    if (sc == 0) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        sc = 4 * (sms > 0 ? sms : 148);
-        schedulers.store(sc);
-    }
     int64_t best = 1;
     double best_t = 0;
     for (int64_t C = 1; C <= std::min(T, most); C++) {
         const int64_t chunks = (T + C - 1) / C;
-        const double warps = (double)(outputs * chunks) / TEAMS / sc;
-        const double time = (73.0 + line * C) * std::max(1.6, warps);
+        const double time = launch_time(73.0 + line * C, (double)(outputs * chunks) / TEAMS);
         if (C == 1 || time < best_t) best = C, best_t = time;
     }
     return best;

@@ -4,9 +4,10 @@
 //   G1 affine 96 B, G2 affine 192 B, Fp12 576 B, Fr scalars as canonical
 //   32-byte little-endian integers, the point at infinity as zero bytes.
 #pragma once
+#include <algorithm>
+#include <atomic>
 #include <cstddef>
 #include <cstdint>
-#include <atomic>
 #include <cuda_runtime.h>
 
 namespace wbte {
@@ -43,6 +44,25 @@ struct Tuning {
     int miller_chunk = 0;  // pairs per thread of the chunked unprepared Miller loops, 1..8
 };
 extern thread_local Tuning g_tune;
+
+// warp schedulers of the current device (four to an SM)
+inline int schedulers() {
+    static std::atomic<int> cache{0};
+    int n = cache.load(std::memory_order_relaxed);
+    if (n == 0) {
+        int dev = 0, sms = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        n = 4 * (sms > 0 ? sms : 148);
+        cache.store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+// The cost models' time of a launch of `warps` warps whose lanes spend `work`
+// wide multiply-adds each.  One warp alone keeps a scheduler's multiply-add
+// pipe 0.6 busy (14.0 of 18.6 and 19.1 of 29.7 G products/s measured at one
+// and at eight warps), so fewer than 1.6 warps a scheduler take as long as 1.6.
+inline double launch_time(double work, double warps) { return work * std::max(1.6, warps / schedulers()); }
 
 constexpr size_t G1_AFF = 96, G2_AFF = 192, G1_XYZZ = 192, G2_XYZZ = 384, GT_SZ = 576, FR_SZ = 32;
 constexpr size_t LINE_SZ = 288;  // three Fp2 coefficients
@@ -128,6 +148,19 @@ void launch_small_msm(Group g, uint8_t* out, const uint8_t* points, const int64_
 void launch_msm_family(Group g, uint8_t* out, const uint8_t* points, const int64_t* pbase, const int32_t* idx,
                        const uint8_t* scalars, const int32_t* vsel, int32_t V, int64_t k, int64_t n,
                        cudaStream_t s, const MsmPlan* forced = nullptr);
+// Kernels over quads (k_quad.cu) for launches that leave schedulers idle:
+// out[j] = sum_w 2^(c w) wins[j windows + w] from XYZZ window sums
+void launch_msm_combine(Group g, uint8_t* out, const uint8_t* wins, int64_t k, int windows, int c, cudaStream_t s);
+// one radix-2 stage over XYZZ points
+void launch_quad_ntt_stage(Group g, uint8_t* work, const uint8_t* tw, int64_t n, int64_t half, int64_t count,
+                           cudaStream_t s);
+// launch_small_msm with the (term, digit) pairs of an output on L points
+void launch_quad_small_msm(Group g, uint8_t* out, const uint8_t* points, const int64_t* pbase, const int32_t* idx,
+                           const uint8_t* scalars, const int32_t* vsel, int64_t k, int64_t n, int L, cudaStream_t s);
+void launch_quad_mul_batch(Group g, uint8_t* out, const uint8_t* pts, int64_t stride, const uint8_t* scalars, int64_t n,
+                           cudaStream_t s);
+void launch_quad_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t* R, const uint8_t* sresp, const uint8_t* c,
+                                int64_t n, const uint8_t* gen_table, cudaStream_t s);
 // Scratch-size query and launch with caller-supplied scratch (no allocation).
 size_t msm_family_scratch_bytes(Group g, int32_t V, int64_t k, int64_t n, const MsmPlan& plan);
 void launch_msm_family_scratch(Group g, uint8_t* out, const uint8_t* points, const int64_t* pbase, const int32_t* idx,

@@ -130,11 +130,7 @@ WBTE_INL void make_cyc_plan(CycPlan& pl, const uint32_t s_in[8]) {
     }
 }
 
-// ------------------------------------------------ lane-split exponentiation
-// The transforms split one exponentiation across a few threads of a warp, one
-// base-|x| digit each, so that every thread of the warp runs the same fixed
-// schedule of squarings (data-dependent NAF lengths otherwise diverge).
-
+// ------------------------------------------------ fixed-schedule recodings
 // s = d0 + d1|x| + d2|x|^2 + d3|x|^3 with 0 <= dc < |x| (s < r < |x|^4)
 WBTE_INL void decompose_base_x(uint64_t d[4], const uint32_t s_in[8]) {
     uint32_t s[8];
@@ -182,31 +178,6 @@ WBTE_INL int r16_digit(uint64_t lo, uint64_t hi, int k, int top) {
     return nib + r16_carry(lo, hi, k) - 16 * cout;
 }
 
-// out = [w]p for w = hi 2^64 + lo < 16^top, over the signed radix-16 digits
-template <class F>
-static __device__ __noinline__ void xyzz_mul_r16(Xyzz<F>& out, const Xyzz<F>& p, uint64_t lo, uint64_t hi, int top) {
-    Xyzz<F> tab[8];  // [1]p .. [8]p
-    tab[0] = p;
-    tab[1] = xyzz_dbl(tab[0]);
-    for (int k = 2; k < 8; k++) tab[k] = xyzz_add(tab[k - 1], tab[0]);
-    Xyzz<F> acc;
-    set_inf(acc);
-    for (int k = top; k >= 0; k--) {
-        acc = xyzz_dbl(acc);
-        acc = xyzz_dbl(acc);
-        acc = xyzz_dbl(acc);
-        acc = xyzz_dbl(acc);
-        int dd = r16_digit(lo, hi, k, top);
-        int ad = dd < 0 ? -dd : dd;
-        if (ad) {
-            Xyzz<F> m = tab[ad - 1];
-            if (dd < 0) m = neg(m);
-            acc = xyzz_add(acc, m);
-        }
-    }
-    out = acc;
-}
-
 // psi (untwist-Frobenius-twist) on G2 in XYZZ coordinates; acts as [x]
 WBTE_INL G2X g2_psi(const G2X& p) {
     G2X r;
@@ -221,29 +192,6 @@ WBTE_INL G1X g1_phi(const G1X& p) {
     G1X r = p;
     r.X = fp_mul(p.X, fp_from_const(C_GLV_BETA));
     return r;
-}
-
-// Lane c (0..3) of [s]v on G2 for s = sum_c d_c |x|^c:
-// out = [d_c]((-1)^c psi^c(v)) = [d_c |x|^c]v.
-WBTE_INL void g2_mul_lane(G2X& out, const G2X& v, const uint64_t d[4], int c) {
-    G2X base = v;
-    for (int i = 0; i < c; i++) base = g2_psi(base);
-    if (c & 1) base = neg(base);
-    xyzz_mul_r16(out, base, d[c], 0, 16);
-}
-
-// Lane c (0 or 1) of [s]v on G1 for s = a + b |x|^2 with a = d0 + d1|x| and
-// b = d2 + d3|x| (both below |x|^2 < 2^128): [a]v, or [b](phi(v) + v) since
-// phi(v) + v = [x^2]v.
-WBTE_INL void g1_mul_lane(G1X& out, const G1X& v, const uint64_t d[4], int c) {
-    G1X base = v;
-    if (c) base = xyzz_add(g1_phi(v), v);
-    uint64_t lo = d[2 * c], hi = d[2 * c + 1];
-    // w = lo + hi |x| as a 128-bit integer
-    uint64_t plo = hi * X_ABS, phi = __umul64hi(hi, X_ABS);
-    uint64_t wlo = plo + lo;
-    uint64_t whi = phi + (wlo < plo ? 1 : 0);
-    xyzz_mul_r16(out, base, wlo, whi, 32);
 }
 
 }  // namespace wbte
