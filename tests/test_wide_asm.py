@@ -19,7 +19,7 @@ def test_wide_product(a):
         assert value(call("fp_mul_wide", a=limbs(a, 12), b=limbs(b, 12))["r"]) == a * b
 
 
-@pytest.mark.parametrize("lo,hi,shift", [(-16, 6, 2), (-14, 8, 2), (-5, 17, 1), (-6, 5, 1), (-2, 7, 1), (-3, 3, 1)])
+@pytest.mark.parametrize("lo,hi,shift", [(-16, 6, 2), (-14, 8, 2), (-5, 17, 1), (-4, 8, 1), (-3, 3, 1)])
 def test_reduction_of_signed_sums(lo, hi, shift):
     """Sums in (lo p^2, hi p^2), shifted by shift * p 2^384, reduce below 4p."""
     rng = random.Random(lo)
@@ -51,3 +51,13 @@ def test_sum_of_two_products():
         a, b, c, d = ([0, 1, P - 1, P][rng.randrange(4)] if k < 30 else rng.randrange(P) for _ in range(4))
         got = call("fp_mont_mul2", a=limbs(a, 12), b=limbs(b, 12), c=limbs(c, 12), d=limbs(d, 12))["r"]
         assert value(got) == (a * b + c * d) * ri % P
+
+
+def test_small_multiples():
+    rng = random.Random(6)
+    for _ in range(40):
+        a = rng.randrange(8 * P)
+        r = call("fp_csub_4p", a=limbs(a, 12))["r"]
+        assert value(r) == (a - 4 * P if a >= 4 * P else a)
+        b = rng.randrange(P + 1)
+        assert value(call("fp_p_minus", a=limbs(b, 12))["r"]) == P - b

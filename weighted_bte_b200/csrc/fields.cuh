@@ -50,6 +50,11 @@ WBTE_INL bool fp_eq(const Fp& a, const Fp& b) {
     _Pragma("unroll") for (int i = 0; i < 12; i++) x |= a.v[i] ^ b.v[i];
     return x == 0;
 }
+WBTE_INL Fp fp_select(bool c, const Fp& a, const Fp& b) {
+    Fp r;
+    _Pragma("unroll") for (int i = 0; i < 12; i++) r.v[i] = c ? a.v[i] : b.v[i];
+    return r;
+}
 WBTE_INL Fp fp_from_const(const uint32_t (&c)[12]) {
     Fp r;
     _Pragma("unroll") for (int i = 0; i < 12; i++) r.v[i] = c[i];

@@ -341,6 +341,21 @@ def gen_add_const(name, c, n):
                          [("a", i) for i in range(n)])
 
 
+def gen_const_minus(name, c, n):
+    """r = c - a modulo 2^(32n)."""
+    cl = limbs32(c, n)
+    lines = []
+    w = lines.append
+    w(".reg .u32 d<%d>;" % n)
+    for j in range(n):
+        op = "sub.cc" if j == 0 else ("subc.cc" if j < n - 1 else "subc")
+        w("%s.u32 d%d, 0x%08x, %%%d;" % (op, j, cl[j], n + j))
+    for j in range(n):
+        w("mov.u32 %%%d, d%d;" % (j, j))
+    return _asm_function(name, "uint32_t r[%d], const uint32_t a[%d]" % (n, n), lines, [("r", i) for i in range(n)],
+                         [("a", i) for i in range(n)])
+
+
 def gen_addsub_nr(name, n, sub):
     """r = a + b or a - b modulo 2^(32n)."""
     o = "sub" if sub else "add"
@@ -738,6 +753,8 @@ def main():
         gen_redc("fp_redc", P, 12),
         gen_cond_sub("fp_csub_p", P, 12),
         gen_cond_sub("fp_csub_2p", 2 * P, 12),
+        gen_cond_sub("fp_csub_4p", 4 * P, 12),
+        gen_const_minus("fp_p_minus", P, 12),
         gen_add_const("fp_add_p", P, 12),
         gen_add_const("fp_add_2p", 2 * P, 12),
         gen_addsub_nr("wide_add", 24, False),

@@ -135,7 +135,7 @@ template <int PER> __device__ __forceinline__ int64_t team_index() {
 // fastest over nbp >= nb = blocks * count slots, so that with nbp a multiple of
 // five a warp has one twiddle.
 template <int L, bool NAF>
-__global__ void __launch_bounds__(WARP) k_gt_radix4_pows(uint8_t* ex, const uint8_t* io, const int8_t* rec, int64_t n,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_pows(uint8_t* ex, const uint8_t* io, const int8_t* rec, int64_t n,
                                                          int64_t h, int64_t J, int64_t nb, int64_t nbp) {
     __shared__ uint4 sh[T6_ROWS * 32];
     constexpr int PER = PerWarp<L>::N;
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(WARP) k_gt_radix4_pows(uint8_t* ex, const uint
 // and the powers ex (null: all twiddles are one, the powers are src's own
 // values), into dst.  prefix: only outputs below `keep` of each array are
 // wanted, of butterflies j < J.
-__global__ void __launch_bounds__(WARP) k_gt_radix4_outputs(uint8_t* dst, const uint8_t* src, const uint8_t* ex,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_outputs(uint8_t* dst, const uint8_t* src, const uint8_t* ex,
                                                             int64_t n, int64_t h, int64_t J, int64_t nb, int inverse,
                                                             int64_t keep) {
     __shared__ uint4 sh[T6_ROWS * 32];
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(WARP) k_gt_radix4_outputs(uint8_t* dst, const 
 }
 
 // the first radix-2 stage (all twiddles one): u v and u / v of neighbours
-__global__ void __launch_bounds__(WARP) k_gt_radix2_first(uint8_t* dst, const uint8_t* src, int64_t total) {
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix2_first(uint8_t* dst, const uint8_t* src, int64_t total) {
     __shared__ uint4 sh[T6_ROWS * 32];
     const Team t = team_init(sh);
     int64_t g = team_index<TEAMS>();
@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(WARP) k_gt_radix2_first(uint8_t* dst, const ui
 // out[q B + i] = base[(q B + i) stride]^(scalar i) for K arrays of B values
 // sharing the B exponents: teams take the arrays fastest over Kp >= K slots
 template <int L, bool NAF>
-__global__ void __launch_bounds__(WARP) k_gt_pow(uint8_t* out, const uint8_t* base, int64_t stride, const int8_t* rec,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_pow(uint8_t* out, const uint8_t* base, int64_t stride, const int8_t* rec,
                                                  int64_t B, int64_t K, int64_t Kp) {
     __shared__ uint4 sh[T6_ROWS * 32];
     constexpr int PER = PerWarp<L>::N;
@@ -241,7 +241,7 @@ __global__ void __launch_bounds__(WARP) k_gt_pow(uint8_t* out, const uint8_t* ba
 // square-and-multiply over the bits of |c_i| with cyclotomic squarings, then
 // the inverse (conjugation) for negative c_i -- mul_cyclotomic_signed_small of
 // weighted_pfe/src/fft.rs:671-699.  c_i = 0 gives one.
-__global__ void __launch_bounds__(WARP) k_gt_pow_small(uint8_t* out, const uint8_t* base, int64_t stride,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_pow_small(uint8_t* out, const uint8_t* base, int64_t stride,
                                                        const int32_t* coeffs, int64_t n) {
     __shared__ uint4 sh[T6_ROWS * 32];
     const Team t = team_init(sh);

@@ -51,7 +51,7 @@ __device__ __forceinline__ int64_t team_index() {
 // (p_per = per: weighted_btx) or each slot with its own T points (p_per = 1:
 // weighted_pfe, and single pairs with T = 1).  The pairs of a run share the 62
 // squarings.
-__global__ void __launch_bounds__(WARP) k_miller_lines_multi(uint8_t* out, const uint8_t* lines, const uint8_t* p,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_miller_lines_multi(uint8_t* out, const uint8_t* lines, const uint8_t* p,
                                                              int64_t n, int64_t per, int64_t p_per, int64_t T, int64_t C,
                                                              int64_t chunks) {
     __shared__ uint4 sh[T6_ROWS * 32];
@@ -87,7 +87,7 @@ __global__ void __launch_bounds__(WARP) k_miller_lines_multi(uint8_t* out, const
 // C pairs; the team of (s, ch) writes the product of its run's Miller loops,
 // lines computed on the fly, one multi-Miller loop sharing the squarings.
 // Pair i is (P[p_mod ? i % p_mod : i], Q[q_mod ? i % q_mod : i]).
-__global__ void __launch_bounds__(WARP) k_miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t per,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t per,
                                                         int64_t K, int C, int64_t chunks, int64_t p_mod, int64_t q_mod) {
     __shared__ uint4 sh[T6_ROWS * 32];
     const Team t = team_init(sh);
@@ -126,7 +126,7 @@ __global__ void __launch_bounds__(WARP) k_miller_chunks(uint8_t* out, const uint
     if (active) t6_store(t, out + GT_SZ * g, f);
 }
 
-__global__ void __launch_bounds__(WARP) k_fp12_segment_product(uint8_t* out, const uint8_t* in, const int64_t* offsets,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_fp12_segment_product(uint8_t* out, const uint8_t* in, const int64_t* offsets,
                                                                int64_t k) {
     __shared__ uint4 sh[T6_ROWS * 32];
     const Team t = team_init(sh);
@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(WARP) k_fp12_segment_product(uint8_t* out, con
     if (active) t6_store(t, out + GT_SZ * j, acc);
 }
 
-__global__ void __launch_bounds__(WARP) k_final_exp(uint8_t* out, const uint8_t* in, int64_t n, int mode) {
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_final_exp(uint8_t* out, const uint8_t* in, int64_t n, int mode) {
     __shared__ uint4 sh[T6_ROWS * 32];
     const Team t = team_init(sh);
     int64_t i = team_index();
@@ -155,7 +155,7 @@ __global__ void __launch_bounds__(WARP) k_final_exp(uint8_t* out, const uint8_t*
     if (active) t6_store(t, out + GT_SZ * i, f);
 }
 
-__global__ void __launch_bounds__(WARP) k_fp12_mul(uint8_t* out, const uint8_t* a, int64_t sa, const uint8_t* b,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_fp12_mul(uint8_t* out, const uint8_t* a, int64_t sa, const uint8_t* b,
                                                    int64_t sb, bool conj_b, int64_t n) {
     __shared__ uint4 sh[T6_ROWS * 32];
     const Team t = team_init(sh);
@@ -168,7 +168,7 @@ __global__ void __launch_bounds__(WARP) k_fp12_mul(uint8_t* out, const uint8_t* 
     if (active) t6_store(t, out + GT_SZ * i, r);
 }
 
-__global__ void __launch_bounds__(WARP) k_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha,
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha,
                                                  const uint8_t* beta, const uint8_t* valid, int64_t n) {
     __shared__ uint4 sh[T6_ROWS * 32];
     const Team t = team_init(sh);

@@ -43,12 +43,6 @@ WBTE_INL Fp fp_shfl_xor(const Fp& a, int m) {
     _Pragma("unroll") for (int i = 0; i < 12; i++) r.v[i] = __shfl_xor_sync(FULL, a.v[i], m);
     return r;
 }
-WBTE_INL Fp fp_select(bool c, const Fp& a, const Fp& b) {
-    Fp r;
-    _Pragma("unroll") for (int i = 0; i < 12; i++) r.v[i] = c ? a.v[i] : b.v[i];
-    return r;
-}
-
 // ------------------------------------------------------------------ fields
 // The field over the lanes of one place: every lane holds one Fp.  LANES lanes
 // per value; product, square and the constants of the curve.

@@ -13,10 +13,12 @@
 // products.
 //
 // Measured on B200 against one thread per element (one batch of B = 512, then
-// 64 of them): truncated GT transform 48 -> 3.3 ms and 82 -> 47 ms, hard parts
-// 10.7 -> 1.85 ms and 15.0 -> 15.4 ms, prepared Miller loops 7.2 -> 1.0 ms and
-// 21.4 -> 15.1 ms, opening multi-Miller loops of three pairs 20.4 -> 16.4 ms
-// (64 batches).
+// 64 of them): truncated GT transform 48 -> 2.8 ms and 82 -> 44 ms, hard parts
+// 10.7 -> 1.4 ms and 15.0 -> 12.3 ms, prepared Miller loops 7.2 -> 0.9 ms and
+// 21.4 -> 15.0 ms, opening multi-Miller loops of three pairs 20.4 -> 15.7 ms
+// (64 batches).  At 64 batches the multiply-add pipe is 55-62 % busy: the
+// rest is the latency of carry chains between products, with two warps per
+// scheduler, and instruction fetch.
 //
 // Lanes meet in shared memory: rows of 32 16-byte vectors, a value of a lane
 // being one column ("slot") of consecutive rows, so that the lanes of a warp
@@ -34,10 +36,16 @@ namespace wbte {
 
 constexpr int TEAM_LANES = 6;
 constexpr int TEAMS = 5;  // per warp
+// Resident one-warp blocks per SM that the team kernels are compiled for: the
+// registers of eight warps, two per scheduler.  Ten and twelve (168 registers)
+// measured 45.9 -> 56 and 57 ms for the GT transform of 64 batches of 512 and
+// changed the hard parts by 1 %: what more warps hide they lose to
+// instruction fetch (the loop's 45 KB) and to the tables' share of L1.
+constexpr int T6_BLOCKS = 8;
 constexpr int T6_ZERO = 31;
-// rows: operands A and B (6 each), three double-width exchange areas (12 each)
-constexpr int T6_A = 0, T6_B = 6, T6_X = 12, T6_Y = 24, T6_Z = 36, T6_ROWS = 48;
-constexpr size_t T6_SMEM = (size_t)T6_ROWS * 32 * sizeof(uint4);
+// rows: three double-width exchange areas (12 each), the first also holding the
+// operands A and B
+constexpr int T6_A = 0, T6_B = 6, T6_X = 0, T6_Y = 12, T6_Z = 24, T6_ROWS = 36;
 
 struct Wide { uint32_t v[24]; };
 struct Wide2 { Wide c0, c1; };
@@ -78,7 +86,8 @@ template <class T> WBTE_INL void team_st(const Team& t, int row, int slot, const
 }
 
 // ------------------------------------------------------------ double width
-static __device__ __noinline__ Wide fp_wide(Fp a, Fp b) { Wide r; fp_mul_wide(r.v, a.v, b.v); return r; }
+WBTE_INL Wide fp_wide_inl(const Fp& a, const Fp& b) { Wide r; fp_mul_wide(r.v, a.v, b.v); return r; }
+static __device__ __noinline__ Wide fp_wide(Fp a, Fp b) { return fp_wide_inl(a, b); }
 // t / 2^384 mod p for 0 <= t < 3 p 2^384
 static __device__ __noinline__ Fp wide_reduce(Wide t) {
     Fp r;
@@ -99,6 +108,14 @@ WBTE_INL Wide2 fp2_wide(const Fp2& a, const Fp2& b) {
     const Wide z = fp_wide(fp_add_lazy(a.c0, a.c1), fp_add_lazy(b.c0, b.c1));
     return Wide2{w_sub(x, y), w_sub(w_sub(z, x), y)};
 }
+// the same in line: faster where a kernel's loop holds few of them (Miller loops
+// of one pair each 1.02 -> 0.89 ms), slower in t6_mul (GT transforms of 64
+// batches 44 -> 57 ms, instruction fetch)
+WBTE_INL Wide2 fp2_wide_inl(const Fp2& a, const Fp2& b) {
+    const Wide x = fp_wide_inl(a.c0, b.c0), y = fp_wide_inl(a.c1, b.c1);
+    const Wide z = fp_wide_inl(fp_add_lazy(a.c0, a.c1), fp_add_lazy(b.c0, b.c1));
+    return Wide2{w_sub(x, y), w_sub(w_sub(z, x), y)};
+}
 // reductions of sums in (-19.6 p^2, 9.8 p^2) and (-9.8 p^2, 19.6 p^2)
 WBTE_INL Fp2 w2_reduce_21(Wide2 t) {
     fp_add_2p(t.c0.v + 12, t.c0.v + 12);
@@ -112,7 +129,7 @@ WBTE_INL Fp2 w2_reduce_11(Wide2 t) {
     return Fp2{wide_reduce(t.c0), wide_reduce(t.c1)};
 }
 // one lane's Fp2 product, components below 4 p: two reductions instead of three
-static __device__ __noinline__ Fp2 t6_fp2_mul(Fp2 a, Fp2 b) { return w2_reduce_11(fp2_wide(a, b)); }
+static __device__ __noinline__ Fp2 t6_fp2_mul(Fp2 a, Fp2 b) { return w2_reduce_11(fp2_wide_inl(a, b)); }
 
 // --------------------------------------------------------- Fp12 products
 // The Karatsuba products of an Fp6 product, one per lane: x0y0, x1y1, x2y2,
@@ -163,13 +180,6 @@ WBTE_INL int t6_vslot(const Team& t) {
     const int i = t.k >> 1;
     return t.base + 2 * (i == 0 ? 2 : i - 1) + 1;
 }
-WBTE_INL void w2_clear_if(Wide2& a, bool clear) {
-    _Pragma("unroll") for (int i = 0; i < 24; i++) {
-        a.c0.v[i] = clear ? 0u : a.c0.v[i];
-        a.c1.v[i] = clear ? 0u : a.c1.v[i];
-    }
-}
-
 // a b.  With a = a0 + a1 w, b = b0 + b1 w: c0 = a0 b0 + v a1 b1 and
 // c1 = (a0 + a1)(b0 + b1) - a0 b0 - a1 b1, every Fp6 product by its Karatsuba
 // products.  As integers the outputs are sums of one product and five
@@ -183,10 +193,11 @@ static __device__ __noinline__ Fp2 t6_mul(Team t, Fp2 a, Fp2 b) {
     __syncwarp();
     const int s0 = t6_term0(t), s1 = t6_term1(t);
     Fp2 u = t6_pair(t, T6_A, s0, s1), v = t6_pair(t, T6_B, s0, s1);
+    const Fp2 u1 = t6_pair(t, T6_A, t6_odd(s0), t6_odd(s1)), v1 = t6_pair(t, T6_B, t6_odd(s0), t6_odd(s1));
+    __syncwarp();
     Wide2 x = fp2_wide(u, v);
     team_st(t, T6_X, own, x);
     {
-        const Fp2 u1 = t6_pair(t, T6_A, t6_odd(s0), t6_odd(s1)), v1 = t6_pair(t, T6_B, t6_odd(s0), t6_odd(s1));
         const Wide2 y = fp2_wide(u1, v1);
         team_st(t, T6_Y, own, y);
         x = w2_add(x, y);
@@ -196,21 +207,21 @@ static __device__ __noinline__ Fp2 t6_mul(Team t, Fp2 a, Fp2 b) {
     team_st(t, T6_Z, own, w2_sub(fp2_wide(u, v), x));
     __syncwarp();
     // first the coefficients of a0 b0 (even lanes) and a1 b1 (odd lanes), then
-    // the odd lanes' own and v a1 b1 on the even ones
+    // the odd lanes' own and, on the even ones, v a1 b1 joining their a0 b0
     T6Comb c = t6_comb_of(t, odd ? T6_Y : T6_X);
-    Wide2 acc = t6_comb(t, c);
-    team_st(t, T6_A, own, acc);
+    const Wide2 e = t6_comb(t, c);
     __syncwarp();
-    w2_clear_if(acc, odd);
+    team_st(t, T6_X, own, e);
+    __syncwarp();
     if (odd) {
         c.row = T6_Z;
     } else {
-        c.row = T6_A;
+        c.row = T6_X;
         c.g0 = t6_vslot(t);
-        c.g1 = c.g2 = c.h = c.m = T6_ZERO;
+        c.g1 = c.g2 = c.m = T6_ZERO;
+        c.h = own;
     }
-    acc = w2_add(acc, t6_comb(t, c));
-    return w2_reduce_21(acc);
+    return w2_reduce_21(t6_comb(t, c));
 }
 
 // a^2 by complex squaring: c1 = 2 a0 a1, c0 = (a0 + a1)(a0 + v a1) - a0 a1 -
@@ -227,72 +238,92 @@ static __device__ __noinline__ Fp2 t6_sqr(Team t, Fp2 a) {
     const int s0 = t6_term0(t), s1 = t6_term1(t);
     const Fp2 u0 = t6_pair(t, T6_A, s0, s1), u1 = t6_pair(t, T6_A, t6_odd(s0), t6_odd(s1));
     const Fp2 v1 = t6_pair(t, T6_B, t6_odd(s0), t6_odd(s1));
-    const Wide2 x = fp2_wide(u0, u1);
+    __syncwarp();
+    const Wide2 x = fp2_wide_inl(u0, u1);
     team_st(t, T6_X, own, x);
-    team_st(t, T6_Y, own, w2_sub(fp2_wide(fp2_add_lazy(u0, u1), fp2_add_lazy(u0, v1)), x));
+    team_st(t, T6_Y, own, w2_sub(fp2_wide_inl(fp2_add_lazy(u0, u1), fp2_add_lazy(u0, v1)), x));
     __syncwarp();
     T6Comb c = t6_comb_of(t, odd ? T6_X : T6_Y);
-    Wide2 acc = t6_comb(t, c);
-    team_st(t, T6_A, own, acc);
+    team_st(t, T6_Z, own, t6_comb(t, c));
     __syncwarp();
     // odd lanes double, even lanes subtract v a0 a1
-    c.row = T6_A;
+    c.row = T6_Z;
     c.g0 = odd ? own : T6_ZERO;
     c.g1 = odd ? T6_ZERO : t6_vslot(t);
-    c.g2 = c.h = c.m = T6_ZERO;
+    c.g2 = c.m = T6_ZERO;
+    c.h = own;
     c.gm = c.gm && !odd;
-    acc = w2_add(acc, t6_comb(t, c));
-    return w2_reduce_21(acc);
+    return w2_reduce_21(t6_comb(t, c));
 }
 
-// Granger-Scott squaring in the cyclotomic subgroup (fp12_cyclotomic_sqr):
-// even lanes hold a^2 + xi b^2, odd lanes 2ab of the pairs (w^0, w^3),
-// (w^1, w^4), (w^2, w^5), four 12 x 12-word products each, and z' = 3t -+ 2z.
-// Lane 1 takes xi 2ab of the pair (w^2, w^5), lane 4 its a^2 + xi b^2.
+// Granger-Scott squaring in the cyclotomic subgroup: even lanes hold
+// a^2 + xi b^2, odd lanes 2ab of the pairs (w^0, w^3), (w^1, w^4), (w^2, w^5),
+// and z' = 3t -+ 2z.  Lane 1 takes xi 2ab of the pair (w^2, w^5), lane 4 its
+// a^2 + xi b^2.  Four 12 x 12-word products on each lane:
+//   even: A = (a0+a1)(a0-a1)  B = 2a0 a1  C = (b0+b1)(b0-b1)  D = 2b0 b1
+//   odd:  A = 2a0 b0          B = 2a0 b1  C = 2a1 b0          D = 2a1 b1
+//   c0 = A + [even] C - D,  c1 = B + C + [even] D
+// Which value a factor starts from differs between the lanes, so they read it
+// from the place it has in shared memory instead of selecting it: c0, c1, p -
+// c1 and (for lane 1) xi z without reduction.  Most lanes' time besides the
+// products goes into carry chains, and this is two thirds of the chains of a
+// form with selections and a branch per parity; the four products stand in
+// line, which lets their chains overlap (hard parts of 32,768 values 15.2 ->
+// 13.7 ms against calls).  Components: (-4 p^2, 8 p^2) and [0, 12 p^2) at lane 1,
+// inside that elsewhere.
 static __device__ __noinline__ Fp2 t6_cyc_sqr(Team t, Fp2 z) {
+    constexpr int C0 = 0, C1 = 3, NEG = 6, XI0 = 9, XI1 = 12;
     const bool even = !(t.k & 1);
+    const int own = t.base + t.k;
+    Fp n, m;
+    fp_p_minus(n.v, z.c1.v);
     __syncwarp();
-    team_st(t, T6_A, t.base + t.k, z);
+    team_st(t, C0, own, z.c0);
+    team_st(t, C1, own, z.c1);
+    team_st(t, NEG, own, n);
+    team_st(t, XI0, own, fp_add_lazy(z.c0, n));
+    team_st(t, XI1, own, fp_add_lazy(z.c0, z.c1));
     __syncwarp();
-    const int ia = t.base + nib(0x120120u, t.k);
-    const Fp2 a = team_ld<Fp2>(t, T6_A, ia), b = team_ld<Fp2>(t, T6_A, ia + 3);
-    // even: (a0+a1)(a0-a1), a0a1, (b0+b1)(b0-b1), b0b1
-    // odd:  (a0+a1)(b0+b1), a0b0, -,              a1b1
-    const Fp sa = fp_add_lazy(a.c0, a.c1), sb = fp_add_lazy(b.c0, b.c1);
-    const Fp da = fp_sub(a.c0, a.c1), db = fp_sub(b.c0, b.c1);
-    Fp v1, v2, u3, u4;
-    _Pragma("unroll") for (int i = 0; i < 12; i++) {
-        v1.v[i] = even ? da.v[i] : sb.v[i];
-        v2.v[i] = even ? a.c1.v[i] : b.c0.v[i];
-        u3.v[i] = even ? sb.v[i] : 0u;
-        u4.v[i] = even ? b.c0.v[i] : a.c1.v[i];
+    const int pa = t.base + nib(0x120120u, t.k), pb = pa + 3;
+    const int a0r = t.k == 1 ? XI0 : C0, a1r = t.k == 1 ? XI1 : C1;
+    const Fp a0 = team_ld<Fp>(t, a0r, pa), b0 = team_ld<Fp>(t, C0, pb), b1 = team_ld<Fp>(t, C1, pb);
+    const Fp d = team_ld<Fp>(t, even ? C0 : a1r, even ? pb : pa);  // b0 or a1
+    const Wide A = fp_wide_inl(fp_add_lazy(a0, team_ld<Fp>(t, even ? C1 : a0r, pa)),
+                               fp_add_lazy(team_ld<Fp>(t, C0, even ? pa : pb), team_ld<Fp>(t, NEG, even ? pa : T6_ZERO)));
+    const Wide B = fp_wide_inl(fp_add_lazy(a0, a0), team_ld<Fp>(t, C1, even ? pa : pb));
+    const Wide C = fp_wide_inl(fp_add_lazy(d, team_ld<Fp>(t, even ? C1 : a1r, even ? pb : pa)),
+                               fp_add_lazy(b0, team_ld<Fp>(t, NEG, even ? pb : T6_ZERO)));
+    const Wide D = fp_wide_inl(fp_add_lazy(d, d), b1);
+    const uint32_t mask = even ? 0xffffffffu : 0u;
+    Wide c, e;
+    _Pragma("unroll") for (int i = 0; i < 24; i++) {
+        c.v[i] = C.v[i] & mask;
+        e.v[i] = D.v[i] & mask;
     }
-    const Wide x1 = fp_wide(sa, v1), x2 = fp_wide(a.c0, v2), x3 = fp_wide(u3, db), x4 = fp_wide(u4, b.c1);
-    Wide2 r;
-    if (even) {  // (-2 p^2, 4 p^2), [0, 6 p^2)
-        const Wide d4 = w_add(x4, x4);
-        r.c0 = w_sub(w_add(x1, x3), d4);
-        r.c1 = w_add(w_add(w_add(x2, x2), x3), d4);
-    } else {  // (-2 p^2, 2 p^2), [0, 4 p^2); lane 1: (-6 p^2, 2 p^2), (-2 p^2, 6 p^2)
-        const Wide d = w_sub(x2, x4), e = w_sub(w_sub(x1, x2), x4);
-        r.c0 = w_add(d, d);
-        r.c1 = w_add(e, e);
-        if (t.k == 1) {
-            const Wide s = w_sub(r.c0, r.c1);
-            r.c1 = w_add(r.c0, r.c1);
-            r.c0 = s;
-        }
-    }
-    const Fp2 q = w2_reduce_11(r);
-    Fp2 m = fp2_neg(z);
-    _Pragma("unroll") for (int i = 0; i < 12; i++) {
-        m.c0.v[i] = even ? m.c0.v[i] : z.c0.v[i];
-        m.c1.v[i] = even ? m.c1.v[i] : z.c1.v[i];
-    }
-    return fp2_add(fp2_dbl(fp2_add(q, m)), q);
+    c = w_sub(w_add(A, c), D);
+    fp_add_p(c.v + 12, c.v + 12);
+    e = w_add(w_add(B, C), e);
+    Fp2 q;
+    fp_redc(q.c0.v, c.v);
+    fp_redc(q.c1.v, e.v);
+    fp_csub_2p(q.c0.v, q.c0.v);
+    fp_csub_2p(q.c1.v, q.c1.v);
+    // 3q -+ 2z = 2 (q + (p - z or z)) + q, below 8p
+    fp_p_minus(m.v, z.c0.v);
+    m = fp_select(even, m, z.c0);
+    q.c0 = fp_add_lazy(fp_add_lazy(q.c0, q.c0), fp_add_lazy(q.c0, fp_add_lazy(m, m)));
+    n = fp_select(even, n, z.c1);
+    q.c1 = fp_add_lazy(fp_add_lazy(q.c1, q.c1), fp_add_lazy(q.c1, fp_add_lazy(n, n)));
+    fp_csub_4p(q.c0.v, q.c0.v);
+    fp_csub_4p(q.c1.v, q.c1.v);
+    fp_csub_2p(q.c0.v, q.c0.v);
+    fp_csub_2p(q.c1.v, q.c1.v);
+    fp_csub_p(q.c0.v, q.c0.v);
+    fp_csub_p(q.c1.v, q.c1.v);
+    return q;
 }
 
-// f (l0 + l1 w^2 + l2 w^3) with the line's six Fp components in rows T6_X.. of
+// f (l0 + l1 w^2 + l2 w^3) with the line's six Fp components in rows T6_Y.. of
 // the team's slots (component c of the record at slot base + c): three Fp2
 // products per lane, no exchange after them.  Components in (-3 p^2, 3 p^2)
 // and [0, 6 p^2).
@@ -304,12 +335,12 @@ static __device__ __noinline__ Fp2 t6_mul_line(Team t, Fp2 f, Fp line_component)
     __syncwarp();
     team_st(t, T6_A, own, f);
     team_st(t, T6_B, own, fp2_mul_xi(f));
-    team_st(t, T6_X, own, line_component);
+    team_st(t, T6_Y, own, line_component);
     __syncwarp();
-    Wide2 acc = fp2_wide(f, team_ld_line(t, T6_X, 0));
+    Wide2 acc = fp2_wide_inl(f, team_ld_line(t, T6_Y, 0));
     const int k2 = t.k < 2 ? t.k + 4 : t.k - 2, k3 = t.k < 3 ? t.k + 3 : t.k - 3;
-    acc = w2_add(acc, fp2_wide(team_ld<Fp2>(t, t.k < 2 ? T6_B : T6_A, t.base + k2), team_ld_line(t, T6_X, 1)));
-    acc = w2_add(acc, fp2_wide(team_ld<Fp2>(t, t.k < 3 ? T6_B : T6_A, t.base + k3), team_ld_line(t, T6_X, 2)));
+    acc = w2_add(acc, fp2_wide_inl(team_ld<Fp2>(t, t.k < 2 ? T6_B : T6_A, t.base + k2), team_ld_line(t, T6_Y, 1)));
+    acc = w2_add(acc, fp2_wide_inl(team_ld<Fp2>(t, t.k < 3 ? T6_B : T6_A, t.base + k3), team_ld_line(t, T6_Y, 2)));
     return w2_reduce_11(acc);
 }
 
