@@ -25,9 +25,10 @@
 #include <atomic>
 #include <cmath>
 #include <mutex>
+#include <type_traits>
 
 #include "launch.h"
-#include "pairing.cuh"
+#include "quad.cuh"
 
 namespace wbte {
 
@@ -106,113 +107,107 @@ __global__ void k_sort(uint64_t* entries, int32_t* nnz, const int16_t* digits, i
     }
 }
 
-// acc += g * run for a small positive g
-template <class F> WBTE_INL Xyzz<F> add_small_multiple(const Xyzz<F>& acc, const Xyzz<F>& run, uint32_t g) {
-    if (g == 1) return xyzz_add(acc, run);
-    Xyzz<F> m;
-    set_inf(m);
-    int top = 31 - __clz(g);
-    for (int b = top; b >= 0; b--) {
-        m = xyzz_dbl(m);
-        if ((g >> b) & 1) m = xyzz_add(m, run);
-    }
-    return xyzz_add(acc, m);
-}
+// One lane (G1) or pair of lanes (G2) per segment of S sorted terms of one
+// (MSM, window): the running sum `run` of the terms seen so far, and at each
+// bucket transition (bucket cur_b to b < cur_b) acc += (cur_b - b) * run; at the
+// end acc += cur_b * run (Abel summation: acc = sum over the segment of
+// |d| * (+-P)).
+// Adding at the transition itself would have a warp run the addition whenever
+// any of its segments does, so every segment would pay an XYZZ addition per term
+// besides its mixed addition.  Instead a lane stores a snapshot of run (and the
+// gap) in a small queue in shared memory, and all segments of the warp add
+// their oldest entry together: when each segment that still has terms holds
+// one, or when one's queue is full.  An entry with a gap above one stays for its
+// next turn unless the warp's largest gap makes double-and-add cheaper.  The sum
+// is the same: the group is commutative and every snapshot is added as often
+// as its gap says.
+// The multiply-add pipe bounds it.  Measured on B200: see Point for why G2 takes
+// pairs; the families of a committee preparation at B = 512 (512 MSMs for each
+// of three parties, 1,382 terms together, and 1,023 of 1,382) 171 -> 102 ms,
+// one MSM of 20,011 points 2.5 -> 1.5 ms; G1 as one thread per segment was,
+// 1.57 ms at 65,536 points.
+constexpr int SEG_QUEUE = 4;
+constexpr size_t SEG_SMEM = (sizeof(Point<OnLane>) + sizeof(uint32_t)) * SEG_QUEUE * SEG_TPB;
 
-// One thread per segment of S sorted terms of one (MSM, window): the running
-// sum `run` of the terms seen so far, and at each bucket transition (bucket
-// cur_b to b < cur_b) acc += (cur_b - b) * run; at the end acc += cur_b * run
-// (Abel summation: acc = sum over the segment of |d| * (+-P)).
-// Adding at the transition itself would diverge: every lane reaches its own
-// transitions at its own terms, and a warp runs the addition whenever any of
-// its 32 lanes does, so every lane would pay an XYZZ addition per term besides
-// its mixed addition.  Instead a lane stores a snapshot of run (and the gap)
-// in a small per-lane queue in shared memory, and the queued additions run
-// when every lane of the warp that still has terms holds one, all lanes
-// together; a full queue adds its oldest entry on its own.  The sum is the
-// same: the group is commutative and every snapshot is added exactly once.
-// Measured on B200 against adding at the transition: G1 and G2 MSMs of 2^16
-// to 2^18 points 15-18 % faster, 2^20 5-7 %, the batched partial decryptions
-// (384 MSMs of 512 terms) 10 %.
-template <class F> struct SegQueue;
-template <> struct SegQueue<Fp> { static constexpr int Q = 4; };
-template <> struct SegQueue<Fp2> { static constexpr int Q = 2; };
-template <class F> constexpr size_t seg_queue_bytes() {
-    return (sizeof(Xyzz<F>) + sizeof(uint32_t)) * SegQueue<F>::Q * SEG_TPB;
-}
-
-template <class F>
+template <class P>
 __global__ void __launch_bounds__(SEG_TPB) k_segments(uint8_t* seg_out, const uint8_t* points, const int64_t* pbase,
                                                         const int32_t* idx, const uint64_t* entries,
                                                         const int32_t* nnz, const int32_t* vsel, int64_t k, int64_t n,
                                                         int windows, int64_t S, int64_t nseg) {
-    constexpr int Q = SegQueue<F>::Q;
+    using Pt = Point<P>;
     extern __shared__ __align__(16) uint8_t seg_sh[];
-    Xyzz<F>* qv = reinterpret_cast<Xyzz<F>*>(seg_sh);
-    uint32_t* qg = reinterpret_cast<uint32_t*>(seg_sh + sizeof(Xyzz<F>) * Q * SEG_TPB);
-    const int tid = threadIdx.x;
-    const int64_t gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    // threads past the grid's work stay in the loop (the warp votes need
-    // every lane) with an empty segment
-    using A = Affine<F>;
+    Pt* qv = reinterpret_cast<Pt*>(seg_sh) + threadIdx.x;
+    uint32_t* qg = reinterpret_cast<uint32_t*>(seg_sh + sizeof(Pt) * SEG_QUEUE * SEG_TPB) + threadIdx.x;
+    const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / P::LANES;
+    // lanes past the grid's work run along with an empty segment
+    const bool real = gid < k * windows * nseg;
     int64_t lo = 0, hi = 0;
     const uint64_t* e = entries;
-    const A* P = reinterpret_cast<const A*>(points);
-    if (gid < k * windows * nseg) {
+    const uint8_t* base = points;
+    if (real) {
         const int64_t seg = gid % nseg;
         const int64_t w = (gid / nseg) % windows;
         const int64_t j = gid / (nseg * windows);
-        const int64_t v = vsel ? vsel[j] : 0;
-        const int64_t vw = v * windows + w;
+        const int64_t vw = (vsel ? (int64_t)vsel[j] : 0) * windows + w;
         lo = seg * S;
         hi = lo + S;
         const int64_t cnt = nnz[vw];
         if (hi > cnt) hi = cnt;
         if (lo > hi) lo = hi;
         e = entries + vw * n;
-        P = reinterpret_cast<const A*>(points) + pbase[j];
+        base = points + 2 * P::FIELD * pbase[j];
     }
-    Xyzz<F> run, acc;
-    set_inf(run);
-    set_inf(acc);
+    Pt run = Pt::infinity(), acc = Pt::infinity();
     uint32_t cur_b = lo < hi ? ((uint32_t)(e[lo] >> 32) & 0x7fffu) : 0u;
     int qh = 0, qn = 0;
-    for (int64_t i = 0; i < S; i++) {
-        const int64_t x = lo + i;
-        if (x < hi) {
-            const uint64_t en = e[x];
-            const uint32_t b = (uint32_t)(en >> 32) & 0x7fffu;
-            const uint32_t t = (uint32_t)en;
-            if (b != cur_b) {
-                if (qn == Q) {
-                    acc = add_small_multiple(acc, qv[qh * SEG_TPB + tid], qg[qh * SEG_TPB + tid]);
-                    qh = qh + 1 == Q ? 0 : qh + 1;
-                    qn--;
-                }
-                const int slot = (qh + qn) % Q;
-                qv[slot * SEG_TPB + tid] = run;
-                qg[slot * SEG_TPB + tid] = cur_b - b;
-                qn++;
-                cur_b = b;
-            }
-            A p = load_affine(P + (idx ? (int64_t)idx[t] : (int64_t)t));
-            if (en >> 63) p = neg(p);
-            run = xyzz_madd(run, p);
-        }
-        // lanes without terms left never hold the warp back
-        if (__all_sync(0xffffffffu, qn > 0 || x + 1 >= hi) && qn > 0) {
-            acc = add_small_multiple(acc, qv[qh * SEG_TPB + tid], qg[qh * SEG_TPB + tid]);
-            qh = qh + 1 == Q ? 0 : qh + 1;
+    // every segment with an entry adds its oldest
+    auto turn = [&]() {
+        const bool has = qn > 0;
+        const int at = qh * SEG_TPB;
+        const uint32_t g = has ? qg[at] : 0u;
+        Pt m = has ? qv[at] : Pt::infinity();
+        uint32_t left = 0;
+        if (__reduce_max_sync(FULL, g) > 2)
+            m = Pt::multiple(m, g);
+        else
+            left = g == 2;
+        acc = Pt::add(acc, m, has);
+        if (left) {
+            qg[at] = left;
+        } else if (has) {
+            qh = (qh + 1) % SEG_QUEUE;
             qn--;
         }
+    };
+    for (int64_t i = 0; i < S; i++) {
+        const int64_t x = lo + i;
+        const bool live = x < hi;
+        const uint64_t en = live ? e[x] : 0;
+        const uint32_t b = (uint32_t)(en >> 32) & 0x7fffu;
+        const bool step = live && b != cur_b;
+        while (__any_sync(FULL, step && qn == SEG_QUEUE)) turn();
+        if (step) {
+            const int at = (qh + qn) % SEG_QUEUE * SEG_TPB;
+            qv[at] = run;
+            qg[at] = cur_b - b;
+            qn++;
+            cur_b = b;
+        }
+        Fp px = fp_zero(), py = fp_zero();
+        if (live) {
+            const uint32_t t = (uint32_t)en;
+            const uint8_t* pt = base + 2 * P::FIELD * (idx ? (int64_t)idx[t] : (int64_t)t);
+            px = load_affine(Pt::at(pt, 0));
+            py = load_affine(Pt::at(pt, 1));
+            if (en >> 63) py = fp_neg(py);
+        }
+        run = Pt::madd(run, px, py, live);
+        // segments without terms left never hold the warp back
+        if (__all_sync(FULL, qn > 0 || x + 1 >= hi) && __any_sync(FULL, qn > 0)) turn();
     }
-    if (lo < hi) acc = add_small_multiple(acc, run, cur_b);
-    while (qn > 0) {
-        acc = add_small_multiple(acc, qv[qh * SEG_TPB + tid], qg[qh * SEG_TPB + tid]);
-        qh = qh + 1 == Q ? 0 : qh + 1;
-        qn--;
-    }
-    if (gid < k * windows * nseg) store_vec(reinterpret_cast<Xyzz<F>*>(seg_out) + gid, acc);
+    acc = Pt::add(acc, Pt::multiple(run, cur_b), lo < hi);
+    while (__any_sync(FULL, qn > 0)) turn();
+    if (real) acc.store(seg_out + 4 * P::FIELD * gid);
 }
 
 // out[i] = sum_{g < G, i*G+g < len} in[row * len + i*G + g] for each row
@@ -307,10 +302,11 @@ void run_family(uint8_t* out, const uint8_t* points, const int64_t* pbase, const
     note_launch();
     // the queues take about 49 KB of shared memory per block, past the 48 KB
     // default, so the kernel opts in once
-    static const bool smem_ok = cudaFuncSetAttribute(k_segments<F>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)seg_queue_bytes<F>()) == cudaSuccess;
+    using P = typename std::conditional<sizeof(F) == sizeof(Fp), OnLane, OnPair>::type;
+    static const bool smem_ok =
+        cudaFuncSetAttribute(k_segments<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SEG_SMEM) == cudaSuccess;
     (void)smem_ok;
-    k_segments<F><<<blocks_for(segthreads, SEG_TPB), SEG_TPB, seg_queue_bytes<F>(), s>>>(
+    k_segments<P><<<blocks_for(segthreads * P::LANES, SEG_TPB), SEG_TPB, SEG_SMEM, s>>>(
         seg, points, pbase, idx, entries, nnz, vsel, k, n, p.windows, p.segment, p.segments);
     prof_end(tok, s);
     prof_begin(g1 ? "msm_reduce_g1" : "msm_reduce_g2", s, &tok);
@@ -338,27 +334,20 @@ void run_family(uint8_t* out, const uint8_t* points, const int64_t* pbase, const
 }
 }  // namespace
 
-// Threads of k_segments<F> resident on the whole device (one wave), from the
+// Segments of k_segments resident on the whole device (one wave), from the
 // occupancy of the compiled kernel; cached per device and group.
-static int64_t segment_wave_threads(Group g) {
-    static std::atomic<int64_t> cache[2][64];
+template <class P> static int64_t segment_wave() {
+    static std::atomic<int64_t> cache[64];
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148 * 256;
-    int gi = g == GROUP_G1 ? 0 : 1;
-    int64_t v = cache[gi][dev].load();
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148 * 256 / P::LANES;
+    int64_t v = cache[dev].load();
     if (v > 0) return v;
     int sms = 0, blocks = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (g == GROUP_G1) {
-        cudaFuncSetAttribute(k_segments<Fp>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)seg_queue_bytes<Fp>());
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_segments<Fp>, SEG_TPB, seg_queue_bytes<Fp>());
-    } else {
-        cudaFuncSetAttribute(k_segments<Fp2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)seg_queue_bytes<Fp2>());
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_segments<Fp2>, SEG_TPB, seg_queue_bytes<Fp2>());
-    }
-    v = (int64_t)(sms > 0 ? sms : 148) * (blocks > 0 ? blocks : 4) * SEG_TPB;
-    cache[gi][dev].store(v);
+    cudaFuncSetAttribute(k_segments<P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SEG_SMEM);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, k_segments<P>, SEG_TPB, SEG_SMEM);
+    v = (int64_t)(sms > 0 ? sms : 148) * (blocks > 0 ? blocks : 4) * SEG_TPB / P::LANES;
+    cache[dev].store(v);
     return v;
 }
 
@@ -379,7 +368,7 @@ MsmPlan msm_plan(Group g, int64_t n, int64_t k) {
     // segment.  Cost model in mixed additions: S terms plus one full addition
     // (~1.43 mixed additions) per bucket change, min(S, buckets), and the
     // tree reduction of the segment sums.
-    const int64_t wave = segment_wave_threads(g);
+    const int64_t wave = g == GROUP_G1 ? segment_wave<OnLane>() : segment_wave<OnPair>();
     const int64_t rows = k * p.windows;
     const double nnz = (double)n * (1.0 - 1.0 / (double)(int64_t(1) << c));
     double best = 1e300;

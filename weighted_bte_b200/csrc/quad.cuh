@@ -52,6 +52,16 @@ struct OnLane {  // Fp
     static constexpr bool G1 = true;
     static WBTE_INL Fp mul(const Fp& a, const Fp& b) { return fp_mul(a, b); }
     static WBTE_INL bool zero(const Fp& a) { return fp_is_zero(a); }
+    // a value that several products use
+    struct Shared { Fp own; };
+    static WBTE_INL Shared share(const Fp& a) { return Shared{a}; }
+    static WBTE_INL Fp mul(const Shared& a, const Shared& b) { return fp_mul(a.own, b.own); }
+    static WBTE_INL Fp sqr(const Shared& a) { return fp_sqr(a.own); }
+    // a b - c d
+    static WBTE_INL Fp mul_sub(const Shared& a, const Shared& b, const Shared& c, const Shared& d) {
+        return fp_mul2(a.own, b.own, fp_neg(c.own), d.own);
+    }
+    static WBTE_INL uint32_t all_lanes(uint32_t ballot) { return ballot; }
     static WBTE_INL Fp one() { return fp_one(); }
     static WBTE_INL Fp inv(const Fp& a) { return fp_inv(a); }
 };
@@ -65,6 +75,25 @@ struct OnPair {  // Fp2, component = lane parity
         const Fp pa = fp_shfl_xor(a, 1), pb = fp_shfl_xor(b, 1);
         const Fp n = fp_neg(pa);
         return fp_mul2(fp_select(odd(), pa, a), b, fp_select(odd(), a, n), pb);
+    }
+    // a value that several products use, with the partner's component
+    struct Shared { Fp own, other; };
+    static WBTE_INL Shared share(const Fp& a) { return Shared{a, fp_shfl_xor(a, 1)}; }
+    static WBTE_INL Fp mul(const Shared& a, const Shared& b) {
+        return fp_mul2(fp_select(odd(), a.other, a.own), b.own, fp_select(odd(), a.own, fp_neg(a.other)), b.other);
+    }
+    // even: (a0 + a1)(a0 - a1), odd: a0 2a1
+    static WBTE_INL Fp sqr(const Shared& a) {
+        return fp_mul(fp_select(odd(), a.other, fp_add_lazy(a.own, a.other)),
+                      fp_select(odd(), fp_add_lazy(a.own, a.own), fp_sub(a.own, a.other)));
+    }
+    static WBTE_INL Fp mul_sub(const Shared& a, const Shared& b, const Shared& c, const Shared& d) {
+        return fp_sub(mul(a, b), mul(c, d));
+    }
+    // bits of the lanes whose pair agrees on a set bit
+    static WBTE_INL uint32_t all_lanes(uint32_t ballot) {
+        const uint32_t both = ballot & (ballot >> 1) & 0x55555555u;
+        return both | (both << 1);
     }
     static WBTE_INL bool zero(const Fp& a) {
         const bool z = fp_is_zero(a);
@@ -240,5 +269,98 @@ template <class P> WBTE_INL void quad_digit(uint64_t& lo, uint64_t& hi, const ui
         hi = 0;
     }
 }
+
+// ------------------------------------------------- a point on one lane or pair
+// For kernels that fill the chip: a lane (G1) or a pair (G2) holds all four
+// coordinates.  In G2 that halves the registers of a point against one thread
+// per point, which spilled its way through 255 of them, and takes an Fp2 product
+// as 888 wide multiply-adds over the pair, none of its factors in local memory.
+// Every lane of the warp runs every step, `live` says whose result counts.
+template <class P> struct Point {
+    Fp X, Y, ZZ, ZZZ;
+
+    static WBTE_INL bool flag(bool mine) {
+        return (P::all_lanes(__ballot_sync(FULL, mine)) >> (threadIdx.x & 31)) & 1;
+    }
+    static WBTE_INL Point infinity() { return Point{fp_zero(), P::one(), fp_zero(), fp_zero()}; }
+    static WBTE_INL Point select(bool c, const Point& a, const Point& b) {
+        return Point{fp_select(c, a.X, b.X), fp_select(c, a.Y, b.Y), fp_select(c, a.ZZ, b.ZZ), fp_select(c, a.ZZZ, b.ZZZ)};
+    }
+    WBTE_INL bool is_inf() const { return flag(fp_is_zero(ZZ)); }
+
+    static __device__ __noinline__ Point dbl(Point p) {
+        const typename P::Shared U = P::share(fp_dbl(p.Y)), X = P::share(p.X);
+        const typename P::Shared V = P::share(P::sqr(U)), W = P::share(P::mul(U, V));
+        const Fp S = P::mul(X, V), x2 = P::sqr(X);
+        const typename P::Shared M = P::share(fp_add(fp_dbl(x2), x2));
+        Point r;
+        r.X = fp_sub(fp_sub(P::sqr(M), S), S);
+        r.Y = P::mul_sub(M, P::share(fp_sub(S, r.X)), W, P::share(p.Y));
+        r.ZZ = P::mul(V, P::share(p.ZZ));
+        r.ZZZ = P::mul(W, P::share(p.ZZZ));
+        return r;
+    }
+    // p + (x, y), zero for infinity
+    static __device__ __noinline__ Point madd(Point p, Fp x, Fp y, bool live) {
+        const typename P::Shared ZZ = P::share(p.ZZ), ZZZ = P::share(p.ZZZ);
+        const Fp d = fp_sub(P::mul(P::share(x), ZZ), p.X), e = fp_sub(P::mul(P::share(y), ZZZ), p.Y);
+        Point r = chord(p.X, p.Y, P::share(d), P::share(e), ZZ, ZZZ);
+        const bool qinf = flag(fp_is_zero(x) && fp_is_zero(y)) || !live, pinf = p.is_inf();
+        const bool same = flag(fp_is_zero(d)) && !pinf && !qinf, twice = flag(fp_is_zero(e));
+        if (__any_sync(FULL, same)) {
+            const Point two = dbl(p);
+            r = select(same, select(twice, two, infinity()), r);
+        }
+        r = select(pinf, Point{x, y, P::one(), P::one()}, r);
+        return select(qinf, p, r);
+    }
+    static __device__ __noinline__ Point add(Point p, Point q, bool live) {
+        const typename P::Shared ZZ1 = P::share(p.ZZ), ZZZ1 = P::share(p.ZZZ);
+        const typename P::Shared ZZ2 = P::share(q.ZZ), ZZZ2 = P::share(q.ZZZ);
+        const Fp u = P::mul(P::share(p.X), ZZ2), s = P::mul(P::share(p.Y), ZZZ2);
+        const Fp d = fp_sub(P::mul(P::share(q.X), ZZ1), u), e = fp_sub(P::mul(P::share(q.Y), ZZZ1), s);
+        Point r = chord(u, s, P::share(d), P::share(e), P::share(P::mul(ZZ1, ZZ2)), P::share(P::mul(ZZZ1, ZZZ2)));
+        const bool pinf = p.is_inf(), qinf = q.is_inf() || !live;
+        const bool same = flag(fp_is_zero(d)) && !pinf && !qinf, twice = flag(fp_is_zero(e));
+        if (__any_sync(FULL, same)) {
+            const Point two = dbl(p);
+            r = select(same, select(twice, two, infinity()), r);
+        }
+        r = select(pinf, q, r);
+        return select(qinf, p, r);
+    }
+    // (u, s) and (u + d, s + e) over the common denominators
+    static WBTE_INL Point chord(const Fp& u, const Fp& s, const typename P::Shared& d, const typename P::Shared& e,
+                                const typename P::Shared& ZZ, const typename P::Shared& ZZZ) {
+        const typename P::Shared PP = P::share(P::sqr(d)), PPP = P::share(P::mul(d, PP));
+        const Fp Q = P::mul(P::share(u), PP);
+        Point r;
+        r.X = fp_sub(fp_sub(fp_sub(P::sqr(e), PPP.own), Q), Q);
+        r.Y = P::mul_sub(e, P::share(fp_sub(Q, r.X)), P::share(s), PPP);
+        r.ZZ = P::mul(ZZ, PP);
+        r.ZZZ = P::mul(ZZZ, PPP);
+        return r;
+    }
+    // [g]p, the lanes running the longest of their multiples' bits
+    static WBTE_INL Point multiple(const Point& p, uint32_t g) {
+        Point r = infinity();
+        for (int b = 31 - __clz(__reduce_or_sync(FULL, g) | 1); b >= 0; b--) {
+            r = dbl(r);
+            if (__any_sync(FULL, (g >> b) & 1)) r = add(r, p, (g >> b) & 1);
+        }
+        return r;
+    }
+
+    // this lane's component of coordinate i of a record in memory
+    static WBTE_INL const Fp* at(const uint8_t* rec, int i) {
+        return reinterpret_cast<const Fp*>(rec + i * P::FIELD + 48 * (threadIdx.x & (P::LANES - 1)));
+    }
+    WBTE_INL void store(uint8_t* rec) const {
+        store_vec(const_cast<Fp*>(at(rec, 0)), X);
+        store_vec(const_cast<Fp*>(at(rec, 1)), Y);
+        store_vec(const_cast<Fp*>(at(rec, 2)), ZZ);
+        store_vec(const_cast<Fp*>(at(rec, 3)), ZZZ);
+    }
+};
 
 }  // namespace wbte
