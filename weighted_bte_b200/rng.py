@@ -56,10 +56,11 @@ def chacha20_block(key_words, counter: int, stream: int = 0):
     return [(w[i] + state[i]) & _M32 for i in range(16)]
 
 
-def chacha20_blocks(key_words, counter: int, n: int):
+def _keystream(key_words, counter: int, n: int) -> bytes:
     """n consecutive keystream blocks (counters counter .. counter + n - 1,
-    stream 0) as one flat list of 16 n words, computed for all blocks at once
-    with numpy uint32 vectors (the same function as chacha20_block)."""
+    stream 0).  The four quarter rounds of a column or diagonal round run as one
+    on (4, n) arrays of words (the same function as chacha20_block): numpy's
+    cost per call, not its arithmetic, bounds blocks by the hundred."""
     import numpy as np
 
     st = np.empty((16, n), dtype=np.uint32)
@@ -68,34 +69,38 @@ def chacha20_blocks(key_words, counter: int, n: int):
     ctr = np.arange(counter, counter + n, dtype=np.uint64)
     st[12] = (ctr & np.uint64(_M32)).astype(np.uint32)
     st[13] = (ctr >> np.uint64(32)).astype(np.uint32)
-    st[14] = 0
-    st[15] = 0
-    w = [st[i].copy() for i in range(16)]
+    st[14:16] = 0
+    a, b, c, d = (st[4 * i : 4 * i + 4].copy() for i in range(4))
+    t = np.empty_like(a)
 
-    def rotl(x, k):
-        return (x << np.uint32(k)) | (x >> np.uint32(32 - k))
+    def xor_rotl(x, y, k):  # x <- rotl(x ^ y, k)
+        np.bitwise_xor(x, y, out=x)
+        np.right_shift(x, np.uint32(32 - k), out=t)
+        np.left_shift(x, np.uint32(k), out=x)
+        np.bitwise_or(x, t, out=x)
 
-    def quarter(a, b, c, d):
-        w[a] += w[b]
-        w[d] = rotl(w[d] ^ w[a], 16)
-        w[c] += w[d]
-        w[b] = rotl(w[b] ^ w[c], 12)
-        w[a] += w[b]
-        w[d] = rotl(w[d] ^ w[a], 8)
-        w[c] += w[d]
-        w[b] = rotl(w[b] ^ w[c], 7)
+    def quarters():
+        nonlocal a, c
+        a += b
+        xor_rotl(d, a, 16)
+        c += d
+        xor_rotl(b, c, 12)
+        a += b
+        xor_rotl(d, a, 8)
+        c += d
+        xor_rotl(b, c, 7)
 
     for _ in range(10):
-        quarter(0, 4, 8, 12)
-        quarter(1, 5, 9, 13)
-        quarter(2, 6, 10, 14)
-        quarter(3, 7, 11, 15)
-        quarter(0, 5, 10, 15)
-        quarter(1, 6, 11, 12)
-        quarter(2, 7, 8, 13)
-        quarter(3, 4, 9, 14)
-    out = np.stack(w) + st
-    return out.T.reshape(-1).tolist()
+        quarters()
+        b, c, d = b[[1, 2, 3, 0]], c[[2, 3, 0, 1]], d[[3, 0, 1, 2]]
+        quarters()
+        b, c, d = b[[3, 0, 1, 2]], c[[2, 3, 0, 1]], d[[1, 2, 3, 0]]
+    return (np.concatenate([a, b, c, d]) + st).T.astype("<u4").tobytes()
+
+
+def chacha20_blocks(key_words, counter: int, n: int):
+    """The words of _keystream as one flat list of 16 n integers."""
+    return list(struct.unpack(f"<{16 * n}I", _keystream(key_words, counter, n)))
 
 
 def _pcg32(state: int):
@@ -112,7 +117,8 @@ class ChaCha20Rng:
             raise ValueError("ChaCha20Rng takes a 32-byte seed")
         self.key = list(struct.unpack("<8I", seed))
         self.counter = 0
-        self.buf = []
+        self._stream, self._at = b"", 0
+        self._refill = 0
 
     @classmethod
     def seed_from_u64(cls, state: int) -> "ChaCha20Rng":
@@ -123,27 +129,32 @@ class ChaCha20Rng:
             words.append(x)
         return cls(struct.pack("<8I", *words))
 
-    # keystream blocks generated per refill: the words come out in the same
-    # order whatever the refill size (blocks depend only on key and counter)
+    # keystream blocks of the first refill, doubled up to 16 times that: the
+    # words come out in the same order whatever the size (blocks depend only on
+    # key and counter)
     REFILL_BLOCKS = 64
 
+    def _take(self, n: int) -> bytes:
+        """The next n bytes of the keystream (n a multiple of four)."""
+        out = self._stream[self._at : self._at + n]
+        self._at += len(out)
+        while len(out) < n:
+            self._refill = min(max(self.REFILL_BLOCKS, 2 * self._refill), 16 * self.REFILL_BLOCKS)
+            self._stream = _keystream(self.key, self.counter, self._refill)
+            self.counter += self._refill
+            self._at = n - len(out)
+            out += self._stream[: self._at]
+            self._at = min(self._at, len(self._stream))
+        return out
+
     def next_u32(self) -> int:
-        if not self.buf:
-            self.buf = chacha20_blocks(self.key, self.counter, self.REFILL_BLOCKS)
-            self.counter += self.REFILL_BLOCKS
-            self.buf.reverse()
-        return self.buf.pop()
+        return int.from_bytes(self._take(4), "little")
 
     def next_u64(self) -> int:
-        lo = self.next_u32()
-        hi = self.next_u32()
-        return lo | (hi << 32)
+        return int.from_bytes(self._take(8), "little")
 
     def fill_bytes(self, n: int) -> bytes:
-        out = bytearray()
-        while len(out) < n:
-            out += struct.pack("<I", self.next_u32())
-        return bytes(out[:n])
+        return self._take((n + 3) // 4 * 4)[:n]
 
 
 class OsRng:
@@ -155,10 +166,8 @@ class OsRng:
 
 
 def random_scalar(rng) -> int:
-    acc = 0
-    for i in range(8):
-        acc |= rng.next_u64() << (64 * i)
-    return acc % R
+    # eight 64-bit words, least significant first, as the 64 bytes they are
+    return int.from_bytes(rng.fill_bytes(64), "little") % R
 
 
 def sample_nonzero(rng) -> int:
