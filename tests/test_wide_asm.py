@@ -61,3 +61,10 @@ def test_small_multiples():
         assert value(r) == (a - 4 * P if a >= 4 * P else a)
         b = rng.randrange(P + 1)
         assert value(call("fp_p_minus", a=limbs(b, 12))["r"]) == P - b
+
+
+def test_square():
+    rng = random.Random(7)
+    ri = pow(R384, -1, P)
+    for a in [0, 1, P - 1, P, 2 * P - 1] + [rng.randrange(2 * P) for _ in range(40)]:
+        assert value(call("fp_mont_sqr", a=limbs(a, 12))["r"]) == a * a * ri % P

@@ -19,6 +19,9 @@ WBTE_INL bool f_is_zero(const Fp& a) { return fp_is_zero(a); }
 WBTE_INL Fp f_inv(const Fp& a) { return fp_inv(a); }
 WBTE_INL void f_set_zero(Fp& a) { a = fp_zero(); }
 WBTE_INL void f_set_one(Fp& a) { a = fp_one(); }
+// a b - c d
+WBTE_INL Fp f_mul_sub(const Fp& a, const Fp& b, const Fp& c, const Fp& d) { return fp_mul2(a, b, fp_minus(c), d); }
+WBTE_INL Fp2 f_mul_sub(const Fp2& a, const Fp2& b, const Fp2& c, const Fp2& d) { return fp2_sub(fp2_mul(a, b), fp2_mul(c, d)); }
 WBTE_INL Fp2 f_add(const Fp2& a, const Fp2& b) { return fp2_add(a, b); }
 WBTE_INL Fp2 f_sub(const Fp2& a, const Fp2& b) { return fp2_sub(a, b); }
 WBTE_INL Fp2 f_mul(const Fp2& a, const Fp2& b) { return fp2_mul(a, b); }
@@ -70,7 +73,7 @@ template <class F> static __device__ __noinline__ Xyzz<F> xyzz_dbl(const Xyzz<F>
     F M = f_add(f_dbl(X2), X2);
     Xyzz<F> r;
     r.X = f_sub(f_sub(f_sqr(M), S), S);
-    r.Y = f_sub(f_mul(M, f_sub(S, r.X)), f_mul(W, p.Y));
+    r.Y = f_mul_sub(M, f_sub(S, r.X), W, p.Y);
     r.ZZ = f_mul(V, p.ZZ);
     r.ZZZ = f_mul(W, p.ZZZ);
     return r;
@@ -87,7 +90,7 @@ template <class F> WBTE_INL Xyzz<F> xyzz_mdbl(const Affine<F>& q) {
     F X2 = f_sqr(q.x);
     F M = f_add(f_dbl(X2), X2);
     r.X = f_sub(f_sub(f_sqr(M), S), S);
-    r.Y = f_sub(f_mul(M, f_sub(S, r.X)), f_mul(W, q.y));
+    r.Y = f_mul_sub(M, f_sub(S, r.X), W, q.y);
     r.ZZ = V;
     r.ZZZ = W;
     return r;
@@ -112,7 +115,7 @@ template <class F> static __device__ __noinline__ Xyzz<F> xyzz_madd(const Xyzz<F
     F Q = f_mul(p.X, PP);
     Xyzz<F> r;
     r.X = f_sub(f_sub(f_sub(f_sqr(R), PPP), Q), Q);
-    r.Y = f_sub(f_mul(R, f_sub(Q, r.X)), f_mul(p.Y, PPP));
+    r.Y = f_mul_sub(R, f_sub(Q, r.X), p.Y, PPP);
     r.ZZ = f_mul(p.ZZ, PP);
     r.ZZZ = f_mul(p.ZZZ, PPP);
     return r;
@@ -139,7 +142,7 @@ template <class F> static __device__ __noinline__ Xyzz<F> xyzz_add(const Xyzz<F>
     F Q = f_mul(U1, PP);
     Xyzz<F> r;
     r.X = f_sub(f_sub(f_sub(f_sqr(R), PPP), Q), Q);
-    r.Y = f_sub(f_mul(R, f_sub(Q, r.X)), f_mul(S1, PPP));
+    r.Y = f_mul_sub(R, f_sub(Q, r.X), S1, PPP);
     r.ZZ = f_mul(f_mul(p.ZZ, q.ZZ), PP);
     r.ZZZ = f_mul(f_mul(p.ZZZ, q.ZZZ), PPP);
     return r;

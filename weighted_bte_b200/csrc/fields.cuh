@@ -29,11 +29,21 @@ WBTE_INL Fp fp_one() { Fp r; _Pragma("unroll") for (int i = 0; i < 12; i++) r.v[
 // inside the instruction cache.
 static __device__ __noinline__ Fp fp_mul_ool(Fp a, Fp b) { Fp r; fp_mont_mul(r.v, a.v, b.v); return r; }
 WBTE_INL Fp fp_mul(const Fp& a, const Fp& b) { return fp_mul_ool(a, b); }
-WBTE_INL Fp fp_sqr(const Fp& a) { return fp_mul_ool(a, a); }
+// 222 wide multiply-adds against the product's 288
+static __device__ __noinline__ Fp fp_sqr_ool(Fp a) { Fp r; fp_mont_sqr(r.v, a.v); return r; }
+WBTE_INL Fp fp_sqr(const Fp& a) { return fp_sqr_ool(a); }
 #else
 WBTE_INL Fp fp_mul(const Fp& a, const Fp& b) { Fp r; fp_mont_mul(r.v, a.v, b.v); return r; }
-WBTE_INL Fp fp_sqr(const Fp& a) { Fp r; fp_mont_mul(r.v, a.v, a.v); return r; }
+WBTE_INL Fp fp_sqr(const Fp& a) { Fp r; fp_mont_sqr(r.v, a.v); return r; }
 #endif
+// (a b + c d) / 2^384 mod p for factors up to p: one reduction for two products
+static __device__ __noinline__ Fp fp_mul2(Fp a, Fp b, Fp c, Fp d) {
+    Fp r;
+    fp_mont_mul2(r.v, a.v, b.v, c.v, d.v);
+    return r;
+}
+// p - a, in (0, p]: a factor
+WBTE_INL Fp fp_minus(const Fp& a) { Fp r; fp_p_minus(r.v, a.v); return r; }
 WBTE_INL Fp fp_add(const Fp& a, const Fp& b) { Fp r; fp_add_raw(r.v, a.v, b.v); return r; }
 WBTE_INL Fp fp_sub(const Fp& a, const Fp& b) { Fp r; fp_sub_raw(r.v, a.v, b.v); return r; }
 // a + b without reduction: only valid as a multiplication input (< 2p).

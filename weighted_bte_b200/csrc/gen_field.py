@@ -262,6 +262,75 @@ def gen_mont_mul2(name, modulus, n):
                          [("r", i) for i in range(n)], [(v, i) for v in "abcd" for i in range(n)])
 
 
+def gen_mont_sqr(name, modulus, n):
+    """Montgomery square of a < 2m: the products a_i a_j, i < j, once (two chains a
+    row over the even and the odd columns), doubled, with the a_i^2 in one chain,
+    then the reduction of gen_redc: n (n - 1) / 2 + n + n^2 wide multiply-adds
+    and n more instructions for the quotient words, 222 + 12 for 12 words
+    against 288 + 12 of the product."""
+    pinv = (-pow(modulus, -1, 1 << 32)) % (1 << 32)
+    ml = limbs32(modulus, n)
+    mw = ["0x%08x" % x for x in ml]
+    lines = []
+    w = lines.append
+    w(Window.regs(n, ""))
+    w(".reg .u32 x<%d>, y<%d>, t<%d>, u<%d>, m, bw, d<%d>;" % (2 * n + 2, 2 * n + 2, 2 * n, n, n))
+    w(".reg .pred nb;")
+    a = ["%%%d" % (n + i) for i in range(n)]
+    # column c of the even-column chains is x_c, of the odd-column ones y_c
+    cols = [{}, {}]
+    names = "xy"
+    for i in range(n - 1):
+        for first in (i + 1, i + 2):
+            js = list(range(first, n, 2))
+            if not js:
+                continue
+            par = (i + first) % 2
+            words = cols[par]
+            for k, j in enumerate(js):
+                lo, hi = i + j, i + j + 1
+                w("%s.lo.cc.u32 %s%d, %s, %s, %s;" % ("madc" if k else "mad", names[par], lo, a[i], a[j], words.get(lo, "0")))
+                w("madc.hi.cc.u32 %s%d, %s, %s, %s;" % (names[par], hi, a[i], a[j], words.get(hi, "0")))
+                words[lo] = "%s%d" % (names[par], lo)
+                words[hi] = "%s%d" % (names[par], hi)
+            top = i + js[-1] + 2
+            w("addc.u32 %s%d, %s, 0;" % (names[par], top, words.get(top, "0")))
+            words[top] = "%s%d" % (names[par], top)
+    # t = 2 (x + y) + sum a_i^2 2^(64 i)
+    s = []
+    for c in range(2 * n):
+        e, o = cols[0].get(c), cols[1].get(c)
+        s.append((e, o))
+    w("mov.u32 t0, 0;")
+    started = False
+    for c in range(1, 2 * n):
+        e, o = s[c]
+        e, o = e or "0", o or "0"
+        w("%s.u32 t%d, %s, %s;" % ("addc.cc" if started else "add.cc", c, e, o))
+        started = True
+    for c in range(1, 2 * n):
+        w("%s.u32 t%d, t%d, t%d;" % ("add.cc" if c == 1 else ("addc.cc" if c < 2 * n - 1 else "addc"), c, c, c))
+    for i in range(n):
+        w("%s.lo.cc.u32 t%d, %s, %s, t%d;" % ("madc" if i else "mad", 2 * i, a[i], a[i], 2 * i))
+        w("madc.hi%s.u32 t%d, %s, %s, t%d;" % (".cc" if i < n - 1 else "", 2 * i + 1, a[i], a[i], 2 * i + 1))
+    t = ["t%d" % i for i in range(2 * n)]
+    win = Window(w, n, "")
+    win.Ein = t[:n]
+    w("mul.lo.u32 m, %s, 0x%08x;" % (t[0], pinv))
+    win.add_row(mw, "m")
+    for i in range(1, n):
+        win.shift()
+        w("mul.lo.u32 m, %s, 0x%08x;" % (win.E[0], pinv))
+        win.add_row(mw, "m")
+    u = ["u%d" % i for i in range(n)]
+    win.merge(u)
+    for j in range(n):
+        w("%s.u32 u%d, u%d, %s;" % ("add.cc" if j == 0 else ("addc.cc" if j < n - 1 else "addc"), j, j, t[n + j]))
+    emit_cond_sub(w, ["%%%d" % i for i in range(n)], u, ml)
+    return _asm_function(name, "uint32_t r[%d], const uint32_t a[%d]" % (n, n), lines, [("r", i) for i in range(n)],
+                         [("a", i) for i in range(n)])
+
+
 def gen_mul_wide(name, n):
     """r (2n words) = a b, any n-word a and b."""
     lines = []
@@ -749,6 +818,7 @@ def main():
         gen_sub("fp_sub_raw", P, 12),
         gen_add_nr("fp_add_nored", 12),
         gen_mont_mul2("fp_mont_mul2", P, 12),
+        gen_mont_sqr("fp_mont_sqr", P, 12),
         gen_mul_wide("fp_mul_wide", 12),
         gen_redc("fp_redc", P, 12),
         gen_cond_sub("fp_csub_p", P, 12),

@@ -24,13 +24,6 @@
 
 namespace wbte {
 
-// (x b + y c) / 2^384 mod p for x, y, b, c <= p (or one product of factors < 2p)
-static __device__ __noinline__ Fp fp_mul2(Fp x, Fp b, Fp y, Fp c) {
-    Fp r;
-    fp_mont_mul2(r.v, x.v, b.v, y.v, c.v);
-    return r;
-}
-
 constexpr uint32_t FULL = 0xffffffffu;
 
 WBTE_INL Fp fp_shfl(const Fp& a, int src) {
@@ -59,7 +52,7 @@ struct OnLane {  // Fp
     static WBTE_INL Fp sqr(const Shared& a) { return fp_sqr(a.own); }
     // a b - c d
     static WBTE_INL Fp mul_sub(const Shared& a, const Shared& b, const Shared& c, const Shared& d) {
-        return fp_mul2(a.own, b.own, fp_neg(c.own), d.own);
+        return fp_mul2(a.own, b.own, fp_minus(c.own), d.own);
     }
     static WBTE_INL uint32_t all_lanes(uint32_t ballot) { return ballot; }
     static WBTE_INL Fp one() { return fp_one(); }
@@ -73,14 +66,14 @@ struct OnPair {  // Fp2, component = lane parity
     // even: a0 b0 + (-a1) b1, odd: a0 b1 + a1 b0
     static WBTE_INL Fp mul(const Fp& a, const Fp& b) {
         const Fp pa = fp_shfl_xor(a, 1), pb = fp_shfl_xor(b, 1);
-        const Fp n = fp_neg(pa);
+        const Fp n = fp_minus(pa);
         return fp_mul2(fp_select(odd(), pa, a), b, fp_select(odd(), a, n), pb);
     }
     // a value that several products use, with the partner's component
     struct Shared { Fp own, other; };
     static WBTE_INL Shared share(const Fp& a) { return Shared{a, fp_shfl_xor(a, 1)}; }
     static WBTE_INL Fp mul(const Shared& a, const Shared& b) {
-        return fp_mul2(fp_select(odd(), a.other, a.own), b.own, fp_select(odd(), a.own, fp_neg(a.other)), b.other);
+        return fp_mul2(fp_select(odd(), a.other, a.own), b.own, fp_select(odd(), a.own, fp_minus(a.other)), b.other);
     }
     // even: (a0 + a1)(a0 - a1), odd: a0 2a1
     static WBTE_INL Fp sqr(const Shared& a) {
