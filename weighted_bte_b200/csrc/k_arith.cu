@@ -107,23 +107,35 @@ __global__ void k_gather(uint8_t* out, const uint8_t* in, const int32_t* idx, in
     }
 }
 
-// L_i(0) = prod_{k != i} (-x_k) / (x_i - x_k)
+// L_i(0) = prod_{k != i} (-x_k) / (x_i - x_k), one warp per i: lane l takes the
+// factors k = l, l + 32, .. (a chain of 2n/32 products instead of 2n)
 __global__ void k_lagrange(uint8_t* out, const uint8_t* x, int64_t n, int32_t* status) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
     if (i >= n) return;
-    Fr xi = load_fr_mont(x + FR_SZ * i);
+    const Fr xi = load_fr_mont(x + FR_SZ * i);
     Fr num = fr_one(), den = fr_one();
-    for (int64_t k = 0; k < n; k++) {
+    for (int64_t k = lane; k < n; k += 32) {
         if (k == i) continue;
-        Fr xk = load_fr_mont(x + FR_SZ * k);
+        const Fr xk = load_fr_mont(x + FR_SZ * k);
         num = fr_mul(num, fr_neg(xk));
         den = fr_mul(den, fr_sub(xi, xk));
     }
+    for (int w = 16; w > 0; w >>= 1) {
+        Fr a, b;
+        _Pragma("unroll") for (int t = 0; t < 8; t++) {
+            a.v[t] = __shfl_xor_sync(0xffffffffu, num.v[t], w);
+            b.v[t] = __shfl_xor_sync(0xffffffffu, den.v[t], w);
+        }
+        num = fr_mul(num, a);
+        den = fr_mul(den, b);
+    }
     if (fr_is_zero(den)) {
-        atomicExch(status, 1);
+        if (lane == 0) atomicExch(status, 1);
         return;
     }
-    store_fr_canonical(out + FR_SZ * i, fr_mul(num, fr_inv(den)));
+    num = fr_mul(num, fr_inv(den));
+    if (lane == 0) store_fr_canonical(out + FR_SZ * i, num);
 }
 
 __global__ void k_domain_twiddles(uint8_t* tw, int log_n, int64_t count, bool inverse) {
@@ -846,7 +858,7 @@ void launch_lagrange_at_zero(uint8_t* out, const uint8_t* x, int64_t n, int32_t*
     ProfScope prof_("lagrange", s);
     if (n <= 0) return;
     note_launch();
-    k_lagrange<<<blocks_for(n, 64), 64, 0, s>>>(out, x, n, status);
+    k_lagrange<<<blocks_for(32 * n, 64), 64, 0, s>>>(out, x, n, status);
 }
 void launch_domain_twiddles(uint8_t* tw, int64_t n, int64_t count, bool inverse, cudaStream_t s) {
     if (count <= 0) return;
@@ -927,22 +939,20 @@ void launch_negate(Group g, uint8_t* out, const uint8_t* in, int64_t n, cudaStre
     else k_negate<Fp2><<<blocks_for(n), TPB, 0, s>>>(out, in, n);
 }
 
-// Whether a transform stage of `butterflies` butterflies runs one thread per
-// butterfly (k_ntt_stage_joint) rather than quads: a cost model of one
-// thread's products (G1: 128 doublings and 81 additions of 9 and 14 products
-// of 300 wide multiply-adds; G2: 64 and 75 of 9 and 14 Fp2 products of 900, at
-// half the pipe rate for their spills) and of a quad lane's rounds (G1: 128
-// doublings of three and 41 additions of four rounds, a fifth more for the
-// exchanges, eight lanes a butterfly; G2: 64 and 24 rounds of 444, 32 lanes).
-// WBTE_NTT_JOINT = 0 or 1 overrides the choice, and so does the calling
-// context's tuning knob.
-static bool ntt_joint(Group g, int64_t butterflies) {
+// Whether a transform of `count` arrays of 2^bits values runs one thread per
+// butterfly (k_ntt_stage_joint) rather than quads (quad_ntt_plan): a cost
+// model of one thread's products (G1: 128 doublings and 81 additions of 9 and
+// 14 products of 300 wide multiply-adds; G2: 64 and 75 of 9 and 14 Fp2 products
+// of 900, at half the pipe rate for their spills).  WBTE_NTT_JOINT = 0 or 1
+// overrides the choice, and so does the calling context's tuning knob.
+static bool ntt_joint(Group g, int bits, int64_t count) {
     if (const char* env = getenv("WBTE_NTT_JOINT")) return atoi(env) != 0;
     if (g_tune.ntt_joint == 0 || g_tune.ntt_joint == 1) return g_tune.ntt_joint == 1;
-    const double n = (double)butterflies;
-    if (g == GROUP_G1)
-        return launch_time((128 * 9 + 81 * 14) * 300.0, n / 32) < launch_time((128 * 3 + 41 * 4) * 360.0, n / 4);
-    return launch_time((64 * 9 + 75 * 14) * 1800.0, n / 32) < launch_time((64 * 3 + 24 * 4) * 530.0, n);
+    const double stage = g == GROUP_G1 ? (128 * 9 + 81 * 14) * 300.0 : (64 * 9 + 75 * 14) * 1800.0;
+    const double butterflies = (double)((int64_t)1 << bits) / 2 * (double)count;
+    int steps[64], nsteps = 0;
+    // the first stage has no multiples
+    return (bits - 1) * launch_time(stage, butterflies / 32) < quad_ntt_plan(g, bits, count, steps, &nsteps);
 }
 
 // work[i] = [c_i] in[i] for small signed c_i (XYZZ out): double-and-add over
@@ -1020,36 +1030,29 @@ void launch_group_ntt(Group g, uint8_t* io, uint8_t* work, const uint8_t* tw, in
     ProfScope prof_(g == GROUP_G1 ? "ntt_g1" : "ntt_g2", s);
     int bits = 0;
     while ((int64_t(1) << bits) < n) bits++;
-    const int64_t total = n * count, butterflies = (n / 2) * count;
-    if (g == GROUP_G1) {
-        note_launch();
-        k_ntt_load<Fp><<<blocks_for(total), TPB, 0, s>>>(work, io, n, bits, count);
-        const bool joint = ntt_joint(g, butterflies);
+    const int64_t total = n * count;
+    const bool g1 = g == GROUP_G1;
+    note_launch();
+    if (g1) k_ntt_load<Fp><<<blocks_for(total), TPB, 0, s>>>(work, io, n, bits, count);
+    else k_ntt_load<Fp2><<<blocks_for(total), TPB, 0, s>>>(work, io, n, bits, count);
+    if (ntt_joint(g, bits, count)) {
         // 24..31 transforms run padded to 32 slots: warp-uniform NAF twiddles
         // with at most a quarter of the lanes idle
-        const int64_t pad = count >= 24 && count < WARP ? (int64_t)WARP : count;
+        const int64_t pad = g1 && count >= 24 && count < WARP ? (int64_t)WARP : count;
         for (int64_t half = 1; half < n; half *= 2) {
-            if (joint) {
-                note_launch();
+            note_launch();
+            if (g1)
                 k_ntt_stage_joint<Fp><<<blocks_for((n / 2) * pad, WARP), WARP, 0, s>>>(work, tw, n, half, count, pad);
-            } else {
-                launch_quad_ntt_stage(g, work, tw, n, half, count, s);
-            }
+            else
+                k_ntt_stage_joint<Fp2><<<blocks_for((n / 2) * pad, WARP), WARP, 0, s>>>(work, tw, n, half, count, pad);
         }
-        launch_xyzz_to_affine(GROUP_G1, io, work, total, s);
+        launch_xyzz_to_affine(g, io, work, total, s);
     } else {
-        note_launch();
-        k_ntt_load<Fp2><<<blocks_for(total), TPB, 0, s>>>(work, io, n, bits, count);
-        const bool joint = ntt_joint(g, butterflies);
-        for (int64_t half = 1; half < n; half *= 2) {
-            if (joint) {
-                note_launch();
-                k_ntt_stage_joint<Fp2><<<blocks_for(butterflies, WARP), WARP, 0, s>>>(work, tw, n, half, count, count);
-            } else {
-                launch_quad_ntt_stage(g, work, tw, n, half, count, s);
-            }
-        }
-        launch_xyzz_to_affine(GROUP_G2, io, work, total, s);
+        uint8_t* other = nullptr;
+        if (cudaMallocAsync(&other, (g1 ? G1_XYZZ : G2_XYZZ) * (size_t)total, s) != cudaSuccess) return;
+        if (const uint8_t* done = launch_quad_ntt(g, work, other, tw, n, count, s))
+            launch_xyzz_to_affine(g, io, done, total, s);
+        cudaFreeAsync(other, s);
     }
 }
 

@@ -17,31 +17,33 @@ inline unsigned blocks_for(int64_t n, int tpb = TPB) { return (unsigned)((n + tp
 WBTE_INL Fp12* as_gt(uint8_t* p) { return reinterpret_cast<Fp12*>(p); }
 WBTE_INL const Fp12* as_gt(const uint8_t* p) { return reinterpret_cast<const Fp12*>(p); }
 
-__global__ void k_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n) {
-    int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    Line* L = reinterpret_cast<Line*>(lines);
-    G2A Q = load_affine(reinterpret_cast<const G2A*>(q + G2_AFF * i));
-    if (is_inf(Q)) {
-        // identity lines: every line value is 1, so the loop returns 1
-        Line one{fp2_one(), fp2_zero(), fp2_zero()};
-        for (int s = 0; s < MILLER_LINES; s++) store_vec(L + (int64_t)s * n + i, one);
-        return;
-    }
-    G2Proj T = g2proj_from_affine(Q);
-    int idx = 0;
-    for (int b = 62; b >= 0; b--) {
-        store_vec(L + (int64_t)(idx++) * n + i, line_double(T));
-        if ((X_ABS >> b) & 1) store_vec(L + (int64_t)(idx++) * n + i, line_add(T, Q));
-    }
-}
-
 // this lane's team in the launch (shadow lanes belong to the warp's last one);
 // teams past the end take the last value again without storing it, which is
 // their own warp's, so that a call may work in place
 __device__ __forceinline__ int64_t team_index() {
     const int tm = (int)(threadIdx.x & 31) / TEAM_LANES;
     return (int64_t)blockIdx.x * TEAMS + (tm < TEAMS ? tm : TEAMS - 1);
+}
+
+// the line table of one point per team: lane k writes component k of each record
+__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n) {
+    __shared__ uint4 sh[T6_ROWS * 32];
+    const Team t = team_init(sh);
+    int64_t i = team_index();
+    const bool active = i < n;
+    if (!active) i = n - 1;
+    const G2A Q = load_affine(reinterpret_cast<const G2A*>(q + G2_AFF * i));
+    // identity lines: every line value is 1, so the loop returns 1
+    const bool inf = is_inf(Q);
+    const Fp one = t.k == 0 ? fp_one() : fp_zero();
+    Fp* L = reinterpret_cast<Fp*>(lines + LINE_SZ * i) + t.k;
+    Fp2 T = t.k == 0 ? Q.x : (t.k == 1 ? Q.y : fp2_one());
+    for (int b = 62; b >= 0; b--)
+        for (int step = 0; step <= (t6_bit(b) ? 1 : 0); step++) {
+            const Fp c = step ? t6_line_add(t, T, Q) : t6_line_double(t, T);
+            if (active) store_vec(L, fp_select(inf, one, c));
+            L += n * (int64_t)(LINE_SZ / sizeof(Fp));
+        }
 }
 
 // out[o chunks + ch] = prod over run ch (at most C of t < T) of
@@ -241,7 +243,7 @@ void launch_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n, cudaStrea
     ProfScope prof_("prepare_lines", s);
     if (n <= 0) return;
     note_launch();
-    k_prepare_lines<<<blocks_for(n), TPB, 0, s>>>(lines, q, n);
+    k_prepare_lines<<<blocks_for(n, TEAMS), WARP, 0, s>>>(lines, q, n);
 }
 // Pairs per team of a launch of `outputs` products of T Miller loops each.
 // Sharing the 62 squarings saves 73 of a first pair's wide multiply-adds (in

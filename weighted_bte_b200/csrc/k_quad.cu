@@ -38,39 +38,90 @@ __global__ void __launch_bounds__(WARP) k_combine(uint8_t* out, const uint8_t* w
     if (active) Q::store_affine(out + SizeOf<P>::AFF * j, acc);
 }
 
-// One radix-2 butterfly per DIGITS points: point j takes digit j of the
-// twiddle (Quad::image), the parts are summed, and the first two points write
-// u + t and u - t.
+// A radix-2^kappa step of a decimation-in-time transform merges the radix-2
+// stages of half sizes h, 2h, .., 2^(kappa-1) h: in a block of rho h values
+// (rho = 2^kappa) and for each offset j < h, with x_k the value at j + q h, q the
+// bit reversal of k, and s = n / (rho h),
+//   out[j + m h] = sum_k w^(k s (j + m h)) x_k.
+// For k = 2^e odd the multiples repeat up to sign after V_k = rho / 2^(e+1)
+// values of m, so a block and offset need sum_k V_k = (4^kappa - 1) / 3 of them,
+// all independent: 5 instead of 4 for two stages, 21 instead of 12 for three.
+// A scalar multiple is a chain of about 550 rounds and a sum one of four, so
+// where schedulers idle a step of three stages takes about a third of their time.
+//
+// Multiple r of a block and offset: those of k = 1, 2, .., rho - 1 in order.
+struct RadixTerm { int k, m; };
+__device__ __forceinline__ int radix_variants(int k, int rho) { return rho / (2 * (k & -k)); }
+__device__ __forceinline__ RadixTerm radix_term(int r, int rho) {
+    int k = 1;
+    for (; r >= radix_variants(k, rho); k++) r -= radix_variants(k, rho);
+    return {k, r};
+}
+__device__ __forceinline__ int radix_slot(int k, int m, int rho) {
+    int r = m;
+    for (int i = 1; i < k; i++) r += radix_variants(i, rho);
+    return r;
+}
+
+// multiples[(t per + r)] for the blocks and offsets t (array-major, then block,
+// then offset) and the per = (4^kappa - 1) / 3 multiples r, DIGITS points each
 template <class P>
-__global__ void __launch_bounds__(WARP) k_ntt_stage(uint8_t* work, const uint8_t* tw, int64_t n, int64_t half,
-                                                    int64_t count) {
+__global__ void __launch_bounds__(WARP) k_ntt_multiples(uint8_t* multiples, const uint8_t* work, const uint8_t* tw, int64_t n,
+                                                        int64_t h, int kappa, int64_t total, int per) {
     using Q = Quad<P>;
     constexpr int D = Q::DIGITS;
-    const int64_t p = point_index<P>(), total = (n / 2) * count;
+    const int rho = 1 << kappa;
+    const int64_t p = point_index<P>();
     const int dig = (int)(p % D);
     const bool active = p / D < total;
-    const int64_t t = active ? p / D : total - 1;
-    const int64_t q = t / (n / 2), tt = t % (n / 2), chunk = tt / half, j = tt % half;
-    const int64_t a = q * n + chunk * 2 * half + j, b = a + half;
-    Fp v = Q::load(work + SizeOf<P>::XYZZ * b);
-    const Fp u = Q::load(work + SizeOf<P>::XYZZ * a);
-    if (half > 1) {
-        uint64_t d[4] = {1, 0, 0, 0};
-        if (j) {
-            uint32_t s[8];
-            load_scalar(s, tw + FR_SZ * (j * (n / (2 * half))));
-            decompose_base_x(d, s);
-        }
+    const int64_t g = active ? p / D : total - 1;
+    const int64_t t = g / per, j = t % h, blk = t / h;
+    const RadixTerm term = radix_term((int)(g % per), rho);
+    const int q = (int)(__brev((uint32_t)term.k) >> (32 - kappa));
+    const Fp v = Q::load(work + SizeOf<P>::XYZZ * (blk * rho * h + j + q * h));
+    int64_t idx = (int64_t)term.k * (n / (rho * h)) * (j + term.m * h) % n;
+    const bool minus = idx >= n / 2;  // w^(i + n/2) = -w^i
+    if (minus) idx -= n / 2;
+    uint64_t d[4] = {1, 0, 0, 0};
+    if (idx) {
+        uint32_t s[8];
+        load_scalar(s, tw + FR_SZ * idx);
+        decompose_base_x(d, s);
+    }
+    Fp r = v;
+    // w^0 alone in the whole warp needs no digits
+    if (__any_sync(FULL, idx != 0)) {
         uint64_t lo[1], hi[1];
         quad_digit<P>(lo[0], hi[0], d, dig);
         const Fp base[1] = {Q::image(v, dig)};
-        v = Q::group_sum(Q::straus(base, lo, hi, 1), D);
+        r = Q::group_sum(Q::straus(base, lo, hi, 1), D);
     }
-    // the sum is valid in the butterfly's first point
-    const int lane = threadIdx.x & 31;
-    const Fp first = fp_shfl(v, (lane & ~(D * Q::WIDTH - 1)) + (lane & (Q::WIDTH - 1)));
-    const Fp r = Q::add(u, dig == 1 ? Q::neg(first) : first, true);
-    if (active && dig < 2) Q::store(work + SizeOf<P>::XYZZ * (dig == 0 ? a : b), r);
+    if (minus) r = Q::neg(r);
+    if (active && dig == 0) Q::store(multiples + SizeOf<P>::XYZZ * g, r);
+}
+
+// the sums of a step, L points (a power of two that a warp holds) per output
+template <class P>
+__global__ void __launch_bounds__(WARP) k_ntt_sums(uint8_t* out, const uint8_t* work, const uint8_t* multiples, int64_t h,
+                                                   int kappa, int64_t total, int per, int L) {
+    using Q = Quad<P>;
+    const int rho = 1 << kappa;
+    const int64_t p = point_index<P>();
+    const int sub = (int)(p % L);
+    const bool active = p / L < total;
+    const int64_t o = active ? p / L : total - 1;
+    const int64_t t = o / rho, j = t % h, blk = t / h;
+    const int m = (int)(o % rho);
+    Fp acc = Q::infinity();
+    for (int k = sub; k < rho; k += L) {
+        const int V = k ? radix_variants(k, rho) : 1;
+        Fp x = Q::load(k ? multiples + SizeOf<P>::XYZZ * (t * per + radix_slot(k, m % V, rho))
+                         : work + SizeOf<P>::XYZZ * (blk * rho * h + j));
+        if (k && (m / V) & 1) x = Q::neg(x);
+        acc = k == sub ? x : Q::add(acc, x, true);
+    }
+    acc = Q::group_sum(acc, L);
+    if (active && sub == 0) Q::store(out + SizeOf<P>::XYZZ * (blk * rho * h + j + m * h), acc);
 }
 
 // out[o] = sum_t scalars[vsel[o] n + t] points[pbase[o] + idx[t]] for n <=
@@ -176,14 +227,75 @@ void launch_msm_combine(Group g, uint8_t* out, const uint8_t* wins, int64_t k, i
         k_combine<OnPair><<<blocks_for(k, SizeOf<OnPair>::PER_WARP), WARP, 0, s>>>(out, wins, k, windows, c);
 }
 
-void launch_quad_ntt_stage(Group g, uint8_t* work, const uint8_t* tw, int64_t n, int64_t half, int64_t count,
-                           cudaStream_t s) {
-    const int64_t butterflies = (n / 2) * count;
-    note_launch();
-    if (g == GROUP_G1)
-        k_ntt_stage<OnLane><<<blocks_for(2 * butterflies, SizeOf<OnLane>::PER_WARP), WARP, 0, s>>>(work, tw, n, half, count);
-    else
-        k_ntt_stage<OnPair><<<blocks_for(4 * butterflies, SizeOf<OnPair>::PER_WARP), WARP, 0, s>>>(work, tw, n, half, count);
+// rounds of a quad's scalar multiple (128 doublings of three and 41 additions of
+// four in G1, 64 and 24 in G2) and the wide multiply-adds of a round with its
+// exchanges
+static constexpr double MULTIPLE_G1 = 548, MULTIPLE_G2 = 288, ROUND_G1 = 360, ROUND_G2 = 530;
+
+// Steps of a transform of `bits` stages over `count` arrays: steps[i] stages each,
+// the cheapest composition by the cost model; returns its time.
+double quad_ntt_plan(Group g, int bits, int64_t count, int* steps, int* nsteps) {
+    const bool g1 = g == GROUP_G1;
+    const double points = (double)((int64_t)1 << bits) * (double)count;
+    const int per_warp = g1 ? SizeOf<OnLane>::PER_WARP : SizeOf<OnPair>::PER_WARP, digits = g1 ? 2 : 4;
+    // a pair's products keep two chains in flight: one warp fills a scheduler
+    // (1,024 points in G2: 0.52 ms a stage at 0.9 warps, 1.05 ms at 2.2)
+    const double alone = g1 ? 1.6 : 1.0;
+    double best[64];
+    int last[64];
+    best[0] = 0;
+    for (int done = 1; done <= bits; done++) {
+        best[done] = -1;
+        for (int kappa = 1; kappa <= 4 && kappa <= done; kappa++) {
+            // a first step multiplies by powers of its own root only: one of a k's V_k is one
+            const double multiples = ((double)((1 << (2 * kappa)) - 1) / 3.0) / (double)(1 << kappa) * points * digits;
+            const double chain = done == kappa && kappa == 1 ? 0.0 : (g1 ? MULTIPLE_G1 : MULTIPLE_G2);
+            const double t = best[done - kappa] +
+                             launch_time(chain * (g1 ? ROUND_G1 : ROUND_G2), multiples / per_warp, alone) +
+                             launch_time(4.0 * kappa * (g1 ? ROUND_G1 : ROUND_G2), points / per_warp, alone);
+            if (best[done] < 0 || t < best[done]) best[done] = t, last[done] = kappa;
+        }
+    }
+    *nsteps = 0;
+    for (int done = bits; done > 0; done -= last[done]) steps[(*nsteps)++] = last[done];
+    std::reverse(steps, steps + *nsteps);
+    return best[bits];
+}
+
+uint8_t* launch_quad_ntt(Group g, uint8_t* work, uint8_t* other, const uint8_t* tw, int64_t n, int64_t count, cudaStream_t s) {
+    int bits = 0;
+    while ((int64_t(1) << bits) < n) bits++;
+    int steps[64], nsteps = 0;
+    quad_ntt_plan(g, bits, count, steps, &nsteps);
+    const bool g1 = g == GROUP_G1;
+    const size_t rec = g1 ? G1_XYZZ : G2_XYZZ;
+    const int per_warp = g1 ? SizeOf<OnLane>::PER_WARP : SizeOf<OnPair>::PER_WARP, digits = g1 ? 2 : 4;
+    int64_t most = 0;
+    for (int i = 0; i < nsteps; i++) most = std::max<int64_t>(most, ((1 << (2 * steps[i])) - 1) / 3 * (n >> steps[i]) * count);
+    uint8_t* multiples = nullptr;
+    if (cudaMallocAsync(&multiples, rec * (size_t)std::max<int64_t>(most, 1), s) != cudaSuccess) return nullptr;
+    int64_t h = 1;
+    for (int i = 0; i < nsteps; i++) {
+        const int kappa = steps[i], per = ((1 << (2 * kappa)) - 1) / 3;
+        const int64_t total = (n >> kappa) * count * per, outs = n * count;
+        // sums: as many points per output as leave no scheduler waiting
+        int L = 1;
+        while (2 * L <= per_warp && 2 * L <= (1 << kappa) && (double)(outs * 2 * L) / per_warp <= 1.6 * schedulers()) L *= 2;
+        note_launch(2);
+        if (g1) {
+            k_ntt_multiples<OnLane><<<blocks_for(total * digits, per_warp), WARP, 0, s>>>(multiples, work, tw, n, h, kappa,
+                                                                                       total, per);
+            k_ntt_sums<OnLane><<<blocks_for(outs * L, per_warp), WARP, 0, s>>>(other, work, multiples, h, kappa, outs, per, L);
+        } else {
+            k_ntt_multiples<OnPair><<<blocks_for(total * digits, per_warp), WARP, 0, s>>>(multiples, work, tw, n, h, kappa,
+                                                                                       total, per);
+            k_ntt_sums<OnPair><<<blocks_for(outs * L, per_warp), WARP, 0, s>>>(other, work, multiples, h, kappa, outs, per, L);
+        }
+        std::swap(work, other);
+        h <<= kappa;
+    }
+    cudaFreeAsync(multiples, s);
+    return work;
 }
 
 void launch_quad_small_msm(Group g, uint8_t* out, const uint8_t* points, const int64_t* pbase, const int32_t* idx,

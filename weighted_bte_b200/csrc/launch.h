@@ -62,7 +62,9 @@ inline int schedulers() {
 // wide multiply-adds each.  One warp alone keeps a scheduler's multiply-add
 // pipe 0.6 busy (14.0 of 18.6 and 19.1 of 29.7 G products/s measured at one
 // and at eight warps), so fewer than 1.6 warps a scheduler take as long as 1.6.
-inline double launch_time(double work, double warps) { return work * std::max(1.6, warps / schedulers()); }
+inline double launch_time(double work, double warps, double alone = 1.6) {
+    return work * std::max(alone, warps / schedulers());
+}
 
 constexpr size_t G1_AFF = 96, G2_AFF = 192, G1_XYZZ = 192, G2_XYZZ = 384, GT_SZ = 576, FR_SZ = 32;
 constexpr size_t LINE_SZ = 288;  // three Fp2 coefficients
@@ -151,9 +153,11 @@ void launch_msm_family(Group g, uint8_t* out, const uint8_t* points, const int64
 // Kernels over quads (k_quad.cu) for launches that leave schedulers idle:
 // out[j] = sum_w 2^(c w) wins[j windows + w] from XYZZ window sums
 void launch_msm_combine(Group g, uint8_t* out, const uint8_t* wins, int64_t k, int windows, int c, cudaStream_t s);
-// one radix-2 stage over XYZZ points
-void launch_quad_ntt_stage(Group g, uint8_t* work, const uint8_t* tw, int64_t n, int64_t half, int64_t count,
-                           cudaStream_t s);
+// all stages of a transform over XYZZ points in bit-reversed order, between two
+// buffers; returns the one with the result, null if there is no memory.
+// quad_ntt_plan: its steps and the cost model's time.
+uint8_t* launch_quad_ntt(Group g, uint8_t* work, uint8_t* other, const uint8_t* tw, int64_t n, int64_t count, cudaStream_t s);
+double quad_ntt_plan(Group g, int bits, int64_t count, int* steps, int* nsteps);
 // launch_small_msm with the (term, digit) pairs of an output on L points
 void launch_quad_small_msm(Group g, uint8_t* out, const uint8_t* points, const int64_t* pbase, const int32_t* idx,
                            const uint8_t* scalars, const int32_t* vsel, int64_t k, int64_t n, int L, cudaStream_t s);
