@@ -217,6 +217,77 @@ __global__ void __launch_bounds__(WARP) k_schnorr_verify(uint8_t* valid, const u
     if (active && sub == 0 && Q::place() == 0) valid[i] = inf ? 1 : 0;
 }
 
+// ------------------------------------------- fixed-base G2 MSMs of few terms
+// For G2 points that stay fixed across many calls (a committee's verification
+// keys), table[p][w][m - 1] = [m 64^w] P_p (w < FB_WINDOWS, 1 <= m <= 32,
+// affine).  A term [s]P then costs one mixed addition per nonzero signed
+// radix-64 digit of each base-|x| digit of s (digit c acting through
+// (-1)^c psi^c, applied to the table entry), and no doublings.
+
+// signed radix-64 digit k of d (d < 2^64): digits in [-31, 32], the carry
+// into digit k set when the low k digits of d exceed 0x20..20 (32 in each)
+WBTE_INL int r64_digit(uint64_t d, int k) {
+    auto carry = [&](int j) -> int {
+        if (j == 0 || 6 * j > 64) return 0;  // above bit 64 the bound exceeds any d < 2^64
+        const uint64_t m = (1ull << (6 * j)) - 1;
+        const uint64_t e = 0x820820820820820ull & m;  // 32 * 64^i summed over i < j
+        return (d & m) > e;
+    };
+    const int nib = 6 * k < 64 ? (int)((d >> (6 * k)) & 63u) : 0;
+    return nib + carry(k) - 64 * carry(k + 1);
+}
+
+// out[o] = sum_t scalars[vsel[o] n + t] * P(tbase[o] + tidx[t]), L pairs of lanes
+// per output.  One pair takes the four digits in turn, applying |x| to its sum
+// between them; of four or sixteen pairs each takes one digit (and of sixteen
+// a quarter of its windows) and applies |x| to its own sum at the end.  Applied
+// to sums instead of table entries, psi is 3 actions an output instead of 66 a
+// term.  Measured on B200: 32,768 outputs of three terms 8.3 -> 6.1 ms; the
+// six classes of 24 uneven weighted_pfe batches 36 -> 3.0 ms.
+__global__ void __launch_bounds__(WARP) k_fixed_msm_g2(uint8_t* out, const uint8_t* tables, const int64_t* tbase,
+                                                      const int32_t* tidx, const uint8_t* scalars, const int32_t* vsel,
+                                                      int64_t k, int64_t n, int L) {
+    using Pt = Point<OnPair>;
+    const int64_t p = ((int64_t)blockIdx.x * WARP + threadIdx.x) / 2;
+    const int sub = (int)(p % L), parts = L > 4 ? L / 4 : 1;
+    const bool active = p / L < k;
+    const int64_t o = active ? p / L : k - 1;
+    const int64_t v = vsel ? (int64_t)vsel[o] : 0;
+    Pt acc = Pt::infinity();
+    const int digits = L == 1 ? 4 : 1;
+    for (int i = 0; i < digits; i++) {
+        const int c = L == 1 ? 3 - i : sub & 3;
+        if (i) acc = Pt::image(acc);
+        for (int64_t t = 0; t < n; t++) {
+            const uint8_t* T = tables + FIXED_TABLE_BYTES * (tbase[o] + (tidx ? (int64_t)tidx[t] : t));
+            uint32_t sc[8];
+            load_scalar(sc, scalars + FR_SZ * (v * n + t));
+            uint64_t d[4];
+            decompose_base_x(d, sc);
+            const uint64_t dc = c < 2 ? (c == 0 ? d[0] : d[1]) : (c == 2 ? d[2] : d[3]);
+            for (int w0 = 0; w0 < FB_WINDOWS; w0 += parts) {
+                const int w = w0 + sub / 4 % parts;
+                const int dd = w < FB_WINDOWS ? r64_digit(dc, w) : 0;
+                if (!__any_sync(FULL, dd != 0)) continue;
+                const int a = dd < 0 ? -dd : dd;
+                const uint8_t* e = T + G2_AFF * ((w < FB_WINDOWS ? w : 0) * FB_ENTRIES + (a ? a - 1 : 0));
+                const Fp x = load_vec(Pt::at(e, 0)), y = load_vec(Pt::at(e, 1));
+                acc = Pt::madd(acc, x, dd < 0 ? fp_neg(y) : y, dd != 0);
+            }
+        }
+    }
+    if (L > 1) {
+        for (int i = 0; i < 3; i++) acc = Pt::select((sub & 3) > i, Pt::image(acc), acc);
+        for (int w = 1; w < L; w *= 2) acc = Pt::add(acc, Pt::above(acc, 2 * w), true);
+    }
+    Fp x, y;
+    acc.affine(x, y);
+    if (active && sub == 0) {
+        store_vec(const_cast<Fp*>(Pt::at(out + G2_AFF * o, 0)), x);
+        store_vec(const_cast<Fp*>(Pt::at(out + G2_AFF * o, 1)), y);
+    }
+}
+
 }  // namespace
 
 void launch_msm_combine(Group g, uint8_t* out, const uint8_t* wins, int64_t k, int windows, int c, cudaStream_t s) {
@@ -322,6 +393,21 @@ void launch_quad_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t*
                                 int64_t n, const uint8_t* gen_table, cudaStream_t s) {
     note_launch();
     k_schnorr_verify<<<blocks_for(4 * n, SizeOf<OnLane>::PER_WARP), WARP, 0, s>>>(valid, X, R, sresp, c, n, gen_table);
+}
+
+void launch_fixed_msm_g2(uint8_t* out, const uint8_t* tables, const int64_t* tbase, const int32_t* tidx,
+                         const uint8_t* scalars, const int32_t* vsel, int64_t k, int64_t n, cudaStream_t s) {
+    ProfScope prof_("fixed_msm_g2", s);
+    if (k <= 0) return;
+    // mixed additions of one pair: 44 a term, or 11 or 3 and the tree's
+    int L = 1;
+    double best = launch_time(44.0 * n, (double)k / 16, 1.25);
+    for (int pairs : {4, 16}) {
+        const double t = launch_time((pairs == 4 ? 11.0 : 3.0) * n + 1.5 * (pairs == 4 ? 2 : 4), (double)k * pairs / 16, 1.25);
+        if (t < best) best = t, L = pairs;
+    }
+    note_launch();
+    k_fixed_msm_g2<<<blocks_for(2 * L * k, WARP), WARP, 0, s>>>(out, tables, tbase, tidx, scalars, vsel, k, n, L);
 }
 
 }  // namespace wbte

@@ -117,7 +117,8 @@ void launch_group_ntt(Group g, uint8_t* io_affine, uint8_t* work_xyzz, const uin
 // compressed (ZCash) encodings
 void launch_compress(Group g, uint8_t* out, const uint8_t* in, int64_t n, cudaStream_t s);
 // fixed-base tables of np G2 points (points[point_index[p]]): FIXED_TABLE_BYTES each
-constexpr size_t FIXED_TABLE_BYTES = G2_AFF * 11 * 32;
+constexpr int FB_WINDOWS = 11, FB_ENTRIES = 32;  // of 64-bit digits in radix 64
+constexpr size_t FIXED_TABLE_BYTES = G2_AFF * FB_WINDOWS * FB_ENTRIES;
 void launch_fixed_tables_g2(uint8_t* tables, const uint8_t* points, const int64_t* point_index, int64_t np,
                             cudaStream_t s);
 // out[o] = sum_t scalars[vsel[o] n + t] * (point of table tbase[o] + tidx[t]), k outputs

@@ -344,6 +344,27 @@ template <class P> struct Point {
         return r;
     }
 
+    // the action of |x| on G2: -psi
+    static WBTE_INL Point image(const Point& p) {
+        const auto conj = [](const Fp& a) { return OnPair::odd() ? fp_neg(a) : a; };
+        const Fp kx = fp_select(OnPair::odd(), fp_from_const(C_PSI_CX[1]), fp_from_const(C_PSI_CX[0]));
+        const Fp ky = fp_select(OnPair::odd(), fp_from_const(C_PSI_CY[1]), fp_from_const(C_PSI_CY[0]));
+        return Point{P::mul(conj(p.X), kx), fp_neg(P::mul(conj(p.Y), ky)), conj(p.ZZ), conj(p.ZZZ)};
+    }
+    // the point `by` lanes further on
+    static WBTE_INL Point above(const Point& p, int by) {
+        const int l = ((threadIdx.x & 31) + by) & 31;
+        return Point{fp_shfl(p.X, l), fp_shfl(p.Y, l), fp_shfl(p.ZZ, l), fp_shfl(p.ZZZ, l)};
+    }
+    // X and Y of the affine point (zero for infinity)
+    WBTE_INL void affine(Fp& x, Fp& y) const {
+        const Fp t = P::inv(P::mul(ZZ, ZZZ));
+        const bool inf = is_inf();
+        const Fp ax = P::mul(X, P::mul(t, ZZZ)), ay = P::mul(Y, P::mul(t, ZZ));
+        x = fp_select(inf, fp_zero(), ax);
+        y = fp_select(inf, fp_zero(), ay);
+    }
+
     // this lane's component of coordinate i of a record in memory
     static WBTE_INL const Fp* at(const uint8_t* rec, int i) {
         return reinterpret_cast<const Fp*>(rec + i * P::FIELD + 48 * (threadIdx.x & (P::LANES - 1)));
