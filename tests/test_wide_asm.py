@@ -61,6 +61,8 @@ def test_small_multiples():
         assert value(r) == (a - 4 * P if a >= 4 * P else a)
         b = rng.randrange(P + 1)
         assert value(call("fp_p_minus", a=limbs(b, 12))["r"]) == P - b
+        b = rng.randrange(3 * P + 1)
+        assert value(call("fp_3p_minus", a=limbs(b, 12))["r"]) == 3 * P - b
 
 
 def test_square():

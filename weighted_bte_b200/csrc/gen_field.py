@@ -825,6 +825,7 @@ def main():
         gen_cond_sub("fp_csub_2p", 2 * P, 12),
         gen_cond_sub("fp_csub_4p", 4 * P, 12),
         gen_const_minus("fp_p_minus", P, 12),
+        gen_const_minus("fp_3p_minus", 3 * P, 12),
         gen_add_const("fp_add_p", P, 12),
         gen_add_const("fp_add_2p", 2 * P, 12),
         gen_addsub_nr("wide_add", 24, False),

@@ -22,16 +22,17 @@ template <class P> __device__ __forceinline__ int64_t point_index() {
     return (int64_t)blockIdx.x * SizeOf<P>::PER_WARP + (threadIdx.x & 31) / Quad<P>::WIDTH;
 }
 
-// out[j] = sum_w 2^(c w) wins[j windows + w], the sums of each window
+// out[j] = sum_w 2^(c w) wins[j windows + w], the sums of each window, of points
+// on the curve.  About 250 doublings in a row bound it, whatever the MSM's size.
 template <class P>
 __global__ void __launch_bounds__(WARP) k_combine(uint8_t* out, const uint8_t* wins, int64_t k, int windows, int c) {
-    using Q = Quad<P>;
-    const int64_t j = point_index<P>();
+    using Q = Quad<P, 8>;
+    const int64_t j = (int64_t)blockIdx.x * (WARP / Q::WIDTH) + (threadIdx.x & 31) / Q::WIDTH;
     const bool active = j < k;
     const uint8_t* W = wins + SizeOf<P>::XYZZ * (active ? j : k - 1) * windows;
     Fp acc = Q::load(W + SizeOf<P>::XYZZ * (windows - 1));
     for (int w = windows - 2; w >= 0; w--) {
-        for (int i = 0; i < c; i++) acc = Q::dbl(acc);
+        for (int i = 0; i < c; i++) acc = Q::dbl_on_curve(acc);
         acc = Q::add(acc, Q::load(W + SizeOf<P>::XYZZ * w), true);
     }
     acc = Q::affine(acc);
@@ -293,9 +294,9 @@ __global__ void __launch_bounds__(WARP) k_fixed_msm_g2(uint8_t* out, const uint8
 void launch_msm_combine(Group g, uint8_t* out, const uint8_t* wins, int64_t k, int windows, int c, cudaStream_t s) {
     note_launch();
     if (g == GROUP_G1)
-        k_combine<OnLane><<<blocks_for(k, SizeOf<OnLane>::PER_WARP), WARP, 0, s>>>(out, wins, k, windows, c);
+        k_combine<OnLane><<<blocks_for(k, WARP / Quad<OnLane, 8>::WIDTH), WARP, 0, s>>>(out, wins, k, windows, c);
     else
-        k_combine<OnPair><<<blocks_for(k, SizeOf<OnPair>::PER_WARP), WARP, 0, s>>>(out, wins, k, windows, c);
+        k_combine<OnPair><<<blocks_for(k, WARP / Quad<OnPair, 8>::WIDTH), WARP, 0, s>>>(out, wins, k, windows, c);
 }
 
 // rounds of a quad's scalar multiple (128 doublings of three and 41 additions of
