@@ -210,49 +210,32 @@ __global__ void __launch_bounds__(SEG_TPB) k_segments(uint8_t* seg_out, const ui
     if (real) acc.store(seg_out + 4 * P::FIELD * gid);
 }
 
-// out[i] = sum_{g < G, i*G+g < len} in[row * len + i*G + g] for each row
+// out[row * out_len + i] = sum of in[row * len + G i .. G i + G - 1], G = 2, 4,
+// .., 32: G lanes per output, a shuffle tree of log2 G additions (lanes past len
+// hold the identity); every lane runs each level, so the warp never diverges
+// around the shuffles.
 template <class F>
-__global__ void k_reduce(uint8_t* out, const uint8_t* in, int64_t rows, int64_t len, int64_t G, int64_t out_len) {
-    int64_t gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (gid >= rows * out_len) return;
-    int64_t row = gid / out_len, i = gid % out_len;
-    const Xyzz<F>* src = reinterpret_cast<const Xyzz<F>*>(in) + row * len;
+__global__ void k_reduce(uint8_t* out, const uint8_t* in, int64_t rows, int64_t len, int64_t out_len, int G) {
+    const int64_t gid = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, sub = lane & (G - 1);
+    const int64_t o = gid / G, row = o / out_len, x = o % out_len * G + sub;
     Xyzz<F> acc;
-    set_inf(acc);
-    for (int64_t g = 0; g < G; g++) {
-        int64_t x = i * G + g;
-        if (x < len) acc = xyzz_add(acc, load_vec(src + x));
-    }
-    store_vec(reinterpret_cast<Xyzz<F>*>(out) + gid, acc);
-}
-
-// out[row * out_len + i] = sum of in[row * len + 32 i .. 32 i + 31]: one warp
-// per output, a shuffle tree of five additions (lanes past len hold the
-// identity); every lane runs each level, so the warp never diverges around
-// the shuffles.
-template <class F>
-__global__ void k_reduce_warp(uint8_t* out, const uint8_t* in, int64_t rows, int64_t len, int64_t out_len) {
-    const int lane = threadIdx.x & 31;
-    const int64_t wid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5;
-    if (wid >= rows * out_len) return;  // whole warps: rows * out_len warps are launched
-    const int64_t row = wid / out_len, i = wid % out_len, x = i * 32 + lane;
-    Xyzz<F> acc;
-    if (x < len) {
+    if (row < rows && x < len) {
         acc = load_vec(reinterpret_cast<const Xyzz<F>*>(in) + row * len + x);
     } else {
         set_inf(acc);
     }
     constexpr int WORDS = sizeof(Xyzz<F>) / 4;
-    for (int off = 16; off > 0; off >>= 1) {
+    for (int off = G / 2; off > 0; off >>= 1) {
         Xyzz<F> other;
         uint32_t* dst = reinterpret_cast<uint32_t*>(&other);
         const uint32_t* src = reinterpret_cast<const uint32_t*>(&acc);
 #pragma unroll
         for (int w = 0; w < WORDS; w++) dst[w] = __shfl_down_sync(0xffffffffu, src[w], off);
-        if (lane + off >= 32) set_inf(other);
+        if (sub + off >= G) set_inf(other);
         acc = xyzz_add(acc, other);
     }
-    if (lane == 0) store_vec(reinterpret_cast<Xyzz<F>*>(out) + wid, acc);
+    if (row < rows && sub == 0) store_vec(reinterpret_cast<Xyzz<F>*>(out) + o, acc);
 }
 
 struct ScratchLayout {
@@ -316,15 +299,12 @@ void run_family(uint8_t* out, const uint8_t* points, const int64_t* pbase, const
     uint8_t* bufs[2] = {red, seg};
     int flip = 0;
     while (len > 1) {
-        // long rows: warp-shuffle trees of 32; the last few per row: one thread
-        const int64_t G = len > 8 ? 32 : len;
+        int G = 2;
+        while (G < 32 && G < len) G *= 2;
         const int64_t out_len = (len + G - 1) / G;
         uint8_t* dst = bufs[flip];
         note_launch();
-        if (G == 32)
-            k_reduce_warp<F><<<blocks_for(rows * out_len * 32, 64), 64, 0, s>>>(dst, src, rows, len, out_len);
-        else
-            k_reduce<F><<<blocks_for(rows * out_len, 64), 64, 0, s>>>(dst, src, rows, len, G, out_len);
+        k_reduce<F><<<blocks_for(rows * out_len * G, 64), 64, 0, s>>>(dst, src, rows, len, out_len, G);
         src = dst;
         flip ^= 1;
         len = out_len;
@@ -351,45 +331,55 @@ template <class P> static int64_t segment_wave() {
     return v;
 }
 
+// Window width and segments per (MSM, window) from a cost model in mixed
+// additions.  Every segment's lanes walk S sorted terms, so the launch takes
+// ceil(segments / wave) waves of S terms, an addition (1.43) per bucket that a
+// segment of terms spread evenly over the buckets meets, and, where a row has
+// several segments, the last bucket's multiple (a doubling and an addition per
+// bit) and a tree of additions; the sort's count of buckets takes one thread, the
+// tail adds the windows' sums in one chain (0.53 each; the doublings do not
+// depend on c).  Narrow windows make few
+// buckets and short multiples, wide ones few rows.  Measured on B200, one G1
+// MSM of 65,536 points: c = 8 2.58 ms, 10 2.60, 13 (the former log2(n) - 2,
+// capped) 2.79; of 32 points c = 8 1.30, 4 1.40.
 MsmPlan msm_plan(Group g, int64_t n, int64_t k) {
-    MsmPlan p;
-    int lg = 0;
-    while ((int64_t(1) << (lg + 1)) <= n) lg++;
-    int c = lg - 1;
-    if (n >= (1 << 14)) c = lg - 2;
-    if (c < 4) c = 4;
-    if (c > 13) c = 13;
-    if (g_tune.msm_window >= 4 && g_tune.msm_window <= 13) c = g_tune.msm_window;
-    p.c = c;
-    p.windows = (256 + c - 1) / c;
-    p.buckets = 1 << (c - 1);
-    // Segments per (MSM, window): every thread of k_segments walks one
-    // segment, so the launch takes ceil(threads / wave) waves of the longest
-    // segment.  Cost model in mixed additions: S terms plus one full addition
-    // (~1.43 mixed additions) per bucket change, min(S, buckets), and the
-    // tree reduction of the segment sums.
-    const int64_t wave = g == GROUP_G1 ? segment_wave<OnLane>() : segment_wave<OnPair>();
-    const int64_t rows = k * p.windows;
-    const double nnz = (double)n * (1.0 - 1.0 / (double)(int64_t(1) << c));
-    double best = 1e300;
-    int64_t best_s = 1;
-    for (int64_t s = 1; s <= 1024 && s <= n; s++) {
-        double S = std::ceil(nnz / (double)s);
-        double per_thread = S + 1.43 * std::min(S, (double)p.buckets);
-        int64_t threads = rows * s;
-        double waves = std::ceil((double)threads / (double)wave);
-        double reduce = s > 1 ? 1.43 * 8.0 * std::ceil((double)threads / (8.0 * (double)wave)) : 0.0;
-        double cost = waves * per_thread + reduce;
-        if (cost < best * 0.999) {
-            best = cost;
-            best_s = s;
-        }
+    const double wave = (double)(g == GROUP_G1 ? segment_wave<OnLane>() : segment_wave<OnPair>());
+    int c0 = 4, c1 = 13;
+    if (g_tune.msm_window >= c0 && g_tune.msm_window <= c1) c0 = c1 = g_tune.msm_window;
+    const int64_t forced = g_tune.msm_segments > 0 ? std::min<int64_t>(std::min<int64_t>(g_tune.msm_segments, 1024), n) : 0;
+    const int64_t most = std::min<int64_t>(1024, n);
+    MsmPlan best;
+    double best_cost = 0;
+    for (int c = c0; c <= c1; c++) {
+        const int windows = (256 + c - 1) / c;
+        const double buckets = (double)(1 << (c - 1)), rows = (double)(k * windows);
+        const double terms = (double)n * (1.0 - 1.0 / (2.0 * buckets));
+        auto consider = [&](int64_t s) {
+            s = forced ? forced : std::max<int64_t>(1, std::min(s, most));
+            const double S = std::ceil(terms / (double)s);
+            // buckets without terms leave gaps of several between those with
+            const double gap = 2.3 * std::max(0.0, std::log2(buckets / (double)n));
+            const double met = std::min(std::min(S, buckets), S * buckets / (double)n + 1.0);
+            double each = S + met * (1.43 + gap) + (s > 1 ? 2.3 * (c - 1) : 0.0), tree = buckets / 900;
+            if (s > 1) {
+                for (double len = (double)s; len > 1; len = std::ceil(len / 32)) tree += 1.43 * std::min(5.0, std::ceil(std::log2(len)));
+            }
+            const double cost = std::ceil(rows * (double)s / wave) * each + tree + 0.53 * windows;
+            if (best.c == 0 || cost < best_cost) {
+                best_cost = cost;
+                best.c = c;
+                best.windows = windows;
+                best.segments = s;
+            }
+        };
+        // counts an eighth apart, and those that just fill whole waves
+        for (int64_t s = 1; s <= most; s += 1 + s / 8) consider(s);
+        for (int w = 1; w <= 4; w++) consider((int64_t)(wave * w / rows));
     }
-    if (g_tune.msm_segments > 0) best_s = std::min<int64_t>(std::min<int64_t>(g_tune.msm_segments, 1024), n);
-    p.segment = (n + best_s - 1) / best_s;
-    p.segments = (n + p.segment - 1) / p.segment;
-    if (p.segments < 1) p.segments = 1;
-    return p;
+    best.buckets = 1 << (best.c - 1);
+    best.segment = (n + best.segments - 1) / best.segments;
+    best.segments = std::max<int64_t>(1, (n + best.segment - 1) / best.segment);
+    return best;
 }
 
 size_t msm_family_scratch_bytes(Group g, int32_t V, int64_t k, int64_t n, const MsmPlan& plan) {
