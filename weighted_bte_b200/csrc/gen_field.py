@@ -425,6 +425,24 @@ def gen_const_minus(name, c, n):
                          [("a", i) for i in range(n)])
 
 
+def gen_add_signed(name, n):
+    """r = a + b (m[0] = 0) or a - b (m[0] all ones) modulo 2^(32n)."""
+    lines = []
+    w = lines.append
+    w(".reg .u32 d<%d>, x<%d>, c;" % (n, n))
+    m = "%%%d" % (3 * n)
+    for j in range(n):
+        w("xor.b32 x%d, %%%d, %s;" % (j, 2 * n + j, m))
+    w("add.cc.u32 c, %s, %s;" % (m, m))
+    for j in range(n):
+        w("%s.u32 d%d, %%%d, x%d;" % ("addc.cc" if j < n - 1 else "addc", j, n + j, j))
+    for j in range(n):
+        w("mov.u32 %%%d, d%d;" % (j, j))
+    return _asm_function(name, "uint32_t r[%d], const uint32_t a[%d], const uint32_t b[%d], const uint32_t m[1]" % (n, n, n),
+                         lines, [("r", i) for i in range(n)],
+                         [("a", i) for i in range(n)] + [("b", i) for i in range(n)] + [("m", 0)])
+
+
 def gen_addsub_nr(name, n, sub):
     """r = a + b or a - b modulo 2^(32n)."""
     o = "sub" if sub else "add"
@@ -830,6 +848,7 @@ def main():
         gen_add_const("fp_add_2p", 2 * P, 12),
         gen_addsub_nr("wide_add", 24, False),
         gen_addsub_nr("wide_sub", 24, True),
+        gen_add_signed("wide_add_signed", 24),
         gen_fp2_mul_lazy("fp2_mont_mul_lazy"),
         gen_mont_mul_rolled("fp_mont_mul_r4", P, 12, 4),
         gen_mont_mul_rolled("fp_mont_mul_r6", P, 12, 6),

@@ -1,4 +1,4 @@
-// GT transforms and GT exponentiation over teams of six lanes (team.cuh): the
+// GT transforms and GT exponentiation over teams of lanes (team.cuh): the
 // radix-4 stages of the (truncated) cyclotomic transforms and batched GT
 // powers.
 //
@@ -9,7 +9,7 @@
 // of five blocks or arrays, so its recoding is uniform in the warp and a
 // width-4 NAF skips zero digits without divergence.  A transform of one array
 // leaves schedulers idle and is bound by the length of the chain, so the
-// digits are spread over two or four teams that meet in a product.
+// digits are spread over teams that meet in a product.
 #include <algorithm>
 #include <cstdlib>
 
@@ -68,41 +68,41 @@ __global__ void k_gt_recode(int8_t* rec, const uint8_t* scalars, int64_t n, int 
 // as |x|), NAF tables 1, 3, 5, 7; the other digits' tables are their images.
 // Digits may differ between the teams of a warp: a product is skipped only
 // where every team's digit is zero, and is by one where a team's is.
-template <int L, bool NAF>
-__device__ __forceinline__ Fp2 t6_pow(const Team& t, Fp2 x, const int8_t* rec, int c0) {
+template <class T, int L, bool NAF>
+__device__ __forceinline__ ElemOf<T> team_pow(const Team& t, ElemOf<T> x, const int8_t* rec, int c0) {
     constexpr int R = 4 / L, ND = NAF ? 4 : 8, TOP = NAF ? NAF_DIGITS : R16_DIGITS, RUN = NAF ? 1 : 4;
     if (L > 1) {
-        const Fp2 y = t6_frobenius(t, x, c0 ? c0 : 1);
-        const Fp2 z = (c0 & 1) ? t6_conj(t, y) : y;
+        const ElemOf<T> y = team_frobenius<T>(t, x, c0 ? c0 : 1);
+        const ElemOf<T> z = (c0 & 1) ? team_conj<T>(t, y) : y;
         x = c0 ? z : x;
     }
-    Fp2 tab[R][ND];
-    const Fp2 two = t6_cyc_sqr(t, x);
+    ElemOf<T> tab[R][ND];
+    const ElemOf<T> two = T::cyc_sqr(t, x);
     tab[0][0] = x;
     if (NAF) {
-        for (int i = 1; i < ND; i++) tab[0][i] = t6_mul(t, tab[0][i - 1], two);
+        for (int i = 1; i < ND; i++) tab[0][i] = T::mul(t, tab[0][i - 1], two);
     } else {
         tab[0][1] = two;
-        for (int i = 2; i < ND; i++) tab[0][i] = t6_mul(t, tab[0][i - 1], x);
+        for (int i = 2; i < ND; i++) tab[0][i] = T::mul(t, tab[0][i - 1], x);
     }
     for (int r = 1; r < R; r++)
         for (int i = 0; i < ND; i++) {
-            const Fp2 y = t6_frobenius(t, tab[0][i], r * L);
-            tab[r][i] = ((r * L) & 1) ? t6_conj(t, y) : y;
+            const ElemOf<T> y = team_frobenius<T>(t, tab[0][i], r * L);
+            tab[r][i] = ((r * L) & 1) ? team_conj<T>(t, y) : y;
         }
-    Fp2 acc = t6_one(t);
+    ElemOf<T> acc = team_one<T>(t);
     bool started = false;  // the same in all lanes
     for (int pos = TOP - 1; pos >= 0; pos--) {
         if (started)
-            for (int i = 0; i < RUN; i++) acc = t6_cyc_sqr(t, acc);
+            for (int i = 0; i < RUN; i++) acc = T::cyc_sqr(t, acc);
         for (int r = 0; r < R; r++) {
             const int d = rec[(c0 + r * L) * REC_DIGITS + pos];
             if (!__any_sync(0xffffffffu, d != 0)) continue;
             const int ad = d < 0 ? -d : d;
-            Fp2 m = t6_one(t);
+            ElemOf<T> m = team_one<T>(t);
             if (d) m = tab[r][NAF ? (ad >> 1) : (ad - 1)];
-            if (d < 0) m = t6_conj(t, m);
-            acc = started ? t6_mul(t, acc, m) : m;
+            if (d < 0) m = team_conj<T>(t, m);
+            acc = started ? T::mul(t, acc, m) : m;
             started = true;
         }
     }
@@ -110,38 +110,32 @@ __device__ __forceinline__ Fp2 t6_pow(const Team& t, Fp2 x, const int8_t* rec, i
 }
 
 // the product over a group of L neighbouring teams, valid in the first
-template <int L> __device__ __forceinline__ Fp2 t6_group_product(const Team& t, Fp2 x, int sub) {
+template <class T, int L> __device__ __forceinline__ ElemOf<T> team_group_product(const Team& t, ElemOf<T> x, int sub) {
     for (int w = 1; w < L; w *= 2) {
         __syncwarp();
-        team_st(t, T6_A, t.base + t.k, x);
+        T::st(t, T6_A, t.base + t.k, x);
         __syncwarp();
-        const Fp2 y = team_ld<Fp2>(t, T6_A, t.base + t.k + (sub % (2 * w) == 0 ? TEAM_LANES * w : 0));
-        x = t6_mul(t, x, y);
+        const ElemOf<T> y = T::ld(t, T6_A, t.base + t.k + (sub % (2 * w) == 0 ? 6 * w : 0));
+        x = T::mul(t, x, y);
     }
     return x;
 }
 
-template <int L> struct PerWarp { static constexpr int N = L == 1 ? TEAMS : 4; };
-
-// this lane's team in the launch, and whether it is one of the launch's
-// `per`-team warps' real teams (shadow lanes belong to the last one)
-template <int PER> __device__ __forceinline__ int64_t team_index() {
-    const int tm = (int)(threadIdx.x & 31) / TEAM_LANES;
-    return (int64_t)blockIdx.x * PER + (tm < PER ? tm : PER - 1);
-}
+// teams per warp where L of them share a power
+template <class T, int L> struct PerWarp { static constexpr int N = T::PER / L * L; };
 
 // The twiddle powers of a radix-4 stage (k_gt_radix4_outputs): power e of
 // butterfly j of block b, for j < J.  Teams take the blocks of all arrays
 // fastest over nbp >= nb = blocks * count slots, so that with nbp a multiple of
 // five a warp has one twiddle.
-template <int L, bool NAF>
+template <class T, int L, bool NAF>
 __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_pows(uint8_t* ex, const uint8_t* io, const int8_t* rec, int64_t n,
                                                          int64_t h, int64_t J, int64_t nb, int64_t nbp) {
     __shared__ uint4 sh[T6_ROWS * 32];
-    constexpr int PER = PerWarp<L>::N;
-    const Team t = team_init(sh, PER);
-    const int64_t g = team_index<PER>() / L;
-    const int sub = (int)(team_index<PER>() % L);
+    constexpr int PER = PerWarp<T, L>::N;
+    const Team t = team_of<T>(sh, PER);
+    const int64_t g = team_index<T>(PER) / L;
+    const int sub = (int)(team_index<T>(PER) % L);
     int64_t je = g / nbp, b = g % nbp;
     const bool active = je < 3 * J && b < nb;
     if (!active) je = 0, b = 0;
@@ -150,11 +144,11 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_pows(uint8_t* ex,
     int64_t idx = (e == 0 ? 2 * j : (e == 1 ? j : 3 * j)) * (n / (4 * h));
     const bool neg = idx >= n / 2;  // w^(k + n/2) = -w^k: the inverse
     if (neg) idx -= n / 2;
-    const Fp2 x = t6_load(t, io + GT_SZ * (q * n + blk * 4 * h + j + (int64_t)(e + 1) * h));
-    Fp2 r = t6_pow<L, NAF>(t, x, rec + REC_SZ * idx, sub);
-    if (L > 1) r = t6_group_product<L>(t, r, sub);
-    if (neg) r = t6_conj(t, r);
-    if (active && sub == 0) t6_store(t, ex + GT_SZ * (3 * (q * (n / 4) + blk * h + j) + e), r);
+    const ElemOf<T> x = team_load<T>(t, io + GT_SZ * (q * n + blk * 4 * h + j + (int64_t)(e + 1) * h));
+    ElemOf<T> r = team_pow<T, L, NAF>(t, x, rec + REC_SZ * idx, sub);
+    if (L > 1) r = team_group_product<T, L>(t, r, sub);
+    if (neg) r = team_conj<T>(t, r);
+    if (active && sub == 0) team_store<T>(t, ex + GT_SZ * (3 * (q * (n / 4) + blk * h + j) + e), r);
 }
 
 // x^(omega_4) under the decomposed action.  The forward domain's primitive
@@ -173,12 +167,13 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_pows(uint8_t* ex,
 // and the powers ex (null: all twiddles are one, the powers are src's own
 // values), into dst.  prefix: only outputs below `keep` of each array are
 // wanted, of butterflies j < J.
+template <class T>
 __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_outputs(uint8_t* dst, const uint8_t* src, const uint8_t* ex,
                                                             int64_t n, int64_t h, int64_t J, int64_t nb, int inverse,
                                                             int64_t keep) {
     __shared__ uint4 sh[T6_ROWS * 32];
-    const Team t = team_init(sh);
-    int64_t g = team_index<TEAMS>();
+    const Team t = team_of<T>(sh);
+    int64_t g = team_index<T>();
     const bool active = g < 2 * J * nb;
     if (!active) g = 2 * J * nb - 1;
     const int par = (int)(g & 1);
@@ -186,107 +181,119 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_outputs(uint8_t* 
     const int64_t at = q * n + blk * 4 * h + j;
     const uint8_t* powers = ex ? ex + GT_SZ * 3 * (q * (n / 4) + blk * h + j) : src + GT_SZ * (at + h);
     const size_t step = ex ? GT_SZ : GT_SZ * h;
-    const Fp2 a = t6_load(t, src + GT_SZ * at);
-    Fp2 t1 = t6_load(t, powers), e2 = t6_load(t, powers + 2 * step);
+    const ElemOf<T> a = team_load<T>(t, src + GT_SZ * at);
+    ElemOf<T> t1 = team_load<T>(t, powers), e2 = team_load<T>(t, powers + 2 * step);
     if (par) {
-        t1 = t6_conj(t, t1);
-        e2 = t6_conj(t, e2);
+        t1 = team_conj<T>(t, t1);
+        e2 = team_conj<T>(t, e2);
     }
-    Fp2 m = t6_mul(t, t6_load(t, powers + step), e2);
-    const Fp2 w = t6_frobenius(t, m, 3);
-    if (par) m = inverse ? w : t6_conj(t, w);
-    const Fp2 at1 = t6_mul(t, a, t1);
+    ElemOf<T> m = T::mul(t, team_load<T>(t, powers + step), e2);
+    const ElemOf<T> w = team_frobenius<T>(t, m, 3);
+    if (par) m = inverse ? w : team_conj<T>(t, w);
+    const ElemOf<T> at1 = T::mul(t, a, t1);
     const int64_t o0 = blk * 4 * h + j + par * h, o1 = o0 + 2 * h;
-    const Fp2 r0 = t6_mul(t, at1, m);
-    if (active && o0 < keep) t6_store(t, dst + GT_SZ * (q * n + o0), r0);
+    const ElemOf<T> r0 = T::mul(t, at1, m);
+    if (active && o0 < keep) team_store<T>(t, dst + GT_SZ * (q * n + o0), r0);
     if (!__any_sync(0xffffffffu, active && o1 < keep)) return;
-    const Fp2 r1 = t6_mul(t, at1, t6_conj(t, m));
-    if (active && o1 < keep) t6_store(t, dst + GT_SZ * (q * n + o1), r1);
+    const ElemOf<T> r1 = T::mul(t, at1, team_conj<T>(t, m));
+    if (active && o1 < keep) team_store<T>(t, dst + GT_SZ * (q * n + o1), r1);
 }
 
 // the first radix-2 stage (all twiddles one): u v and u / v of neighbours
+template <class T>
 __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix2_first(uint8_t* dst, const uint8_t* src, int64_t total) {
     __shared__ uint4 sh[T6_ROWS * 32];
-    const Team t = team_init(sh);
-    int64_t g = team_index<TEAMS>();
+    const Team t = team_of<T>(sh);
+    int64_t g = team_index<T>();
     const bool active = g < total;
     if (!active) g = total - 1;
     const uint8_t* pair = src + GT_SZ * (g & ~(int64_t)1);
-    Fp2 v = t6_load(t, pair + GT_SZ);
-    if (g & 1) v = t6_conj(t, v);
-    const Fp2 r = t6_mul(t, t6_load(t, pair), v);
-    if (active) t6_store(t, dst + GT_SZ * g, r);
+    ElemOf<T> v = team_load<T>(t, pair + GT_SZ);
+    if (g & 1) v = team_conj<T>(t, v);
+    const ElemOf<T> r = T::mul(t, team_load<T>(t, pair), v);
+    if (active) team_store<T>(t, dst + GT_SZ * g, r);
 }
 
 // out[q B + i] = base[(q B + i) stride]^(scalar i) for K arrays of B values
 // sharing the B exponents: teams take the arrays fastest over Kp >= K slots
-template <int L, bool NAF>
+template <class T, int L, bool NAF>
 __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_pow(uint8_t* out, const uint8_t* base, int64_t stride, const int8_t* rec,
                                                  int64_t B, int64_t K, int64_t Kp) {
     __shared__ uint4 sh[T6_ROWS * 32];
-    constexpr int PER = PerWarp<L>::N;
-    const Team t = team_init(sh, PER);
-    const int64_t g = team_index<PER>() / L;
-    const int sub = (int)(team_index<PER>() % L);
+    constexpr int PER = PerWarp<T, L>::N;
+    const Team t = team_of<T>(sh, PER);
+    const int64_t g = team_index<T>(PER) / L;
+    const int sub = (int)(team_index<T>(PER) % L);
     int64_t i = g / Kp, q = g % Kp;
     const bool active = i < B && q < K;
     if (!active) i = 0, q = 0;
-    const Fp2 x = t6_load(t, base + GT_SZ * stride * (q * B + i));
-    Fp2 r = t6_pow<L, NAF>(t, x, rec + REC_SZ * i, sub);
-    if (L > 1) r = t6_group_product<L>(t, r, sub);
-    if (active && sub == 0) t6_store(t, out + GT_SZ * (q * B + i), r);
+    const ElemOf<T> x = team_load<T>(t, base + GT_SZ * stride * (q * B + i));
+    ElemOf<T> r = team_pow<T, L, NAF>(t, x, rec + REC_SZ * i, sub);
+    if (L > 1) r = team_group_product<T, L>(t, r, sub);
+    if (active && sub == 0) team_store<T>(t, out + GT_SZ * (q * B + i), r);
 }
 
 // out[i] = base[i stride]^c_i for small signed c_i on cyclotomic values:
 // square-and-multiply over the bits of |c_i| with cyclotomic squarings, then
 // the inverse (conjugation) for negative c_i -- mul_cyclotomic_signed_small of
 // weighted_pfe/src/fft.rs:671-699.  c_i = 0 gives one.
+template <class T>
 __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_pow_small(uint8_t* out, const uint8_t* base, int64_t stride,
                                                        const int32_t* coeffs, int64_t n) {
     __shared__ uint4 sh[T6_ROWS * 32];
-    const Team t = team_init(sh);
-    int64_t i = team_index<TEAMS>();
+    const Team t = team_of<T>(sh);
+    int64_t i = team_index<T>();
     const bool active = i < n;
     if (!active) i = n - 1;
     const int32_t c = coeffs[i];
     const uint32_t mag = c < 0 ? (uint32_t)(-(int64_t)c) : (uint32_t)c;
-    const Fp2 x = t6_load(t, base + GT_SZ * stride * i);
+    const ElemOf<T> x = team_load<T>(t, base + GT_SZ * stride * i);
     const uint32_t all = __reduce_or_sync(0xffffffffu, mag);
-    Fp2 acc = t6_one(t);
+    ElemOf<T> acc = team_one<T>(t);
     for (int b = 31 - __clz(all | 1); b >= 0; b--) {
-        acc = t6_cyc_sqr(t, acc);
+        acc = T::cyc_sqr(t, acc);
         if (!__any_sync(0xffffffffu, (mag >> b) & 1)) continue;
-        acc = t6_mul(t, acc, ((mag >> b) & 1) ? x : t6_one(t));
+        acc = T::mul(t, acc, ((mag >> b) & 1) ? x : team_one<T>(t));
     }
-    if (c < 0) acc = t6_conj(t, acc);
-    if (active) t6_store(t, out + GT_SZ * i, acc);
+    if (c < 0) acc = team_conj<T>(t, acc);
+    if (active) team_store<T>(t, out + GT_SZ * i, acc);
 }
 
-// Teams per exponentiation for E of them, from a cost model: the wide
-// multiply-adds of one lane, in thousands (64 squarings of 888; products of
-// 1,608: 52 and three for the table with the warp-uniform NAF, 17 a digit and
-// seven for the table in radix 16; table images of 744).  WBTE_GT_LANES = 1, 2 or 4 overrides it, and so does the
-// calling context's tuning knob.
-int gt_pow_teams(int64_t E, bool uniform) {
+// How the powers of a launch of E are spread: over teams of six or twelve lanes,
+// L teams each.
+struct PowSpread { bool twelve; int L; };
+// From a cost model: the wide multiply-adds of one lane, in thousands.  Teams
+// of six: 64 squarings of 888; products of 1,608, 52 and three for the table with
+// the warp-uniform NAF, 17 a digit and seven for the table in radix 16; table
+// images of 744.  Teams of twelve: 444, 1,020 and 444; they win up to about 800
+// powers (transform of 1,024 values with 768 powers a stage 2.81 -> 2.70 ms, of
+// 256 with 192 a stage 1.60 -> 1.38 ms).  WBTE_GT_LANES = 1, 2 or 4
+// forces that many teams of six, and so does the calling context's tuning knob.
+PowSpread gt_pow_spread(int64_t E, bool uniform) {
     if (const char* env = getenv("WBTE_GT_LANES")) {
         const int v = atoi(env);
-        if (v == 1 || v == 2 || v == 4) return v;
+        if (v == 1 || v == 2 || v == 4) return {false, v};
     }
-    if (g_tune.gt_lanes == 1 || g_tune.gt_lanes == 2 || g_tune.gt_lanes == 4) return g_tune.gt_lanes;
-    const double work[3] = {uniform ? 156.0 : 195.0, 130.0, 98.0};
-    const int per[3] = {TEAMS, 4, 4};
-    int best = 1;
+    if (g_tune.gt_lanes == 1 || g_tune.gt_lanes == 2 || g_tune.gt_lanes == 4) return {false, g_tune.gt_lanes};
+    struct Way { PowSpread spread; double work, per; };
+    const Way ways[] = {{{false, 1}, uniform ? 156.0 : 195.0, 5.0}, {{false, 2}, 130.0, 2.0}, {{false, 4}, 98.0, 1.0},
+                        {{true, 1}, 115.0, 2.0},                    {{true, 2}, 74.0, 1.0}};
+    const Way* best = ways;
     double best_t = 0;
-    for (int i = 0, L = 1; L <= 4; i++, L *= 2) {
-        const double time = launch_time(work[i], (double)(E * L) / per[i]);
-        if (L == 1 || time < best_t) best = L, best_t = time;
+    for (const Way& w : ways) {
+        const double t = launch_time(w.work, (double)E / w.per);
+        if (&w == ways || t < best_t) best = &w, best_t = t;
     }
-    return best;
+    return best->spread;
 }
+
+// Launches of single products take teams of twelve while two to a warp leave no
+// scheduler more than one warp's work.
+bool few_values(int64_t n) { return n <= 2 * (int64_t)schedulers(); }
 
 int64_t pad5(int64_t x) { return (x + TEAMS - 1) / TEAMS * TEAMS; }
 // One exponent for every five neighbouring teams: worth idle teams up to the
-// difference between the recodings (156 against 195 of gt_pow_teams).
+// difference between the recodings (156 against 195 of gt_pow_spread).
 bool uniform_pays(int64_t same) { return same >= TEAMS && 5 * same >= 4 * pad5(same); }
 
 // rec <- the recodings of n scalars; null if there is no memory
@@ -301,20 +308,24 @@ int8_t* recode(const uint8_t* scalars, int64_t n, bool naf, cudaStream_t s) {
 void gt_pow_run(uint8_t* out, const uint8_t* base, int64_t stride, const uint8_t* scalars, int64_t B, int64_t K,
                 cudaStream_t s) {
     const bool uniform = uniform_pays(K);
-    const int L = gt_pow_teams(B * K, uniform);
-    const bool naf = L == 1 && uniform;
+    const PowSpread how = gt_pow_spread(B * K, uniform);
+    const bool naf = !how.twelve && how.L == 1 && uniform;
     int8_t* rec = recode(scalars, B, naf, s);
     if (!rec) return;
-    const int64_t Kp = naf ? pad5(K) : K;
+    const int64_t Kp = naf ? pad5(K) : K, items = B * Kp;
     note_launch();
     if (naf)
-        k_gt_pow<1, true><<<blocks_for(B * Kp, TEAMS), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
-    else if (L == 1)
-        k_gt_pow<1, false><<<blocks_for(B * Kp, TEAMS), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
-    else if (L == 2)
-        k_gt_pow<2, false><<<blocks_for(B * Kp * 2, 4), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+        k_gt_pow<Six, 1, true><<<blocks_for(items, 5), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+    else if (how.twelve && how.L == 1)
+        k_gt_pow<Twelve, 1, false><<<blocks_for(items, 2), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+    else if (how.twelve)
+        k_gt_pow<Twelve, 2, false><<<blocks_for(items, 1), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+    else if (how.L == 1)
+        k_gt_pow<Six, 1, false><<<blocks_for(items, 5), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+    else if (how.L == 2)
+        k_gt_pow<Six, 2, false><<<blocks_for(items, 2), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
     else
-        k_gt_pow<4, false><<<blocks_for(B * Kp * 4, 4), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+        k_gt_pow<Six, 4, false><<<blocks_for(items, 1), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
     cudaFreeAsync(rec, s);
 }
 
@@ -338,7 +349,10 @@ void launch_gt_pow_small(uint8_t* out, const uint8_t* base, int64_t stride, cons
     ProfScope prof_("gt_pow_small", s);
     if (n <= 0) return;
     note_launch();
-    k_gt_pow_small<<<blocks_for(n, TEAMS), WARP, 0, s>>>(out, base, stride, coeffs, n);
+    if (few_values(n))
+        k_gt_pow_small<Twelve><<<blocks_for(n, Twelve::PER), WARP, 0, s>>>(out, base, stride, coeffs, n);
+    else
+        k_gt_pow_small<Six><<<blocks_for(n, Six::PER), WARP, 0, s>>>(out, base, stride, coeffs, n);
 }
 
 // The unscaled transform of `count` arrays of n values, keeping the first
@@ -362,7 +376,10 @@ static void gt_transform(uint8_t* io, const uint8_t* tw, int64_t n, int64_t keep
     if (ok && (bits & 1)) {
         // an odd number of stages starts with one radix-2 stage, the rest pair up
         note_launch();
-        k_gt_radix2_first<<<blocks_for(n * count, TEAMS), WARP, 0, s>>>(other, cur, n * count);
+        if (few_values(n * count))
+            k_gt_radix2_first<Twelve><<<blocks_for(n * count, Twelve::PER), WARP, 0, s>>>(other, cur, n * count);
+        else
+            k_gt_radix2_first<Six><<<blocks_for(n * count, Six::PER), WARP, 0, s>>>(other, cur, n * count);
         std::swap(cur, other);
         half = 2;
     }
@@ -373,8 +390,8 @@ static void gt_transform(uint8_t* io, const uint8_t* tw, int64_t n, int64_t keep
         const int64_t J = last ? std::min(half, keep) : half;
         if (half > 1) {
             const bool uniform = uniform_pays(nb);
-            const int L = gt_pow_teams(3 * J * nb, uniform);
-            const bool use_naf = L == 1 && uniform;
+            const PowSpread how = gt_pow_spread(3 * J * nb, uniform);
+            const bool use_naf = !how.twelve && how.L == 1 && uniform;
             int8_t*& rec = use_naf ? naf : r16;
             if (!rec) rec = recode(tw, n / 2, use_naf, s);
             if (!rec || (!ex && cudaMallocAsync(&ex, GT_SZ * 3 * (size_t)(n / 4 * count), s) != cudaSuccess)) {
@@ -384,17 +401,26 @@ static void gt_transform(uint8_t* io, const uint8_t* tw, int64_t n, int64_t keep
             const int64_t nbp = use_naf ? pad5(nb) : nb, items = 3 * J * nbp;
             note_launch();
             if (use_naf)
-                k_gt_radix4_pows<1, true><<<blocks_for(items, TEAMS), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
-            else if (L == 1)
-                k_gt_radix4_pows<1, false><<<blocks_for(items, TEAMS), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
-            else if (L == 2)
-                k_gt_radix4_pows<2, false><<<blocks_for(2 * items, 4), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+                k_gt_radix4_pows<Six, 1, true><<<blocks_for(items, 5), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+            else if (how.twelve && how.L == 1)
+                k_gt_radix4_pows<Twelve, 1, false><<<blocks_for(items, 2), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+            else if (how.twelve)
+                k_gt_radix4_pows<Twelve, 2, false><<<blocks_for(items, 1), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+            else if (how.L == 1)
+                k_gt_radix4_pows<Six, 1, false><<<blocks_for(items, 5), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+            else if (how.L == 2)
+                k_gt_radix4_pows<Six, 2, false><<<blocks_for(items, 2), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
             else
-                k_gt_radix4_pows<4, false><<<blocks_for(4 * items, 4), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+                k_gt_radix4_pows<Six, 4, false><<<blocks_for(items, 1), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
         }
         note_launch();
-        k_gt_radix4_outputs<<<blocks_for(2 * J * nb, TEAMS), WARP, 0, s>>>(other, cur, half > 1 ? ex : nullptr, n, half,
-                                                                           J, nb, inverse ? 1 : 0, last ? keep : n);
+        const uint8_t* powers = half > 1 ? ex : nullptr;
+        if (few_values(2 * J * nb))
+            k_gt_radix4_outputs<Twelve><<<blocks_for(2 * J * nb, Twelve::PER), WARP, 0, s>>>(
+                other, cur, powers, n, half, J, nb, inverse ? 1 : 0, last ? keep : n);
+        else
+            k_gt_radix4_outputs<Six><<<blocks_for(2 * J * nb, Six::PER), WARP, 0, s>>>(other, cur, powers, n, half, J, nb,
+                                                                                  inverse ? 1 : 0, last ? keep : n);
         std::swap(cur, other);
     }
     if (ok) {

@@ -1,5 +1,6 @@
 // Fp12 arithmetic with one element spread over a team of six lanes: lane k
-// holds the Fp2 coefficient of w^k (w^6 = xi = 1 + u), five teams per warp.
+// holds the Fp2 coefficient of w^k (w^6 = xi = 1 + u), five teams per warp.  Calls
+// of few values take teams of twelve (below).
 //
 // What bounds it: the wide multiply-add pipe (a 32 x 32 + 64-bit multiply-add
 // every four cycles per scheduler).  One thread per element needs 288 words
@@ -30,12 +31,11 @@
 // are reduced are bounded integers (bounds at each use), shifted to be
 // non-negative by a multiple of p 2^384 before the reduction.
 #pragma once
-#include "pairing.cuh"
+#include "quad.cuh"
 
 namespace wbte {
 
-constexpr int TEAM_LANES = 6;
-constexpr int TEAMS = 5;  // per warp
+constexpr int TEAMS = 5;  // of six lanes per warp
 // Resident one-warp blocks per SM that the team kernels are compiled for: the
 // registers of eight warps, two per scheduler.  Ten and twelve (168 registers)
 // measured 45.9 -> 56 and 57 ms for the GT transform of 64 batches of 512 and
@@ -53,20 +53,23 @@ struct Wide2 { Wide c0, c1; };
 struct Team {
     uint4* sh;  // this warp's rows
     int k;      // this lane's power of w
-    int base;   // slot of the team's lane 0
+    int h;      // this lane's component of the coefficient (teams of twelve)
+    int base;   // slot of the team's coefficient 0
 };
 
 WBTE_INL int nib(uint32_t packed, int k) { return (int)((packed >> (4 * k)) & 15u); }
 
-// `per` teams per warp (4 or 5); lanes past them shadow the last team's
-WBTE_INL Team team_init(uint4* sh, int per = TEAMS) {
+// `per` teams per warp of `lanes` lanes (a multiple of six: one lane or two
+// neighbours per coefficient); lanes past them shadow the last team's
+WBTE_INL Team team_init(uint4* sh, int lanes, int per) {
     const int lane = threadIdx.x & 31;
-    const int used = TEAM_LANES * per;
-    const int l = lane < used ? lane : used - TEAM_LANES + (lane - used) % TEAM_LANES;
+    const int used = lanes * per, each = lanes / 6;
+    const int l = lane < used ? lane : used - lanes + (lane - used) % lanes;
     Team t;
     t.sh = sh;
-    t.k = l % TEAM_LANES;
-    t.base = l - t.k;
+    t.k = l % lanes / each;
+    t.h = l % each;
+    t.base = 6 * (l / lanes);
     for (int r = lane; r < T6_ROWS; r += 32) sh[r * 32 + T6_ZERO] = make_uint4(0, 0, 0, 0);
     __syncwarp();
     return t;
@@ -344,177 +347,404 @@ static __device__ __noinline__ Fp2 t6_mul_line(Team t, Fp2 f, Fp line_component)
     return w2_reduce_11(acc);
 }
 
-WBTE_INL Fp2 t6_one(const Team& t) {
-    Fp2 r = fp2_zero();
-    if (t.k == 0) r.c0 = fp_one();
+// ------------------------------------------------------------- teams of twelve
+// Two lanes per coefficient, one Fp component each: for calls of so few values
+// that a team's own chain is all that counts.  An Fp2 product is two 12 x
+// 12-word products on each lane, without Karatsuba (c0 = a0 b0 - a1 b1, c1 = a0
+// b1 + a1 b0): 1,020 wide multiply-adds per lane and Fp12 product against 1,608,
+// 444 per cyclotomic squaring against 888, at two teams per warp instead of
+// five: slower once every scheduler has its warps.  Measured on B200, 100 values
+// (six lanes, twelve): final exponentiations 1.49 and 0.92 ms, Miller loops of
+// computed lines 1.76 and 1.04 ms, of prepared ones 0.89 and 0.63 ms; 500
+// products of three pairings 3.6 and 2.65 ms with the call.
+WBTE_INL Wide w_add_signed(const Wide& a, const Wide& b, bool minus) {
+    const uint32_t m[1] = {minus ? 0xffffffffu : 0u};
+    Wide r;
+    wide_add_signed(r.v, a.v, b.v, m);
     return r;
 }
-WBTE_INL Fp2 t6_conj(const Team& t, const Fp2& a) {
-    const Fp2 n = fp2_neg(a);
+WBTE_INL Wide w_partner(const Wide& a) {
+    Wide r;
+    _Pragma("unroll") for (int i = 0; i < 24; i++) r.v[i] = __shfl_xor_sync(FULL, a.v[i], 1);
+    return r;
+}
+// this lane's component of u v
+WBTE_INL Wide t12_wide(const Team& t, const Fp2& u, const Fp2& v) {
+    const Wide x = fp_wide_inl(u.c0, fp_select(t.h, v.c1, v.c0)), y = fp_wide_inl(u.c1, fp_select(t.h, v.c0, v.c1));
+    return w_add_signed(x, y, !t.h);
+}
+WBTE_INL Fp t12_reduce(const Team& t, Wide s, bool two) {
+    fp_add_p(s.v + 12, s.v + 12);
+    if (two) {  // the first component's sums reach -16 p^2
+        Fp hi, more;
+        _Pragma("unroll") for (int i = 0; i < 12; i++) hi.v[i] = s.v[12 + i];
+        fp_add_p(more.v, hi.v);
+        _Pragma("unroll") for (int i = 0; i < 12; i++) s.v[12 + i] = t.h ? hi.v[i] : more.v[i];
+    }
+    return wide_reduce(s);
+}
+WBTE_INL Wide t12_comb(const Team& t, const T6Comb& c) {
+    const int row = c.row + 6 * t.h;
+    Wide G = w_sub(w_sub(team_ld<Wide>(t, row, c.g0), team_ld<Wide>(t, row, c.g1)), team_ld<Wide>(t, row, c.g2));
+    Wide M = team_ld<Wide>(t, row, c.m);
+    _Pragma("unroll") for (int i = 0; i < 24; i++) M.v[i] = c.gm ? G.v[i] : M.v[i];
+    G = w_add(G, team_ld<Wide>(t, row, c.h));
+    return w_add_signed(G, w_partner(M), !t.h);
+}
+static __device__ __noinline__ Fp t12_mul(Team t, Fp a, Fp b) {
+    const int own = t.base + t.k;
+    const bool odd = t.k & 1;
+    __syncwarp();
+    team_st(t, T6_A + 3 * t.h, own, a);
+    team_st(t, T6_B + 3 * t.h, own, b);
+    __syncwarp();
+    const int s0 = t6_term0(t), s1 = t6_term1(t);
+    const Fp2 u = t6_pair(t, T6_A, s0, s1), v = t6_pair(t, T6_B, s0, s1);
+    const Fp2 u1 = t6_pair(t, T6_A, t6_odd(s0), t6_odd(s1)), v1 = t6_pair(t, T6_B, t6_odd(s0), t6_odd(s1));
+    __syncwarp();
+    const Wide x = t12_wide(t, u, v);
+    team_st(t, T6_X + 6 * t.h, own, x);
+    const Wide y = t12_wide(t, u1, v1);
+    team_st(t, T6_Y + 6 * t.h, own, y);
+    const Wide z = t12_wide(t, fp2_add_lazy(u, u1), fp2_add_lazy(v, v1));
+    team_st(t, T6_Z + 6 * t.h, own, w_sub(w_sub(z, x), y));
+    __syncwarp();
+    T6Comb c = t6_comb_of(t, odd ? T6_Y : T6_X);
+    const Wide e = t12_comb(t, c);
+    __syncwarp();
+    team_st(t, T6_X + 6 * t.h, own, e);
+    __syncwarp();
+    if (odd) {
+        c.row = T6_Z;
+    } else {
+        c.row = T6_X;
+        c.g0 = t6_vslot(t);
+        c.g1 = c.g2 = c.m = T6_ZERO;
+        c.h = own;
+    }
+    return t12_reduce(t, t12_comb(t, c), true);
+}
+WBTE_INL Fp t12_xi(const Team& t, const Fp& a) {
+    const Fp o = fp_shfl_xor(a, 1);
+    return fp_select(t.h, fp_add(a, o), fp_sub(a, o));
+}
+static __device__ __noinline__ Fp t12_sqr(Team t, Fp a) {
+    const int own = t.base + t.k;
+    const bool odd = t.k & 1;
+    const Fp xa = t12_xi(t, a);
+    __syncwarp();
+    team_st(t, T6_A + 3 * t.h, own, a);
+    if (odd) team_st(t, T6_B + 3 * t.h, t.base + 2 * (t.k == 5 ? 0 : (t.k >> 1) + 1) + 1, t.k == 5 ? xa : a);
+    __syncwarp();
+    const int s0 = t6_term0(t), s1 = t6_term1(t);
+    const Fp2 u0 = t6_pair(t, T6_A, s0, s1), u1 = t6_pair(t, T6_A, t6_odd(s0), t6_odd(s1));
+    const Fp2 v1 = t6_pair(t, T6_B, t6_odd(s0), t6_odd(s1));
+    __syncwarp();
+    const Wide x = t12_wide(t, u0, u1);
+    team_st(t, T6_X + 6 * t.h, own, x);
+    team_st(t, T6_Y + 6 * t.h, own, w_sub(t12_wide(t, fp2_add_lazy(u0, u1), fp2_add_lazy(u0, v1)), x));
+    __syncwarp();
+    T6Comb c = t6_comb_of(t, odd ? T6_X : T6_Y);
+    team_st(t, T6_Z + 6 * t.h, own, t12_comb(t, c));
+    __syncwarp();
+    c.row = T6_Z;
+    c.g0 = odd ? own : T6_ZERO;
+    c.g1 = odd ? T6_ZERO : t6_vslot(t);
+    c.g2 = c.m = T6_ZERO;
+    c.h = own;
+    c.gm = c.gm && !odd;
+    return t12_reduce(t, t12_comb(t, c), true);
+}
+// the four products of t6_cyc_sqr, A and D on the first lane, B and C on the
+// second; even coefficients exchange C and D
+static __device__ __noinline__ Fp t12_cyc_sqr(Team t, Fp z) {
+    constexpr int C0 = 0, C1 = 3, NEG = 6, XI0 = 9, XI1 = 12, UNUSED = 15;
+    const bool even = !(t.k & 1), h = t.h;
+    const int own = t.base + t.k;
+    const Fp o = fp_shfl_xor(z, 1);
+    const Fp n = fp_minus(h ? z : o);  // p - c1
+    __syncwarp();
+    team_st(t, h ? C1 : C0, own, z);
+    team_st(t, h ? NEG : XI0, own, h ? n : fp_add_lazy(z, n));
+    team_st(t, h ? XI1 : UNUSED, own, fp_add_lazy(z, o));
+    __syncwarp();
+    const int pa = t.base + nib(0x120120u, t.k), pb = pa + 3;
+    const int a0r = t.k == 1 ? XI0 : C0, a1r = t.k == 1 ? XI1 : C1;
+    const Fp a0 = team_ld<Fp>(t, a0r, pa);
+    const Fp d = team_ld<Fp>(t, even ? C0 : a1r, even ? pb : pa);  // b0 or a1
+    // A = (a0 + a1 or a0)(a0 or b0, less a1 or not) and B = 2a0 (a1 or b1)
+    const Wide x = fp_wide_inl(fp_add_lazy(a0, team_ld<Fp>(t, even && !h ? C1 : a0r, pa)),
+                               fp_add_lazy(team_ld<Fp>(t, h ? C1 : C0, even ? pa : pb),
+                                           team_ld<Fp>(t, NEG, even && !h ? pa : T6_ZERO)));
+    // D = 2d b1 and C = (d + b1 or a1)(b0, less b1 or not)
+    const Wide y = fp_wide_inl(fp_add_lazy(d, team_ld<Fp>(t, even ? (h ? C1 : C0) : a1r, even ? pb : pa)),
+                               fp_add_lazy(team_ld<Fp>(t, h ? C0 : C1, pb),
+                                           team_ld<Fp>(t, NEG, even && h ? pb : T6_ZERO)));
+    Wide w = w_partner(y);
+    const uint32_t mask = even ? 0xffffffffu : 0u;
+    _Pragma("unroll") for (int i = 0; i < 24; i++) w.v[i] &= mask;
+    w = w_add_signed(w_add(x, w), y, !h);
+    fp_add_p(w.v + 12, w.v + 12);
+    Fp q;
+    fp_redc(q.v, w.v);
+    fp_csub_2p(q.v, q.v);
+    const Fp m = fp_select(even, fp_minus(z), z);
+    q = fp_add_lazy(fp_add_lazy(q, q), fp_add_lazy(q, fp_add_lazy(m, m)));
+    fp_csub_4p(q.v, q.v);
+    fp_csub_2p(q.v, q.v);
+    fp_csub_p(q.v, q.v);
+    return q;
+}
+static __device__ __noinline__ Fp t12_mul_line(Team t, Fp f, int component, Fp line_component) {
+    const int own = t.base + t.k;
+    const Fp xf = t12_xi(t, f);
+    __syncwarp();
+    team_st(t, T6_A + 3 * t.h, own, f);
+    team_st(t, T6_B + 3 * t.h, own, xf);
+    team_st(t, T6_Y, t.base + component, line_component);
+    __syncwarp();
+    const int k2 = t.k < 2 ? t.k + 4 : t.k - 2, k3 = t.k < 3 ? t.k + 3 : t.k - 3;
+    Wide acc = t12_wide(t, team_ld<Fp2>(t, T6_A, own), team_ld_line(t, T6_Y, 0));
+    acc = w_add(acc, t12_wide(t, team_ld<Fp2>(t, t.k < 2 ? T6_B : T6_A, t.base + k2), team_ld_line(t, T6_Y, 1)));
+    acc = w_add(acc, t12_wide(t, team_ld<Fp2>(t, t.k < 3 ? T6_B : T6_A, t.base + k3), team_ld_line(t, T6_Y, 2)));
+    return t12_reduce(t, acc, false);
+}
+
+// --------------------------------------------------- what both kinds of team do
+// E: what a lane holds of an Fp12 value's coefficient, and so of any Fp2 value
+// that the team computes with.
+struct Six {
+    using E = Fp2;
+    static constexpr int LANES = 6, PER = TEAMS;
+    static WBTE_INL E mul(const Team& t, const E& a, const E& b) { return t6_mul(t, a, b); }
+    static WBTE_INL E sqr(const Team& t, const E& a) { return t6_sqr(t, a); }
+    static WBTE_INL E cyc_sqr(const Team& t, const E& a) { return t6_cyc_sqr(t, a); }
+    static WBTE_INL E mul_line(const Team& t, const E& f, const Fp& c) { return t6_mul_line(t, f, c); }
+    // the record component that this lane brings of a line
+    static WBTE_INL int line_index(const Team& t) { return t.k; }
+    static WBTE_INL Fp component(const E& a, int c) { return c ? a.c1 : a.c0; }
+    static WBTE_INL E of(const Team&, const Fp2& a) { return a; }
+    static WBTE_INL E load(const Team&, const uint8_t* v) { return load_vec(reinterpret_cast<const Fp2*>(v)); }
+    static WBTE_INL void store(const Team&, uint8_t* v, const E& a) { store_vec(reinterpret_cast<Fp2*>(v), a); }
+    static WBTE_INL E ld(const Team& t, int row, int slot) { return team_ld<Fp2>(t, row, slot); }
+    static WBTE_INL void st(const Team& t, int row, int slot, const E& a) { team_st(t, row, slot, a); }
+    static WBTE_INL E f_add(const E& a, const E& b) { return fp2_add(a, b); }
+    static WBTE_INL E f_sub(const E& a, const E& b) { return fp2_sub(a, b); }
+    static WBTE_INL E f_neg(const E& a) { return fp2_neg(a); }
+    static WBTE_INL E f_xi(const Team&, const E& a) { return fp2_mul_xi(a); }
+    static WBTE_INL E f_conj(const Team&, const E& a) { return fp2_conj(a); }
+    static WBTE_INL E f_mul(const E& a, const E& b) { return t6_fp2_mul(a, b); }
+};
+struct Twelve {
+    using E = Fp;
+    static constexpr int LANES = 12, PER = 2;
+    static WBTE_INL E mul(const Team& t, const E& a, const E& b) { return t12_mul(t, a, b); }
+    static WBTE_INL E sqr(const Team& t, const E& a) { return t12_sqr(t, a); }
+    static WBTE_INL E cyc_sqr(const Team& t, const E& a) { return t12_cyc_sqr(t, a); }
+    static WBTE_INL E mul_line(const Team& t, const E& f, const Fp& c) { return t12_mul_line(t, f, line_index(t), c); }
+    static WBTE_INL int line_index(const Team& t) { return 2 * (t.k % 3) + t.h; }
+    static WBTE_INL Fp component(const E& a, int) { return a; }
+    static WBTE_INL E of(const Team& t, const Fp2& a) { return fp_select(t.h, a.c1, a.c0); }
+    static WBTE_INL E load(const Team& t, const uint8_t* v) { return load_vec(reinterpret_cast<const Fp*>(v) + t.h); }
+    static WBTE_INL void store(const Team& t, uint8_t* v, const E& a) { store_vec(reinterpret_cast<Fp*>(v) + t.h, a); }
+    static WBTE_INL E ld(const Team& t, int row, int slot) { return team_ld<Fp>(t, row + 3 * t.h, slot); }
+    static WBTE_INL void st(const Team& t, int row, int slot, const E& a) { team_st(t, row + 3 * t.h, slot, a); }
+    static WBTE_INL E f_add(const E& a, const E& b) { return fp_add(a, b); }
+    static WBTE_INL E f_sub(const E& a, const E& b) { return fp_sub(a, b); }
+    static WBTE_INL E f_neg(const E& a) { return fp_neg(a); }
+    static WBTE_INL E f_xi(const Team& t, const E& a) { return t12_xi(t, a); }
+    static WBTE_INL E f_conj(const Team& t, const E& a) { return fp_select(t.h, fp_neg(a), a); }
+    static WBTE_INL E f_mul(const E& a, const E& b) { return OnPair::mul(a, b); }
+};
+template <class T> using ElemOf = typename T::E;
+template <class T> WBTE_INL ElemOf<T> team_dbl(const ElemOf<T>& a) { return T::f_add(a, a); }
+template <class T> WBTE_INL ElemOf<T> team_mul3(const ElemOf<T>& a) { return T::f_add(T::f_add(a, a), a); }
+template <class T> WBTE_INL ElemOf<T> team_mul4(const ElemOf<T>& a) { return team_dbl<T>(team_dbl<T>(a)); }
+
+template <class T> WBTE_INL Team team_of(uint4* sh, int per = T::PER) { return team_init(sh, T::LANES, per); }
+// this lane's team in the launch (shadow lanes belong to the warp's last one);
+// kernels have teams past the end take the last value again without storing it,
+// which is their own warp's, so that a call may work in place
+template <class T> __device__ __forceinline__ int64_t team_index(int per = T::PER) {
+    const int tm = (int)(threadIdx.x & 31) / T::LANES;
+    return (int64_t)blockIdx.x * per + (tm < per ? tm : per - 1);
+}
+
+template <class T> WBTE_INL ElemOf<T> team_one(const Team& t) {
+    Fp2 r = fp2_zero();
+    if (t.k == 0) r.c0 = fp_one();
+    return T::of(t, r);
+}
+template <class T> WBTE_INL ElemOf<T> team_conj(const Team& t, const ElemOf<T>& a) {
+    const ElemOf<T> n = T::f_neg(a);
     return (t.k & 1) ? n : a;
 }
 // x^(p^pw), pw in 1..3
-static __device__ __noinline__ Fp2 t6_frobenius(Team t, Fp2 a, int pw) {
-    if (pw & 1) a.c1 = fp_neg(a.c1);
-    const Fp2 c = fp2_from_const(C_FROB[pw - 1][t.k]);
-    return t6_fp2_mul(a, c);
+template <class T> static __device__ __noinline__ ElemOf<T> team_frobenius(Team t, ElemOf<T> a, int pw) {
+    const ElemOf<T> c = T::f_conj(t, a);
+    a = (pw & 1) ? c : a;
+    return T::f_mul(a, T::of(t, fp2_from_const(C_FROB[pw - 1][t.k])));
 }
 
-// lane k's coefficient in blst's Fp12 layout (c0.c0, c0.c1, c0.c2, c1.c0, ..)
-WBTE_INL size_t t6_offset(const Team& t) { return 96 * (size_t)((t.k & 1) * 3 + (t.k >> 1)); }
-WBTE_INL Fp2 t6_load(const Team& t, const uint8_t* gt) {
-    return load_vec(reinterpret_cast<const Fp2*>(gt + t6_offset(t)));
-}
-WBTE_INL void t6_store(const Team& t, uint8_t* gt, const Fp2& a) {
-    store_vec(reinterpret_cast<Fp2*>(gt + t6_offset(t)), a);
+// coefficient k in blst's Fp12 layout (c0.c0, c0.c1, c0.c2, c1.c0, ..)
+WBTE_INL size_t team_offset(const Team& t) { return 96 * (size_t)((t.k & 1) * 3 + (t.k >> 1)); }
+template <class T> WBTE_INL ElemOf<T> team_load(const Team& t, const uint8_t* gt) { return T::load(t, gt + team_offset(t)); }
+template <class T> WBTE_INL void team_store(const Team& t, uint8_t* gt, const ElemOf<T>& a) {
+    T::store(t, gt + team_offset(t), a);
 }
 
 // ------------------------------------------------------ final exponentiation
-// 1/d for the Fp2 value that lane 0 of the team holds, on every lane
-WBTE_INL Fp2 t6_inverse_of_lane0(const Team& t, const Fp2& a) {
+// 1/d for the Fp2 value d that is coefficient 0
+template <class T> WBTE_INL ElemOf<T> team_inverse_of_first(const Team& t, const ElemOf<T>& a) {
     __syncwarp();
-    team_st(t, T6_A, t.base + t.k, a);
+    T::st(t, T6_A, t.base + t.k, a);
     __syncwarp();
-    return fp2_inv(team_ld<Fp2>(t, T6_A, t.base));
+    return T::of(t, fp2_inv(team_ld<Fp2>(t, T6_A, t.base)));
 }
 // f^((p^6 - 1)(p^2 + 1)) = (conj(f)^2 / (f conj(f)))^(p^2 + 1).  N = f conj(f)
 // lies in Fp6, and 1/N = N^(p^2) N^(p^4) / (N N^(p^2) N^(p^4)), whose
-// denominator lies in Fp2 (lane 0).  f = 0 gives 0.
-static __device__ __noinline__ Fp2 t6_final_exp_easy(Team t, Fp2 f) {
-    const Fp2 g = t6_conj(t, f);
-    const Fp2 n = t6_mul(t, f, g);
-    const Fp2 n2 = t6_frobenius(t, n, 2);
-    const Fp2 m = t6_mul(t, n2, t6_frobenius(t, n2, 2));
-    const Fp2 d = t6_inverse_of_lane0(t, t6_mul(t, n, m));
-    Fp2 r = t6_mul(t, t6_mul(t, g, g), t6_fp2_mul(m, d));
-    return t6_mul(t, r, t6_frobenius(t, r, 2));
+// denominator lies in Fp2.  f = 0 gives 0.
+template <class T> static __device__ __noinline__ ElemOf<T> team_final_exp_easy(Team t, ElemOf<T> f) {
+    const ElemOf<T> g = team_conj<T>(t, f);
+    const ElemOf<T> n = T::mul(t, f, g);
+    const ElemOf<T> n2 = team_frobenius<T>(t, n, 2);
+    const ElemOf<T> m = T::mul(t, n2, team_frobenius<T>(t, n2, 2));
+    const ElemOf<T> d = team_inverse_of_first<T>(t, T::mul(t, n, m));
+    const ElemOf<T> r = T::mul(t, T::mul(t, g, g), T::f_mul(m, d));
+    return T::mul(t, r, team_frobenius<T>(t, r, 2));
 }
 // x^(|z|/2) conjugated: squaring runs between the set bits of |z|
-static __device__ __noinline__ Fp2 t6_raise_to_z_div_by_2(Team t, Fp2 x) {
-    Fp2 acc = t6_cyc_sqr(t, x);
+template <class T> static __device__ __noinline__ ElemOf<T> team_raise_to_z_div_by_2(Team t, ElemOf<T> x) {
+    ElemOf<T> acc = T::cyc_sqr(t, x);
     const uint64_t runs = 2ull | (3ull << 8) | (9ull << 16) | (32ull << 24) | (15ull << 32);
     for (int r = 0; r < 5; r++) {
-        acc = t6_mul(t, acc, x);
-        for (int i = (int)((runs >> (8 * r)) & 255u); i > 0; i--) acc = t6_cyc_sqr(t, acc);
+        acc = T::mul(t, acc, x);
+        for (int i = (int)((runs >> (8 * r)) & 255u); i > 0; i--) acc = T::cyc_sqr(t, acc);
     }
-    return t6_conj(t, acc);
+    return team_conj<T>(t, acc);
 }
-WBTE_INL Fp2 t6_raise_to_z(const Team& t, const Fp2& x) { return t6_cyc_sqr(t, t6_raise_to_z_div_by_2(t, x)); }
-// the chain of final_exp_hard
-static __device__ __noinline__ Fp2 t6_final_exp_hard(Team t, Fp2 in) {
-    const Fp2 y0 = t6_cyc_sqr(t, in);
-    Fp2 y1 = t6_raise_to_z(t, y0);
-    Fp2 y2 = t6_raise_to_z_div_by_2(t, y1);
-    y1 = t6_conj(t, t6_mul(t, y1, t6_conj(t, in)));
-    y1 = t6_mul(t, y1, y2);
-    y2 = t6_raise_to_z(t, y1);
-    Fp2 y3 = t6_raise_to_z(t, y2);
-    y1 = t6_conj(t, y1);
-    y3 = t6_mul(t, y3, y1);
-    y1 = t6_frobenius(t, t6_conj(t, y1), 3);
-    y1 = t6_mul(t, y1, t6_frobenius(t, y2, 2));
-    y2 = t6_mul(t, t6_raise_to_z(t, y3), y0);
-    y1 = t6_mul(t, y1, t6_mul(t, y2, in));
-    return t6_mul(t, y1, t6_frobenius(t, y3, 1));
+template <class T> WBTE_INL ElemOf<T> team_raise_to_z(const Team& t, const ElemOf<T>& x) {
+    return T::cyc_sqr(t, team_raise_to_z_div_by_2<T>(t, x));
+}
+// the addition chain of btx/src/final_exponentiation.rs:255-283
+template <class T> static __device__ __noinline__ ElemOf<T> team_final_exp_hard(Team t, ElemOf<T> in) {
+    const ElemOf<T> y0 = T::cyc_sqr(t, in);
+    ElemOf<T> y1 = team_raise_to_z<T>(t, y0);
+    ElemOf<T> y2 = team_raise_to_z_div_by_2<T>(t, y1);
+    y1 = team_conj<T>(t, T::mul(t, y1, team_conj<T>(t, in)));
+    y1 = T::mul(t, y1, y2);
+    y2 = team_raise_to_z<T>(t, y1);
+    ElemOf<T> y3 = team_raise_to_z<T>(t, y2);
+    y1 = team_conj<T>(t, y1);
+    y3 = T::mul(t, y3, y1);
+    y1 = team_frobenius<T>(t, team_conj<T>(t, y1), 3);
+    y1 = T::mul(t, y1, team_frobenius<T>(t, y2, 2));
+    y2 = T::mul(t, team_raise_to_z<T>(t, y3), y0);
+    y1 = T::mul(t, y1, T::mul(t, y2, in));
+    return T::mul(t, y1, team_frobenius<T>(t, y3, 1));
 }
 
 // -------------------------------------------------------------- Miller loops
-// Lines (pairing.cuh) enter as their six Fp components, component k on lane
-// k, already scaled by (1, 1, xP, xP, yP, yP).
-WBTE_INL bool t6_bit(int i) { return (X_ABS >> i) & 1; }
+// Lines (pairing.cuh) enter as their six Fp components, already scaled by (1, 1,
+// xP, xP, yP, yP).
+WBTE_INL bool miller_bit(int i) { return (X_ABS >> i) & 1; }
 
 // this lane's scale for lines through P; identities get the line 1
-struct T6Point { Fp scale; bool inf; };
-WBTE_INL T6Point t6_point(const Team& t, const G1A& P) {
-    T6Point r;
+struct TeamPoint { Fp scale; bool inf; };
+template <class T> WBTE_INL TeamPoint team_point(const Team& t, const G1A& P) {
+    const int c = T::line_index(t);
+    TeamPoint r;
     r.inf = is_inf(P);
-    r.scale = t.k < 2 ? fp_one() : (t.k < 4 ? P.x : P.y);
+    r.scale = c < 2 ? fp_one() : (c < 4 ? P.x : P.y);
     return r;
 }
-WBTE_INL Fp t6_line_value(const Team& t, const Fp& component, const T6Point& P) {
+template <class T> WBTE_INL Fp team_line_value(const Team& t, const Fp& component, const TeamPoint& P) {
     const Fp v = fp_mul(component, P.scale);
-    const Fp id = t.k == 0 ? fp_one() : fp_zero();
+    const Fp id = T::line_index(t) == 0 ? fp_one() : fp_zero();
     return P.inf ? id : v;
 }
 
-// G2 point of a running loop in homogeneous coordinates: X, Y, Z on lanes 0, 1,
-// 2 (the others carry anything).  The products of a step go one to a lane;
-// every lane forms the sums it needs from shared memory.
+// G2 point of a running loop in homogeneous coordinates: X, Y, Z at
+// coefficients 0, 1, 2 (the others carry anything).  The products of a step go
+// one to a coefficient; every lane forms the sums it needs from shared memory.
 constexpr int T6_P = T6_Y, T6_Q = T6_Y + 6, T6_R = T6_Z, T6_S = T6_Z + 6;
-WBTE_INL Fp2 t6_exchange(const Team& t, int row, const Fp2& v) {
-    team_st(t, row, t.base + t.k, v);
+template <class T> WBTE_INL void team_exchange(const Team& t, int row, const ElemOf<T>& v) {
+    T::st(t, row, t.base + t.k, v);
     __syncwarp();
-    return v;
 }
-// T <- 2T; returns this lane's component of the tangent line (line_double)
-static __device__ __noinline__ Fp t6_line_double(Team t, Fp2& T) {
+// S <- 2S; returns this lane's component of the tangent line
+template <class T> static __device__ __noinline__ Fp team_line_double(Team t, ElemOf<T>& S) {
+    using E = ElemOf<T>;
     __syncwarp();
-    t6_exchange(t, T6_P, T);
+    team_exchange<T>(t, T6_P, S);
     // Y Y, Z Z, X X, Y Z, X Y
-    t6_exchange(t, T6_Q, t6_fp2_mul(team_ld<Fp2>(t, T6_P, t.base + nib(0x001021u, t.k)),
-                                    team_ld<Fp2>(t, T6_P, t.base + nib(0x112021u, t.k))));
-    const Fp2 t0 = team_ld<Fp2>(t, T6_Q, t.base);
-    const Fp2 t2 = fp2_mul4(fp2_mul3(fp2_mul_xi(team_ld<Fp2>(t, T6_Q, t.base + 1))));  // 3 b' Z^2
-    const Fp2 t23 = fp2_mul3(t2);
-    const Fp2 YZ = team_ld<Fp2>(t, T6_Q, t.base + 3);
+    team_exchange<T>(t, T6_Q, T::f_mul(T::ld(t, T6_P, t.base + nib(0x001021u, t.k)),
+                                       T::ld(t, T6_P, t.base + nib(0x112021u, t.k))));
+    const E t0 = T::ld(t, T6_Q, t.base);
+    const E t2 = team_mul4<T>(team_mul3<T>(T::f_xi(t, T::ld(t, T6_Q, t.base + 1))));  // 3 b' Z^2
+    const E t23 = team_mul3<T>(t2);
+    const E YZ = T::ld(t, T6_Q, t.base + 3);
     // XY (t0 - t23), (t0 + t23)^2, t2^2, t0 YZ
-    Fp2 a = t0, b = YZ;
+    E a = t0, b = YZ;
     if (t.k == 0) {
-        a = team_ld<Fp2>(t, T6_Q, t.base + 4);
-        b = fp2_sub(t0, t23);
+        a = T::ld(t, T6_Q, t.base + 4);
+        b = T::f_sub(t0, t23);
     } else if (t.k == 1) {
-        a = b = fp2_add(t0, t23);
+        a = b = T::f_add(t0, t23);
     } else if (t.k == 2) {
         a = b = t2;
     }
-    t6_exchange(t, T6_R, t6_fp2_mul(a, b));
-    if (t.k == 0) {
-        T = fp2_dbl(team_ld<Fp2>(t, T6_R, t.base));
-    } else if (t.k == 1) {
-        T = fp2_sub(team_ld<Fp2>(t, T6_R, t.base + 1), fp2_mul4(fp2_mul3(team_ld<Fp2>(t, T6_R, t.base + 2))));
-    } else {
-        T = fp2_mul4(fp2_dbl(team_ld<Fp2>(t, T6_R, t.base + 3)));
-    }
-    Fp2 l;
-    if (t.k < 2) {
-        l = fp2_sub(t2, t0);
-    } else if (t.k < 4) {
-        l = fp2_mul3(team_ld<Fp2>(t, T6_Q, t.base + 2));
-    } else {
-        l = fp2_neg(fp2_dbl(YZ));
-    }
-    return (t.k & 1) ? l.c1 : l.c0;
-}
-// T <- T + Q; returns this lane's component of the chord (line_add)
-static __device__ __noinline__ Fp t6_line_add(Team t, Fp2& T, const G2A& Q) {
     __syncwarp();
-    t6_exchange(t, T6_P, T);
-    const Fp2 X = team_ld<Fp2>(t, T6_P, t.base), Y = team_ld<Fp2>(t, T6_P, t.base + 1);
-    const Fp2 Z = team_ld<Fp2>(t, T6_P, t.base + 2);
-    const Fp2 qx = Q.x, qy = Q.y;
-    t6_exchange(t, T6_Q, t6_fp2_mul(t.k == 0 ? qy : qx, Z));
-    const Fp2 u = fp2_sub(team_ld<Fp2>(t, T6_Q, t.base), Y);
-    const Fp2 v = fp2_sub(team_ld<Fp2>(t, T6_Q, t.base + 1), X);
-    // u u, v v, u xQ, v yQ
-    t6_exchange(t, T6_R, t6_fp2_mul((t.k == 0 || t.k == 2) ? u : v,
-                                    t.k == 0 ? u : (t.k == 1 ? v : (t.k == 2 ? qx : qy))));
-    const Fp2 v2 = team_ld<Fp2>(t, T6_R, t.base + 1);
-    // v2 v, v2 X, u2 Z
-    t6_exchange(t, T6_S, t6_fp2_mul(t.k < 2 ? v2 : team_ld<Fp2>(t, T6_R, t.base), t.k == 0 ? v : (t.k == 1 ? X : Z)));
-    const Fp2 v3 = team_ld<Fp2>(t, T6_S, t.base), v2X = team_ld<Fp2>(t, T6_S, t.base + 1);
-    const Fp2 A = fp2_sub(fp2_sub(team_ld<Fp2>(t, T6_S, t.base + 2), v3), fp2_dbl(v2X));
-    // v A, u (v2X - A), v3 Y, v3 Z
-    const Fp2 r = t6_fp2_mul(t.k == 0 ? v : (t.k == 1 ? u : v3), t.k == 0 ? A : (t.k == 1 ? fp2_sub(v2X, A) : (t.k == 2 ? Y : Z)));
-    t6_exchange(t, T6_Q, r);
-    T = team_ld<Fp2>(t, T6_Q, t.base + (t.k < 2 ? t.k : 3));
-    if (t.k == 1) T = fp2_sub(T, team_ld<Fp2>(t, T6_Q, t.base + 2));
-    Fp2 l;
-    if (t.k < 2) {
-        l = fp2_sub(team_ld<Fp2>(t, T6_R, t.base + 2), team_ld<Fp2>(t, T6_R, t.base + 3));
+    team_exchange<T>(t, T6_R, T::f_mul(a, b));
+    if (t.k == 0) {
+        S = team_dbl<T>(T::ld(t, T6_R, t.base));
+    } else if (t.k == 1) {
+        S = T::f_sub(T::ld(t, T6_R, t.base + 1), team_mul4<T>(team_mul3<T>(T::ld(t, T6_R, t.base + 2))));
     } else {
-        l = t.k < 4 ? fp2_neg(u) : v;
+        S = team_mul4<T>(team_dbl<T>(T::ld(t, T6_R, t.base + 3)));
     }
-    return (t.k & 1) ? l.c1 : l.c0;
+    const int c = T::line_index(t);
+    E l;
+    if (c < 2) {
+        l = T::f_sub(t2, t0);
+    } else if (c < 4) {
+        l = team_mul3<T>(T::ld(t, T6_Q, t.base + 2));
+    } else {
+        l = T::f_neg(team_dbl<T>(YZ));
+    }
+    return T::component(l, c & 1);
+}
+// S <- S + Q; returns this lane's component of the chord
+template <class T> static __device__ __noinline__ Fp team_line_add(Team t, ElemOf<T>& S, const G2A& Q) {
+    using E = ElemOf<T>;
+    __syncwarp();
+    team_exchange<T>(t, T6_P, S);
+    const E X = T::ld(t, T6_P, t.base), Y = T::ld(t, T6_P, t.base + 1), Z = T::ld(t, T6_P, t.base + 2);
+    const E qx = T::of(t, Q.x), qy = T::of(t, Q.y);
+    team_exchange<T>(t, T6_Q, T::f_mul(t.k == 0 ? qy : qx, Z));
+    const E u = T::f_sub(T::ld(t, T6_Q, t.base), Y), v = T::f_sub(T::ld(t, T6_Q, t.base + 1), X);
+    // u u, v v, u xQ, v yQ
+    team_exchange<T>(t, T6_R, T::f_mul((t.k == 0 || t.k == 2) ? u : v, t.k == 0 ? u : (t.k == 1 ? v : (t.k == 2 ? qx : qy))));
+    const E v2 = T::ld(t, T6_R, t.base + 1);
+    // v2 v, v2 X, u2 Z
+    team_exchange<T>(t, T6_S, T::f_mul(t.k < 2 ? v2 : T::ld(t, T6_R, t.base), t.k == 0 ? v : (t.k == 1 ? X : Z)));
+    const E v3 = T::ld(t, T6_S, t.base), v2X = T::ld(t, T6_S, t.base + 1);
+    const E A = T::f_sub(T::f_sub(T::ld(t, T6_S, t.base + 2), v3), team_dbl<T>(v2X));
+    // v A, u (v2X - A), v3 Y, v3 Z
+    const E w = T::f_sub(v2X, A);
+    const E r = T::f_mul(t.k == 0 ? v : (t.k == 1 ? u : v3), t.k == 0 ? A : (t.k == 1 ? w : (t.k == 2 ? Y : Z)));
+    team_exchange<T>(t, T6_Q, r);
+    S = T::ld(t, T6_Q, t.base + (t.k < 2 ? t.k : 3));
+    const E y = T::f_sub(S, T::ld(t, T6_Q, t.base + 2));
+    if (t.k == 1) S = y;
+    const int c = T::line_index(t);
+    E l;
+    if (c < 2) {
+        l = T::f_sub(T::ld(t, T6_R, t.base + 2), T::ld(t, T6_R, t.base + 3));
+    } else {
+        l = c < 4 ? T::f_neg(u) : v;
+    }
+    return T::component(l, c & 1);
 }
 
 }  // namespace wbte
