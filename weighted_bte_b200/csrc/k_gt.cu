@@ -93,6 +93,7 @@ __device__ __forceinline__ ElemOf<T> team_pow(const Team& t, ElemOf<T> x, const 
     ElemOf<T> acc = team_one<T>(t);
     bool started = false;  // the same in all lanes
     for (int pos = TOP - 1; pos >= 0; pos--) {
+        T::step();
         if (started)
             for (int i = 0; i < RUN; i++) acc = T::cyc_sqr(t, acc);
         for (int r = 0; r < R; r++) {
@@ -129,9 +130,9 @@ template <class T, int L> struct PerWarp { static constexpr int N = T::PER / L *
 // fastest over nbp >= nb = blocks * count slots, so that with nbp a multiple of
 // five a warp has one twiddle.
 template <class T, int L, bool NAF>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_pows(uint8_t* ex, const uint8_t* io, const int8_t* rec, int64_t n,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_gt_radix4_pows(uint8_t* ex, const uint8_t* io, const int8_t* rec, int64_t n,
                                                          int64_t h, int64_t J, int64_t nb, int64_t nbp) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     constexpr int PER = PerWarp<T, L>::N;
     const Team t = team_of<T>(sh, PER);
     const int64_t g = team_index<T>(PER) / L;
@@ -168,10 +169,10 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_pows(uint8_t* ex,
 // values), into dst.  prefix: only outputs below `keep` of each array are
 // wanted, of butterflies j < J.
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_outputs(uint8_t* dst, const uint8_t* src, const uint8_t* ex,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_gt_radix4_outputs(uint8_t* dst, const uint8_t* src, const uint8_t* ex,
                                                             int64_t n, int64_t h, int64_t J, int64_t nb, int inverse,
                                                             int64_t keep) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t g = team_index<T>();
     const bool active = g < 2 * J * nb;
@@ -201,8 +202,8 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix4_outputs(uint8_t* 
 
 // the first radix-2 stage (all twiddles one): u v and u / v of neighbours
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix2_first(uint8_t* dst, const uint8_t* src, int64_t total) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_gt_radix2_first(uint8_t* dst, const uint8_t* src, int64_t total) {
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t g = team_index<T>();
     const bool active = g < total;
@@ -217,9 +218,9 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_radix2_first(uint8_t* ds
 // out[q B + i] = base[(q B + i) stride]^(scalar i) for K arrays of B values
 // sharing the B exponents: teams take the arrays fastest over Kp >= K slots
 template <class T, int L, bool NAF>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_pow(uint8_t* out, const uint8_t* base, int64_t stride, const int8_t* rec,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_gt_pow(uint8_t* out, const uint8_t* base, int64_t stride, const int8_t* rec,
                                                  int64_t B, int64_t K, int64_t Kp) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     constexpr int PER = PerWarp<T, L>::N;
     const Team t = team_of<T>(sh, PER);
     const int64_t g = team_index<T>(PER) / L;
@@ -238,9 +239,9 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_pow(uint8_t* out, const 
 // the inverse (conjugation) for negative c_i -- mul_cyclotomic_signed_small of
 // weighted_pfe/src/fft.rs:671-699.  c_i = 0 gives one.
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_gt_pow_small(uint8_t* out, const uint8_t* base, int64_t stride,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_gt_pow_small(uint8_t* out, const uint8_t* base, int64_t stride,
                                                        const int32_t* coeffs, int64_t n) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t i = team_index<T>();
     const bool active = i < n;
@@ -315,17 +316,17 @@ void gt_pow_run(uint8_t* out, const uint8_t* base, int64_t stride, const uint8_t
     const int64_t Kp = naf ? pad5(K) : K, items = B * Kp;
     note_launch();
     if (naf)
-        k_gt_pow<Six, 1, true><<<blocks_for(items, 5), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+        team_launch<SixBlock>(k_gt_pow<SixBlock, 1, true>, items, 5, s, out, base, stride, rec, B, K, Kp);
     else if (how.twelve && how.L == 1)
-        k_gt_pow<Twelve, 1, false><<<blocks_for(items, 2), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+        team_launch<Twelve>(k_gt_pow<Twelve, 1, false>, items, 2, s, out, base, stride, rec, B, K, Kp);
     else if (how.twelve)
-        k_gt_pow<Twelve, 2, false><<<blocks_for(items, 1), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+        team_launch<Twelve>(k_gt_pow<Twelve, 2, false>, items, 1, s, out, base, stride, rec, B, K, Kp);
     else if (how.L == 1)
-        k_gt_pow<Six, 1, false><<<blocks_for(items, 5), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+        team_launch<SixBlock>(k_gt_pow<SixBlock, 1, false>, items, 5, s, out, base, stride, rec, B, K, Kp);
     else if (how.L == 2)
-        k_gt_pow<Six, 2, false><<<blocks_for(items, 2), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+        team_launch<Six>(k_gt_pow<Six, 2, false>, items, 2, s, out, base, stride, rec, B, K, Kp);
     else
-        k_gt_pow<Six, 4, false><<<blocks_for(items, 1), WARP, 0, s>>>(out, base, stride, rec, B, K, Kp);
+        team_launch<Six>(k_gt_pow<Six, 4, false>, items, 1, s, out, base, stride, rec, B, K, Kp);
     cudaFreeAsync(rec, s);
 }
 
@@ -350,9 +351,9 @@ void launch_gt_pow_small(uint8_t* out, const uint8_t* base, int64_t stride, cons
     if (n <= 0) return;
     note_launch();
     if (few_values(n))
-        k_gt_pow_small<Twelve><<<blocks_for(n, Twelve::PER), WARP, 0, s>>>(out, base, stride, coeffs, n);
+        team_launch<Twelve>(k_gt_pow_small<Twelve>, n, Twelve::PER, s, out, base, stride, coeffs, n);
     else
-        k_gt_pow_small<Six><<<blocks_for(n, Six::PER), WARP, 0, s>>>(out, base, stride, coeffs, n);
+        team_launch<Six>(k_gt_pow_small<Six>, n, Six::PER, s, out, base, stride, coeffs, n);
 }
 
 // The unscaled transform of `count` arrays of n values, keeping the first
@@ -377,9 +378,9 @@ static void gt_transform(uint8_t* io, const uint8_t* tw, int64_t n, int64_t keep
         // an odd number of stages starts with one radix-2 stage, the rest pair up
         note_launch();
         if (few_values(n * count))
-            k_gt_radix2_first<Twelve><<<blocks_for(n * count, Twelve::PER), WARP, 0, s>>>(other, cur, n * count);
+            team_launch<Twelve>(k_gt_radix2_first<Twelve>, n * count, Twelve::PER, s, other, cur, n * count);
         else
-            k_gt_radix2_first<Six><<<blocks_for(n * count, Six::PER), WARP, 0, s>>>(other, cur, n * count);
+            team_launch<Six>(k_gt_radix2_first<Six>, n * count, Six::PER, s, other, cur, n * count);
         std::swap(cur, other);
         half = 2;
     }
@@ -401,25 +402,24 @@ static void gt_transform(uint8_t* io, const uint8_t* tw, int64_t n, int64_t keep
             const int64_t nbp = use_naf ? pad5(nb) : nb, items = 3 * J * nbp;
             note_launch();
             if (use_naf)
-                k_gt_radix4_pows<Six, 1, true><<<blocks_for(items, 5), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+                team_launch<SixBlock>(k_gt_radix4_pows<SixBlock, 1, true>, items, 5, s, ex, cur, rec, n, half, J, nb, nbp);
             else if (how.twelve && how.L == 1)
-                k_gt_radix4_pows<Twelve, 1, false><<<blocks_for(items, 2), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+                team_launch<Twelve>(k_gt_radix4_pows<Twelve, 1, false>, items, 2, s, ex, cur, rec, n, half, J, nb, nbp);
             else if (how.twelve)
-                k_gt_radix4_pows<Twelve, 2, false><<<blocks_for(items, 1), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+                team_launch<Twelve>(k_gt_radix4_pows<Twelve, 2, false>, items, 1, s, ex, cur, rec, n, half, J, nb, nbp);
             else if (how.L == 1)
-                k_gt_radix4_pows<Six, 1, false><<<blocks_for(items, 5), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+                team_launch<SixBlock>(k_gt_radix4_pows<SixBlock, 1, false>, items, 5, s, ex, cur, rec, n, half, J, nb, nbp);
             else if (how.L == 2)
-                k_gt_radix4_pows<Six, 2, false><<<blocks_for(items, 2), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+                team_launch<Six>(k_gt_radix4_pows<Six, 2, false>, items, 2, s, ex, cur, rec, n, half, J, nb, nbp);
             else
-                k_gt_radix4_pows<Six, 4, false><<<blocks_for(items, 1), WARP, 0, s>>>(ex, cur, rec, n, half, J, nb, nbp);
+                team_launch<Six>(k_gt_radix4_pows<Six, 4, false>, items, 1, s, ex, cur, rec, n, half, J, nb, nbp);
         }
         note_launch();
         const uint8_t* powers = half > 1 ? ex : nullptr;
         if (few_values(2 * J * nb))
-            k_gt_radix4_outputs<Twelve><<<blocks_for(2 * J * nb, Twelve::PER), WARP, 0, s>>>(
-                other, cur, powers, n, half, J, nb, inverse ? 1 : 0, last ? keep : n);
+            team_launch<Twelve>(k_gt_radix4_outputs<Twelve>, 2 * J * nb, Twelve::PER, s, other, cur, powers, n, half, J, nb, inverse ? 1 : 0, last ? keep : n);
         else
-            k_gt_radix4_outputs<Six><<<blocks_for(2 * J * nb, Six::PER), WARP, 0, s>>>(other, cur, powers, n, half, J, nb,
+            team_launch<Six>(k_gt_radix4_outputs<Six>, 2 * J * nb, Six::PER, s, other, cur, powers, n, half, J, nb,
                                                                                   inverse ? 1 : 0, last ? keep : n);
         std::swap(cur, other);
     }

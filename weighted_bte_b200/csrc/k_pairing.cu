@@ -19,8 +19,8 @@ WBTE_INL const Fp12* as_gt(const uint8_t* p) { return reinterpret_cast<const Fp1
 
 // the line table of one point per team: lane k writes component k of each record
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n) {
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t i = team_index<T>();
     const bool active = i < n;
@@ -48,10 +48,10 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_prepare_lines(uint8_t* line
 // weighted_pfe, and single pairs).  The pairs of a run share the 62
 // squarings.
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_miller_lines_multi(uint8_t* out, const uint8_t* lines, const uint8_t* p,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_miller_lines_multi(uint8_t* out, const uint8_t* lines, const uint8_t* p,
                                                              int64_t n, int64_t per, int64_t p_per, int64_t pairs, int64_t C,
                                                              int64_t chunks) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t g = team_index<T>();
     const bool active = g < n * chunks;
@@ -68,6 +68,7 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_miller_lines_multi(uint8_t*
             // runs of one launch differ in length only at the end; the
             // shorter ones take lines of value one
             for (int64_t r = 0; r < C; r++) {
+                T::step();
                 const int64_t x = r < cnt ? r : 0;
                 TeamPoint pt = team_point<T>(t, load_affine(P + x));
                 pt.inf |= r >= cnt;
@@ -85,9 +86,9 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_miller_lines_multi(uint8_t*
 // lines computed on the fly, one multi-Miller loop sharing the squarings.
 // Pair i is (P[p_mod ? i % p_mod : i], Q[q_mod ? i % q_mod : i]).
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t per,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t per,
                                                         int64_t K, int C, int64_t chunks, int64_t p_mod, int64_t q_mod) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t g = team_index<T>();
     const bool active = g < K * chunks;
@@ -114,6 +115,7 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_miller_chunks(uint8_t* out,
         if (i != 62) f = T::sqr(t, f);
         for (int step = 0; step <= (miller_bit(i) ? 1 : 0); step++)
             for (int r = 0; r < C; r++) {
+                T::step();
                 const Fp c = step ? team_line_add<T>(t, S[r], Q_of(r)) : team_line_double<T>(t, S[r]);
                 TeamPoint pt = team_point<T>(t, P_of(r));
                 pt.inf |= (dead >> r) & 1;
@@ -125,9 +127,9 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_miller_chunks(uint8_t* out,
 }
 
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_fp12_segment_product(uint8_t* out, const uint8_t* in, const int64_t* offsets,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_fp12_segment_product(uint8_t* out, const uint8_t* in, const int64_t* offsets,
                                                                int64_t k) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t j = team_index<T>();
     const bool active = j < k;
@@ -143,8 +145,8 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_fp12_segment_product(uint8_
 }
 
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_final_exp(uint8_t* out, const uint8_t* in, int64_t n, int mode) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_final_exp(uint8_t* out, const uint8_t* in, int64_t n, int mode) {
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t i = team_index<T>();
     const bool active = i < n;
@@ -156,9 +158,9 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_final_exp(uint8_t* out, con
 }
 
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_fp12_mul(uint8_t* out, const uint8_t* a, int64_t sa, const uint8_t* b,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_fp12_mul(uint8_t* out, const uint8_t* a, int64_t sa, const uint8_t* b,
                                                    int64_t sb, bool conj_b, int64_t n) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t i = team_index<T>();
     const bool active = i < n;
@@ -170,9 +172,9 @@ __global__ void __launch_bounds__(WARP, T6_BLOCKS) k_fp12_mul(uint8_t* out, cons
 }
 
 template <class T>
-__global__ void __launch_bounds__(WARP, T6_BLOCKS) k_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha,
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha,
                                                  const uint8_t* beta, const uint8_t* valid, int64_t n) {
-    __shared__ uint4 sh[T6_ROWS * 32];
+    extern __shared__ uint4 sh[];
     const Team t = team_of<T>(sh);
     int64_t i = team_index<T>();
     const bool active = i < n;
@@ -269,17 +271,17 @@ void launch_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n, cudaStrea
     if (n <= 0) return;
     note_launch();
     if (launch_time(95.0, (double)n / Twelve::PER) < launch_time(150.0, (double)n / Six::PER))
-        k_prepare_lines<Twelve><<<blocks_for(n, Twelve::PER), WARP, 0, s>>>(lines, q, n);
+        team_launch<Twelve>(k_prepare_lines<Twelve>, n, Twelve::PER, s, lines, q, n);
     else
-        k_prepare_lines<Six><<<blocks_for(n, Six::PER), WARP, 0, s>>>(lines, q, n);
+        team_launch<Six>(k_prepare_lines<Six>, n, Six::PER, s, lines, q, n);
 }
 
 static void segment_product(uint8_t* out, const uint8_t* in, const int64_t* offsets, int64_t k, cudaStream_t s) {
     note_launch();
     if (few_values(k))
-        k_fp12_segment_product<Twelve><<<blocks_for(k, Twelve::PER), WARP, 0, s>>>(out, in, offsets, k);
+        team_launch<Twelve>(k_fp12_segment_product<Twelve>, k, Twelve::PER, s, out, in, offsets, k);
     else
-        k_fp12_segment_product<Six><<<blocks_for(k, Six::PER), WARP, 0, s>>>(out, in, offsets, k);
+        team_launch<Six>(k_fp12_segment_product<Six>, k, Six::PER, s, out, in, offsets, k);
 }
 
 static bool miller_lines(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, int64_t per, int64_t p_per,
@@ -293,10 +295,10 @@ static bool miller_lines(uint8_t* out, const uint8_t* lines, const uint8_t* p, i
         return false;
     note_launch();
     if (how.twelve)
-        k_miller_lines_multi<Twelve><<<blocks_for(n * chunks, Twelve::PER), WARP, 0, s>>>(runs, lines, p, n, per, p_per, pairs,
+        team_launch<Twelve>(k_miller_lines_multi<Twelve>, n * chunks, Twelve::PER, s, runs, lines, p, n, per, p_per, pairs,
                                                                                       how.C, chunks);
     else
-        k_miller_lines_multi<Six><<<blocks_for(n * chunks, Six::PER), WARP, 0, s>>>(runs, lines, p, n, per, p_per, pairs,
+        team_launch<SixBlock>(k_miller_lines_multi<SixBlock>, n * chunks, Six::PER, s, runs, lines, p, n, per, p_per, pairs,
                                                                                 how.C, chunks);
     if (chunks > 1) {
         note_launch();
@@ -327,9 +329,9 @@ static void miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int6
     note_launch();
     if (launch_time(45.0 + LINE_COMPUTED.twelve * C, (double)runs / Twelve::PER) <
         launch_time(73.0 + LINE_COMPUTED.six * C, (double)runs / Six::PER))
-        k_miller_chunks<Twelve><<<blocks_for(runs, Twelve::PER), WARP, 0, s>>>(out, p, q, per, K, C, chunks, p_mod, q_mod);
+        team_launch<Twelve>(k_miller_chunks<Twelve>, runs, Twelve::PER, s, out, p, q, per, K, C, chunks, p_mod, q_mod);
     else
-        k_miller_chunks<Six><<<blocks_for(runs, Six::PER), WARP, 0, s>>>(out, p, q, per, K, C, chunks, p_mod, q_mod);
+        team_launch<SixBlock>(k_miller_chunks<SixBlock>, runs, Six::PER, s, out, p, q, per, K, C, chunks, p_mod, q_mod);
 }
 void launch_miller(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t n, cudaStream_t s, int64_t p_mod,
                    int64_t q_mod) {
@@ -369,18 +371,18 @@ void launch_final_exp(uint8_t* out, const uint8_t* in, int64_t n, FinalExpMode m
     note_launch();
     // 315 cyclotomic squarings and 35 products of the hard part
     if (launch_time(176.0, (double)n / Twelve::PER) < launch_time(336.0, (double)n / Six::PER))
-        k_final_exp<Twelve><<<blocks_for(n, Twelve::PER), WARP, 0, s>>>(out, in, n, (int)mode);
+        team_launch<Twelve>(k_final_exp<Twelve>, n, Twelve::PER, s, out, in, n, (int)mode);
     else
-        k_final_exp<Six><<<blocks_for(n, Six::PER), WARP, 0, s>>>(out, in, n, (int)mode);
+        team_launch<Six>(k_final_exp<Six>, n, Six::PER, s, out, in, n, (int)mode);
 }
 
 void launch_fp12_mul(uint8_t* out, const uint8_t* a, int64_t sa, const uint8_t* b, int64_t sb, bool conj_b, int64_t n, cudaStream_t s) {
     if (n <= 0) return;
     note_launch();
     if (few_values(n))
-        k_fp12_mul<Twelve><<<blocks_for(n, Twelve::PER), WARP, 0, s>>>(out, a, sa, b, sb, conj_b, n);
+        team_launch<Twelve>(k_fp12_mul<Twelve>, n, Twelve::PER, s, out, a, sa, b, sb, conj_b, n);
     else
-        k_fp12_mul<Six><<<blocks_for(n, Six::PER), WARP, 0, s>>>(out, a, sa, b, sb, conj_b, n);
+        team_launch<Six>(k_fp12_mul<Six>, n, Six::PER, s, out, a, sa, b, sb, conj_b, n);
 }
 void launch_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha, const uint8_t* beta, const uint8_t* valid,
                    int64_t n, cudaStream_t s) {
@@ -388,9 +390,9 @@ void launch_unmask(uint8_t* out, const uint8_t* second, const uint8_t* alpha, co
     if (n <= 0) return;
     note_launch();
     if (few_values(n))
-        k_unmask<Twelve><<<blocks_for(n, Twelve::PER), WARP, 0, s>>>(out, second, alpha, beta, valid, n);
+        team_launch<Twelve>(k_unmask<Twelve>, n, Twelve::PER, s, out, second, alpha, beta, valid, n);
     else
-        k_unmask<Six><<<blocks_for(n, Six::PER), WARP, 0, s>>>(out, second, alpha, beta, valid, n);
+        team_launch<Six>(k_unmask<Six>, n, Six::PER, s, out, second, alpha, beta, valid, n);
 }
 void launch_gt_compress(uint8_t* out, const uint8_t* in, int64_t n, cudaStream_t s) {
     ProfScope prof_("gt_compress", s);
