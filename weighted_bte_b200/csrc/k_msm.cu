@@ -123,9 +123,14 @@ __global__ void k_sort(uint64_t* entries, int32_t* nnz, const int16_t* digits, i
 // as its gap says.
 // The multiply-add pipe bounds it.  Measured on B200: see Point for why G2 takes
 // pairs; the families of a committee preparation at B = 512 (512 MSMs for each
-// of three parties, 1,382 terms together, and 1,023 of 1,382) 171 -> 102 ms,
-// one MSM of 20,011 points 2.5 -> 1.5 ms; G1 as one thread per segment was,
-// 1.57 ms at 65,536 points.
+// of three parties, 1,382 terms together, and 1,023 of 1,382) 171 -> 84 ms,
+// one MSM of 20,011 points 2.5 -> 1.3 ms; G1 as one thread per segment was,
+// 1.3 ms at 65,536 points.
+// The MSMs of a family run fastest over the lanes: those that share a scalar
+// vector have the same transitions, so a warp's segments queue and add
+// together (84 -> 81 ms), and the block's warps meet before each term, which
+// lets them share instruction fetches (81 -> 79 ms; blocks of 128 threads 79.5,
+// of 256 84 ms).
 constexpr int SEG_QUEUE = 4;
 constexpr size_t SEG_SMEM = (sizeof(Point<OnLane>) + sizeof(uint32_t)) * SEG_QUEUE * SEG_TPB;
 
@@ -141,13 +146,14 @@ __global__ void __launch_bounds__(SEG_TPB) k_segments(uint8_t* seg_out, const ui
     const int64_t gid = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) / P::LANES;
     // lanes past the grid's work run along with an empty segment
     const bool real = gid < k * windows * nseg;
-    int64_t lo = 0, hi = 0;
+    int64_t lo = 0, hi = 0, out = 0;
     const uint64_t* e = entries;
     const uint8_t* base = points;
     if (real) {
-        const int64_t seg = gid % nseg;
-        const int64_t w = (gid / nseg) % windows;
-        const int64_t j = gid / (nseg * windows);
+        const int64_t j = gid % k;
+        const int64_t seg = (gid / k) % nseg;
+        const int64_t w = gid / (k * nseg);
+        out = (j * windows + w) * nseg + seg;
         const int64_t vw = (vsel ? (int64_t)vsel[j] : 0) * windows + w;
         lo = seg * S;
         hi = lo + S;
@@ -180,6 +186,7 @@ __global__ void __launch_bounds__(SEG_TPB) k_segments(uint8_t* seg_out, const ui
         }
     };
     for (int64_t i = 0; i < S; i++) {
+        __syncthreads();
         const int64_t x = lo + i;
         const bool live = x < hi;
         const uint64_t en = live ? e[x] : 0;
@@ -207,7 +214,7 @@ __global__ void __launch_bounds__(SEG_TPB) k_segments(uint8_t* seg_out, const ui
     }
     acc = Pt::add(acc, Pt::multiple(run, cur_b), lo < hi);
     while (__any_sync(FULL, qn > 0)) turn();
-    if (real) acc.store(seg_out + 4 * P::FIELD * gid);
+    if (real) acc.store(seg_out + 4 * P::FIELD * out);
 }
 
 // out[row * out_len + i] = sum of in[row * len + G i .. G i + G - 1], G = 2, 4,
