@@ -70,3 +70,15 @@ def test_square():
     ri = pow(R384, -1, P)
     for a in [0, 1, P - 1, P, 2 * P - 1] + [rng.randrange(2 * P) for _ in range(40)]:
         assert value(call("fp_mont_sqr", a=limbs(a, 12))["r"]) == a * a * ri % P
+
+
+@pytest.mark.parametrize("ka,kb", [(8, 1), (1, 8), (7, 1), (1, 7), (4, 2), (2, 4), (3, 3)])
+def test_product_of_sums_without_reduction(ka, kb):
+    """Factors below ka p and kb p with ka kb < 2^384 / p give a reduced product;
+    the first factor plus p has to stay below 2^384 as well."""
+    rng = random.Random(10 * ka + kb)
+    ri = pow(R384, -1, P)
+    for k in range(30):
+        a = [ka * P - 1, ka * P - 2, 0, P][k % 4] if k < 8 else rng.randrange(ka * P)
+        b = [kb * P - 1, kb * P - 1, P, kb * P - 3][k % 4] if k < 12 else rng.randrange(kb * P)
+        assert value(call("fp_mont_mul", a=limbs(a, 12), b=limbs(b, 12))["r"]) == a * b * ri % P

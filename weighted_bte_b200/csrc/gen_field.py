@@ -740,6 +740,9 @@ def gen_constants():
                 if (G1X * cand % P, G1Y) == ec_mul(g1, lam, FP_OPS):
                     beta = cand
         gg += 1
+    # u^6 = 1/6: (x, y) -> (u^2 x, u^3 y) maps y^2 = x^3 + 4 to y^2 = x^3 + 2/3
+    u = 0x9f64800c4c997af191289fe6b29921022cec61a41342277f518a80c214d2fab652cd036108b697526c934ce9eb1bb94
+    assert 6 * pow(u, 6, P) % P == 1
     # Frobenius coefficients FROB[k][i] = xi^{i (p^k - 1)/6}, xi = 1 + u
     xi = (1, 1)
     frob = []
@@ -768,6 +771,9 @@ def gen_constants():
     w("__device__ __constant__ const uint32_t C_G2_GEN[4][12] = {%s, %s, %s, %s};" % (
         fp_lit(G2X0), fp_lit(G2X1), fp_lit(G2Y0), fp_lit(G2Y1)))
     w("__device__ __constant__ const uint32_t C_GLV_BETA[12] = %s;" % fp_lit(beta))
+    w("// u^2, u^3 and their inverses for the u with u^6 = 1/6")
+    w("__device__ __constant__ const uint32_t C_ISO_IN[2][12] = %s;" % fp2_lit((pow(u, 2, P), pow(u, 3, P))))
+    w("__device__ __constant__ const uint32_t C_ISO_OUT[2][12] = %s;" % fp2_lit((pow(u, -2, P), pow(u, -3, P))))
     w("__device__ __constant__ const uint32_t C_PSI_CX[2][12] = %s;" % fp2_lit(cx))
     w("__device__ __constant__ const uint32_t C_PSI_CY[2][12] = %s;" % fp2_lit(cy))
     rows = []

@@ -871,12 +871,12 @@ void launch_domain_twiddles(uint8_t* tw, int64_t n, int64_t count, bool inverse,
 void launch_mul_batch(Group g, uint8_t* out, const uint8_t* pts, int64_t stride, const uint8_t* scalars, int64_t n, cudaStream_t s) {
     ProfScope prof_("mul_batch", s);
     if (n <= 0) return;
-    // 252 doublings and 76 additions by one thread or one quad (the measures
-    // of ntt_joint)
+    // 252 doublings and 76 additions by one thread or by the lanes of one point
+    // (the measures of ntt_joint)
     const bool g1 = g == GROUP_G1;
-    if (launch_time((252 * 3 + 76 * 4) * (g1 ? 360.0 : 530.0), (double)n / (g1 ? 8 : 4)) <
-        launch_time((252 * 9 + 76 * 14) * (g1 ? 300.0 : 1800.0), (double)n / 32)) {
-        launch_quad_mul_batch(g, out, pts, stride, scalars, n, s);
+    const ChainTime chain = chain_time(g1, 252, 76, (double)n);
+    if (chain.time < launch_time((252 * 9 + 76 * 14) * (g1 ? 300.0 : 1800.0), (double)n / 32)) {
+        launch_quad_mul_batch(g, out, pts, stride, scalars, n, chain.eight, s);
         return;
     }
     note_launch();
@@ -1073,8 +1073,8 @@ __global__ void k_fixed_tables_g2(uint8_t* tables, const uint8_t* points, const 
 }
 
 // How a small MSM's outputs are spread: over L lanes of one thread per pair
-// group (quads false) or over L quads.
-struct SmallMsmSpread { bool quads; int L; };
+// group (quads false) or over L quads (or points on eight lanes each).
+struct SmallMsmSpread { bool quads; int L; bool eight = false; };
 // From a cost model of one lane's work: its tables (7 additions per term it
 // touches; 15 on G1, two tables; on quads 7 per pair), the shared doublings and
 // one addition per window and pair it holds, in the measures of ntt_joint.
@@ -1089,7 +1089,7 @@ static SmallMsmSpread small_msm_spread(Group g, int64_t k, int64_t n) {
     const bool g1 = g == GROUP_G1;
     const int D = g1 ? SmallMsmDigits<Fp>::D : SmallMsmDigits<Fp2>::D;
     const int windows = (g1 ? SmallMsmDigits<Fp>::TOP : SmallMsmDigits<Fp2>::TOP) + 1;
-    const double product = g1 ? 300.0 : 1800.0, round = g1 ? 360.0 : 530.0, table = g1 ? 15.0 : 7.0;
+    const double product = g1 ? 300.0 : 1800.0, table = g1 ? 15.0 : 7.0;
     const int64_t pairs = n * D;
     SmallMsmSpread best = {false, 1};
     double best_t = 0;
@@ -1101,8 +1101,8 @@ static SmallMsmSpread small_msm_spread(Group g, int64_t k, int64_t n) {
         const double t = launch_time((dbls * 9 + (terms * table + mine * windows) * 14) * product, (double)(k * L) / 32);
         if (L == 1 || t < best_t) best = {false, L}, best_t = t;
         if (L <= (g1 ? 8 : 4)) {
-            const double q = launch_time((dbls * 3 + mine * (windows + 7) * 4) * round, (double)(k * L) / (g1 ? 8 : 4));
-            if (q < best_t) best = {true, L}, best_t = q;
+            const ChainTime q = chain_time(g1, dbls, mine * (windows + 7), (double)(k * L));
+            if (q.time < best_t && L <= (q.eight ? 4 : 8)) best = {true, L, q.eight}, best_t = q.time;
         }
         if (L >= pairs) break;
     }
@@ -1117,7 +1117,7 @@ void launch_small_msm(Group g, uint8_t* out, const uint8_t* points, const int64_
     const SmallMsmSpread spread = small_msm_spread(g, k, n);
     const int L = spread.L;
     if (spread.quads) {
-        launch_quad_small_msm(g, out, points, pbase, idx, scalars, vsel, k, n, L, s);
+        launch_quad_small_msm(g, out, points, pbase, idx, scalars, vsel, k, n, L, spread.eight, s);
         return;
     }
     note_launch();
@@ -1158,9 +1158,10 @@ void launch_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t* R, c
     const uint8_t* table = generator_table(GROUP_G1, st);
     if (!table) return;
     // 128 doublings and about 130 additions by one thread, or 128 and 60 on
-    // each of four quads
-    if (launch_time((128 * 3 + 60 * 4) * 360.0, (double)n / 2) < launch_time((128 * 9 + 130 * 13) * 300.0, (double)n / 32)) {
-        launch_quad_schnorr_verify(valid, X, R, sresp, c, n, table, st);
+    // each of four points
+    const ChainTime chain = chain_time(true, 128, 60, 4.0 * n);
+    if (chain.time < launch_time((128 * 9 + 130 * 13) * 300.0, (double)n / 32)) {
+        launch_quad_schnorr_verify(valid, X, R, sresp, c, n, table, chain.eight, st);
         return;
     }
     note_launch();

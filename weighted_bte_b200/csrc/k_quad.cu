@@ -13,30 +13,34 @@ namespace {
 constexpr int WARP = 32;
 inline unsigned blocks_for(int64_t n, int64_t per) { return (unsigned)((n + per - 1) / per); }
 
-template <class P> struct SizeOf {
-    static constexpr size_t AFF = 2 * P::FIELD, XYZZ = 4 * P::FIELD;
-    static constexpr int PER_WARP = WARP / Quad<P>::WIDTH;
+template <class Q> struct SizeOf {
+    static constexpr size_t AFF = 2 * Q::Field::FIELD, XYZZ = 4 * Q::Field::FIELD;
+    static constexpr int PER_WARP = WARP / Q::WIDTH;
 };
+using G1Quad = Quad<OnLane>;
+using G2Quad = Quad<OnPair>;
 // this lane's point among all the launch's
-template <class P> __device__ __forceinline__ int64_t point_index() {
-    return (int64_t)blockIdx.x * SizeOf<P>::PER_WARP + (threadIdx.x & 31) / Quad<P>::WIDTH;
+template <class Q> __device__ __forceinline__ int64_t point_index() {
+    return (int64_t)blockIdx.x * SizeOf<Q>::PER_WARP + (threadIdx.x & 31) / Q::WIDTH;
 }
+// a doubling of a Horner chain
+__device__ __forceinline__ Fp horner_dbl(Oct, const Fp& p) { return Oct::dbl(p); }
+__device__ __forceinline__ Fp horner_dbl(Quad<OnPair, 8>, const Fp& p) { return Quad<OnPair, 8>::dbl_on_curve(p); }
 
 // out[j] = sum_w 2^(c w) wins[j windows + w], the sums of each window, of points
 // on the curve.  About 250 doublings in a row bound it, whatever the MSM's size.
-template <class P>
+template <class Q>
 __global__ void __launch_bounds__(WARP) k_combine(uint8_t* out, const uint8_t* wins, int64_t k, int windows, int c) {
-    using Q = Quad<P, 8>;
     const int64_t j = (int64_t)blockIdx.x * (WARP / Q::WIDTH) + (threadIdx.x & 31) / Q::WIDTH;
     const bool active = j < k;
-    const uint8_t* W = wins + SizeOf<P>::XYZZ * (active ? j : k - 1) * windows;
-    Fp acc = Q::load(W + SizeOf<P>::XYZZ * (windows - 1));
+    const uint8_t* W = wins + SizeOf<Q>::XYZZ * (active ? j : k - 1) * windows;
+    Fp acc = Q::load(W + SizeOf<Q>::XYZZ * (windows - 1));
     for (int w = windows - 2; w >= 0; w--) {
-        for (int i = 0; i < c; i++) acc = Q::dbl_on_curve(acc);
-        acc = Q::add(acc, Q::load(W + SizeOf<P>::XYZZ * w), true);
+        for (int i = 0; i < c; i++) acc = horner_dbl(Q(), acc);
+        acc = Q::add(acc, Q::load(W + SizeOf<Q>::XYZZ * w), true);
     }
     acc = Q::affine(acc);
-    if (active) Q::store_affine(out + SizeOf<P>::AFF * j, acc);
+    if (active) Q::store_affine(out + SizeOf<Q>::AFF * j, acc);
 }
 
 // A radix-2^kappa step of a decimation-in-time transform merges the radix-2
@@ -66,20 +70,19 @@ __device__ __forceinline__ int radix_slot(int k, int m, int rho) {
 
 // multiples[(t per + r)] for the blocks and offsets t (array-major, then block,
 // then offset) and the per = (4^kappa - 1) / 3 multiples r, DIGITS points each
-template <class P>
+template <class Q>
 __global__ void __launch_bounds__(WARP) k_ntt_multiples(uint8_t* multiples, const uint8_t* work, const uint8_t* tw, int64_t n,
                                                         int64_t h, int kappa, int64_t total, int per) {
-    using Q = Quad<P>;
-    constexpr int D = Q::DIGITS;
+    constexpr int D = QuadDigits<Q>::DIGITS;
     const int rho = 1 << kappa;
-    const int64_t p = point_index<P>();
+    const int64_t p = point_index<Q>();
     const int dig = (int)(p % D);
     const bool active = p / D < total;
     const int64_t g = active ? p / D : total - 1;
     const int64_t t = g / per, j = t % h, blk = t / h;
     const RadixTerm term = radix_term((int)(g % per), rho);
     const int q = (int)(__brev((uint32_t)term.k) >> (32 - kappa));
-    const Fp v = Q::load(work + SizeOf<P>::XYZZ * (blk * rho * h + j + q * h));
+    const Fp v = Q::load(work + SizeOf<Q>::XYZZ * (blk * rho * h + j + q * h));
     int64_t idx = (int64_t)term.k * (n / (rho * h)) * (j + term.m * h) % n;
     const bool minus = idx >= n / 2;  // w^(i + n/2) = -w^i
     if (minus) idx -= n / 2;
@@ -93,21 +96,20 @@ __global__ void __launch_bounds__(WARP) k_ntt_multiples(uint8_t* multiples, cons
     // w^0 alone in the whole warp needs no digits
     if (__any_sync(FULL, idx != 0)) {
         uint64_t lo[1], hi[1];
-        quad_digit<P>(lo[0], hi[0], d, dig);
-        const Fp base[1] = {Q::image(v, dig)};
-        r = Q::group_sum(Q::straus(base, lo, hi, 1), D);
+        quad_digit<typename Q::Field>(lo[0], hi[0], d, dig);
+        const Fp base[1] = {quad_image<Q>(v, dig)};
+        r = quad_sum<Q>(quad_straus<Q>(base, lo, hi, 1), D);
     }
     if (minus) r = Q::neg(r);
-    if (active && dig == 0) Q::store(multiples + SizeOf<P>::XYZZ * g, r);
+    if (active && dig == 0) Q::store(multiples + SizeOf<Q>::XYZZ * g, r);
 }
 
 // the sums of a step, L points (a power of two that a warp holds) per output
-template <class P>
+template <class Q>
 __global__ void __launch_bounds__(WARP) k_ntt_sums(uint8_t* out, const uint8_t* work, const uint8_t* multiples, int64_t h,
                                                    int kappa, int64_t total, int per, int L) {
-    using Q = Quad<P>;
     const int rho = 1 << kappa;
-    const int64_t p = point_index<P>();
+    const int64_t p = point_index<Q>();
     const int sub = (int)(p % L);
     const bool active = p / L < total;
     const int64_t o = active ? p / L : total - 1;
@@ -116,25 +118,24 @@ __global__ void __launch_bounds__(WARP) k_ntt_sums(uint8_t* out, const uint8_t* 
     Fp acc = Q::infinity();
     for (int k = sub; k < rho; k += L) {
         const int V = k ? radix_variants(k, rho) : 1;
-        Fp x = Q::load(k ? multiples + SizeOf<P>::XYZZ * (t * per + radix_slot(k, m % V, rho))
-                         : work + SizeOf<P>::XYZZ * (blk * rho * h + j));
+        Fp x = Q::load(k ? multiples + SizeOf<Q>::XYZZ * (t * per + radix_slot(k, m % V, rho))
+                         : work + SizeOf<Q>::XYZZ * (blk * rho * h + j));
         if (k && (m / V) & 1) x = Q::neg(x);
         acc = k == sub ? x : Q::add(acc, x, true);
     }
-    acc = Q::group_sum(acc, L);
-    if (active && sub == 0) Q::store(out + SizeOf<P>::XYZZ * (blk * rho * h + j + m * h), acc);
+    acc = quad_sum<Q>(acc, L);
+    if (active && sub == 0) Q::store(out + SizeOf<Q>::XYZZ * (blk * rho * h + j + m * h), acc);
 }
 
 // out[o] = sum_t scalars[vsel[o] n + t] points[pbase[o] + idx[t]] for n <=
 // SMALL_MSM_MAX: the (term, digit) pairs of an output are dealt to L points
 // (a power of two that a warp holds), the sums meet in a tree
-template <class P>
+template <class Q>
 __global__ void __launch_bounds__(WARP) k_small_msm(uint8_t* out, const uint8_t* points, const int64_t* pbase,
                                                     const int32_t* idx, const uint8_t* scalars, const int32_t* vsel,
                                                     int64_t k, int64_t n, int L) {
-    using Q = Quad<P>;
-    constexpr int D = Q::DIGITS, MOST = SMALL_MSM_MAX * D;
-    const int64_t p = point_index<P>();
+    constexpr int D = QuadDigits<Q>::DIGITS, MOST = SMALL_MSM_MAX * D;
+    const int64_t p = point_index<Q>();
     const int sub = (int)(p % L);
     const bool active = p / L < k;
     const int64_t o = active ? p / L : k - 1;
@@ -144,32 +145,31 @@ __global__ void __launch_bounds__(WARP) k_small_msm(uint8_t* out, const uint8_t*
     uint64_t lo[MOST], hi[MOST];
     for (int r = 0; r < mine; r++) {
         const int x = sub + r * L, t = x < pairs ? x / D : 0, c = x % D;
-        base[r] = Q::image(Q::load_affine(points + SizeOf<P>::AFF * (pbase[o] + (idx ? (int64_t)idx[t] : t))), c);
+        base[r] = quad_image<Q>(Q::load_affine(points + SizeOf<Q>::AFF * (pbase[o] + (idx ? (int64_t)idx[t] : t))), c);
         uint32_t s[8];
         load_scalar(s, scalars + FR_SZ * (v * n + t));
         uint64_t d[4];
         decompose_base_x(d, s);
-        quad_digit<P>(lo[r], hi[r], d, c);
+        quad_digit<typename Q::Field>(lo[r], hi[r], d, c);
         if (x >= pairs) lo[r] = hi[r] = 0;
     }
-    const Fp r = Q::affine(Q::group_sum(Q::straus(base, lo, hi, mine), L));
-    if (active && sub == 0) Q::store_affine(out + SizeOf<P>::AFF * o, r);
+    const Fp r = Q::affine(quad_sum<Q>(quad_straus<Q>(base, lo, hi, mine), L));
+    if (active && sub == 0) Q::store_affine(out + SizeOf<Q>::AFF * o, r);
 }
 
 // out[i] = scalars[i] points[i stride] for any points of the curve (no
 // endomorphism): 4-bit windows of the 256-bit scalar
-template <class P>
+template <class Q>
 __global__ void __launch_bounds__(WARP) k_mul_batch(uint8_t* out, const uint8_t* pts, int64_t stride,
                                                     const uint8_t* scalars, int64_t n) {
-    using Q = Quad<P>;
-    int64_t i = point_index<P>();
+    int64_t i = point_index<Q>();
     const bool active = i < n;
     if (!active) i = n - 1;
     uint32_t s[8];
     load_scalar(s, scalars + FR_SZ * i);
     Fp tab[16];
     tab[0] = Q::infinity();
-    tab[1] = Q::load_affine(pts + SizeOf<P>::AFF * stride * i);
+    tab[1] = Q::load_affine(pts + SizeOf<Q>::AFF * stride * i);
     tab[2] = Q::dbl(tab[1]);
     for (int d = 3; d < 16; d++) tab[d] = Q::add(tab[d - 1], tab[1], true);
     Fp acc = Q::infinity();
@@ -183,16 +183,16 @@ __global__ void __launch_bounds__(WARP) k_mul_batch(uint8_t* out, const uint8_t*
         acc = Q::add(acc, tab[d], d != 0);
     }
     const Fp r = Q::affine(acc);
-    if (active) Q::store_affine(out + SizeOf<P>::AFF * i, r);
+    if (active) Q::store_affine(out + SizeOf<Q>::AFF * i, r);
 }
 
 // valid[i] = ([s_i] G == R_i + [c_i] X_i), four points per check: two take the
 // digits of [c]X, two the even and odd bytes of [s]G from the generator table
+template <class Q>
 __global__ void __launch_bounds__(WARP) k_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t* R,
                                                          const uint8_t* sresp, const uint8_t* c, int64_t n,
                                                          const uint8_t* gen_table) {
-    using Q = Quad<OnLane>;
-    const int64_t p = point_index<OnLane>();
+    const int64_t p = point_index<Q>();
     const int sub = (int)(p & 3);
     const bool active = p / 4 < n;
     const int64_t i = active ? p / 4 : n - 1;
@@ -202,8 +202,8 @@ __global__ void __launch_bounds__(WARP) k_schnorr_verify(uint8_t* valid, const u
     decompose_base_x(d, s);
     quad_digit<OnLane>(lo[0], hi[0], d, sub & 1);
     if (sub >= 2) lo[0] = hi[0] = 0;
-    const Fp base[1] = {Q::image(Q::load_affine(X + G1_AFF * i), sub & 1)};
-    Fp acc = Q::straus(base, lo, hi, 1);
+    const Fp base[1] = {quad_image<Q>(Q::load_affine(X + G1_AFF * i), sub & 1)};
+    Fp acc = quad_straus<Q>(base, lo, hi, 1);
     // R joins the first point's sum; -[s]G gathers on the third and fourth
     const uint8_t* sb = sresp + FR_SZ * i;
     for (int w = 0; w < 16; w++) {
@@ -213,7 +213,7 @@ __global__ void __launch_bounds__(WARP) k_schnorr_verify(uint8_t* valid, const u
         if (sub >= 2) m = Q::neg(m);
         acc = Q::add(acc, m, sub >= 2 ? by != 0 : (sub == 0 && w == 0));
     }
-    acc = Q::group_sum(acc, 4);
+    acc = quad_sum<Q>(acc, 4);
     const bool inf = Q::is_inf(acc);
     if (active && sub == 0 && Q::place() == 0) valid[i] = inf ? 1 : 0;
 }
@@ -294,22 +294,23 @@ __global__ void __launch_bounds__(WARP) k_fixed_msm_g2(uint8_t* out, const uint8
 void launch_msm_combine(Group g, uint8_t* out, const uint8_t* wins, int64_t k, int windows, int c, cudaStream_t s) {
     note_launch();
     if (g == GROUP_G1)
-        k_combine<OnLane><<<blocks_for(k, WARP / Quad<OnLane, 8>::WIDTH), WARP, 0, s>>>(out, wins, k, windows, c);
+        k_combine<Oct><<<blocks_for(k, SizeOf<Oct>::PER_WARP), WARP, 0, s>>>(out, wins, k, windows, c);
     else
-        k_combine<OnPair><<<blocks_for(k, WARP / Quad<OnPair, 8>::WIDTH), WARP, 0, s>>>(out, wins, k, windows, c);
+        k_combine<Quad<OnPair, 8>><<<blocks_for(k, SizeOf<Quad<OnPair, 8>>::PER_WARP), WARP, 0, s>>>(out, wins, k, windows, c);
 }
 
-// rounds of a quad's scalar multiple (128 doublings of three and 41 additions of
-// four in G1, 64 and 24 in G2) and the wide multiply-adds of a round with its
-// exchanges
-static constexpr double MULTIPLE_G1 = 548, MULTIPLE_G2 = 288, ROUND_G1 = 360, ROUND_G2 = 530;
+// doublings and additions of a multiple of one digit: 128 and 41 in G1, 64 and 24
+// in G2
+static ChainTime multiples_time(bool g1, double points, double alone) {
+    return g1 ? chain_time(true, 128, 41, points, alone) : chain_time(false, 64, 24, points, alone);
+}
 
 // Steps of a transform of `bits` stages over `count` arrays: steps[i] stages each,
 // the cheapest composition by the cost model; returns its time.
 double quad_ntt_plan(Group g, int bits, int64_t count, int* steps, int* nsteps) {
     const bool g1 = g == GROUP_G1;
     const double points = (double)((int64_t)1 << bits) * (double)count;
-    const int per_warp = g1 ? SizeOf<OnLane>::PER_WARP : SizeOf<OnPair>::PER_WARP, digits = g1 ? 2 : 4;
+    const int digits = g1 ? 2 : 4;
     // a pair's products keep two chains in flight: one warp fills a scheduler
     // (1,024 points in G2: 0.52 ms a stage at 0.9 warps, 1.05 ms at 2.2)
     const double alone = g1 ? 1.6 : 1.0;
@@ -321,10 +322,9 @@ double quad_ntt_plan(Group g, int bits, int64_t count, int* steps, int* nsteps) 
         for (int kappa = 1; kappa <= 4 && kappa <= done; kappa++) {
             // a first step multiplies by powers of its own root only: one of a k's V_k is one
             const double multiples = ((double)((1 << (2 * kappa)) - 1) / 3.0) / (double)(1 << kappa) * points * digits;
-            const double chain = done == kappa && kappa == 1 ? 0.0 : (g1 ? MULTIPLE_G1 : MULTIPLE_G2);
-            const double t = best[done - kappa] +
-                             launch_time(chain * (g1 ? ROUND_G1 : ROUND_G2), multiples / per_warp, alone) +
-                             launch_time(4.0 * kappa * (g1 ? ROUND_G1 : ROUND_G2), points / per_warp, alone);
+            const double chain = done == kappa && kappa == 1 ? 0.0 : multiples_time(g1, multiples, alone).time;
+            const double t = best[done - kappa] + chain +
+                             launch_time(4.0 * kappa * (g1 ? 360.0 : 530.0), points / (g1 ? 8 : 4), alone);
             if (best[done] < 0 || t < best[done]) best[done] = t, last[done] = kappa;
         }
     }
@@ -341,7 +341,7 @@ uint8_t* launch_quad_ntt(Group g, uint8_t* work, uint8_t* other, const uint8_t* 
     quad_ntt_plan(g, bits, count, steps, &nsteps);
     const bool g1 = g == GROUP_G1;
     const size_t rec = g1 ? G1_XYZZ : G2_XYZZ;
-    const int per_warp = g1 ? SizeOf<OnLane>::PER_WARP : SizeOf<OnPair>::PER_WARP, digits = g1 ? 2 : 4;
+    const int per_warp = g1 ? SizeOf<G1Quad>::PER_WARP : SizeOf<G2Quad>::PER_WARP, digits = g1 ? 2 : 4;
     int64_t most = 0;
     for (int i = 0; i < nsteps; i++) most = std::max<int64_t>(most, ((1 << (2 * steps[i])) - 1) / 3 * (n >> steps[i]) * count);
     uint8_t* multiples = nullptr;
@@ -355,13 +355,17 @@ uint8_t* launch_quad_ntt(Group g, uint8_t* work, uint8_t* other, const uint8_t* 
         while (2 * L <= per_warp && 2 * L <= (1 << kappa) && (double)(outs * 2 * L) / per_warp <= 1.6 * schedulers()) L *= 2;
         note_launch(2);
         if (g1) {
-            k_ntt_multiples<OnLane><<<blocks_for(total * digits, per_warp), WARP, 0, s>>>(multiples, work, tw, n, h, kappa,
-                                                                                       total, per);
-            k_ntt_sums<OnLane><<<blocks_for(outs * L, per_warp), WARP, 0, s>>>(other, work, multiples, h, kappa, outs, per, L);
+            if (multiples_time(true, (double)(total * digits), 1.6).eight)
+                k_ntt_multiples<Oct><<<blocks_for(total * digits, SizeOf<Oct>::PER_WARP), WARP, 0, s>>>(
+                    multiples, work, tw, n, h, kappa, total, per);
+            else
+                k_ntt_multiples<G1Quad><<<blocks_for(total * digits, per_warp), WARP, 0, s>>>(multiples, work, tw, n, h, kappa,
+                                                                                           total, per);
+            k_ntt_sums<G1Quad><<<blocks_for(outs * L, per_warp), WARP, 0, s>>>(other, work, multiples, h, kappa, outs, per, L);
         } else {
-            k_ntt_multiples<OnPair><<<blocks_for(total * digits, per_warp), WARP, 0, s>>>(multiples, work, tw, n, h, kappa,
+            k_ntt_multiples<G2Quad><<<blocks_for(total * digits, per_warp), WARP, 0, s>>>(multiples, work, tw, n, h, kappa,
                                                                                        total, per);
-            k_ntt_sums<OnPair><<<blocks_for(outs * L, per_warp), WARP, 0, s>>>(other, work, multiples, h, kappa, outs, per, L);
+            k_ntt_sums<G2Quad><<<blocks_for(outs * L, per_warp), WARP, 0, s>>>(other, work, multiples, h, kappa, outs, per, L);
         }
         std::swap(work, other);
         h <<= kappa;
@@ -371,29 +375,38 @@ uint8_t* launch_quad_ntt(Group g, uint8_t* work, uint8_t* other, const uint8_t* 
 }
 
 void launch_quad_small_msm(Group g, uint8_t* out, const uint8_t* points, const int64_t* pbase, const int32_t* idx,
-                           const uint8_t* scalars, const int32_t* vsel, int64_t k, int64_t n, int L, cudaStream_t s) {
+                           const uint8_t* scalars, const int32_t* vsel, int64_t k, int64_t n, int L, bool eight, cudaStream_t s) {
     note_launch();
-    if (g == GROUP_G1)
-        k_small_msm<OnLane><<<blocks_for(L * k, SizeOf<OnLane>::PER_WARP), WARP, 0, s>>>(out, points, pbase, idx, scalars,
+    if (g == GROUP_G2)
+        k_small_msm<G2Quad><<<blocks_for(L * k, SizeOf<G2Quad>::PER_WARP), WARP, 0, s>>>(out, points, pbase, idx, scalars,
                                                                                       vsel, k, n, L);
+    else if (eight)
+        k_small_msm<Oct><<<blocks_for(L * k, SizeOf<Oct>::PER_WARP), WARP, 0, s>>>(out, points, pbase, idx, scalars, vsel,
+                                                                                k, n, L);
     else
-        k_small_msm<OnPair><<<blocks_for(L * k, SizeOf<OnPair>::PER_WARP), WARP, 0, s>>>(out, points, pbase, idx, scalars,
+        k_small_msm<G1Quad><<<blocks_for(L * k, SizeOf<G1Quad>::PER_WARP), WARP, 0, s>>>(out, points, pbase, idx, scalars,
                                                                                       vsel, k, n, L);
 }
 
 void launch_quad_mul_batch(Group g, uint8_t* out, const uint8_t* pts, int64_t stride, const uint8_t* scalars, int64_t n,
-                           cudaStream_t s) {
+                           bool eight, cudaStream_t s) {
     note_launch();
-    if (g == GROUP_G1)
-        k_mul_batch<OnLane><<<blocks_for(n, SizeOf<OnLane>::PER_WARP), WARP, 0, s>>>(out, pts, stride, scalars, n);
+    if (g == GROUP_G2)
+        k_mul_batch<G2Quad><<<blocks_for(n, SizeOf<G2Quad>::PER_WARP), WARP, 0, s>>>(out, pts, stride, scalars, n);
+    else if (eight)
+        k_mul_batch<Oct><<<blocks_for(n, SizeOf<Oct>::PER_WARP), WARP, 0, s>>>(out, pts, stride, scalars, n);
     else
-        k_mul_batch<OnPair><<<blocks_for(n, SizeOf<OnPair>::PER_WARP), WARP, 0, s>>>(out, pts, stride, scalars, n);
+        k_mul_batch<G1Quad><<<blocks_for(n, SizeOf<G1Quad>::PER_WARP), WARP, 0, s>>>(out, pts, stride, scalars, n);
 }
 
 void launch_quad_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t* R, const uint8_t* sresp, const uint8_t* c,
-                                int64_t n, const uint8_t* gen_table, cudaStream_t s) {
+                                int64_t n, const uint8_t* gen_table, bool eight, cudaStream_t s) {
     note_launch();
-    k_schnorr_verify<<<blocks_for(4 * n, SizeOf<OnLane>::PER_WARP), WARP, 0, s>>>(valid, X, R, sresp, c, n, gen_table);
+    if (eight)
+        k_schnorr_verify<Oct><<<blocks_for(4 * n, SizeOf<Oct>::PER_WARP), WARP, 0, s>>>(valid, X, R, sresp, c, n, gen_table);
+    else
+        k_schnorr_verify<G1Quad><<<blocks_for(4 * n, SizeOf<G1Quad>::PER_WARP), WARP, 0, s>>>(valid, X, R, sresp, c, n,
+                                                                                           gen_table);
 }
 
 void launch_fixed_msm_g2(uint8_t* out, const uint8_t* tables, const int64_t* tbase, const int32_t* tidx,

@@ -66,6 +66,18 @@ inline double launch_time(double work, double warps, double alone = 1.6) {
     return work * std::max(alone, warps / schedulers());
 }
 
+// The time, in launch_time's measure, of `points` chains of `dbls` doublings and
+// `adds` additions on quads or, in G1, on eight lanes each (quad.cuh); `eight`
+// tells which is the shorter.  A quad's doubling is three rounds of products and
+// its addition four, 360 wide multiply-adds a lane with their exchanges (530 in
+// G2); eight lanes take two rounds of 380 for either.
+struct ChainTime { double time; bool eight; };
+inline ChainTime chain_time(bool g1, double dbls, double adds, double points, double alone = 1.6) {
+    const double quads = launch_time((3 * dbls + 4 * adds) * (g1 ? 360.0 : 530.0), points / (g1 ? 8 : 4), alone);
+    const double eights = launch_time(2 * (dbls + adds) * 380.0, points / 4, alone);
+    return g1 && eights < quads ? ChainTime{eights, true} : ChainTime{quads, false};
+}
+
 constexpr size_t G1_AFF = 96, G2_AFF = 192, G1_XYZZ = 192, G2_XYZZ = 384, GT_SZ = 576, FR_SZ = 32;
 constexpr size_t LINE_SZ = 288;  // three Fp2 coefficients
 constexpr int LINES_PER_POINT = 68;
@@ -161,11 +173,11 @@ uint8_t* launch_quad_ntt(Group g, uint8_t* work, uint8_t* other, const uint8_t* 
 double quad_ntt_plan(Group g, int bits, int64_t count, int* steps, int* nsteps);
 // launch_small_msm with the (term, digit) pairs of an output on L points
 void launch_quad_small_msm(Group g, uint8_t* out, const uint8_t* points, const int64_t* pbase, const int32_t* idx,
-                           const uint8_t* scalars, const int32_t* vsel, int64_t k, int64_t n, int L, cudaStream_t s);
+                           const uint8_t* scalars, const int32_t* vsel, int64_t k, int64_t n, int L, bool eight, cudaStream_t s);
 void launch_quad_mul_batch(Group g, uint8_t* out, const uint8_t* pts, int64_t stride, const uint8_t* scalars, int64_t n,
-                           cudaStream_t s);
+                           bool eight, cudaStream_t s);
 void launch_quad_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t* R, const uint8_t* sresp, const uint8_t* c,
-                                int64_t n, const uint8_t* gen_table, cudaStream_t s);
+                                int64_t n, const uint8_t* gen_table, bool eight, cudaStream_t s);
 // Scratch-size query and launch with caller-supplied scratch (no allocation).
 size_t msm_family_scratch_bytes(Group g, int32_t V, int64_t k, int64_t n, const MsmPlan& plan);
 void launch_msm_family_scratch(Group g, uint8_t* out, const uint8_t* points, const int64_t* pbase, const int32_t* idx,

@@ -13,9 +13,10 @@
 // multiply-adds per lane against 900 for three products on one lane).
 //
 // Measured on B200 against one thread per point (or per digit of it): the tail
-// of a G1 MSM 4.0 -> 1.25 ms and of a G2 MSM 9.1 -> 2.1 ms, transforms of 1,024
-// points 16.5 -> 6.1 ms in G1 and 26.0 -> 4.7 ms in G2, 512 Schnorr checks
-// 2.9 -> 0.8 ms, 128 multiples in G1 3.3 -> 1.05 ms.
+// of a G1 MSM 4.0 -> 1.25 ms and of a G2 MSM 9.1 -> 1.8 ms, transforms of 1,024
+// points 16.5 -> 2.9 ms in G1 and 26.0 -> 4.7 ms in G2, 512 Schnorr checks
+// 2.9 -> 0.8 ms, 128 multiples in G1 3.3 -> 1.05 ms; G1 calls of fewer points take
+// eight lanes (Oct).
 //
 // All lanes of a warp run every step (shuffles name the whole warp); special
 // cases are selected afterwards.
@@ -57,8 +58,6 @@ struct OnLane {  // Fp
     static WBTE_INL uint32_t all_lanes(uint32_t ballot) { return ballot; }
     static WBTE_INL Fp one() { return fp_one(); }
     static WBTE_INL Fp inv(const Fp& a) { return fp_inv(a); }
-    // the curve's b / 4 times a
-    static WBTE_INL Fp times_b4(const Fp& a) { return a; }
 };
 struct OnPair {  // Fp2, component = lane parity
     static constexpr int LANES = 2;
@@ -113,6 +112,7 @@ struct OnPair {  // Fp2, component = lane parity
 // With PLACES = 8 the places past the coordinates make room for the fifth
 // product of a doubling in two rounds (dbl_on_curve).
 template <class P, int PLACES = 4> struct Quad {
+    using Field = P;
     static constexpr int L = P::LANES, WIDTH = PLACES * L;  // lanes per point
     static WBTE_INL int lane() { return threadIdx.x & 31; }
     static WBTE_INL int place() { return (lane() / L) & (PLACES - 1); }  // 0 X, 1 Y, 2 ZZ, 3 ZZZ
@@ -241,65 +241,183 @@ template <class P, int PLACES = 4> struct Quad {
     }
     // the value of the point `points` further on in the warp
     static WBTE_INL Fp above(const Fp& p, int points) { return fp_shfl(p, (lane() + points * WIDTH) & 31); }
-    // sum over groups of n neighbouring points, valid in the first of each
-    static WBTE_INL Fp group_sum(Fp p, int n) {
-        for (int w = 1; w < n; w *= 2) p = add(p, above(p, w), true);
-        return p;
+};
+
+// G1 points for the calls with the fewest: homogeneous X, Y, Z at the first three
+// of eight lanes, the others carry anything between operations.  Both operations
+// are two rounds of products: the complete addition for odd order and a = 0 of
+// Renes, Costello and Batina (six products in each round, no special cases to
+// select) and the doubling that goes with it, on the isomorphic curve
+// y^2 = x^3 + 2/3, where their 3b is 2: (x, y) -> (u^2 x, u^3 y), u^6 = 1/6.  That
+// small constant and factors that are sums without reduction (their product
+// below 9 p^2) leave the second round's factors a few carry chains away from the
+// first's results, and one reduction at the end.
+// Measured on B200 against quads: 512 Schnorr checks 0.81 -> 0.51 ms, 128
+// multiples 1.05 -> 0.68 ms, transforms of 32 points 1.5 -> 1.05 ms, the tail of an
+// MSM 1.11 -> 0.95 ms.  Eight lanes cost as many product slots as a quad for an
+// addition and a third more for a doubling, so calls with more points than
+// schedulers take quads (chain_time).
+struct Oct {
+    using Field = OnLane;
+    static constexpr int WIDTH = 8;
+    static WBTE_INL int lane() { return threadIdx.x & 31; }
+    static WBTE_INL int place() { return lane() & 7; }
+    static WBTE_INL Fp from(const Fp& a, int s) { return fp_shfl(a, (lane() & ~7) + s); }
+    static WBTE_INL Fp above(const Fp& p, int points) { return fp_shfl(p, (lane() + points * WIDTH) & 31); }
+    static WBTE_INL Fp infinity() { return place() == 1 ? fp_one() : fp_zero(); }
+    static WBTE_INL bool is_inf(const Fp& p) { return (__ballot_sync(FULL, fp_is_zero(p)) >> ((lane() & ~7) + 2)) & 1; }
+    static WBTE_INL Fp neg(const Fp& p) { return place() == 1 ? fp_neg(p) : p; }
+    static WBTE_INL Fp reduce4(Fp a) {
+        fp_csub_2p(a.v, a.v);
+        fp_csub_p(a.v, a.v);
+        return a;
     }
 
-    // The acting of |x|^j: on G2 (-1)^j psi^j, psi acting as [x].  G1 splits
-    // scalars in two 128-bit digits, the second acting as |x|^2 on phi(p) + p.
-    static constexpr int DIGITS = P::G1 ? 2 : 4, TOP = P::G1 ? 32 : 16;
-    static WBTE_INL Fp image(Fp p, int j) {
+    // in line: the two operations together are four products (0.54 -> 0.51 ms for
+    // Schnorr checks against calls)
+    static WBTE_INL Fp mul(const Fp& a, const Fp& b) {
+        Fp r;
+        fp_mont_mul(r.v, a.v, b.v);
+        return r;
+    }
+
+    // with B = Y^2 and z = Z^2: 2 XY (B - 6z), B^2 + 12 z (B - z), 8 YZ B
+    static __device__ __noinline__ Fp dbl(Fp p) {
         const int c = place();
-        if constexpr (P::G1) {
-            const Fp f = c == 0 ? fp_mul(p, fp_from_const(C_GLV_BETA)) : p;
-            const Fp s = add(f, p, true);
-            return j ? s : p;
-        } else {
-            for (int i = 0; i < 3; i++) {
-                // conjugate every coordinate, scale x and y
-                const Fp k = OnPair::odd() ? (c == 0 ? fp_from_const(C_PSI_CX[1]) : fp_from_const(C_PSI_CY[1]))
-                                           : (c == 0 ? fp_from_const(C_PSI_CX[0]) : fp_from_const(C_PSI_CY[0]));
-                const Fp cj = OnPair::odd() ? fp_neg(p) : p;
-                const Fp m = P::mul(cj, k);
-                const Fp n = neg(c < 2 ? m : cj);
-                if (i < j) p = n;
-            }
-            return p;
-        }
+        const Fp s = from(p, c == 3 ? 2 : 1);
+        const Fp r1 = mul(c == 3 ? s : p, s);  // XY, YY, ZY, ZZ
+        const Fp B = from(r1, 1), z = from(r1, 3), n = fp_minus(z);
+        const Fp n2 = fp_add_lazy(n, n), n6 = fp_add_lazy(fp_add_lazy(n2, n2), n2);
+        const Fp z2 = fp_add_lazy(z, z), B2 = fp_add_lazy(B, B), B4 = fp_add_lazy(B2, B2);
+        // XY (B - 6z), B B, YZ 8B, 4z (B - z)
+        const Fp b = c == 1 ? B : fp_add_lazy(c == 2 ? B4 : B, c == 0 ? n6 : (c == 2 ? B4 : n));
+        const Fp r2 = mul(c == 3 ? fp_add_lazy(z2, z2) : r1, b);
+        const Fp t = from(r2, 3);
+        const Fp more = c == 0 ? r2 : (c == 1 ? fp_add_lazy(fp_add_lazy(t, t), t) : fp_zero());
+        return reduce4(fp_add_lazy(r2, more));
     }
 
-    // sum over r < n of [w_r] p_r for w_r = hi_r 2^64 + lo_r < 16^TOP, signed
-    // radix-16 digits over one run of doublings; terms past this point's own
-    // count have zero scalars
-    template <int N> static WBTE_INL Fp straus(const Fp (&p)[N], const uint64_t (&lo)[N], const uint64_t (&hi)[N], int n) {
-        Fp tab[N][8];
-        for (int r = 0; r < n; r++) {
-            tab[r][0] = p[r];
-            tab[r][1] = dbl(p[r]);
-            for (int k = 2; k < 8; k++) tab[r][k] = add(tab[r][k - 1], p[r], true);
-        }
-        Fp acc = infinity();
-        bool started = false;
-        for (int k = TOP; k >= 0; k--) {
-            if (started)
-                for (int i = 0; i < 4; i++) acc = dbl(acc);
-            for (int r = 0; r < n; r++) {
-                const int d = r16_digit(lo[r], hi[r], k, TOP);
-                if (!__any_sync(FULL, d != 0)) continue;
-                started = true;
-                const int a = d < 0 ? -d : d;
-                Fp m = tab[r][a ? a - 1 : 0];
-                if (d < 0) m = neg(m);
-                acc = add(acc, m, d != 0);
-            }
-        }
-        return acc;
+    // with t0, t1, t2 = X1X2, Y1Y2, Z1Z2 and the mixed sums t3 = X1Y2 + X2Y1, t4 of
+    // Y and Z, t5 of X and Z: X = t3 (t1 - 2 t2) - 2 t4 t5, Y = (t1 + 2 t2)(t1 - 2 t2)
+    // + 6 t0 t5, Z = t4 (t1 + 2 t2) + 3 t0 t3.  Lanes of a point agree on `live`
+    // (false: p).
+    static __device__ __noinline__ Fp add(Fp p, Fp q, bool live) {
+        const int c = place();
+        const int i = (int)((0x00010210u >> (4 * c)) & 15u), j = (int)((0x00221000u >> (4 * c)) & 15u);
+        const bool mixed = c >= 3;
+        const Fp pj = from(p, j), qj = from(q, j), none = fp_zero();
+        const Fp r1 = mul(fp_add_lazy(from(p, i), fp_select(mixed, pj, none)),
+                             fp_add_lazy(from(q, i), fp_select(mixed, qj, none)));
+        const Fp g = fp_minus(from(r1, i)), h = fp_minus(from(r1, j));
+        const Fp t = fp_add_lazy(r1, fp_select(mixed, fp_add_lazy(g, h), none));  // below 3p
+        // t3, t1 - 2 t2, t4 | t4, t5, t3 times t1 - 2 t2, t1 + 2 t2, t1 + 2 t2 | t5, 3 t0, 3 t0
+        const Fp f = from(t, (int)((0x00354413u >> (4 * c)) & 15u)), e = from(t, (int)((0x00005111u >> (4 * c)) & 15u));
+        const Fp t2 = from(t, 2), n = fp_minus(t2), n2 = fp_add_lazy(n, n);
+        const Fp x = c == 3 ? none : (c > 3 ? e : (c == 0 ? n : t2));
+        const Fp r2 = mul(fp_add_lazy(f, fp_select(c == 1, n2, none)), fp_add_lazy(e, fp_add_lazy(x, x)));
+        const Fp o = from(r2, c < 3 ? c + 3 : c);
+        const Fp y = c == 0 ? fp_minus(o) : o;
+        const Fp r = reduce4(fp_add_lazy(fp_add_lazy(r2, y), c == 2 ? none : y));
+        return live ? r : p;
+    }
+
+    // from and to memory: affine points in blst's layout, XYZZ records
+    static WBTE_INL Fp load_affine(const uint8_t* pt) {
+        const Fp v = load_vec(reinterpret_cast<const Fp*>(pt + 48 * (place() & 1)));
+        const uint32_t zeros = __ballot_sync(FULL, fp_is_zero(v)) >> (lane() & ~7);
+        const Fp k = fp_mul(v, fp_from_const(C_ISO_IN[place() & 1]));
+        return (zeros & 3) == 3 ? infinity() : (place() < 2 ? k : (place() == 2 ? fp_one() : fp_zero()));
+    }
+    // x / zz and y / zzz over the common denominator zz zzz
+    static WBTE_INL Fp load(const uint8_t* xyzz) {
+        const Fp v = load_vec(reinterpret_cast<const Fp*>(xyzz + 48 * (place() & 3)));
+        const Fp w = fp_mul(v, from(v, place() == 1 ? 2 : 3));
+        const Fp r = fp_mul(w, place() < 2 ? fp_from_const(C_ISO_IN[place() & 1]) : fp_one());
+        return is_inf(v) ? infinity() : r;
+    }
+    static WBTE_INL void store(uint8_t* xyzz, const Fp& p) {
+        const int c = place();
+        const Fp z = from(p, 2);
+        const Fp z2 = fp_mul(z, z);
+        // X z, Y z^2, z^2, z^3
+        const Fp a = fp_mul(c < 2 ? p : z2, c == 1 ? z2 : z);
+        const Fp r = fp_mul(c == 2 ? z2 : a, c < 2 ? fp_from_const(C_ISO_OUT[c & 1]) : fp_one());
+        const Fp s = is_inf(p) ? infinity() : r;
+        if (c < 4) store_vec(reinterpret_cast<Fp*>(xyzz + 48 * c), s);
+    }
+    static WBTE_INL Fp affine(const Fp& p) {
+        const Fp r = fp_mul(fp_mul(p, fp_inv(from(p, 2))), fp_from_const(C_ISO_OUT[place() & 1]));
+        return is_inf(p) ? fp_zero() : r;
+    }
+    static WBTE_INL void store_affine(uint8_t* pt, const Fp& a) {
+        if (place() < 2) store_vec(reinterpret_cast<Fp*>(pt + 48 * place()), a);
     }
 };
 
-// the digits of a canonical scalar that act through Quad::image
+// ----------------------------------------------------- sums and multiples
+// Q: a point's spread, Quad or Oct.
+// sum over groups of n neighbouring points, valid in the first of each
+template <class Q> WBTE_INL Fp quad_sum(Fp p, int n) {
+    for (int w = 1; w < n; w *= 2) p = Q::add(p, Q::above(p, w), true);
+    return p;
+}
+
+// The acting of |x|^j: on G2 (-1)^j psi^j, psi acting as [x].  G1 splits scalars
+// in two 128-bit digits, the second acting as |x|^2 on phi(p) + p.
+template <class Q> struct QuadDigits {
+    static constexpr int DIGITS = Q::Field::G1 ? 2 : 4, TOP = Q::Field::G1 ? 32 : 16;
+};
+template <class Q> WBTE_INL Fp quad_image(Fp p, int j) {
+    const int c = Q::place();
+    if constexpr (Q::Field::G1) {
+        const Fp f = c == 0 ? fp_mul(p, fp_from_const(C_GLV_BETA)) : p;
+        const Fp s = Q::add(f, p, true);
+        return j ? s : p;
+    } else {
+        for (int i = 0; i < 3; i++) {
+            // conjugate every coordinate, scale x and y
+            const Fp k = OnPair::odd() ? (c == 0 ? fp_from_const(C_PSI_CX[1]) : fp_from_const(C_PSI_CY[1]))
+                                       : (c == 0 ? fp_from_const(C_PSI_CX[0]) : fp_from_const(C_PSI_CY[0]));
+            const Fp cj = OnPair::odd() ? fp_neg(p) : p;
+            const Fp m = Q::Field::mul(cj, k);
+            const Fp n = Q::neg(c < 2 ? m : cj);
+            if (i < j) p = n;
+        }
+        return p;
+    }
+}
+
+// sum over r < n of [w_r] p_r for w_r = hi_r 2^64 + lo_r < 16^TOP, signed
+// radix-16 digits over one run of doublings; terms past this point's own
+// count have zero scalars
+template <class Q, int N>
+WBTE_INL Fp quad_straus(const Fp (&p)[N], const uint64_t (&lo)[N], const uint64_t (&hi)[N], int n) {
+    constexpr int TOP = QuadDigits<Q>::TOP;
+    Fp tab[N][8];
+    for (int r = 0; r < n; r++) {
+        tab[r][0] = p[r];
+        tab[r][1] = Q::dbl(p[r]);
+        for (int k = 2; k < 8; k++) tab[r][k] = Q::add(tab[r][k - 1], p[r], true);
+    }
+    Fp acc = Q::infinity();
+    bool started = false;
+    for (int k = TOP; k >= 0; k--) {
+        if (started)
+            for (int i = 0; i < 4; i++) acc = Q::dbl(acc);
+        for (int r = 0; r < n; r++) {
+            const int d = r16_digit(lo[r], hi[r], k, TOP);
+            if (!__any_sync(FULL, d != 0)) continue;
+            started = true;
+            const int a = d < 0 ? -d : d;
+            Fp m = tab[r][a ? a - 1 : 0];
+            if (d < 0) m = Q::neg(m);
+            acc = Q::add(acc, m, d != 0);
+        }
+    }
+    return acc;
+}
+
+// the digits of a canonical scalar that act through quad_image
 template <class P> WBTE_INL void quad_digit(uint64_t& lo, uint64_t& hi, const uint64_t d[4], int j) {
     if constexpr (P::G1) {
         const uint64_t plo = d[2 * j + 1] * X_ABS, phi = __umul64hi(d[2 * j + 1], X_ABS);
