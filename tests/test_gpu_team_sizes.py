@@ -48,3 +48,16 @@ def test_transforms(n, count):
         got = ops.split(ops.gt_ntt_many(b"".join(v for a in _tile(arrays, count) for v in a), n, inverse=inv), 576)
         want = [orc.gt_ntt(a, inverse=inv) for a in arrays]
         assert got == [v for a in _tile(want, count) for v in a]
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 7, 1184])
+def test_torus_encodings_of_few_values(n):
+    """Against one thread per value, which longer calls take."""
+    rng = random.Random(n)
+    one = orc.fp12_one()
+    kinds = orc.gt_pow_many(orc.pairing(orc.g1_generator(), orc.g2_generator()), _rs(rng, 4))
+    kinds += [one, bytes(288) + kinds[0][288:], kinds[1][:288] + bytes(288), bytes(576)]
+    many = 1500
+    want = ops.split(ops.gt_compress(b"".join(_tile(kinds, many)), many), 289)
+    assert ops.split(ops.gt_compress(b"".join(_tile(kinds, n)), n), 289) == want[:n]
+    assert want[4] == bytes(289)

@@ -191,11 +191,6 @@ __global__ void k_offsets(int64_t* off, int64_t n, int64_t step) {
     if (i < n) off[i] = i * step;
 }
 
-WBTE_INL void fp_store_be48(uint8_t* out, const Fp& m) {
-    Fp c = fp_from_mont(m);
-    for (int i = 0; i < 48; i++) out[47 - i] = (uint8_t)(c.v[i >> 2] >> (8 * (i & 3)));
-}
-
 // Tagged torus compression of GT: identity -> 0; otherwise 1 followed by the
 // six Fp2 coefficients of (c0 + 1) / c1, each Fp as 48 big-endian bytes.
 __global__ void k_gt_compress(uint8_t* out, const uint8_t* in, int64_t n) {
@@ -217,6 +212,34 @@ __global__ void k_gt_compress(uint8_t* out, const uint8_t* in, int64_t n) {
         fp_store_be48(o + 1 + 96 * k, cs[k]->c0);
         fp_store_be48(o + 1 + 96 * k + 48, cs[k]->c1);
     }
+}
+
+// The same by teams, for few values: 1 / c1 = N^(p^2) N^(p^4) / (N N^(p^2) N^(p^4))
+// for N = c1 in Fp6.  Measured on B200: 512 values 0.14 -> 0.07 ms; one thread per value
+// once a team's copies of the inversion no longer run on idle schedulers.
+template <class T>
+__global__ void __launch_bounds__(32 * T::WARPS, T6_BLOCKS / T::WARPS) k_gt_compress_team(uint8_t* out, const uint8_t* in, int64_t n) {
+    extern __shared__ uint4 sh[];
+    const Team t = team_of<T>(sh);
+    int64_t i = team_index<T>();
+    const bool active = i < n;
+    if (!active) i = n - 1;
+    const ElemOf<T> f = team_load<T>(t, in + GT_SZ * i), one = team_one<T>(t), zero = T::f_sub(one, one);
+    const uint32_t differ = __ballot_sync(FULL, !T::same(f, one));
+    const bool odd = t.k & 1, is_one = !((differ >> (t.base / 6 * T::LANES)) & ((1u << T::LANES) - 1u));
+    __syncwarp();
+    T::st(t, T6_A, t.base + t.k, f);
+    __syncwarp();
+    const ElemOf<T> above = T::ld(t, T6_A, t.base + (t.k | 1));
+    const ElemOf<T> c1 = odd ? zero : above, sum = T::f_add(f, one), c0 = odd ? zero : sum;
+    const ElemOf<T> c2 = team_frobenius<T>(t, c1, 2);
+    const ElemOf<T> m = T::mul(t, c2, team_frobenius<T>(t, c2, 2));
+    const ElemOf<T> d = team_inverse_of_first<T>(t, T::mul(t, c1, m));
+    const ElemOf<T> r = T::mul(t, c0, T::f_mul(m, d));
+    if (!active || odd) return;
+    uint8_t* o = out + 289 * i;
+    if (t.k == 0 && t.h == 0) o[0] = is_one ? 0 : 1;
+    T::store_be(t, o + 1 + 48 * t.k, is_one ? zero : r);
 }
 
 __global__ void k_fp12_conj(uint8_t* out, const uint8_t* in, int64_t n) {
@@ -398,7 +421,10 @@ void launch_gt_compress(uint8_t* out, const uint8_t* in, int64_t n, cudaStream_t
     ProfScope prof_("gt_compress", s);
     if (n <= 0) return;
     note_launch();
-    k_gt_compress<<<blocks_for(n), TPB, 0, s>>>(out, in, n);
+    if (few_values(n))
+        team_launch<Twelve>(k_gt_compress_team<Twelve>, n, Twelve::PER, s, out, in, n);
+    else
+        k_gt_compress<<<blocks_for(n), TPB, 0, s>>>(out, in, n);
 }
 void launch_fp12_conj(uint8_t* out, const uint8_t* in, int64_t n, cudaStream_t s) {
     if (n <= 0) return;

@@ -511,6 +511,12 @@ static __device__ __noinline__ Fp t12_mul_line(Team t, Fp f, int component, Fp l
     return t12_reduce(t, acc, false);
 }
 
+// the canonical value as 48 big-endian bytes
+WBTE_INL void fp_store_be48(uint8_t* out, const Fp& m) {
+    Fp c = fp_from_mont(m);
+    for (int i = 0; i < 48; i++) out[47 - i] = (uint8_t)(c.v[i >> 2] >> (8 * (i & 3)));
+}
+
 // --------------------------------------------------- what both kinds of team do
 // E: what a lane holds of an Fp12 value's coefficient, and so of any Fp2 value
 // that the team computes with.
@@ -528,6 +534,11 @@ struct Six {
     static WBTE_INL E of(const Team&, const Fp2& a) { return a; }
     static WBTE_INL E load(const Team&, const uint8_t* v) { return load_vec(reinterpret_cast<const Fp2*>(v)); }
     static WBTE_INL void store(const Team&, uint8_t* v, const E& a) { store_vec(reinterpret_cast<Fp2*>(v), a); }
+    static WBTE_INL void store_be(const Team&, uint8_t* v, const E& a) {
+        fp_store_be48(v, a.c0);
+        fp_store_be48(v + 48, a.c1);
+    }
+    static WBTE_INL bool same(const E& a, const E& b) { return fp_eq(a.c0, b.c0) && fp_eq(a.c1, b.c1); }
     static WBTE_INL E ld(const Team& t, int row, int slot) { return team_ld<Fp2>(t, row, slot); }
     static WBTE_INL void st(const Team& t, int row, int slot, const E& a) { team_st(t, row, slot, a); }
     static WBTE_INL E f_add(const E& a, const E& b) { return fp2_add(a, b); }
@@ -550,6 +561,8 @@ struct Twelve {
     static WBTE_INL E of(const Team& t, const Fp2& a) { return fp_select(t.h, a.c1, a.c0); }
     static WBTE_INL E load(const Team& t, const uint8_t* v) { return load_vec(reinterpret_cast<const Fp*>(v) + t.h); }
     static WBTE_INL void store(const Team& t, uint8_t* v, const E& a) { store_vec(reinterpret_cast<Fp*>(v) + t.h, a); }
+    static WBTE_INL void store_be(const Team& t, uint8_t* v, const E& a) { fp_store_be48(v + 48 * t.h, a); }
+    static WBTE_INL bool same(const E& a, const E& b) { return fp_eq(a, b); }
     static WBTE_INL E ld(const Team& t, int row, int slot) { return team_ld<Fp>(t, row + 3 * t.h, slot); }
     static WBTE_INL void st(const Team& t, int row, int slot, const E& a) { team_st(t, row + 3 * t.h, slot, a); }
     static WBTE_INL E f_add(const E& a, const E& b) { return fp_add(a, b); }
