@@ -892,16 +892,16 @@ def main():
     ms_of = {k: v[0] for k, v in prof_g.items()}
     top_g = max(prof_g.items(), key=lambda kv: kv[1][0])
     traffic = load_traffic()
-    peak_basis = (f"measured {float(rate[0]) / 1e12:.2f} T IMAD/s (calibration kernel, mad.lo/mad.hi mix) / "
+    peak_basis = (f"measured {float(rate[0]) / 1e12:.2f} T IMAD/s (calibration kernel, carry-joined mad.lo/mad.hi pairs) / "
                   f"{IMAD_PER_FP_MUL} IMAD per Fp product")
     with open(os.path.join(ROOT, "weighted_bte_b200", "algorithmic_work.json")) as f:
         work = json.load(f)
     gt_own = wc.gt_prefix_ifft(m, B, G) if G % 32 == 0 and G >= 32 else None
-    roofline = roof("gt_ifft (truncated cyclotomic inverse transform of a group: k_gt_radix4_pows_plan + "
+    roofline = roof("gt_ifft (truncated cyclotomic inverse transform of a group: k_gt_radix4_pows + "
                     "k_gt_radix4_outputs per radix-4 stage)", ms_of.get("gt_ifft"), gt_own or 0, peak,
                     peak_basis=peak_basis, batches_per_launch=G, dominant_in_group=top_g[0] == "gt_ifft",
-                    work_basis="exact count of the Fp products the kernels run (warp-uniform NAF plans of the "
-                               "twiddles, butterfly outputs); Fp additions not counted")
+                    work_basis="Fp products of the tower formulas over the twiddles' NAF digits and the butterfly "
+                               "outputs; the kernels reduce sums of products once, so they run fewer multiply-adds")
     tr = traffic.get("gt_ifft")
     if tr and ms_of.get("gt_ifft") and tr.get("group") == G and tr.get("batch_size") == B:
         # DRAM bytes of the phase's launches in one group, from the committed

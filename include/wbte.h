@@ -65,14 +65,16 @@ int32_t wbte_ctx_set_stream(wbte_ctx *ctx, void *cuda_stream);
 int32_t wbte_ctx_synchronize(wbte_ctx *ctx);
 /* Knobs of the launchers' cost models for every later call on this context
  * (the per-size-class autotuner sets them; results never depend on them):
- *   WBTE_TUNE_GT_LANES     lanes per GT exponentiation in the radix-4 stages
- *                          of the GT transforms: 1, 2 or 4 (0: cost model)
+ *   WBTE_TUNE_GT_LANES     teams of six lanes per GT exponentiation in the
+ *                          GT transforms and powers: 1, 2 or 4 (0: cost
+ *                          model, which may also take teams of twelve)
  *   WBTE_TUNE_MSM_WINDOW   Pippenger window width c, 4..13 (0: cost model)
  *   WBTE_TUNE_MSM_SEGMENTS sorted-term segments per (MSM, window), 1..1024
  *                          (0: cost model)
  *   WBTE_TUNE_NTT_JOINT    G1/G2 transform stages: 1 one thread per
- *                          butterfly, 0 the lane split (-1: cost model)
- *   WBTE_TUNE_MILLER_CHUNK pairs per thread of the share checks' unprepared
+ *                          butterfly, 0 several lanes per point (-1: cost
+ *                          model)
+ *   WBTE_TUNE_MILLER_CHUNK pairs per team of the share checks' unprepared
  *                          multi-Miller loops, 1..8 (0: cost model)
  * WBTE_ERR_INVALID_ARG for an unknown knob or a value out of range. */
 #define WBTE_TUNE_GT_LANES 1
@@ -92,8 +94,8 @@ uint64_t wbte_thread_launch_count(void);
  * the summed milliseconds and the number of launches (names are written as
  * NUL-terminated strings name_stride bytes apart). */
 int32_t wbte_profile_enable(int32_t on);
-/* Measures the sustained rate of 32-bit integer multiply-add instructions
- * (mad.lo/mad.hi) on the context's GPU with a calibration kernel; the
+/* Measures the sustained rate of 32-bit integer multiply-adds (mad.lo/mad.hi
+ * pairs joined by a carry, counted as two) on the context's GPU with a calibration kernel; the
  * denominator of the integer-pipe roofline.  Synchronous. */
 int32_t wbte_measure_imad_rate(wbte_ctx *ctx, double *imad_per_s);
 int32_t wbte_profile_read(char *names, int32_t name_stride, double *ms, int64_t *counts,

@@ -1,8 +1,8 @@
 """Per-size-class autotuner for the batched decryption path.
 
 The kernel launchers choose their shapes from cost models (Pippenger window
-width and segment count, lanes per GT exponentiation in the transforms,
-joint or lane-split G1/G2 transform stages).  A cost model is only as good as
+width and segment count, teams per GT exponentiation in the transforms, one
+thread or several lanes per point in the G1/G2 transform stages).  A cost model is only as good as
 its constants, and the best choice moves with the batch size and with how
 many batches share a launch.  For each size class the autotuner times a few
 candidate knob settings on a trial group of that class (coordinate descent

@@ -768,15 +768,16 @@ __global__ void k_schnorr_verify(uint8_t* valid, const uint8_t* X, const uint8_t
     valid[i] = is_inf(diff) ? 1 : 0;
 }
 
-// Integer-pipe calibration: eight independent chains of 32-bit multiply-adds
-// per thread, half low and half high products (the mix of the CIOS kernel).
+// Integer-pipe calibration: four independent chains per thread of multiply-add
+// pairs that a carry joins, the field products' instruction.
 __global__ void k_imad_probe(uint32_t* sink, int iters) {
-    uint32_t a[8], b = 0x9e3779b9u + threadIdx.x;
+    uint32_t a[8], b = 0x9e3779b9u + threadIdx.x, c = 0x85ebca6bu + blockIdx.x;
     for (int k = 0; k < 8; k++) a[k] = threadIdx.x * 7u + blockIdx.x + (uint32_t)k;
     for (int i = 0; i < iters; i++) {
         _Pragma("unroll") for (int k = 0; k < 8; k += 2) {
-            asm volatile("mad.lo.u32 %0, %0, %1, %0;" : "+r"(a[k]) : "r"(b));
-            asm volatile("mad.hi.u32 %0, %0, %1, %0;" : "+r"(a[k + 1]) : "r"(b));
+            asm volatile("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;"
+                         : "+r"(a[k]), "+r"(a[k + 1])
+                         : "r"(b), "r"(c));
         }
     }
     uint32_t x = 0;
@@ -786,7 +787,8 @@ __global__ void k_imad_probe(uint32_t* sink, int iters) {
 
 }  // namespace
 
-// IMAD instructions per second sustained by the integer pipe (measured).
+// Multiply-adds per second sustained by the integer pipe (measured): pairs of
+// mad.lo and madc.hi that a carry joins, as in the field products, two each.
 double measure_imad_rate(cudaStream_t s) {
     int dev = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -978,8 +980,8 @@ __global__ void k_mul_small(uint8_t* work, const uint8_t* in, const int32_t* coe
     store_vec(reinterpret_cast<Xyzz<F>*>(work) + i, acc);
 }
 
-// Points per thread of the batched conversions: one inversion (about 485
-// Fp products) per chunk against about 7 products per point, so chunks grow
+// Points per thread of the batched conversions: one inversion (50 us by division
+// steps, the time of about 40 dependent products) per chunk against about 7 products per point, so chunks grow
 // only while the launch still fills the resident threads.
 static int64_t normalize_chunk(int64_t n) {
     int dev = 0, sms = 148;

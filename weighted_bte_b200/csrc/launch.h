@@ -37,10 +37,10 @@ struct ProfScope {
 // context's knobs (wbte_ctx_set_tuning) here for its duration; the
 // per-size-class autotuner measures candidate values through them.
 struct Tuning {
-    int gt_lanes = 0;      // lanes per GT exponentiation in the radix-4 transform stages: 1, 2 or 4
+    int gt_lanes = 0;      // teams of six lanes per GT exponentiation in the radix-4 transform stages: 1, 2 or 4
     int msm_window = 0;    // Pippenger window width c, 4..13
     int msm_segments = 0;  // sorted-term segments per (MSM, window), 1..1024
-    int ntt_joint = -1;    // G1/G2 transform stages: 1 one thread per butterfly, 0 the lane split
+    int ntt_joint = -1;    // G1/G2 transform stages: 1 one thread per butterfly, 0 quads
     int miller_chunk = 0;  // pairs per thread of the chunked unprepared Miller loops, 1..8
 };
 extern thread_local Tuning g_tune;

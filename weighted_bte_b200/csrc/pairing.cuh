@@ -1,5 +1,6 @@
-// Optimal-ate Miller loop over the M-type twist E'(Fp2): y^2 = x^3 + 4(1+u),
-// split final exponentiation, and the decomposed GT exponentiation.
+// What the pairing and the decomposed exponentiations rest on: the lines of the
+// optimal-ate Miller loop over the M-type twist E'(Fp2): y^2 = x^3 + 4(1+u), which
+// team.cuh computes, and the recodings of scalars in base |x|.
 //
 // Lines.  For T on E' and P = (xP, yP) in G1 the line through the untwisted
 // points, scaled by w^3 and by an Fp2 factor (both killed by the easy part
@@ -8,10 +9,6 @@
 //   addition (T + Q, Q affine):          c0 = u xQ - v yQ,  c1 = -u,   c2 = v
 // where u = yQ Z - Y, v = xQ Z - X.  Only final-exponentiated values are
 // canonical, so this scaling is free to differ from any other implementation.
-//
-// The hard part follows the addition chain of the reference,
-// btx/src/final_exponentiation.rs:255-283 (with raise_to_z at :399-413),
-// which computes f^(3 (p^4 - p^2 + 1) / r).
 #pragma once
 #include "curves.cuh"
 
@@ -19,50 +16,8 @@ namespace wbte {
 
 constexpr int MILLER_LINES = 68;  // 63 doublings + 5 additions for |x|
 
-struct Line { Fp2 c0, c1, c2; };
-struct G2Proj { Fp2 X, Y, Z; };
-
 WBTE_INL Fp2 fp2_mul3(const Fp2& a) { return fp2_add(fp2_dbl(a), a); }
 WBTE_INL Fp2 fp2_mul4(const Fp2& a) { return fp2_dbl(fp2_dbl(a)); }
-
-// T <- 2T, returns the tangent line.
-static __device__ __noinline__ Line line_double(G2Proj& T) {
-    Fp2 t0 = fp2_sqr(T.Y);
-    Fp2 t1 = fp2_sqr(T.Z);
-    Fp2 t2 = fp2_mul4(fp2_mul3(fp2_mul_xi(t1)));  // 3 b' Z^2, b' = 4 (1 + u)
-    Fp2 X2 = fp2_sqr(T.X);
-    Fp2 YZ = fp2_mul(T.Y, T.Z);
-    Fp2 XY = fp2_mul(T.X, T.Y);
-    Line l;
-    l.c0 = fp2_sub(t2, t0);
-    l.c1 = fp2_mul3(X2);
-    l.c2 = fp2_neg(fp2_dbl(YZ));
-    Fp2 t23 = fp2_mul3(t2);
-    T.X = fp2_dbl(fp2_mul(XY, fp2_sub(t0, t23)));
-    T.Y = fp2_sub(fp2_sqr(fp2_add(t0, t23)), fp2_mul4(fp2_mul3(fp2_sqr(t2))));
-    T.Z = fp2_mul4(fp2_dbl(fp2_mul(t0, YZ)));
-    return l;
-}
-
-// T <- T + Q, returns the chord.
-static __device__ __noinline__ Line line_add(G2Proj& T, const G2A& Q) {
-    Fp2 u = fp2_sub(fp2_mul(Q.y, T.Z), T.Y);
-    Fp2 v = fp2_sub(fp2_mul(Q.x, T.Z), T.X);
-    Line l;
-    l.c0 = fp2_sub(fp2_mul(u, Q.x), fp2_mul(v, Q.y));
-    l.c1 = fp2_neg(u);
-    l.c2 = v;
-    Fp2 v2 = fp2_sqr(v);
-    Fp2 v3 = fp2_mul(v2, v);
-    Fp2 v2X = fp2_mul(v2, T.X);
-    Fp2 A = fp2_sub(fp2_sub(fp2_mul(fp2_sqr(u), T.Z), v3), fp2_dbl(v2X));
-    T.X = fp2_mul(v, A);
-    T.Y = fp2_sub(fp2_mul(u, fp2_sub(v2X, A)), fp2_mul(v3, T.Y));
-    T.Z = fp2_mul(v3, T.Z);
-    return l;
-}
-
-WBTE_INL G2Proj g2proj_from_affine(const G2A& q) { return G2Proj{q.x, q.y, fp2_one()}; }
 
 // pairs of one run of a Miller loop that computes its lines
 constexpr int MULTI_MILLER_MAX = 8;

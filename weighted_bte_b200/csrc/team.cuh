@@ -657,7 +657,8 @@ template <class T> static __device__ __noinline__ ElemOf<T> team_raise_to_z_div_
 template <class T> WBTE_INL ElemOf<T> team_raise_to_z(const Team& t, const ElemOf<T>& x) {
     return T::cyc_sqr(t, team_raise_to_z_div_by_2<T>(t, x));
 }
-// the addition chain of btx/src/final_exponentiation.rs:255-283
+// the addition chain of btx/src/final_exponentiation.rs:255-283 (raise_to_z at
+// :399-413), which computes f^(3 (p^4 - p^2 + 1) / r)
 template <class T> static __device__ __noinline__ ElemOf<T> team_final_exp_hard(Team t, ElemOf<T> in) {
     const ElemOf<T> y0 = T::cyc_sqr(t, in);
     ElemOf<T> y1 = team_raise_to_z<T>(t, y0);

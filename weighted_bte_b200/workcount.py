@@ -1,15 +1,15 @@
 """Fp-product counts of the library's kernels: the numerators of the
 integer-pipe roofline.
 
-The unit is one 12-limb Montgomery product in Fp (588 multiply-add
-instructions in the CIOS sequence of csrc/field_asm.cuh); Fp additions are
-not counted.  Counts follow the kernels' own formulas (Karatsuba Fp2 / Fp6 /
-Fp12 tower, XYZZ curve formulas, the hard-part chain, warp-uniform NAF plans),
-so `achieved / peak` measures how well the kernel runs the work it does, not
-how much work it avoids.  Counts are exact where the schedule is static
-(Miller loops, final exponentiation, GT transforms whose plans depend only on
-public twiddles); the MSM counts are the expected values of the Pippenger
-plan (nonzero digits of uniform scalars), stated as such.
+The unit is one 12-limb Montgomery product in Fp (288 pairs of multiply-adds and
+12 quotient words, 588 instructions, in csrc/field_asm.cuh); Fp additions are not
+counted.  Counts are those of the textbook formulas over reduced products
+(Karatsuba Fp2 / Fp6 / Fp12 tower, XYZZ curve formulas, the hard-part chain, NAF
+digits of public twiddles, the expected Pippenger digits of uniform scalars), one
+measure for all builds.  The kernels take a different route to the same values
+(double-width sums with one reduction, squarings of their own, eight-lane
+homogeneous chains), so a fraction of peak on these counts compares builds and
+can exceed the pipe's own utilisation.
 """
 from __future__ import annotations
 
@@ -95,7 +95,7 @@ def _naf_len_nonzero(v: int, w: int):
 
 
 def gt_plan_power(s: int) -> int:
-    """k_gt_radix4_pows_plan: the four base-|x| digits of s in width-4 NAF
+    """k_gt_radix4_pows: the four base-|x| digits of s in width-4 NAF
     over one shared run of squarings, with a table of odd powers (1 squaring,
     3 products, 12 Frobenius maps)."""
     longest, nonzero = 0, 0
@@ -226,7 +226,7 @@ def _twiddles(n: int, inverse: bool):
 
 
 def group_ntt_lanes(n: int, g2: bool, inverse: bool = False) -> int:
-    """k_ntt_stage (one transform, the lane split): per butterfly with
+    """One transform with the digits of a multiple apart: per butterfly with
     twiddle t != 1 each lane runs xyzz_mul_r16 on its base-|x| digit group
     (G1: [a]v and [b](phi(v) + v), 128-bit; G2: [d_c] psi^c(v), 64-bit),
     the lanes' parts are added in a tree, and two additions give the outputs."""
@@ -297,7 +297,7 @@ def group_ntt_joint(n: int, g2: bool, inverse: bool = False) -> int:
 
 
 def _gt_lane(d: int, c: int) -> int:
-    """gt_pow_lane: table (Frobenius^c for c > 0, one squaring, six
+    """One digit of a power: table (Frobenius^c for c > 0, one squaring, six
     products), 64 cyclotomic squarings, one product per nonzero digit of the
     17 signed radix-16 digits (the accumulator starts at one)."""
     nz = sum(1 for x in r16_digits(d, 16) if x)
@@ -305,7 +305,7 @@ def _gt_lane(d: int, c: int) -> int:
 
 
 def _gt_one_lane(s: int) -> int:
-    """gt_pow_digits with all four digits on one lane: one table, the shared
+    """All four digits of a power together: one table, the shared
     squarings, per nonzero digit one product (and a Frobenius map for c > 0)."""
     total = CYC_SQR + 6 * FP12_MUL + 64 * CYC_SQR
     for c, d in enumerate(decompose_base_x(s)):
@@ -315,11 +315,9 @@ def _gt_one_lane(s: int) -> int:
 
 
 def gt_ntt_single(n: int, lanes: int, inverse: bool = False) -> int:
-    """One GT transform (gt_transform with count 1): a radix-2 first stage
-    for an odd number of stages (k_gt_stage, four lanes per power, three
-    combine products, two outputs), then radix-4 stages with three powers
-    per butterfly on `lanes` = 4 (k_gt_radix4: four lanes and three combine
-    products per power) or 1 (k_gt_radix4_pows<1>), and four outputs of
+    """One GT transform with each power's digits on `lanes` = 4 teams, which meet in
+    three products, or on 1: a radix-2 first stage for an odd number of stages,
+    then radix-4 stages with three powers per butterfly and four outputs of
     three products, two of them with a Frobenius map (omega_4)."""
     assert lanes in (1, 4) and n >= 4
     w = _twiddles(n, inverse)
