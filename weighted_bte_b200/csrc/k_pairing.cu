@@ -272,7 +272,8 @@ static bool few_values(int64_t n) { return n <= 2 * (int64_t)schedulers(); }
 // teams of six or twelve lanes, C pairs to a team.  Sharing the 62 squarings
 // saves 73 thousand of a lane's wide multiply-adds (45 in a team of twelve) for
 // each further pair of a run; `line` is one pair's 68 lines (LINE_PREPARED,
-// LINE_COMPUTED; the second figure for teams of twelve).
+// LINE_COMPUTED; the second figure for teams of twelve).  Whole turns count (65,664
+// pairs, runs of six instead of eight 28.8 -> 23.0 ms; 49,248, of three 27.5 -> 18.0).
 struct MillerSpread { bool twelve; int64_t C; };
 struct LineWork { double six, twelve; };
 static constexpr LineWork LINE_PREPARED = {130.0, 90.0}, LINE_COMPUTED = {245.0, 160.0};
@@ -281,8 +282,8 @@ static MillerSpread miller_spread(int64_t outputs, int64_t pairs, LineWork line,
     double best_t = 0;
     for (int64_t C = 1; C <= std::min(pairs, most); C++) {
         const double runs = (double)outputs * (double)((pairs + C - 1) / C);
-        const double six = launch_time(73.0 + line.six * C, runs / Six::PER);
-        const double twelve = launch_time(45.0 + line.twelve * C, runs / Twelve::PER);
+        const double six = run_time(73.0 + line.six * C, runs / Six::PER);
+        const double twelve = run_time(45.0 + line.twelve * C, runs / Twelve::PER);
         if (C == 1 || six < best_t) best = {false, C}, best_t = six;
         if (twelve < best_t) best = {true, C}, best_t = twelve;
     }
@@ -350,8 +351,8 @@ static void miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int6
                           int64_t q_mod, cudaStream_t s) {
     const int64_t chunks = (per + C - 1) / C, runs = K * chunks;
     note_launch();
-    if (launch_time(45.0 + LINE_COMPUTED.twelve * C, (double)runs / Twelve::PER) <
-        launch_time(73.0 + LINE_COMPUTED.six * C, (double)runs / Six::PER))
+    if (run_time(45.0 + LINE_COMPUTED.twelve * C, (double)runs / Twelve::PER) <
+        run_time(73.0 + LINE_COMPUTED.six * C, (double)runs / Six::PER))
         team_launch<Twelve>(k_miller_chunks<Twelve>, runs, Twelve::PER, s, out, p, q, per, K, C, chunks, p_mod, q_mod);
     else
         team_launch<SixBlock>(k_miller_chunks<SixBlock>, runs, Six::PER, s, out, p, q, per, K, C, chunks, p_mod, q_mod);

@@ -5,6 +5,7 @@
 //   32-byte little-endian integers, the point at infinity as zero bytes.
 #pragma once
 #include <algorithm>
+#include <cmath>
 #include <atomic>
 #include <cstddef>
 #include <cstdint>
@@ -64,6 +65,14 @@ inline int schedulers() {
 // and at eight warps), so fewer than 1.6 warps a scheduler take as long as 1.6.
 inline double launch_time(double work, double warps, double alone = 1.6) {
     return work * std::max(alone, warps / schedulers());
+}
+
+// The same for kernels with two warps of registers per scheduler and long runs in
+// each: a launch takes whole turns of two warps and a last one of one or two, so a
+// little more than a turn costs most of another.
+inline double run_time(double work, double warps) {
+    const double each = warps / schedulers(), whole = 2 * std::floor(each / 2), rest = each - whole;
+    return work * (whole + (rest > 1 ? 2.0 : (rest > 0 ? 1.6 : 0.0)));
 }
 
 // The time, in launch_time's measure, of `points` chains of `dbls` doublings and
