@@ -266,9 +266,10 @@ struct PowSpread { bool twelve; int L; };
 // From a cost model: the wide multiply-adds of one lane, in thousands.  Teams
 // of six: 64 squarings of 888; products of 1,608, 52 and three for the table with
 // the warp-uniform NAF, 17 a digit and seven for the table in radix 16; table
-// images of 744.  Teams of twelve: 444, 1,020 and 444; they win up to about 800
-// powers (transform of 1,024 values with 768 powers a stage 2.81 -> 2.70 ms, of
-// 256 with 192 a stage 1.60 -> 1.38 ms).  WBTE_GT_LANES = 1, 2 or 4
+// images of 744.  Teams of twelve: 444, 1,020 and 444, one team a power with a tenth
+// more for its share of other instructions.  Measured on B200, powers of as many
+// exponents: 300 0.41 ms, 900 0.67, 2,400 1.10, 4,800 1.51, 6,000 2.54; counted by warps per
+// scheduler instead of turns 2,400 1.72.  WBTE_GT_LANES = 1, 2 or 4
 // forces that many teams of six, and so does the calling context's tuning knob.
 PowSpread gt_pow_spread(int64_t E, bool uniform) {
     if (const char* env = getenv("WBTE_GT_LANES")) {
@@ -278,11 +279,11 @@ PowSpread gt_pow_spread(int64_t E, bool uniform) {
     if (g_tune.gt_lanes == 1 || g_tune.gt_lanes == 2 || g_tune.gt_lanes == 4) return {false, g_tune.gt_lanes};
     struct Way { PowSpread spread; double work, per; };
     const Way ways[] = {{{false, 1}, uniform ? 156.0 : 195.0, 5.0}, {{false, 2}, 130.0, 2.0}, {{false, 4}, 98.0, 1.0},
-                        {{true, 1}, 115.0, 2.0},                    {{true, 2}, 74.0, 1.0}};
+                        {{true, 1}, 125.0, 2.0},                    {{true, 2}, 74.0, 1.0}};
     const Way* best = ways;
     double best_t = 0;
     for (const Way& w : ways) {
-        const double t = launch_time(w.work, (double)E / w.per);
+        const double t = run_time(w.work, (double)E / w.per);
         if (&w == ways || t < best_t) best = &w, best_t = t;
     }
     return best->spread;

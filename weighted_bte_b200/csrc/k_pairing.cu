@@ -294,7 +294,7 @@ void launch_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n, cudaStrea
     ProfScope prof_("prepare_lines", s);
     if (n <= 0) return;
     note_launch();
-    if (launch_time(95.0, (double)n / Twelve::PER) < launch_time(150.0, (double)n / Six::PER))
+    if (run_time(95.0, (double)n / Twelve::PER) < run_time(150.0, (double)n / Six::PER))
         team_launch<Twelve>(k_prepare_lines<Twelve>, n, Twelve::PER, s, lines, q, n);
     else
         team_launch<Six>(k_prepare_lines<Six>, n, Six::PER, s, lines, q, n);
@@ -393,8 +393,10 @@ void launch_final_exp(uint8_t* out, const uint8_t* in, int64_t n, FinalExpMode m
     ProfScope prof_(mode == FE_EASY ? "final_exp_easy" : (mode == FE_HARD ? "final_exp_hard" : "final_exp"), s);
     if (n <= 0) return;
     note_launch();
-    // 315 cyclotomic squarings and 35 products of the hard part
-    if (launch_time(176.0, (double)n / Twelve::PER) < launch_time(336.0, (double)n / Six::PER))
+    // 315 cyclotomic squarings and 35 products of the hard part, an eighth more for
+    // a team of twelve's share of other instructions (2,400 hard parts 1.42 ms, 6,000
+    // 3.28; counted by warps per scheduler instead of turns 2.01 and 3.29)
+    if (run_time(198.0, (double)n / Twelve::PER) < run_time(336.0, (double)n / Six::PER))
         team_launch<Twelve>(k_final_exp<Twelve>, n, Twelve::PER, s, out, in, n, (int)mode);
     else
         team_launch<Six>(k_final_exp<Six>, n, Six::PER, s, out, in, n, (int)mode);

@@ -68,11 +68,12 @@ inline double launch_time(double work, double warps, double alone = 1.6) {
 }
 
 // The same for kernels with two warps of registers per scheduler and long runs in
-// each: a launch takes whole turns of two warps and a last one of one or two, so a
-// little more than a turn costs most of another.
+// each: a launch takes whole turns of two warps and a last one of one (seven tenths
+// of a turn: hard parts on teams of six take 1.4 ms with one warp per scheduler, 2.0
+// with two, 3.3 with a few more) or two.
 inline double run_time(double work, double warps) {
     const double each = warps / schedulers(), whole = 2 * std::floor(each / 2), rest = each - whole;
-    return work * (whole + (rest > 1 ? 2.0 : (rest > 0 ? 1.6 : 0.0)));
+    return work * (whole + (rest > 1 ? 2.0 : (rest > 0 ? 1.4 : 0.0)));
 }
 
 // The time, in launch_time's measure, of `points` chains of `dbls` doublings and
