@@ -926,7 +926,7 @@ def main():
         "miller_lines_multi": roof("k_miller_lines_multi (opening: one multi-Miller loop of T pairings per slot)",
                                    ms_of.get("miller_lines_multi"), wc.multi_miller_with_lines(T) * B * G, peak),
         "miller": roof(f"k_miller_chunks (share check: unprepared multi-Miller loops of B + 1 pairs per batch in "
-                       f"runs of {miller_run} pairs per thread)", ms_of.get(f"miller_c{miller_run}"),
+                       f"runs of {miller_run} pairs per team)", ms_of.get(f"miller_c{miller_run}"),
                        wc.multi_miller_unprepared(B + 1, miller_run) * G, peak),
         "final_exp_hard": roof("k_final_exp hard part (one per slot)", ms_of.get("final_exp_hard"),
                                wc.FINAL_EXP_HARD * B * G, peak),
