@@ -101,6 +101,12 @@ int32_t wbte_measure_imad_rate(wbte_ctx *ctx, double *imad_per_s);
 int32_t wbte_profile_read(char *names, int32_t name_stride, double *ms, int64_t *counts,
                           int32_t max_entries, int32_t *n_out);
 
+/* Points are taken as they are; only the decoders below check them.  A point on
+ * no curve of the library has multiples and sums by the group law of the curve
+ * y^2 = x^3 + b' that it is on, whatever the size of the call.  MSMs of up to four
+ * terms and signature checks split scalars by the endomorphism, and transforms
+ * take roots of unity of order n in Fr: outside the subgroup of order r they do not
+ * give the scalars' multiples. */
 /* --------------------------------------------------------------- MSM */
 /* Replaces blst_p1s_mult_pippenger with nbits = 255, one contiguous block
  * (weighted_btx/src/blst_utils.rs:43-67 g1_multi_exp_affine_bytes).

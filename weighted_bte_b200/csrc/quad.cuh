@@ -58,6 +58,8 @@ struct OnLane {  // Fp
     static WBTE_INL uint32_t all_lanes(uint32_t ballot) { return ballot; }
     static WBTE_INL Fp one() { return fp_one(); }
     static WBTE_INL Fp inv(const Fp& a) { return fp_inv(a); }
+    // the curve's constant times a
+    static WBTE_INL Fp times_b(const Fp& a) { return fp_dbl(fp_dbl(a)); }
 };
 struct OnPair {  // Fp2, component = lane parity
     static constexpr int LANES = 2;
@@ -106,6 +108,7 @@ struct OnPair {  // Fp2, component = lane parity
         const Fp o = fp_shfl_xor(a, 1);
         return fp_select(odd(), fp_add(a, o), fp_sub(a, o));
     }
+    static WBTE_INL Fp times_b(const Fp& a) { return fp_dbl(fp_dbl(times_b4(a))); }
 };
 
 // ------------------------------------------------------------------- points
@@ -126,6 +129,13 @@ template <class P, int PLACES = 4> struct Quad {
     static WBTE_INL Fp infinity() { return place() == 1 ? P::one() : fp_zero(); }
     static WBTE_INL bool is_inf(const Fp& p) { return zero_at(p, 2); }
     static WBTE_INL Fp neg(const Fp& p) { return place() == 1 ? fp_neg(p) : p; }
+    // whether p is infinity or on the curve, Y^2 = X^3 + b ZZZ^2
+    static WBTE_INL bool on_curve(const Fp& p) {
+        const Fp s = P::mul(p, p), x3 = P::mul(s, p);
+        const Fp d = fp_sub(fp_sub(from(s, 1), from(x3, 0)), P::times_b(from(s, 3)));
+        const bool zero = zero_at(d, 0), inf = is_inf(p);
+        return zero || inf;
+    }
 
     // 2p (infinity stays infinity: ZZ = 0 is kept)
     static __device__ __noinline__ Fp dbl(Fp p) {
@@ -257,8 +267,15 @@ template <class P, int PLACES = 4> struct Quad {
 // MSM 1.11 -> 0.95 ms.  Eight lanes cost as many product slots as a quad for an
 // addition and a third more for a doubling, so calls with more points than
 // schedulers take quads (chain_time).
+// These formulas use the curve's constant: of a point elsewhere they make another
+// value than the XYZZ ones, or (0, 0, 0), which swallows every sum it enters and
+// reads as infinity.  Kernels that multiply or add a caller's points look at them
+// first and run General, an XYZZ point on the same lanes, where a warp holds one off
+// the curve: two products of a chain of five hundred.  (Transforms do not look: outside
+// the subgroup of order r their roots of unity are none.)
 struct Oct {
     using Field = OnLane;
+    using General = Quad<OnLane, 8>;
     static constexpr int WIDTH = 8;
     static WBTE_INL int lane() { return threadIdx.x & 31; }
     static WBTE_INL int place() { return lane() & 7; }
