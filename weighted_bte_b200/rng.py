@@ -166,8 +166,15 @@ class OsRng:
 
 
 def random_scalar(rng) -> int:
-    # eight 64-bit words, least significant first, as the 64 bytes they are
-    return int.from_bytes(rng.fill_bytes(64), "little") % R
+    """A scalar from eight 64-bit words of `rng`, least significant first.  `rng` is
+    anything with next_u64; the generators of this file give the words as the 64
+    bytes they are, in one call."""
+    if type(rng) in (ChaCha20Rng, OsRng):
+        return int.from_bytes(rng.fill_bytes(64), "little") % R
+    acc = 0
+    for i in range(8):
+        acc |= rng.next_u64() << (64 * i)
+    return acc % R
 
 
 def sample_nonzero(rng) -> int:
