@@ -308,15 +308,21 @@ static void segment_product(uint8_t* out, const uint8_t* in, const int64_t* offs
         team_launch<Six>(k_fp12_segment_product<Six>, k, Six::PER, s, out, in, offsets, k);
 }
 
+// false (nothing launched, the runtime's error pending) if there is no memory for
+// the runs' products
 static bool miller_lines(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, int64_t per, int64_t p_per,
                          int64_t pairs, cudaStream_t s) {
     const MillerSpread how = miller_spread(n, pairs, LINE_PREPARED, pairs);
     const int64_t chunks = (pairs + how.C - 1) / how.C;
     uint8_t* runs = out;
     int64_t* offs = nullptr;
-    if (chunks > 1 && (cudaMallocAsync(&runs, GT_SZ * (size_t)(n * chunks), s) != cudaSuccess ||
-                       cudaMallocAsync(&offs, sizeof(int64_t) * (size_t)(n + 1), s) != cudaSuccess))
-        return false;
+    if (chunks > 1) {
+        if (cudaMallocAsync(&runs, GT_SZ * (size_t)(n * chunks), s) != cudaSuccess) return false;
+        if (cudaMallocAsync(&offs, sizeof(int64_t) * (size_t)(n + 1), s) != cudaSuccess) {
+            cudaFreeAsync(runs, s);
+            return false;
+        }
+    }
     note_launch();
     if (how.twelve)
         team_launch<Twelve>(k_miller_lines_multi<Twelve>, n * chunks, Twelve::PER, s, runs, lines, p, n, per, p_per, pairs,
@@ -337,15 +343,14 @@ void launch_miller_lines(uint8_t* out, const uint8_t* lines, const uint8_t* p, i
                          int64_t lines_n) {
     ProfScope prof_("miller_lines", s);
     if (n <= 0) return;
-    miller_lines(out, lines, p, n, lines_n > 0 ? lines_n : n, 1, 1, s);
+    miller_lines(out, lines, p, n, lines_n > 0 ? lines_n : n, 1, 1, s);  // one run a value: no scratch
 }
 bool launch_miller_lines_multi(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, int64_t per, int T,
                                cudaStream_t s, int64_t p_per) {
     ProfScope prof_("miller_lines_multi", s);
     if (T < 1 || per < 1) return false;
     if (n <= 0) return true;
-    miller_lines(out, lines, p, n, per, p_per > 0 ? p_per : per, T, s);
-    return true;
+    return miller_lines(out, lines, p, n, per, p_per > 0 ? p_per : per, T, s);
 }
 static void miller_chunks(uint8_t* out, const uint8_t* p, const uint8_t* q, int64_t per, int64_t K, int C, int64_t p_mod,
                           int64_t q_mod, cudaStream_t s) {

@@ -202,7 +202,8 @@ void launch_prepare_lines(uint8_t* lines, const uint8_t* q, int64_t n, cudaStrea
 // out[i] = Miller(p[i], lines of pair i), lines laid out as above with n pairs
 // out[o] = prod_{t<T} Miller(p[(o / p_per) T + t], line table (o % per) T + t) for o < n
 // (tables line-major, stride per * T; p_per <= 0 means per); any T >= 1, the
-// pairs sharing their squarings in chunks of 8; returns false for T < 1.
+// pairs sharing their squarings in runs); false if T < 1 or if there is no memory
+// for the runs' products, and then nothing is launched.
 bool launch_miller_lines_multi(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, int64_t per, int T,
                                cudaStream_t s, int64_t p_per = 0);
 void launch_miller_lines(uint8_t* out, const uint8_t* lines, const uint8_t* p, int64_t n, cudaStream_t s,

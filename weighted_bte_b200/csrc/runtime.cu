@@ -173,7 +173,9 @@ struct Call {
     }
     int32_t finish() {
         cudaError_t e = cudaGetLastError();
-        if (e != cudaSuccess) fail(WBTE_ERR_CUDA, cudaGetErrorString(e));
+        // a launcher that finds no memory for its scratch launches nothing and leaves
+        // the runtime's error
+        if (e != cudaSuccess) fail(e == cudaErrorMemoryAllocation ? WBTE_ERR_OOM : WBTE_ERR_CUDA, cudaGetErrorString(e));
         for (auto& o : outs) cudaMemcpyAsync(o.host, o.dev, o.bytes, cudaMemcpyDeviceToHost, s);
         for (void* p : temps) cudaFreeAsync(p, s);
         if (!outs.empty() || sync || status != WBTE_OK) {
@@ -1626,7 +1628,7 @@ static bool wpfe_open_core(Call& c, uint8_t* dm, const uint8_t* ds, uint64_t T, 
     // first terms: per slot the T pairings with the committee's keys of that
     // slot, one multi-Miller loop over their line tables when given
     if (prepared) {
-        launch_miller_lines_multi(ft, dbl, left, (int64_t)n, (int64_t)B, (int)T, c.s, 1);
+        if (!launch_miller_lines_multi(ft, dbl, left, (int64_t)n, (int64_t)B, (int)T, c.s, 1)) return false;
     } else {
         std::vector<int64_t> offs_T(n + 1);
         for (uint64_t o = 0; o <= n; o++) offs_T[o] = (int64_t)(o * T);
@@ -2193,8 +2195,7 @@ static bool opening_miller(Call& c, uint8_t* alpha, const uint8_t* dk, const voi
     if (opening_lines) {
         const uint8_t* dl = c.in(opening_lines, LINE_SZ * LINES_PER_POINT * BT);
         if (!c.ok()) return false;
-        launch_miller_lines_multi(alpha, dl, ds, (int64_t)(B * K), (int64_t)B, (int)T, c.s);
-        return true;
+        return launch_miller_lines_multi(alpha, dl, ds, (int64_t)(B * K), (int64_t)B, (int)T, c.s);
     }
     uint8_t* P = c.alloc(G1_AFF * BT * K);
     uint8_t* f = c.alloc(GT_SZ * BT * K);
