@@ -96,9 +96,12 @@ size_t request_bytes(const wbte_crs* crs, uint64_t B, uint64_t T) {
     if (crs->scheme == WBTE_SCHEME_WBTX) {
         uint64_t m = 1;
         while (m < 2 * B) m <<= 1;
-        return B * (G1B + GTB + 1) + m * (3 * G1B + GTB) + B * GTB * 3 + T * G1B + (1u << 20);
+        // the transform's two further copies of its values, a stage's powers and the
+        // twiddles' recodings, or the products of the opening's pairing runs
+        const size_t scratch = std::max(m * (2 * GTB + 3 * GTB / 4 + 2 * 136), B * (T * GTB + 8));
+        return B * (G1B + GTB + 1) + m * (3 * G1B + GTB) + B * GTB * 3 + T * G1B + scratch + (1u << 20);
     }
-    return B * (6400 + 480 * T) + (1u << 20);
+    return B * (6400 + (480 + GTB) * T) + (1u << 20);
 }
 
 size_t committee_bytes(const wbte_crs* crs, uint64_t B, uint64_t T) {

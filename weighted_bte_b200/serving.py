@@ -55,15 +55,18 @@ GTB, G1B, G2B = wb.GTB, wb.G1B, wb.G2B
 
 def request_bytes(batch_size: int, parties: int) -> int:
     """Device memory one request holds while it runs, without its committee
-    preparation: the resident batch (first/second/commitment/response), the
-    cross-term transform (G1 XYZZ work + GT values over the transform size),
-    the per-slot pairing products of the opening and the outputs."""
+    preparation: the resident batch (first/second/commitment/response), its
+    place in a group's arrays and in the output, the cross-term transform (G1
+    XYZZ work + GT values over the transform size, two further copies of the
+    values that the stages go between, the stage's powers and the twiddles'
+    recodings), the products of the opening's pairing runs and its sums."""
     B, T = batch_size, parties
     m = wb.transform_size_for(B)
-    batch = B * (G1B + GTB + G1B + 32 + 1)
+    batch = B * (G1B + GTB + G1B + 32 + 1) + B * (G1B + GTB + 1) + B * GTB
     precompute = m * (G1B + 2 * G1B + GTB) + B * GTB
+    stages = m * (2 * GTB + 3 * GTB // 4 + 2 * 136)
     opening = B * T * GTB + 2 * B * GTB
-    return batch + precompute + opening + (1 << 20)
+    return batch + precompute + stages + opening + (1 << 20)
 
 
 def preparation_bytes(batch_size: int, parties: int, committee_weight: int) -> int:

@@ -325,8 +325,8 @@ def request_bytes(B: int, T: int) -> int:
     """Device memory one weighted_pfe request of class B (committee of T)
     holds while it runs: the batch and its encodings, the validation MSM, the
     Cauchy transforms (G1 work, two GT arrays), the opening's per-(slot,
-    party) G1 points and GT values, and the output."""
-    return B * (6400 + 480 * T) + (1 << 20)
+    party) G1 points, the products of its pairing runs, and the output."""
+    return B * (6400 + (480 + GTB) * T) + (1 << 20)
 
 
 def preparation_bytes(B: int, T: int) -> int:
