@@ -21,7 +21,8 @@ std::map<const void*, std::string> kernels;  // by host stub
 std::map<uintptr_t, size_t> blocks;          // device memory
 std::string log_text;
 uint64_t live = 0, peak = 0, allocations = 0;
-int fail_at = 0, device = 0, per_sm = 4, sms[8] = {148, 148, 148, 148, 148, 148, 148, 148};
+int fail_at = 0, device = 0, per_sm = 4;
+std::vector<int> sms(64, 148);
 cudaError_t last = cudaSuccess;
 struct Config { dim3 grid, block; size_t shmem; cudaStream_t s; };
 thread_local std::vector<Config> configs;
@@ -134,7 +135,7 @@ cudaError_t cudaSetDevice(int d) {
     return cudaSuccess;
 }
 cudaError_t cudaGetDeviceCount(int* n) {
-    *n = 8;
+    *n = 64;
     return cudaSuccess;
 }
 cudaError_t cudaGetLastError() {
@@ -195,5 +196,10 @@ using namespace wbte;
 static uint8_t* const ANY = reinterpret_cast<uint8_t*>(uintptr_t(1) << 40);
 int h_miller_lines_multi(int64_t n, int64_t per, int64_t T) {
     return launch_miller_lines_multi(ANY, ANY, ANY, n, per, (int)T, nullptr);
+}
+// window, segments per window and scratch of a plan (the window 0: none within `limit`)
+void h_msm_plan(int g, int64_t n, int64_t k, uint64_t limit, int64_t* out) {
+    const MsmPlan p = msm_plan((Group)g, n, k, limit ? limit : SIZE_MAX);
+    out[0] = p.c, out[1] = p.segments, out[2] = p.c ? (int64_t)msm_family_scratch_bytes((Group)g, 1, k, n, p) : 0;
 }
 }

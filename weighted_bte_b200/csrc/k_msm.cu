@@ -349,7 +349,8 @@ template <class P> static int64_t segment_wave() {
 // buckets and short multiples, wide ones few rows.  Measured on B200, one G1
 // MSM of 65,536 points: c = 8 2.58 ms, 10 2.60, 13 (the former log2(n) - 2,
 // capped) 2.79; of 32 points c = 8 1.30, 4 1.40.
-MsmPlan msm_plan(Group g, int64_t n, int64_t k) {
+// `limit`: plans whose scratch is larger are left out; none left, c = 0.
+MsmPlan msm_plan(Group g, int64_t n, int64_t k, size_t limit) {
     const double wave = (double)(g == GROUP_G1 ? segment_wave<OnLane>() : segment_wave<OnPair>());
     int c0 = 4, c1 = 13;
     if (g_tune.msm_window >= c0 && g_tune.msm_window <= c1) c0 = c1 = g_tune.msm_window;
@@ -372,20 +373,21 @@ MsmPlan msm_plan(Group g, int64_t n, int64_t k) {
                 for (double len = (double)s; len > 1; len = std::ceil(len / 32)) tree += 1.43 * std::min(5.0, std::ceil(std::log2(len)));
             }
             const double cost = std::ceil(rows * (double)s / wave) * each + tree + 0.53 * windows;
-            if (best.c == 0 || cost < best_cost) {
-                best_cost = cost;
-                best.c = c;
-                best.windows = windows;
-                best.segments = s;
-            }
+            if (best.c != 0 && cost >= best_cost) return;
+            MsmPlan p;
+            p.c = c;
+            p.windows = windows;
+            p.buckets = 1 << (c - 1);
+            p.segment = (n + s - 1) / s;
+            p.segments = std::max<int64_t>(1, (n + p.segment - 1) / p.segment);
+            if (limit != SIZE_MAX && msm_family_scratch_bytes(g, 1, k, n, p) > limit) return;
+            best_cost = cost;
+            best = p;
         };
         // counts an eighth apart, and those that just fill whole waves
         for (int64_t s = 1; s <= most; s += 1 + s / 8) consider(s);
         for (int w = 1; w <= 4; w++) consider((int64_t)(wave * w / rows));
     }
-    best.buckets = 1 << (best.c - 1);
-    best.segment = (n + best.segments - 1) / best.segments;
-    best.segments = std::max<int64_t>(1, (n + best.segment - 1) / best.segment);
     return best;
 }
 
@@ -457,22 +459,21 @@ bool static_is_device(const void* p, int dev) {
     return a.type == cudaMemoryTypeDevice && a.device == dev;
 }
 
-// The plan of wbte_g1_msm with fewer, longer segments where its scratch would
-// not fit the array: every n <= STATIC_MSM_MAX_POINTS fits (at n = 16384 the
-// digits and sorted entries take 3.6 MB and at most about 1000 segments of
-// the 22 windows fit the rest).
+// The best plan whose scratch fits the array.  One exists for every n <=
+// STATIC_MSM_MAX_POINTS: the widest windows take 10 bytes a point and window for
+// digits and sorted entries (3.3 MB for 16,384 points), and one segment a window is
+// 0.4 KB with its place in the tree.  Measured on B200 against the general plan with
+// its segments cut until they fit: 16,384 points 1.69 -> 1.58 ms, 12,000 1.61 -> 1.58,
+// 4,096 1.40 -> 1.42, fewer the same plan.
+constexpr size_t STATIC_MSM_LEAST = (sizeof(int16_t) + sizeof(uint64_t)) * 20 * STATIC_MSM_MAX_POINTS + (size_t(1) << 16);
+static_assert(STATIC_MSM_LEAST <= STATIC_MSM_BYTES - STATIC_MSM_TAIL, "windows of 13 bits fit");
 bool static_plan(wbte::MsmPlan& p, int64_t n, size_t avail) {
     using namespace wbte;
     const Tuning saved = g_tune;
     g_tune = Tuning();
-    p = msm_plan(GROUP_G1, n, 1);
+    p = msm_plan(GROUP_G1, n, 1, avail);
     g_tune = saved;
-    while (msm_family_scratch_bytes(GROUP_G1, 1, 1, n, p) > avail) {
-        if (p.segments <= 1) return false;
-        p.segment += std::max<int64_t>(1, p.segment / 8);
-        p.segments = (n + p.segment - 1) / p.segment;
-    }
-    return true;
+    return p.c != 0;
 }
 }  // namespace
 

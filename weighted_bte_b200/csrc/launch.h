@@ -163,7 +163,7 @@ struct MsmPlan {
     int c = 0, windows = 0, buckets = 0;
     int64_t segment = 0, segments = 0;
 };
-MsmPlan msm_plan(Group g, int64_t n, int64_t k);
+MsmPlan msm_plan(Group g, int64_t n, int64_t k, size_t limit = SIZE_MAX);
 // MSMs of at most SMALL_MSM_MAX terms by a Straus loop over the base-|x|
 // digits of every term, the digit pairs spread over 1..16 lanes per output
 // (launch_msm_family dispatches here).

@@ -13,6 +13,8 @@ can exceed the pipe's own utilisation.
 """
 from __future__ import annotations
 
+import math
+
 R_FR = 0x73EDA753299D7D483339D80809A1D80553BDA402FFFE5BFEFFFFFFFF00000001
 P_FP = int("1a0111ea397fe69a4b1ba7b6434bacd764774b84f38512bf6730d2a0f6b0f6241eabfffeb153ffffb9feffffffffaaab", 16)
 X_ABS = 0xD201000000010000
@@ -160,6 +162,56 @@ def g1_ntt_batched(m: int, count: int, inverse: bool = False) -> int:
             total += (m // (2 * half)) * (tw + 2 * G1_ADD)
         half *= 2
     return total * count
+
+
+# segments of one wave of k_segments on a B200: 148 SMs of four blocks of 64
+# threads, a lane (G1) or a pair (G2) each
+SEGMENT_WAVE = {False: 148 * 4 * 64, True: 148 * 4 * 32}
+
+
+def msm_scratch_bytes(n: int, k: int, g2: bool, windows: int, segments: int) -> int:
+    """layout_for of csrc/k_msm.cu for one scalar vector."""
+    align = lambda x: (x + 255) & ~255  # noqa: E731
+    xyzz = 384 if g2 else 192
+    rows = k * windows
+    return (align(2 * windows * n) + align(8 * windows * n) + align(4 * windows) + align(xyzz * rows * segments)
+            + align(xyzz * rows * max(1, (segments + 7) // 8)))
+
+
+def msm_plan(n: int, k: int, g2: bool, wave: int = 0, limit: int = 0):
+    """msm_plan of csrc/k_msm.cu: (window, segments per window), the cheapest by its
+    cost model among those whose scratch is within `limit` (0: any), or None."""
+    wave = float(wave or SEGMENT_WAVE[g2])
+    most = min(1024, n)
+    best, best_cost = None, 0.0
+    for c in range(4, 14):
+        windows = (256 + c - 1) // c
+        buckets, rows = float(1 << (c - 1)), float(k * windows)
+        terms = n * (1.0 - 1.0 / (2.0 * buckets))
+        counts, s = [], 1
+        while s <= most:
+            counts.append(s)
+            s += 1 + s // 8
+        counts += [int(wave * w / rows) for w in range(1, 5)]
+        for s in counts:
+            s = max(1, min(s, most))
+            S = float(math.ceil(terms / s))
+            gap = 2.3 * max(0.0, math.log2(buckets / n))
+            met = min(min(S, buckets), S * buckets / n + 1.0)
+            each = S + met * (1.43 + gap) + (2.3 * (c - 1) if s > 1 else 0.0)
+            tree, length = buckets / 900, float(s)
+            while length > 1:
+                tree += 1.43 * min(5.0, math.ceil(math.log2(length)))
+                length = float(math.ceil(length / 32))
+            cost = math.ceil(rows * s / wave) * each + tree + 0.53 * windows
+            if best is not None and cost >= best_cost:
+                continue
+            segment = -(-n // s)
+            segments = max(1, -(-n // segment))
+            if limit and msm_scratch_bytes(n, k, g2, windows, segments) > limit:
+                continue
+            best, best_cost = (c, segments), cost
+    return best
 
 
 def msm_plan_window(n: int) -> int:
