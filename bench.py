@@ -589,8 +589,8 @@ def sweep_section(torch, wb, peak):
                                          work="expected Pippenger count of the plan")
         del pts, sc
     # group transforms of random elements, each path forced through the
-    # context's knobs so that its exact count (workcount) applies; the entry
-    # is the faster path, both are reported
+    # context's knobs; the entry is the faster path, both are reported, with
+    # the products of the radix-2 (GT: radix-4) schedule over the path's digits
     for lg in (8, 10, 12, 14, 16):
         n = 1 << lg
         for name, call, size, g2, knob, paths in (
@@ -611,7 +611,8 @@ def sweep_section(torch, wb, peak):
                     prod = wc.gt_ntt_single(n, v)
                 else:
                     prod = wc.group_ntt_joint(n, g2) if v == 1 else wc.group_ntt_lanes(n, g2)
-                res[pname] = roof(call, ms, prod, peak, path=pname, work="exact count of the forced path")
+                res[pname] = roof(call, ms, prod, peak, path=pname,
+                                  work="textbook products of the forced path's digits")
             ctx.set_tuning(_lib.TUNE_NTT_JOINT, -1)
             ctx.set_tuning(_lib.TUNE_GT_LANES, 0)
             best = min(res.values(), key=lambda r: r["ms"])
@@ -921,8 +922,8 @@ def main():
     # run length of the share check's multi-Miller loops, from its profile tag
     miller_run = next((int(k[len("miller_c"):]) for k in ms_of if k.startswith("miller_c")), 1)
     rooflines = {
-        "miller_lines": roof("k_miller_lines (precompute: prepared Miller loops of the transformed first "
-                             "components)", ms_of.get("miller_lines"), wc.MILLER_WITH_LINES * m * G, peak),
+        "miller_lines": roof("k_miller_lines_multi, single pairs (precompute: prepared Miller loops of the "
+                             "transformed first components)", ms_of.get("miller_lines"), wc.MILLER_WITH_LINES * m * G, peak),
         "miller_lines_multi": roof("k_miller_lines_multi (opening: one multi-Miller loop of T pairings per slot)",
                                    ms_of.get("miller_lines_multi"), wc.multi_miller_with_lines(T) * B * G, peak),
         "miller": roof(f"k_miller_chunks (share check: unprepared multi-Miller loops of B + 1 pairs per batch in "
@@ -932,8 +933,9 @@ def main():
                                wc.FINAL_EXP_HARD * B * G, peak),
         "ntt_g1": roof("k_ntt_stage_joint<Fp> (batched G1 transforms of the first components)",
                        ms_of.get("ntt_g1"), wc.g1_ntt_batched(m, G) if G % 32 == 0 else 0, peak),
-        "msm_segments_g1": roof("k_segments<Fp> (partial decryptions: T x G G1 MSMs of B terms)",
-                                ms_of.get("msm_segments_g1"), wc.msm_expected(B, T * G, False), peak,
+        "msm_segments_g1": roof("k_segments in G1 (partial decryptions: T x G G1 MSMs of B terms)",
+                                ms_of.get("msm_segments_g1"),
+                                wc.msm_expected(B, T * G, False, wc.msm_plan_window(B, T * G, False)), peak,
                                 work_basis="expected Pippenger count of the plan"),
     }
     group_kernels = {k: round(v[0], 2) for k, v in sorted(prof_g.items(), key=lambda kv: -kv[1][0])}
@@ -941,8 +943,9 @@ def main():
     # the plain path's dominant kernel: the preparation's G2 MSM segments
     top = max(prof.items(), key=lambda kv: kv[1][0]) if prof else ("none", (0.0, 0))
     msm_g2_ms = prof.get("msm_segments_g2", (0.0, 0))[0] / args.steps if prof else None
-    msm_g2_work = sum(wc.msm_expected(weights[j], B, True) for j in committee) + wc.msm_expected(W_T, B - 1, True)
-    roofline_plain = roof("k_segments<Fp2> (committee preparation: B x T party-block G2 MSMs and B - 1 kernel "
+    prep = [(weights[j], B) for j in committee] + [(W_T, B - 1)]  # families of the committee's preparation
+    msm_g2_work = sum(wc.msm_expected(n, k, True, wc.msm_plan_window(n, k, True)) for n, k in prep)
+    roofline_plain = roof("k_segments in G2 (committee preparation: B x T party-block G2 MSMs and B - 1 kernel "
                           "G2 MSMs of W_T terms per batch)", msm_g2_ms, msm_g2_work, peak,
                           work_basis="expected Pippenger count of the plan", top_kernel_of_plain=top[0])
 

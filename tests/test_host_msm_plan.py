@@ -28,6 +28,10 @@ def test_the_restatement_is_the_library_s(g2, k):
         assert scratch == wc.msm_scratch_bytes(n, k, g2, (256 + c - 1) // c, segments)
 
 
+def test_plans_of_the_measured_sizes():
+    assert wc.msm_plan_window(65536) == 8 and wc.msm_plan_window(1 << 20) == 7
+
+
 @pytest.mark.parametrize("n", [1, 2, 40, 517, 1000, 3000, 4096, 8191, 12000, 16000, 16383, 16384])
 def test_the_fixed_footprint_takes_the_best_plan_that_fits(n):
     h = library()

@@ -214,17 +214,16 @@ def msm_plan(n: int, k: int, g2: bool, wave: int = 0, limit: int = 0):
     return best
 
 
-def msm_plan_window(n: int) -> int:
-    lg = max(0, n.bit_length() - 1)
-    c = lg - 1 if n < (1 << 14) else lg - 2
-    return max(4, min(13, c))
+def msm_plan_window(n: int, k: int = 1, g2: bool = False) -> int:
+    """The window that the library takes for k MSMs of n points in one call."""
+    return msm_plan(n, k, g2)[0]
 
 
 def msm_expected(n: int, k: int, g2: bool, c: int = 0) -> int:
     """Expected products of k Pippenger MSMs of n uniform scalars with window
-    c (default: the cost model's): one mixed addition per nonzero signed
+    c (default: the cost model's for one MSM): one mixed addition per nonzero signed
     digit, one addition per occupied bucket, the window combination."""
-    c = c or msm_plan_window(n)
+    c = c or msm_plan_window(n, 1, g2)
     windows = -(-256 // c)
     buckets = 1 << (c - 1)
     nnz = n * (1.0 - 1.0 / (1 << c))
