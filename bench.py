@@ -28,7 +28,9 @@ Every form is bit-exact against the plaintexts (asserted after timing).
                 all requests submitted at once, and p50/p99 request latency
                 under Poisson arrivals at half that rate (continuous batching)
 
-Further sections (flat keys, so every figure survives in the parsed line):
+The JSON line holds the headline and one figure of each section below, at most
+HEADLINE_BYTES long; the record with every figure goes to standard error, one
+line after "record: ".  Its sections:
   roofline / rooflines   the batched form's kernels on their own Fp-product
                 counts (weighted_bte_b200/workcount.py) against the measured
                 integer-pipe peak; `traffic` from the committed ncu capture
@@ -77,6 +79,7 @@ os.environ.setdefault("CUDA_DEVICE_MAX_CONNECTIONS", "32")
 # a*b_i + 24 for m*p + 1) 32-bit IMAD instructions (lo and hi halves).
 IMAD_PER_FP_MUL = 12 * 49
 METRIC = "ciphertexts decrypted/s (weighted_btx batch decryption, B=512)"
+HEADLINE_BYTES = 2000  # of the JSON line, so that whoever keeps the end of the output keeps all of it
 TRAFFIC_FILE = os.path.join(ROOT, "profiles", "roofline_traffic.json")
 
 
@@ -640,6 +643,37 @@ def sweep_section(torch, wb, peak):
     return out
 
 
+def headline(record):
+    """The JSON line of a record: its required keys and a figure of each section,
+    numbers to seven digits."""
+    def short(v):
+        return float(f"{v:.7g}") if isinstance(v, float) else v
+
+    def of(section, *keys):
+        section = section or {}
+        return {k: short(section[k]) for k in keys if k in section}
+
+    config, roofs = record["config"], record["rooflines"]
+    line = {k: record[k] for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                                   "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "gpu_launches")}
+    line["config"] = of(config, "workload", "batch_size", "committee_weight", "parallelism", "form", "l2")
+    line["e2e"] = of(record["e2e"], "value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "p50_ms",
+                     "p99_ms") or None
+    line["clocks"] = record["clocks"]
+    line["roofline"] = of(record["roofline"], "kernel", "bound", "unit", "ms", "achieved", "peak", "frac", "traffic")
+    line["roofline_fracs"] = {k: short(r.get("frac")) for k, r in roofs.items()}
+    line["cpu_baseline"] = of(record["cpu_baseline"], "value", "unit", "cores", "kind") or None
+    for k in ("plain", "plain_cached", "batched_graph", "wpfe_batched", "wpfe_served"):
+        line[k] = short((record[k] or {}).get("value"))
+    if record["sweep"]:
+        line["sweep_ms"] = {k: short(record["sweep"][k]["ms"]) for k in
+                            ("g1_msm_2^16", "g1_msm_2^20", "g2_msm_2^20", "gt_ntt_2^16", "multi_pairing_k4096")}
+    for k in ("sweep_ms", "roofline_fracs", "wpfe_served", "wpfe_batched", "batched_graph", "plain_cached", "plain"):
+        if len(json.dumps(line)) > HEADLINE_BYTES:
+            line.pop(k, None)
+    return line
+
+
 def _lib_i64(v):
     from weighted_bte_b200 import _lib
 
@@ -980,9 +1014,8 @@ def main():
             "vs_baseline": None, "dtype": "u32 limbs (Fp/Fr Montgomery)", "data": "synthetic",
             "config": {"workload": cfg.name, "batch_size": B, "parties": cfg.parties, "total_weight": cfg.total_weight,
                        "threshold": t, "committee": committee, "committee_weight": W_T,
-                       "parallelism": f"replicas x{world}", "form": f"batched: {C} concurrent groups per step (one "
-                       f"CUDA stream each), {G} batches per group with every GPU phase launched once per group; "
-                       f"committee preparation cached (the timed region's first group prepares)",
+                       "parallelism": f"replicas x{world}", "form": f"batched: {C} concurrent groups per step, {G} batches "
+                       f"per group, committee preparation cached (the first timed group prepares)",
                        "l2": "flushed before every step (256 MB write)"},
             "plain": {"value": plain_value, "unit": "ciphertexts/s",
                       "ms_per_batch": ms_plain / args.steps if ms_plain else None,
@@ -999,7 +1032,8 @@ def main():
             "kernel_ms_per_batch_plain": phases, "kernel_ms_per_group": group_kernels,
             "wpfe_batched": wpfe, "wpfe_served": served, "sweep": sweep, "setup_s": round(setup_s, 2), "crs_load": crs_load,
         }
-        print(json.dumps(line), flush=True)
+        print("record: " + json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(headline(line)), flush=True)
     ranks.close()
 
 
