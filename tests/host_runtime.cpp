@@ -202,4 +202,5 @@ void h_msm_plan(int g, int64_t n, int64_t k, uint64_t limit, int64_t* out) {
     const MsmPlan p = msm_plan((Group)g, n, k, limit ? limit : SIZE_MAX);
     out[0] = p.c, out[1] = p.segments, out[2] = p.c ? (int64_t)msm_family_scratch_bytes((Group)g, 1, k, n, p) : 0;
 }
+void h_fp12_mul(int64_t n) { launch_fp12_mul(ANY, ANY, 1, ANY, 1, false, n, nullptr); }
 }

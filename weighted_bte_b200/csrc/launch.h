@@ -42,20 +42,21 @@ struct Tuning {
     int msm_window = 0;    // Pippenger window width c, 4..13
     int msm_segments = 0;  // sorted-term segments per (MSM, window), 1..1024
     int ntt_joint = -1;    // G1/G2 transform stages: 1 one thread per butterfly, 0 quads
-    int miller_chunk = 0;  // pairs per thread of the chunked unprepared Miller loops, 1..8
+    int miller_chunk = 0;  // pairs per team of the chunked unprepared Miller loops, 1..8
 };
 extern thread_local Tuning g_tune;
 
-// warp schedulers of the current device (four to an SM)
+// warp schedulers of the current device (four to an SM), looked up once per device
 inline int schedulers() {
-    static std::atomic<int> cache{0};
-    int n = cache.load(std::memory_order_relaxed);
+    static std::atomic<int> cache[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 4 * 148;
+    int n = cache[dev].load(std::memory_order_relaxed);
     if (n == 0) {
-        int dev = 0, sms = 0;
-        cudaGetDevice(&dev);
+        int sms = 0;
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         n = 4 * (sms > 0 ? sms : 148);
-        cache.store(n, std::memory_order_relaxed);
+        cache[dev].store(n, std::memory_order_relaxed);
     }
     return n;
 }
