@@ -116,7 +116,10 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p) {
     a->device = device;
     return cudaSuccess;
 }
-cudaError_t cudaGetSymbolAddress(void** p, const void*) { return allocate(p, size_t(8) << 20); }
+cudaError_t cudaGetSymbolAddress(void** p, const void* symbol) {
+    *p = const_cast<void*>(symbol);  // part of the image, not allocated
+    return cudaSuccess;
+}
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int dev) {
     *v = a == cudaDevAttrMultiProcessorCount ? sms[dev] : 0;
     return cudaSuccess;
