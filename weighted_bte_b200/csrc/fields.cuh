@@ -36,7 +36,8 @@ WBTE_INL Fp fp_sqr(const Fp& a) { return fp_sqr_ool(a); }
 WBTE_INL Fp fp_mul(const Fp& a, const Fp& b) { Fp r; fp_mont_mul(r.v, a.v, b.v); return r; }
 WBTE_INL Fp fp_sqr(const Fp& a) { Fp r; fp_mont_sqr(r.v, a.v); return r; }
 #endif
-// (a b + c d) / 2^384 mod p for factors up to p: one reduction for two products
+// (a b + c d) / 2^384 mod p for a, c up to p and b + d up to 2^384 (factors below
+// 4p, sums that are not reduced, among them): one reduction for two products
 static __device__ __noinline__ Fp fp_mul2(Fp a, Fp b, Fp c, Fp d) {
     Fp r;
     fp_mont_mul2(r.v, a.v, b.v, c.v, d.v);

@@ -244,9 +244,9 @@ def _asm_function(name, args, lines, outs, ins):
 
 
 def gen_mont_mul2(name, modulus, n):
-    """r = (a b + c d) / 2^(32n) mod m for factors up to m (the sum before each
-    shift stays below 5 m 2^32 < 2^(32(n+1)), the result before the last
-    subtraction below 1.3 m)."""
+    """r = (a b + c d) / 2^(32n) mod m for a, c up to m and any b, d with b + d at
+    most 2^(32n): the sum before each shift stays below 4 m 2^32 < 2^(32(n+1)),
+    the result before the last subtraction below 2 m."""
     pinv = (-pow(modulus, -1, 1 << 32)) % (1 << 32)
     ml = limbs32(modulus, n)
     mw = ["0x%08x" % x for x in ml]
