@@ -2,9 +2,10 @@
 // R = 2^384, byte-identical to blst's blst_fp), Fr (8 x 32-bit limbs),
 // Fp2 = Fp[u]/(u^2+1), Fp6 = Fp2[v]/(v^3-(1+u)), Fp12 = Fp6[w]/(w^2-v).
 //
-// Fp operations are inlined single PTX blocks (field_asm.cuh).  Fp2 products
-// are inlined; Fp6/Fp12 products are out-of-line so that kernels built from
-// them stay within the instruction cache.
+// Fp operations are single PTX blocks (field_asm.cuh); products and squares of
+// Fp, and in the curve files of Fp2, are out of line so that kernels built from
+// them stay within the instruction cache.  Fp12 arithmetic runs over teams of
+// lanes (team.cuh); the Fp6 product and inverse serve the torus encodings.
 #pragma once
 #include <cstdint>
 #include "field_asm.cuh"
@@ -122,21 +123,11 @@ WBTE_INL Fp2 fp2_neg(const Fp2& a) { return Fp2{fp_neg(a.c0), fp_neg(a.c1)}; }
 WBTE_INL Fp2 fp2_conj(const Fp2& a) { return Fp2{a.c0, fp_neg(a.c1)}; }
 WBTE_INL bool fp2_is_zero(const Fp2& a) { return fp_is_zero(a.c0) && fp_is_zero(a.c1); }
 WBTE_INL bool fp2_eq(const Fp2& a, const Fp2& b) { return fp_eq(a.c0, b.c0) && fp_eq(a.c1, b.c1); }
-#if defined(WBTE_FP2_NOINLINE) || defined(WBTE_FP2_LAZY)
+#if defined(WBTE_FP2_NOINLINE)
 #define WBTE_FP2_MUL static __device__ __noinline__
 #else
 #define WBTE_FP2_MUL WBTE_INL
 #endif
-#if defined(WBTE_FP2_LAZY)
-// Karatsuba with lazy reduction (field_asm.cuh): three double-width products
-// and two Montgomery reductions, 1,464 multiply-adds instead of 1,764.  One
-// out-of-line copy: the block is about 1,800 instructions.
-WBTE_FP2_MUL Fp2 fp2_mul(const Fp2& a, const Fp2& b) {
-    Fp2 r;
-    fp2_mont_mul_lazy(r.c0.v, r.c1.v, a.c0.v, a.c1.v, b.c0.v, b.c1.v);
-    return r;
-}
-#else
 // Karatsuba: 3 Fp products; the operand sums stay unreduced (< 2p).
 WBTE_FP2_MUL Fp2 fp2_mul(const Fp2& a, const Fp2& b) {
     Fp t0 = fp_mul(a.c0, b.c0);
@@ -144,14 +135,12 @@ WBTE_FP2_MUL Fp2 fp2_mul(const Fp2& a, const Fp2& b) {
     Fp t2 = fp_mul(fp_add_lazy(a.c0, a.c1), fp_add_lazy(b.c0, b.c1));
     return Fp2{fp_sub(t0, t1), fp_sub(fp_sub(t2, t0), t1)};
 }
-#endif
 // (a0 + a1 u)^2 = (a0 + a1)(a0 - a1) + 2 a0 a1 u
 WBTE_FP2_MUL Fp2 fp2_sqr(const Fp2& a) {
     Fp t = fp_mul(a.c0, a.c1);
     Fp c0 = fp_mul(fp_add_lazy(a.c0, a.c1), fp_sub(a.c0, a.c1));
     return Fp2{c0, fp_dbl(t)};
 }
-WBTE_INL Fp2 fp2_mul_fp(const Fp2& a, const Fp& b) { return Fp2{fp_mul(a.c0, b), fp_mul(a.c1, b)}; }
 // multiply by xi = 1 + u
 WBTE_INL Fp2 fp2_mul_xi(const Fp2& a) { return Fp2{fp_sub(a.c0, a.c1), fp_add(a.c0, a.c1)}; }
 WBTE_INL Fp2 fp2_from_const(const uint32_t (&c)[2][12]) { return Fp2{fp_from_const(c[0]), fp_from_const(c[1])}; }
@@ -159,11 +148,7 @@ WBTE_INL Fp2 fp2_from_const(const uint32_t (&c)[2][12]) { return Fp2{fp_from_con
 // ----------------------------------------------------------------- Fp6
 WBTE_INL Fp6 fp6_zero() { return Fp6{fp2_zero(), fp2_zero(), fp2_zero()}; }
 WBTE_INL Fp6 fp6_one() { return Fp6{fp2_one(), fp2_zero(), fp2_zero()}; }
-WBTE_INL Fp6 fp6_add(const Fp6& a, const Fp6& b) { return Fp6{fp2_add(a.c0, b.c0), fp2_add(a.c1, b.c1), fp2_add(a.c2, b.c2)}; }
-WBTE_INL Fp6 fp6_sub(const Fp6& a, const Fp6& b) { return Fp6{fp2_sub(a.c0, b.c0), fp2_sub(a.c1, b.c1), fp2_sub(a.c2, b.c2)}; }
 WBTE_INL Fp6 fp6_neg(const Fp6& a) { return Fp6{fp2_neg(a.c0), fp2_neg(a.c1), fp2_neg(a.c2)}; }
-// (c0 + c1 v + c2 v^2) v = xi c2 + c0 v + c1 v^2
-WBTE_INL Fp6 fp6_mul_v(const Fp6& a) { return Fp6{fp2_mul_xi(a.c2), a.c0, a.c1}; }
 
 // ---------------------------------------------------------------- Fp12
 WBTE_INL Fp12 fp12_one() { return Fp12{fp6_one(), fp6_zero()}; }

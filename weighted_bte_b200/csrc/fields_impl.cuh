@@ -6,7 +6,8 @@ namespace wbte {
 
 // Modular inversion by division steps (Bernstein and Yang, "Fast constant-time
 // gcd computation and modular inversion", 2019), in the variant that starts
-// from delta = 1/2.  A chain of about 480 dependent Fp products (a^(p-2))
+// from delta = 1/2, with its bound on the number of steps (Wuille and Maxwell,
+// "Bounds on divsteps iterations in safegcd", 2021).  A chain of about 480 dependent Fp products (a^(p-2))
 // bounds every kernel with one inversion per value from below: about 490 us on
 // one warp.  The division steps work on the low word of f and g, 30 at a
 // time, in about 23 one-word instructions each; their 2 x 2 matrix is then

@@ -542,7 +542,10 @@ def gen_add_nr(name, n):
 
 
 def gen_fp2_mul_lazy(name):
-    """Fp2 product (a0 + a1 u)(b0 + b1 u), u^2 = -1, with lazy reduction.
+    """Fp2 product (a0 + a1 u)(b0 + b1 u), u^2 = -1, with lazy reduction.  No
+    kernel uses it: a pair of lanes takes fp_mont_mul2 twice and a team reduces
+    after the tower (team.cuh).  It stays, as the rolled products do, for the
+    interpreter test.
 
     Karatsuba over double-width products: x = a0 b0, y = a1 b1 and
     z = (a0 + a1)(b0 + b1) are formed as full 768-bit products, and only the

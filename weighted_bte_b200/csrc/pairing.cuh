@@ -14,11 +14,6 @@
 
 namespace wbte {
 
-constexpr int MILLER_LINES = 68;  // 63 doublings + 5 additions for |x|
-
-WBTE_INL Fp2 fp2_mul3(const Fp2& a) { return fp2_add(fp2_dbl(a), a); }
-WBTE_INL Fp2 fp2_mul4(const Fp2& a) { return fp2_dbl(fp2_dbl(a)); }
-
 // pairs of one run of a Miller loop that computes its lines
 constexpr int MULTI_MILLER_MAX = 8;
 
@@ -31,7 +26,6 @@ constexpr int MULTI_MILLER_MAX = 8;
 // hard part of the final exponentiation.
 struct CycPlan {
     int8_t naf[4][65];
-    int digits;
 };
 
 // |x| = 2^16 * X_ODD with X_ODD < 2^48
@@ -40,7 +34,6 @@ constexpr uint64_t X_ODD = X_ABS >> 16;
 WBTE_INL void make_cyc_plan(CycPlan& pl, const uint32_t s_in[8]) {
     uint32_t s[8];
     _Pragma("unroll") for (int i = 0; i < 8; i++) s[i] = s_in[i];
-    pl.digits = 0;
     for (int c = 0; c < 4; c++) {
         // s = q |x| + rem:  q = (s >> 16) div X_ODD, rem = ((s >> 16) mod X_ODD) 2^16 + (s & 0xffff)
         uint32_t lo16 = s[0] & 0xffffu;
@@ -81,7 +74,6 @@ WBTE_INL void make_cyc_plan(CycPlan& pl, const uint32_t s_in[8]) {
             carry_bit = 0;
             pos++;
         }
-        if (pos > pl.digits) pl.digits = pos;
     }
 }
 
