@@ -11,7 +11,8 @@
 // the per-window bucket sort are done once per (vector, window).
 //
 // Pipeline:
-//  1. digits:  signed c-bit windows, digit in (-2^(c-1), 2^(c-1)]
+//  1. digits:  signed c-bit windows, digit in (-2^(c-1), 2^(c-1)], the highest
+//              as it is
 //  2. sort:    one CTA per (vector, window) counting-sorts term indices by
 //              |digit| in descending order (zero digits dropped)
 //  3. segments: one thread per (MSM, window, segment of S sorted terms)
@@ -63,7 +64,8 @@ __global__ void k_digits(int16_t* digits, const uint8_t* scalars, int64_t total,
             val = (uint32_t)(two >> off) & (uint32_t)(full - 1);
         }
         int d = (int)val + carry;
-        if (d > half) {
+        // the highest digit has no window to carry into
+        if (d > half && w + 1 < windows) {
             d -= full;
             carry = 1;
         } else {
@@ -73,9 +75,14 @@ __global__ void k_digits(int16_t* digits, const uint8_t* scalars, int64_t total,
     }
 }
 
-// One CTA per (vector, window).  counts lives in dynamic shared memory.
-__global__ void k_sort(uint64_t* entries, int32_t* nnz, const int16_t* digits, int64_t n, int buckets) {
+// One CTA per (vector, window).  counts lives in dynamic shared memory.  `top`:
+// the highest window's buckets.  They are the others' unless the windows end at bit
+// 256 (c = 4 and 8), where its digits, recoded no further, go up to 2^c: those of
+// scalars from 2^255 on, which are no residues but multiply all the same.
+__global__ void k_sort(uint64_t* entries, int32_t* nnz, const int16_t* digits, int64_t n, int buckets, int top,
+                       int windows) {
     extern __shared__ int32_t sh[];
+    if (blockIdx.x % windows == windows - 1) buckets = top;
     int32_t* cnt = sh;                // buckets + 1
     int32_t* cur = sh + buckets + 1;  // buckets + 1
     int64_t vw = blockIdx.x;
@@ -283,9 +290,10 @@ void run_family(uint8_t* out, const uint8_t* points, const int64_t* pbase, const
     prof_begin(g1 ? "msm_sort_g1" : "msm_sort_g2", s, &tok);
     note_launch();
     k_digits<<<blocks_for(total), TPB, 0, s>>>(digits, scalars, total, n, p.c, p.windows);
-    size_t shmem = sizeof(int32_t) * 2 * (p.buckets + 1);
+    const int top = p.windows * p.c == 256 ? 2 * p.buckets : p.buckets;
+    size_t shmem = sizeof(int32_t) * 2 * (top + 1);
     note_launch();
-    k_sort<<<(unsigned)((int64_t)V * p.windows), 256, shmem, s>>>(entries, nnz, digits, n, p.buckets);
+    k_sort<<<(unsigned)((int64_t)V * p.windows), 256, shmem, s>>>(entries, nnz, digits, n, p.buckets, top, p.windows);
     prof_end(tok, s);
     prof_begin(g1 ? "msm_segments_g1" : "msm_segments_g2", s, &tok);
     int64_t segthreads = k * p.windows * p.segments;
