@@ -289,10 +289,6 @@ PowSpread gt_pow_spread(int64_t E, bool uniform) {
     return best->spread;
 }
 
-// Launches of single products take teams of twelve while two to a warp leave no
-// scheduler more than one warp's work.
-bool few_values(int64_t n) { return n <= 2 * (int64_t)schedulers(); }
-
 int64_t pad5(int64_t x) { return (x + TEAMS - 1) / TEAMS * TEAMS; }
 // One exponent for every five neighbouring teams: worth idle teams up to the
 // difference between the recodings (156 against 195 of gt_pow_spread).

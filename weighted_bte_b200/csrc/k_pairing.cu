@@ -264,10 +264,6 @@ __global__ void k_fp12_is_one(uint8_t* flags, const uint8_t* in, int64_t n) {
 }  // namespace
 
 // ============================================================ launchers
-// Launches of single products take teams of twelve while two to a warp leave no
-// scheduler more than one warp's work.
-static bool few_values(int64_t n) { return n <= 2 * (int64_t)schedulers(); }
-
 // How a launch of `outputs` products of `pairs` Miller loops each is spread: over
 // teams of six or twelve lanes, C pairs to a team.  Sharing the 62 squarings
 // saves 73 thousand of a lane's wide multiply-adds (45 in a team of twelve) for

@@ -77,6 +77,15 @@ inline double run_time(double work, double warps) {
     return work * (whole + (rest > 1 ? 2.0 : (rest > 0 ? 1.4 : 0.0)));
 }
 
+// Launches of single products take teams of twelve while two to a warp leave no
+// scheduler more than one warp's work.  Measured on B200 with 592 schedulers, a call
+// on twelve lanes against six (encodings: one thread): products of 1,184 values 11.1
+// against 13.5 us, of 2,368 15.5 against 13.9, of 2,960 24.1 against 14.7; radix-2
+// stages of 1,184 values 19.8 against 22.0 us, of 2,960 35.6 against 27.4; encodings of
+// 1,184 values 77 against 136 us, of 2,368 118 against 136, of 2,960 173 against 136.
+// Between one and two warps a scheduler the sides are within 2 us but for the encodings.
+inline bool few_values(int64_t n) { return n <= 2 * (int64_t)schedulers(); }
+
 // The time, in launch_time's measure, of `points` chains of `dbls` doublings and
 // `adds` additions on quads or, in G1, on eight lanes each (quad.cuh); `eight`
 // tells which is the shorter.  A quad's doubling is three rounds of products and
